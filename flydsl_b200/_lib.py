@@ -6,8 +6,11 @@ package raises.
 
 from __future__ import annotations
 
+import contextlib
 import ctypes
 import threading
+
+import torch
 
 from . import build as _build
 
@@ -56,6 +59,8 @@ SIGNATURES = {
     "flyb200_gemm_mxfp8": (_i, [_vp, _vp, _vp, _vp, _vp, _i, _i, _i, _i, _vp]),
     "flyb200_gemm_mx_mixed": (_i, [_vp, _vp, _vp, _vp, _vp, _i, _i, _i, _i, _i, _i, _vp]),
     "flyb200_gemm_mxfp4": (_i, [_vp, _vp, _vp, _vp, _vp, _i, _i, _i, _i, _vp]),
+    "flyb200_mx_quant": (_i, [_vp, _vp, _vp, _vp, ctypes.c_longlong, _i, _i, _vp]),
+    "flyb200_mx_fp6_containers": (_i, [_vp, _vp, ctypes.c_longlong, _vp]),
     "flyb200_mx_scale_image": (_i, [_vp, _vp, _i, _i, _vp]),
     "flyb200_mx_scale_image_bytes": (_sz, [_i, _i]),
     "flyb200_strerror": (ctypes.c_char_p, [_i]),
@@ -65,6 +70,7 @@ SIGNATURES = {
 
 _lock = threading.Lock()
 _lib = None
+_NO_GUARD = contextlib.nullcontext()
 
 
 class FlyB200Error(RuntimeError):
@@ -98,6 +104,16 @@ def check(code: int, what: str = "libflyb200") -> None:
     if code == E_CUDA:
         msg += ": " + lib.flyb200_last_cuda_error().decode()
     raise FlyB200Error(code, f"{what}: {msg} (code {code})")
+
+
+def on_device(device):
+    """Context that makes ``device`` current, free of cost where it already is."""
+    return _NO_GUARD if torch.cuda.current_device() == device.index else torch.cuda.device(device)
+
+
+def current_stream(device) -> int:
+    """Raw handle of torch's current stream on ``device`` (0 = default)."""
+    return torch.cuda.current_stream(device).cuda_stream
 
 
 PLAN_FIELDS = ("kernel", "bn", "split_k", "kb_per_split", "reduce", "stages", "pdl", "token_blocks")

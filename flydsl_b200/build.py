@@ -44,6 +44,7 @@ HEADERS = [
     "quant_kernel.cuh",
     "moe_kernel.cuh",
     "mx_kernel.cuh",
+    "mx_quant_kernel.cuh",
     "launch.h",
     "decode_launch.h",
     "host_common.h",

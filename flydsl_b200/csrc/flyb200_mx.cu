@@ -3,6 +3,7 @@
 #include "../../include/flyb200.h"
 #include "host_common.h"
 #include "mx_kernel.cuh"
+#include "mx_quant_kernel.cuh"
 
 #include <atomic>
 #include <cstdlib>
@@ -43,6 +44,14 @@ int launch_mx(const CUtensorMap& tmA, const MxParams& p, cudaStream_t s) {
 
 }  // namespace
 
+template <typename TIn>
+void launch_mx_quant(uint8_t* codes, uint8_t* scale, uint8_t* raw, const TIn* x, long long units, int fmt, cudaStream_t s) {
+  const unsigned grid = static_cast<unsigned>((units + 255) / 256);
+  if (fmt == MXQ_FP8) mx_quant_kernel<TIn, MXQ_FP8><<<grid, 256, 0, s>>>(codes, scale, raw, x, units);
+  else if (fmt == MXQ_FP4) mx_quant_kernel<TIn, MXQ_FP4><<<grid, 256, 0, s>>>(codes, scale, raw, x, units);
+  else mx_quant_kernel<TIn, MXQ_FP6><<<grid, 256, 0, s>>>(codes, scale, raw, x, units);
+}
+
 extern "C" {
 
 size_t flyb200_mx_scale_image_bytes(int rows, int K) {
@@ -50,15 +59,49 @@ size_t flyb200_mx_scale_image_bytes(int rows, int K) {
   return static_cast<size_t>(K / KBLOCK_BYTES) * ((rows + 127) / 128) * MX_SF_ATOM;
 }
 
+int flyb200_mx_quant(void* codes, void* scale, void* raw, const void* x, long long elements, int x_dtype, int format,
+                     void* stream) {
+  if (!codes || !scale || !x || elements < 0) return FLYB200_E_BAD_ARG;
+  if (format != FLYB200_MXFMT_E4M3 && format != FLYB200_MXFMT_E2M3 && format != FLYB200_MXFMT_E2M1) return FLYB200_E_UNSUPPORTED;
+  if (format == FLYB200_MXFMT_E2M3 && !raw) return FLYB200_E_BAD_ARG;
+  if (x_dtype < 0 || x_dtype > 2) return FLYB200_E_BAD_ARG;
+  if (elements % 32 != 0 || elements / MXQ_UNIT > 0x7fffffffll * 256) return FLYB200_E_UNSUPPORTED;
+  if (!aligned16(codes) || !aligned16(x) || (raw && !aligned16(raw))) return FLYB200_E_BAD_ALIGN;
+  if (elements == 0) return FLYB200_OK;
+  const long long units = elements / MXQ_UNIT;
+  cudaStream_t s = static_cast<cudaStream_t>(stream);
+  uint8_t *c = static_cast<uint8_t*>(codes), *sc = static_cast<uint8_t*>(scale), *r = static_cast<uint8_t*>(raw);
+  if (x_dtype == 0) launch_mx_quant(c, sc, r, static_cast<const float*>(x), units, format, s);
+  else if (x_dtype == 1) launch_mx_quant(c, sc, r, static_cast<const __half*>(x), units, format, s);
+  else launch_mx_quant(c, sc, r, static_cast<const __nv_bfloat16*>(x), units, format, s);
+  CUDA_TRY(cudaGetLastError());
+  return FLYB200_OK;
+}
+
+int flyb200_mx_fp6_containers(void* dst, const void* src, long long bytes, void* stream) {
+  if (!dst || !src || bytes < 0) return FLYB200_E_BAD_ARG;
+  if (bytes % 32 != 0) return FLYB200_E_UNSUPPORTED;
+  if (!aligned16(dst) || !aligned16(src)) return FLYB200_E_BAD_ALIGN;
+  if (bytes == 0) return FLYB200_OK;
+  const long long blocks32 = bytes / 32;
+  long long grid = (blocks32 + 255) / 256;
+  if (grid > 148 * 16) grid = 148 * 16;
+  mx_fp6_containers_kernel<<<static_cast<int>(grid), 256, 0, static_cast<cudaStream_t>(stream)>>>(
+      static_cast<uint4*>(dst), static_cast<const uint4*>(src), blocks32);
+  CUDA_TRY(cudaGetLastError());
+  return FLYB200_OK;
+}
+
 int flyb200_mx_scale_image(void* dst, const void* src, int rows, int K, void* stream) {
   if (!dst || !src || rows <= 0 || K <= 0) return FLYB200_E_BAD_ARG;
   if (K % KBLOCK_BYTES != 0) return FLYB200_E_UNSUPPORTED;
   const int row_tiles = (rows + 127) / 128;
-  const long long total = static_cast<long long>(flyb200_mx_scale_image_bytes(rows, K));
+  if (reinterpret_cast<uintptr_t>(dst) & 3u) return FLYB200_E_BAD_ALIGN;
+  const long long total = static_cast<long long>(flyb200_mx_scale_image_bytes(rows, K)) / 4;
   long long blocks = (total + 255) / 256;
   if (blocks > 148 * 8) blocks = 148 * 8;
   mx_scale_image_kernel<<<static_cast<int>(blocks), 256, 0, static_cast<cudaStream_t>(stream)>>>(
-      static_cast<uint8_t*>(dst), static_cast<const uint8_t*>(src), rows, K / 32, row_tiles);
+      static_cast<uint32_t*>(dst), static_cast<const uint8_t*>(src), rows, K / 32, row_tiles);
   CUDA_TRY(cudaGetLastError());
   return FLYB200_OK;
 }

@@ -304,20 +304,28 @@ __global__ void __launch_bounds__(NUM_THREADS, 1) mx_gemm_kernel(const __grid_co
   }
 }
 
-// Scale image from row-major scales [rows, K/32] (uint8): see the layout above.
-// One thread per byte of the image; rows past `rows` read as zero.
-static __global__ void mx_scale_image_kernel(uint8_t* __restrict__ dst, const uint8_t* __restrict__ src, int rows, int kb32,
+// Scale image from row-major scales [rows, K/32] (uint8): see the layout above; rows past `rows` read
+// as zero.  A thread moves the four scales of one row and 128-element k-block, a 4-byte word on both
+// sides (at an odd base, where the source words are not aligned, byte by byte).  A call of 1 to 1024
+// rows of K = 8192 takes 2.0 to 2.4 us, the floor of a launch.
+static __global__ void mx_scale_image_kernel(uint32_t* __restrict__ dst, const uint8_t* __restrict__ src, int rows, int kb32,
                                       int row_tiles) {
-  const long long total = static_cast<long long>(kb32 / 4) * row_tiles * MX_SF_ATOM;
+  const long long total = static_cast<long long>(kb32 / 4) * row_tiles * (MX_SF_ATOM / 4);
+  const bool aligned = (reinterpret_cast<uintptr_t>(src) & 3u) == 0;  // rows of kb32 bytes, a multiple of four
   for (long long i = blockIdx.x * static_cast<long long>(blockDim.x) + threadIdx.x; i < total;
        i += static_cast<long long>(gridDim.x) * blockDim.x) {
-    const int in_atom = static_cast<int>(i % MX_SF_ATOM);
-    const long long atom = i / MX_SF_ATOM;
+    const int w = static_cast<int>(i % (MX_SF_ATOM / 4));  // (r % 32) * 4 + r / 32
+    const long long atom = i / (MX_SF_ATOM / 4);
     const int tile = static_cast<int>(atom % row_tiles);
     const int kblk = static_cast<int>(atom / row_tiles);
-    const int r = tile * 128 + (in_atom >> 4) + 32 * ((in_atom >> 2) & 3);
-    const int j = in_atom & 3;
-    dst[i] = r < rows ? __ldg(src + static_cast<size_t>(r) * kb32 + kblk * 4 + j) : 0;
+    const int r = tile * 128 + (w >> 2) + 32 * (w & 3);
+    uint32_t v = 0;
+    if (r < rows) {
+      const uint8_t* s = src + static_cast<size_t>(r) * kb32 + kblk * 4;
+      v = aligned ? __ldg(reinterpret_cast<const uint32_t*>(s))
+                  : (__ldg(s) | (__ldg(s + 1) << 8) | (__ldg(s + 2) << 16) | (static_cast<uint32_t>(__ldg(s + 3)) << 24));
+    }
+    dst[i] = v;
   }
 }
 

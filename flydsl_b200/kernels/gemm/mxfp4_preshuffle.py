@@ -32,12 +32,13 @@ import torch
 
 from ... import _lib
 from ...utils import shuffle_weight
-from .mxfp8_preshuffle import shuffle_scale
+from .mxfp8_preshuffle import quant_kernel, scale_image_bytes, shuffle_scale
 from .preshuffle_gemm import _stream_handle
 
 _TORCH_OUT = {"bf16": torch.bfloat16, "fp16": torch.float16, "f16": torch.float16}
 _FP4_MIDPOINTS = (0.25, 0.75, 1.25, 1.75, 2.5, 3.5, 5.0)  # between E2M1 code c and c + 1
 _FP4_VALUES = (0.0, 0.5, 1.0, 1.5, 2.0, 3.0, 4.0, 6.0)
+_FORMATS = {"fp8": 0, "fp6": 3, "fp4": 5}  # FLYB200_MXFMT_E4M3 / E2M3 / E2M1
 
 
 def _e8m0_of(x: torch.Tensor) -> torch.Tensor:
@@ -51,14 +52,24 @@ def _e8m0_of(x: torch.Tensor) -> torch.Tensor:
 
 
 def per_1x32_f4_quant(x: torch.Tensor):
-    """Per-1x32 MXFP4 quantiser, torch ops on the tensor's device: (packed E2M1 codes
-    uint8 [..., K/2], E8M0 scales uint8 [..., K/32]).  Scale = E8M0 of blockmax / 4, codes =
-    x / scale rounded to nearest (ties to the even code, magnitudes >= 6 saturate), the even
-    element in the low nibble - the arithmetic of the reference helper
-    (tests/kernels/utils/gemm_common_utils.py:675-705)."""
+    """Per-1x32 MXFP4 quantiser on the tensor's device: (packed E2M1 codes uint8 [..., K/2],
+    E8M0 scales uint8 [..., K/32]).  Scale = E8M0 of blockmax / 4, codes = x / scale rounded to
+    nearest (ties to the even code, magnitudes >= 6 saturate), the even element in the low
+    nibble - the arithmetic of the reference helper
+    (tests/kernels/utils/gemm_common_utils.py:675-705).  CUDA tensors of fp32, fp16 or bf16 take
+    the library's kernel, bit-identical to :func:`per_1x32_f4_quant_torch` on that tensor."""
     shape = x.shape
     if shape[-1] % 32 != 0:
         raise ValueError("K must be a multiple of 32")
+    q = quant_kernel(x, _FORMATS["fp4"])
+    if q is None:
+        return per_1x32_f4_quant_torch(x)
+    return q[0].view(*shape[:-1], shape[-1] // 2), q[1].view(*shape[:-1], shape[-1] // 32)
+
+
+def per_1x32_f4_quant_torch(x: torch.Tensor):
+    """The same quantiser as torch ops."""
+    shape = x.shape
     flat = x.contiguous().view(-1, 32).float()
     exponent = _e8m0_of(torch.amax(torch.abs(flat), dim=-1) / 4.0)
     bits = exponent << 23
@@ -95,6 +106,14 @@ def fp6_containers_from_padded(a_pad: torch.Tensor) -> torch.Tensor:
     bytes, tests/kernels/utils/gemm_common_utils.py:744-770) -> byte containers [M, K]: every 16
     codes (12 bytes) followed by 4 bytes of padding."""
     m, k = a_pad.shape
+    if a_pad.is_cuda and a_pad.is_contiguous() and a_pad.element_size() == 1 and a_pad.data_ptr() % 16 == 0 and m * k > 0:
+        dev = a_pad.device
+        out = torch.empty(m, k, dtype=torch.uint8, device=dev)
+        with _lib.on_device(dev):
+            rc = _lib.load().flyb200_mx_fp6_containers(out.data_ptr(), a_pad.data_ptr(), m * k, _lib.current_stream(dev))
+        if rc:
+            _lib.check(rc, "mx_fp6_containers")
+        return out
     v = a_pad.view(torch.uint8).view(m, k // 32, 32)
     out = torch.zeros(m, k // 32, 2, 16, dtype=torch.uint8, device=a_pad.device)
     out[:, :, 0, :12] = v[:, :, 0:12]
@@ -120,12 +139,22 @@ def fp6_e2m3_to_f32(codes: torch.Tensor) -> torch.Tensor:
 
 
 def per_1x32_f6_quant(x: torch.Tensor):
-    """Per-1x32 MXFP6 (E2M3) quantiser of an activation matrix [M, K], torch ops on the tensor's
-    device; returns what the reference helper returns (gemm_common_utils.py:744-770): the padded
+    """Per-1x32 MXFP6 (E2M3) quantiser of an activation matrix [M, K] on the tensor's device;
+    returns what the reference helper returns (gemm_common_utils.py:744-770): the padded
     packed codes uint8 [M, K] (per 32 elements 24 bytes + 8 zero bytes), the E8M0 scales uint8
-    [M, K/32], and the unpacked codes uint8 [M, K]."""
+    [M, K/32], and the unpacked codes uint8 [M, K].  CUDA tensors of fp32, fp16 or bf16 take the
+    library's kernel, bit-identical to :func:`per_1x32_f6_quant_torch` on that tensor."""
     if x.dim() != 2 or x.shape[-1] % 32 != 0:
         raise ValueError("x must be [M, K] with K a multiple of 32")
+    m, k = x.shape
+    q = quant_kernel(x, _FORMATS["fp6"])
+    if q is None:
+        return per_1x32_f6_quant_torch(x)
+    return q[0].view(m, k), q[1].view(m, k // 32), q[2].view(m, k)
+
+
+def per_1x32_f6_quant_torch(x: torch.Tensor):
+    """The same quantiser as torch ops."""
     m, k = x.shape
     flat = x.contiguous().view(-1, 32).float()
     exponent = _e8m0_of(torch.amax(torch.abs(flat), dim=-1) / 4.0)
@@ -171,9 +200,6 @@ def shuffle_scale_w4(src: torch.Tensor, experts_cnt: int = 1, gate_up: bool = Fa
     return shuffle_scale(src)
 
 
-_FORMATS = {"fp8": 0, "fp6": 3, "fp4": 5}  # FLYB200_MXFMT_E4M3 / E2M3 / E2M1
-
-
 class MxMixedGemm:
     """The callable returned by :func:`compile_mxfp4_preshuffle_gemm` for ``a_dtype`` "fp6" or "fp8"
     with ``b_dtype="fp4"``: same call shape; activations in the reference's layout for that dtype."""
@@ -214,8 +240,7 @@ class MxMixedGemm:
             raise ValueError(f"c must be {_TORCH_OUT[self.out_dtype]}, got {arg_c.dtype}")
         if arg_c.numel() < M * self.N or arg_a.numel() < M * self.K or arg_a.element_size() != 1:
             raise ValueError("c or a is smaller than the launch needs (a: one byte per code)")
-        if arg_scale_a.numel() < int(lib.flyb200_mx_scale_image_bytes(max(M, 1), self.K)) or \
-                arg_scale_b.numel() < int(lib.flyb200_mx_scale_image_bytes(self.N, self.K)):
+        if arg_scale_a.numel() < scale_image_bytes(max(M, 1), self.K) or arg_scale_b.numel() < scale_image_bytes(self.N, self.K):
             raise ValueError("a scale image is smaller than the launch needs")
         if arg_bias is not None and arg_bias.numel() != 0:
             raise ValueError("the block-scaled GEMMs have no bias epilogue")
@@ -228,20 +253,23 @@ class MxMixedGemm:
         if M == 0:
             return None
         s = _stream_handle(stream)
-        with torch.cuda.device(arg_c.device):
-            a = arg_a.view(torch.uint8).view(-1)[: M * self.K].view(M, self.K)
+        dev = arg_c.device
+        with _lib.on_device(dev):
+            a = arg_a
             if self.a_dtype == "fp6":
-                ext = torch.cuda.ExternalStream(s, device=arg_c.device) if s else torch.cuda.default_stream(arg_c.device)
-                with torch.cuda.stream(ext):  # the conversion runs on the launch stream, ahead of the GEMM
+                # the conversion runs on the launch stream, ahead of the GEMM; the temporary belongs to that
+                # stream's memory pool, so it cannot be handed out again before the kernel that reads it is done
+                a = arg_a.view(torch.uint8).view(-1)[: M * self.K].view(M, self.K)
+                if s == _lib.current_stream(dev):
                     a = fp6_containers_from_padded(a)
-            _lib.check(
-                lib.flyb200_gemm_mx_mixed(arg_c.data_ptr(), a.data_ptr(), w.data_ptr(), arg_scale_a.data_ptr(),
-                                          arg_scale_b.data_ptr(), M, self.N, self.K, _FORMATS[self.a_dtype], _FORMATS["fp4"],
-                                          self._out, s or None),
-                "gemm_mx_mixed",
-            )
-            if self.a_dtype == "fp6":
-                a.record_stream(ext)  # the temporary must outlive the kernel that reads it
+                else:
+                    with torch.cuda.stream(torch.cuda.ExternalStream(s, device=dev) if s else torch.cuda.default_stream(dev)):
+                        a = fp6_containers_from_padded(a)
+            rc = lib.flyb200_gemm_mx_mixed(arg_c.data_ptr(), a.data_ptr(), w.data_ptr(), arg_scale_a.data_ptr(),
+                                           arg_scale_b.data_ptr(), M, self.N, self.K, _FORMATS[self.a_dtype], _FORMATS["fp4"],
+                                           self._out, s or None)
+        if rc:
+            _lib.check(rc, "gemm_mx_mixed")
         return None
 
 
@@ -261,8 +289,8 @@ class MxFp4Gemm:
         lib = _lib.load()
         need = (
             ("c", arg_c, M * self.N), ("a", arg_a, M * self.K // 2), ("b", arg_b, self.N * self.K // 2),
-            ("scale_a", arg_scale_a, int(lib.flyb200_mx_scale_image_bytes(max(M, 1), self.K))),
-            ("scale_b", arg_scale_b, int(lib.flyb200_mx_scale_image_bytes(self.N, self.K))),
+            ("scale_a", arg_scale_a, scale_image_bytes(max(M, 1), self.K)),
+            ("scale_b", arg_scale_b, scale_image_bytes(self.N, self.K)),
         )  # fmt: skip
         for name, t, n in need:
             if not isinstance(t, torch.Tensor) or not t.is_cuda or not t.is_contiguous():
@@ -278,12 +306,11 @@ class MxFp4Gemm:
             raise ValueError("the MXFP4 GEMM has no bias epilogue")
         if M == 0:
             return None
-        with torch.cuda.device(arg_c.device):
-            _lib.check(
-                lib.flyb200_gemm_mxfp4(arg_c.data_ptr(), arg_a.data_ptr(), arg_b.data_ptr(), arg_scale_a.data_ptr(),
-                                       arg_scale_b.data_ptr(), M, self.N, self.K, self._out, _stream_handle(stream) or None),
-                "gemm_mxfp4",
-            )
+        with _lib.on_device(arg_c.device):
+            rc = lib.flyb200_gemm_mxfp4(arg_c.data_ptr(), arg_a.data_ptr(), arg_b.data_ptr(), arg_scale_a.data_ptr(),
+                                        arg_scale_b.data_ptr(), M, self.N, self.K, self._out, _stream_handle(stream) or None)
+        if rc:
+            _lib.check(rc, "gemm_mxfp4")
         return None
 
 

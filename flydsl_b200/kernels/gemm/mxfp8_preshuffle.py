@@ -27,13 +27,49 @@ _TORCH_OUT = {"bf16": torch.bfloat16, "fp16": torch.float16, "f16": torch.float1
 FP8_MAX = 448.0
 
 
+_QUANT_IN = {torch.float32: 0, torch.float16: 1, torch.bfloat16: 2}
+
+
+def quant_kernel(x: torch.Tensor, fmt: int):
+    """The per-1x32 quantisers as ONE kernel (the torch statements launch 30 to 250): ``(codes, scales, raw)``
+    as flat uint8 tensors on x's device, or None where the kernel cannot take ``x`` (CPU tensors, other
+    dtypes, no elements).  ``fmt``: 0 E4M3, 3 E2M3, 5 E2M1; ``raw`` (the codes one per byte) is None unless E2M3."""
+    if not x.is_cuda or x.dtype not in _QUANT_IN:
+        return None
+    n = x.numel()
+    x = x.contiguous()
+    ptr = x.data_ptr()
+    if n == 0 or ptr % 16 != 0:
+        return None
+    dev = x.device
+    codes = torch.empty(n // 2 if fmt == 5 else n, dtype=torch.uint8, device=dev)
+    scale = torch.empty(n // 32, dtype=torch.uint8, device=dev)
+    raw = torch.empty(n, dtype=torch.uint8, device=dev) if fmt == 3 else None
+    with _lib.on_device(dev):
+        rc = _lib.load().flyb200_mx_quant(codes.data_ptr(), scale.data_ptr(), raw.data_ptr() if fmt == 3 else None, ptr, n,
+                                          _QUANT_IN[x.dtype], fmt, _lib.current_stream(dev))
+    if rc:
+        _lib.check(rc, "mx_quant")
+    return codes, scale, raw
+
+
 def per_1x32_f8_quant(x: torch.Tensor):
-    """Per-1x32 MXFP8 quantiser, torch ops on the tensor's device: (codes
-    float8_e4m3fn [..., K], E8M0 scales uint8 [..., K/32]); same arithmetic as the
-    reference helper (tests/kernels/utils/gemm_common_utils.py:53-72, 773-790)."""
+    """Per-1x32 MXFP8 quantiser on the tensor's device: (codes float8_e4m3fn [..., K], E8M0 scales
+    uint8 [..., K/32]); same arithmetic as the reference helper
+    (tests/kernels/utils/gemm_common_utils.py:53-72, 773-790).  CUDA tensors of fp32, fp16 or bf16
+    take the library's kernel, bit-identical to :func:`per_1x32_f8_quant_torch` on that tensor."""
     shape = x.shape
     if shape[-1] % 32 != 0:
         raise ValueError("K must be a multiple of 32")
+    q = quant_kernel(x, 0)
+    if q is None:
+        return per_1x32_f8_quant_torch(x)
+    return q[0].view(torch.float8_e4m3fn).view(shape), q[1].view(*shape[:-1], shape[-1] // 32)
+
+
+def per_1x32_f8_quant_torch(x: torch.Tensor):
+    """The same quantiser as torch ops."""
+    shape = x.shape
     flat = x.contiguous().view(-1, 32).float()
     max_abs = torch.amax(torch.abs(flat), dim=-1).clamp_min(1e-30)
     u32 = (max_abs / FP8_MAX).view(torch.int32)
@@ -59,16 +95,19 @@ def shuffle_scale(scale: torch.Tensor) -> torch.Tensor:
         raise ValueError("K must be a multiple of 128")
     if not scale.is_cuda:
         raise ValueError("scale must be a CUDA tensor")
-    lib = _lib.load()
-    src = scale.contiguous().view(torch.uint8)
-    out = torch.empty(int(lib.flyb200_mx_scale_image_bytes(rows, kb32 * 32)), dtype=torch.uint8, device=scale.device)
-    with torch.cuda.device(scale.device):
-        _lib.check(
-            lib.flyb200_mx_scale_image(out.data_ptr(), src.data_ptr(), rows, kb32 * 32,
-                                       torch.cuda.current_stream(scale.device).cuda_stream),
-            "mx_scale_image",
-        )
+    dev = scale.device
+    src = scale.contiguous()
+    out = torch.empty(scale_image_bytes(rows, kb32 * 32), dtype=torch.uint8, device=dev)
+    with _lib.on_device(dev):
+        rc = _lib.load().flyb200_mx_scale_image(out.data_ptr(), src.data_ptr(), rows, kb32 * 32, _lib.current_stream(dev))
+    if rc:
+        _lib.check(rc, "mx_scale_image")
     return out
+
+
+def scale_image_bytes(rows: int, k: int) -> int:
+    """flyb200_mx_scale_image_bytes: one 512-byte atom per 128 rows and 128 elements of K."""
+    return k // 128 * ((rows + 127) // 128) * 512
 
 
 class MxFp8Gemm:
@@ -87,8 +126,8 @@ class MxFp8Gemm:
         lib = _lib.load()
         need = (
             ("c", arg_c, M * self.N), ("a", arg_a, M * self.K), ("b", arg_b, self.N * self.K),
-            ("scale_a", arg_scale_a, int(lib.flyb200_mx_scale_image_bytes(max(M, 1), self.K))),
-            ("scale_b", arg_scale_b, int(lib.flyb200_mx_scale_image_bytes(self.N, self.K))),
+            ("scale_a", arg_scale_a, scale_image_bytes(max(M, 1), self.K)),
+            ("scale_b", arg_scale_b, scale_image_bytes(self.N, self.K)),
         )
         for name, t, n in need:
             if not isinstance(t, torch.Tensor) or not t.is_cuda or not t.is_contiguous():
@@ -104,12 +143,11 @@ class MxFp8Gemm:
             raise ValueError("the MXFP8 GEMM has no bias epilogue")
         if M == 0:
             return None
-        with torch.cuda.device(arg_c.device):
-            _lib.check(
-                lib.flyb200_gemm_mxfp8(arg_c.data_ptr(), arg_a.data_ptr(), arg_b.data_ptr(), arg_scale_a.data_ptr(),
-                                       arg_scale_b.data_ptr(), M, self.N, self.K, self._out, _stream_handle(stream) or None),
-                "gemm_mxfp8",
-            )
+        with _lib.on_device(arg_c.device):
+            rc = lib.flyb200_gemm_mxfp8(arg_c.data_ptr(), arg_a.data_ptr(), arg_b.data_ptr(), arg_scale_a.data_ptr(),
+                                        arg_scale_b.data_ptr(), M, self.N, self.K, self._out, _stream_handle(stream) or None)
+        if rc:
+            _lib.check(rc, "gemm_mxfp8")
         return None
 
 

@@ -381,6 +381,19 @@ int flyb200_gemm_mxfp4(void* c, const void* a, const void* w_shuf, const void* s
 #define FLYB200_MXFMT_E2M1 5
 int flyb200_gemm_mx_mixed(void* c, const void* a, const void* w_shuf, const void* scale_a_image, const void* scale_w_image,
                           int M, int N, int K, int a_format, int w_format, int out_dtype, void* stream);
+/* Per-1x32 quantisers of the MX formats: codes and one E8M0 scale per 32 consecutive elements, rounding
+ * as in the reference helpers per_1x32_f8_quant, per_1x32_f4_quant and per_1x32_f6_quant
+ * (tests/kernels/utils/gemm_common_utils.py:675-705, 744-790).
+ *   x         `elements` (a multiple of 32) contiguous values, x_dtype 0 = fp32, 1 = fp16, 2 = bf16
+ *   format    FLYB200_MXFMT_E4M3: codes one per byte; FLYB200_MXFMT_E2M1: two per byte, the even element
+ *             in the low nibble; FLYB200_MXFMT_E2M3: per 32 elements 24 bytes of 6-bit codes and 8 zero
+ *             bytes, and the codes one per byte in `raw` (NULL for the other formats)
+ *   scale     [elements / 32] bytes.   x, codes and raw 16-byte aligned. */
+int flyb200_mx_quant(void* codes, void* scale, void* raw, const void* x, long long elements, int x_dtype, int format,
+                     void* stream);
+/* The 32-byte units that FLYB200_MXFMT_E2M3 quantisation writes -> byte containers for flyb200_gemm_mx_mixed
+ * (12 bytes of codes, 4 of padding, twice); `bytes` is the size of both buffers, a multiple of 32. */
+int flyb200_mx_fp6_containers(void* dst, const void* src, long long bytes, void* stream);
 int flyb200_mx_scale_image(void* dst, const void* src, int rows, int K, void* stream);
 size_t flyb200_mx_scale_image_bytes(int rows, int K);
 

@@ -153,6 +153,21 @@ int launch_moe_bn(int bn, int stage, int out_dtype, bool accumulate, const CUten
   return FLYB200_E_UNSUPPORTED;
 }
 
+// Vectors of eight where every row starts on a 16-byte boundary, else pairs.
+template <typename T>
+void launch_moe_reduce(void* y, const void* x, int tokens, int topk, int dim, const int* expert_mask, const int* topk_ids,
+                       int num_experts, cudaStream_t s) {
+  T* yt = static_cast<T*>(y);
+  const T* xt = static_cast<const T*>(x);
+  if (dim % 8 == 0 && aligned16(y) && aligned16(x)) {
+    const dim3 grid(tokens, (dim / 8 + 255) / 256);
+    moe_reduce_kernel<T, 8><<<grid, 256, 0, s>>>(yt, xt, topk, dim, expert_mask, topk_ids, num_experts);
+  } else {
+    const dim3 grid(tokens, (dim / 2 + 255) / 256);
+    moe_reduce_kernel<T, 2><<<grid, 256, 0, s>>>(yt, xt, topk, dim, expert_mask, topk_ids, num_experts);
+  }
+}
+
 }  // namespace
 
 extern "C" {
@@ -278,21 +293,10 @@ int flyb200_moe_reduce(void* y, const void* x, int tokens, int topk, int dim, in
   if (dim % 2 != 0) return FLYB200_E_UNSUPPORTED;
   if ((reinterpret_cast<uintptr_t>(y) & 3u) || (reinterpret_cast<uintptr_t>(x) & 3u)) return FLYB200_E_BAD_ALIGN;
   if (tokens == 0) return FLYB200_OK;
-  const long long total = static_cast<long long>(tokens) * dim / 2;
-  long long blocks = (total + 255) / 256;
-  if (blocks > 148 * 16) blocks = 148 * 16;
   cudaStream_t s = static_cast<cudaStream_t>(stream);
-  if (dtype == FLYB200_OUT_BF16) {
-    moe_reduce_kernel<__nv_bfloat16><<<static_cast<int>(blocks), 256, 0, s>>>(
-        static_cast<__nv_bfloat16*>(y), static_cast<const __nv_bfloat16*>(x), tokens, topk, dim, expert_mask, topk_ids,
-        num_experts);
-  } else if (dtype == FLYB200_OUT_FP16) {
-    moe_reduce_kernel<__half><<<static_cast<int>(blocks), 256, 0, s>>>(static_cast<__half*>(y),
-                                                                       static_cast<const __half*>(x), tokens, topk, dim,
-                                                                       expert_mask, topk_ids, num_experts);
-  } else {
-    return FLYB200_E_UNSUPPORTED;
-  }
+  if (dtype != FLYB200_OUT_BF16 && dtype != FLYB200_OUT_FP16) return FLYB200_E_UNSUPPORTED;
+  if (dtype == FLYB200_OUT_BF16) launch_moe_reduce<__nv_bfloat16>(y, x, tokens, topk, dim, expert_mask, topk_ids, num_experts, s);
+  else launch_moe_reduce<__half>(y, x, tokens, topk, dim, expert_mask, topk_ids, num_experts, s);
   CUDA_TRY(cudaGetLastError());
   return FLYB200_OK;
 }

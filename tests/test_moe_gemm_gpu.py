@@ -310,6 +310,18 @@ def test_topk_reduction(dev, dtype_str):
     assert torch.all(y[tokens:] == 7.0)
 
 
+@pytest.mark.parametrize("tokens,topk,dim,shift", [(1, 1, 2, 0), (3, 5, 250, 0), (9, 9, 2056, 0), (5, 2, 4104, 2)])
+def test_topk_reduction_vector_forms(dev, tokens, topk, dim, shift):
+    """Dimensions and bases on both sides of the 16-byte form, more slots than one batch of loads, ragged last block."""
+    x = torch.randn(tokens * topk * dim + shift, device=dev).to(torch.bfloat16)[shift:].view(tokens, topk, dim)
+    y = torch.full((tokens + 1, dim), 7.0, dtype=torch.bfloat16, device=dev)
+    compile_moe_reduction(topk=topk, model_dim=dim, dtype_str="bf16")(x, y, None, None, tokens, torch.cuda.current_stream())
+    want = torch.zeros(tokens, dim, device=dev)
+    for s in range(topk):  # fp32 sum in slot order
+        want += x[:, s].float()
+    assert torch.equal(y[:tokens], want.to(torch.bfloat16)) and torch.all(y[tokens:] == 7.0)
+
+
 def test_two_stage_pipeline_end_to_end(dev):
     """x -> stage 1 -> per-token quantisation on the GPU -> stage 2 (per slot) -> top-k reduction."""
     from flydsl_b200 import pertoken_quant

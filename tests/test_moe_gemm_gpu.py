@@ -178,6 +178,19 @@ def test_large_routing_blocks_all_outputs(dev, in_dtype, out_dtype):
         assert torch.all(out2[rows:] == 7.0)
 
 
+@pytest.mark.parametrize("out_dtype", ["f16", "bf16", "f32"])
+@pytest.mark.parametrize("tile_m", [16, 64, 128])
+def test_accumulate_ragged_channels(dev, tile_m, out_dtype):
+    """16-byte reductions at the end of a row: 400 channels = a full pair of tiles, one full tile and 16 channels."""
+    tokens, model_dim, inter_dim, experts, topk = 150, 400, 128, 4, 2
+    d = moe_oracle.make_inputs(tokens, model_dim, inter_dim, experts, topk, "int8", seed=35)
+    out = run_stage2(dev, d, model_dim=model_dim, inter_dim=inter_dim, experts=experts, topk=topk, tile_m=tile_m,
+                     in_dtype="int8", out_dtype=out_dtype, accumulate=True, extra_rows=8)
+    # fp32 sums: the products are exact in fp32 up to their order; 16-bit: one rounding per added slot
+    close_enough(out[:tokens], ref_stage2(d, model_dim), "stage 2", rel=1e-4 if out_dtype == "f32" else 2e-2)
+    assert torch.all(out[tokens:] == 7.0)
+
+
 @pytest.mark.parametrize("tile_m,experts,tokens", [(128, 4, 500), (64, 4, 500), (64, 16, 90), (64, 3, 33)])
 def test_both_kernel_forms_agree(dev, monkeypatch, tile_m, experts, tokens):
     """The persistent form and the two-tiles-per-CTA form do the same arithmetic per output element.

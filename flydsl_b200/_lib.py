@@ -56,6 +56,7 @@ SIGNATURES = {
     "flyb200_moe_gemm": (_i, [_i, _vp, _vp, _vp, _vp, _vp, _vp, _vp, _vp, _vp] + [_i] * 12 + [_vp]),
     "flyb200_moe_reduce": (_i, [_vp, _vp, _i, _i, _i, _i, _vp, _vp, _i, _vp]),
     "flyb200_moe_sorting": (_i, [_vp, _vp, _i, _i, _i, _i, _vp, _vp, _vp, _vp, _vp, _vp]),
+    "flyb200_moe_sorting_range": (_i, [_vp, _i, _vp, _i, _i, _i, ctypes.c_longlong, _i, _vp, _vp, _vp, _vp, _vp]),
     "flyb200_gemm_mxfp8": (_i, [_vp, _vp, _vp, _vp, _vp, _i, _i, _i, _i, _vp]),
     "flyb200_gemm_mx_mixed": (_i, [_vp, _vp, _vp, _vp, _vp, _i, _i, _i, _i, _i, _i, _vp]),
     "flyb200_gemm_mxfp4": (_i, [_vp, _vp, _vp, _vp, _vp, _i, _i, _i, _i, _vp]),

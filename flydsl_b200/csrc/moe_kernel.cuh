@@ -805,79 +805,138 @@ static __global__ void moe_gather_rows_kernel(uint8_t* __restrict__ dst, float* 
 // reference describes): counting sort of the (token, slot) pairs by expert,
 // stable, every expert's run padded to a multiple of block_size.
 // ---------------------------------------------------------------------------
-// Pass 1: fill the outputs with their padding values and count the pairs of every expert
-// (`counts` must be zero on entry).
-static __global__ void moe_sort_count_kernel(const int* __restrict__ topk_ids, int n_pairs, int experts, int* __restrict__ counts,
-                                      int* __restrict__ sorted_ids, float* __restrict__ sorted_weights, int max_padded,
-                                      int* __restrict__ sorted_expert_ids, int max_blocks, int sentinel) {
-  const int stride = gridDim.x * blockDim.x;
-  const int t0 = blockIdx.x * blockDim.x + threadIdx.x;
-  for (int i = t0; i < max_padded; i += stride) {
-    sorted_ids[i] = sentinel;
-    sorted_weights[i] = 0.0f;
+// One launch, one CTA per expert, no scratch.  Every CTA counts all pairs into a
+// shared-memory histogram (so it knows where its run starts and where the list ends
+// without talking to the others), then walks the pairs once more and writes its own
+// run, its padding and its share of the tail behind the last run.  Latency-bound: a
+// chunk is four pairs per thread, one barrier, so 4096 pairs cost about a microsecond.
+// Measured (pairs / experts, one kernel against memset + count + a walk of 256 pairs at
+// a time, us): 64 / 8 4.4 against 5.0, 2060 / 16 5.4 against 11.5, 8192 / 8 9.5 against 29.
+constexpr int MOE_SORT_MAX_THREADS = 1024;
+constexpr int MOE_SORT_BINS = 4096;  // experts counted per pass over the pairs
+
+// ids of the four pairs at `i` (a multiple of four), -1 past the end; made relative to `first_expert`
+template <typename ID>
+__device__ __forceinline__ void moe_load_ids(const ID* __restrict__ ids, long long i, long long n_pairs, long long first_expert,
+                                             int experts, bool vec, int (&e)[4]) {
+  long long v[4];
+  if (vec && i + 3 < n_pairs) {
+    if constexpr (sizeof(ID) == 4) {
+      const int4 q = __ldg(reinterpret_cast<const int4*>(ids + i));
+      v[0] = q.x, v[1] = q.y, v[2] = q.z, v[3] = q.w;
+    } else {
+      const longlong2 q0 = __ldg(reinterpret_cast<const longlong2*>(ids + i)), q1 = __ldg(reinterpret_cast<const longlong2*>(ids + i + 2));
+      v[0] = q0.x, v[1] = q0.y, v[2] = q1.x, v[3] = q1.y;
+    }
+  } else {
+#pragma unroll
+    for (int j = 0; j < 4; ++j) v[j] = i + j < n_pairs ? static_cast<long long>(__ldg(ids + i + j)) : -1ll;
   }
-  for (int i = t0; i < max_blocks; i += stride) sorted_expert_ids[i] = -1;
-  for (int i = t0; i < n_pairs; i += stride) {
-    const int e = __ldg(topk_ids + i);
-    if (e >= 0 && e < experts) atomicAdd(counts + e, 1);
+#pragma unroll
+  for (int j = 0; j < 4; ++j) {
+    const long long local = v[j] - first_expert;
+    e[j] = v[j] >= 0 && local >= 0 && local < experts ? static_cast<int>(local) : -1;
   }
 }
 
-// Pass 2: one CTA per expert walks the pairs in order and writes its run.
-constexpr int MOE_SORT_THREADS = 256;
-static __global__ void __launch_bounds__(MOE_SORT_THREADS)
-moe_sort_place_kernel(const int* __restrict__ topk_ids, const float* __restrict__ topk_weights, int n_pairs, int topk,
-                      int tokens, int experts, int block_size, const int* __restrict__ counts,
-                      int* __restrict__ sorted_ids, float* __restrict__ sorted_weights,
-                      int* __restrict__ sorted_expert_ids, int* __restrict__ post_pad) {
-  __shared__ int warp_sums[MOE_SORT_THREADS / 32];
-  __shared__ int s_start;
-  const int e = blockIdx.x;
+template <typename ID>
+__global__ void __launch_bounds__(MOE_SORT_MAX_THREADS)
+moe_sort_kernel(const ID* __restrict__ topk_ids, const float* __restrict__ topk_weights, int n_pairs, int topk, int tokens,
+                int experts, long long first_expert, int block_size, int* __restrict__ sorted_ids,
+                float* __restrict__ sorted_weights, int* __restrict__ sorted_expert_ids, int* __restrict__ post_pad,
+                int max_padded, int max_blocks) {
+  __shared__ int bins[MOE_SORT_BINS];
+  __shared__ int warp_sums[2][32];
+  __shared__ int s_start, s_total, s_mine;
+  const int me = blockIdx.x;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  // first row of this expert: padded sizes of the experts before it
-  int part = 0;
-  for (int i = tid; i < e; i += MOE_SORT_THREADS) {
-    const int c = __ldg(counts + i);
-    part += (c + block_size - 1) / block_size * block_size;
+  const int threads = blockDim.x, warps = threads >> 5;
+  const bool vec = (reinterpret_cast<uintptr_t>(topk_ids) & 15u) == 0;
+  if (tid == 0) s_start = s_total = s_mine = 0;
+  for (int b0 = 0; b0 < experts; b0 += MOE_SORT_BINS) {
+    const int nb = min(MOE_SORT_BINS, experts - b0);
+    __syncthreads();  // the previous pass has been read
+    for (int i = tid; i < nb; i += threads) bins[i] = 0;
+    __syncthreads();
+    for (long long i = 4 * tid; i < n_pairs; i += 4 * threads) {
+      int e[4];
+      moe_load_ids(topk_ids, i, n_pairs, first_expert, experts, vec, e);
+#pragma unroll
+      for (int j = 0; j < 4; ++j)
+        if (e[j] >= b0 && e[j] < b0 + nb) atomicAdd(&bins[e[j] - b0], 1);
+    }
+    __syncthreads();
+    int before = 0, all = 0;
+    for (int i = tid; i < nb; i += threads) {
+      const int c = bins[i];
+      const int padded = (c + block_size - 1) / block_size * block_size;
+      all += padded;
+      if (b0 + i < me) before += padded;
+      if (b0 + i == me) s_mine = c;
+    }
+    for (int o = 16; o > 0; o >>= 1) {
+      before += __shfl_xor_sync(0xffffffffu, before, o);
+      all += __shfl_xor_sync(0xffffffffu, all, o);
+    }
+    if (lane == 0) {
+      atomicAdd(&s_start, before);
+      atomicAdd(&s_total, all);
+    }
   }
-  for (int o = 16; o > 0; o >>= 1) part += __shfl_xor_sync(0xffffffffu, part, o);
-  if (lane == 0) warp_sums[warp] = part;
   __syncthreads();
-  if (tid == 0) {
-    int t = 0;
-    for (int w = 0; w < MOE_SORT_THREADS / 32; ++w) t += warp_sums[w];
-    s_start = t;
+  const int start = s_start, mine = s_mine, total = s_total;
+  const int padded = (mine + block_size - 1) / block_size * block_size;
+  const int sentinel = (topk << 24) | tokens;
+  for (int i = tid; i < padded / block_size; i += threads) sorted_expert_ids[start / block_size + i] = me;
+  for (int i = start + mine + tid; i < start + padded; i += threads) {
+    sorted_ids[i] = sentinel;
+    sorted_weights[i] = 0.0f;
   }
-  __syncthreads();
-  const int start = s_start;
-  const int mine = __ldg(counts + e);
-  const int n_blk = (mine + block_size - 1) / block_size;
-  for (int i = tid; i < n_blk; i += MOE_SORT_THREADS) sorted_expert_ids[start / block_size + i] = e;
-  if (e == experts - 1 && tid == 0) {
-    post_pad[0] = start + n_blk * block_size;
+  const long long tail0 = static_cast<long long>(me) * threads + tid, tail_step = static_cast<long long>(experts) * threads;
+  for (long long i = total + tail0; i < max_padded; i += tail_step) {
+    sorted_ids[i] = sentinel;
+    sorted_weights[i] = 0.0f;
+  }
+  for (long long i = total / block_size + tail0; i < max_blocks; i += tail_step) sorted_expert_ids[i] = -1;
+  if (me == experts - 1 && tid == 0) {
+    post_pad[0] = total;
     post_pad[1] = tokens;
   }
   int base = 0;  // pairs of this expert seen so far
-  for (int c0 = 0; c0 < n_pairs && base < mine; c0 += MOE_SORT_THREADS) {
-    const int i = c0 + tid;
-    const bool hit = i < n_pairs && __ldg(topk_ids + i) == e;
-    const unsigned ballot = __ballot_sync(0xffffffffu, hit);
-    const int in_warp = __popc(ballot & ((1u << lane) - 1u));
-    __syncthreads();  // warp_sums of the previous chunk have been read
-    if (lane == 0) warp_sums[warp] = __popc(ballot);
-    __syncthreads();
-    int before = 0, total = 0;
-    for (int w = 0; w < MOE_SORT_THREADS / 32; ++w) {
-      const int v = warp_sums[w];
-      if (w < warp) before += v;
-      total += v;
+  int buf = 0;
+  for (long long c0 = 0; c0 < n_pairs && base < mine; c0 += 4 * threads) {
+    const long long i = c0 + 4 * tid;
+    int e[4];
+    moe_load_ids(topk_ids, i, n_pairs, first_expert, experts, vec, e);
+    int hits = 0;
+#pragma unroll
+    for (int j = 0; j < 4; ++j) hits += e[j] == me ? 1 : 0;
+    int scan = hits;  // inclusive over the warp
+    for (int o = 1; o < 32; o <<= 1) {
+      const int up = __shfl_up_sync(0xffffffffu, scan, o);
+      if (lane >= o) scan += up;
     }
-    if (hit) {
-      const int dst = start + base + before + in_warp;
-      sorted_ids[dst] = ((i % topk) << 24) | (i / topk);
-      sorted_weights[dst] = __ldg(topk_weights + i);
+    if (lane == 31) warp_sums[buf][warp] = scan;
+    __syncthreads();  // two buffers: the next chunk writes the other one
+    int ws = lane < warps ? warp_sums[buf][lane] : 0;
+    for (int o = 1; o < 32; o <<= 1) {
+      const int up = __shfl_up_sync(0xffffffffu, ws, o);
+      if (lane >= o) ws += up;
     }
-    base += total;
+    const int before_warp = warp == 0 ? 0 : __shfl_sync(0xffffffffu, ws, warp - 1);
+    const int in_chunk = __shfl_sync(0xffffffffu, ws, 31);
+    int dst = start + base + before_warp + scan - hits;
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+      if (e[j] == me) {
+        const int pair = static_cast<int>(i) + j;
+        sorted_ids[dst] = ((pair % topk) << 24) | (pair / topk);
+        sorted_weights[dst] = __ldg(topk_weights + pair);
+        ++dst;
+      }
+    }
+    base += in_chunk;
+    buf ^= 1;
   }
 }
 

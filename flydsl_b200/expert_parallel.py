@@ -111,18 +111,19 @@ class ExpertParallelMoe:
     def forward_local(self, x_q, scale_x, topk_ids, topk_weights):
         """This rank's partial output [tokens, model_dim] (routes to other ranks' experts contribute nothing)."""
         from . import pertoken_quant
-        from .kernels.moe.moe_gemm_2stage import moe_sorting
+        from .kernels.moe.moe_gemm_2stage import sort_on_device
 
         if self._w1 is None:
             raise RuntimeError("load_expert_weights has not been called")
         tokens = x_q.shape[0]
         dev = x_q.device
-        ids = local_routing(topk_ids, self.shard)
-        srt, wts, e_ids, post = moe_sorting(ids, topk_weights, num_experts=self.shard.experts_local, block_size=self.tile_m)
+        # routes of this rank's experts only, in their numbering (local_routing inside the sort)
+        srt, wts, e_ids, post = sort_on_device(topk_ids, topk_weights, self.shard.experts_local, self.tile_m, self.shard.e0)
         blocks = int(e_ids.numel())
         st = torch.cuda.current_stream(dev)
-        # rows of routes that belong to other ranks are never written nor read: zero keeps the quantiser finite
-        out1 = torch.zeros(tokens * self.topk, self.inter_dim, dtype=torch.bfloat16, device=dev)
+        # rows of routes that belong to other ranks are not written; the quantiser takes whatever they hold
+        # (Inf and NaN included) and nothing reads what it makes of them
+        out1 = torch.empty(tokens * self.topk, self.inter_dim, dtype=torch.bfloat16, device=dev)
         self._g1(out1, x_q.reshape(-1), self._w1.reshape(-1), scale_x.reshape(-1), self._sw1, srt, e_ids, wts, post, tokens,
                  self.inter_dim, self.model_dim, blocks, st)
         qd = torch.float8_e4m3fn if self.in_dtype == "fp8" else torch.int8

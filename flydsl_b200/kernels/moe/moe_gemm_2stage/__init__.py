@@ -92,24 +92,7 @@ def moe_sorting(
     max_padded = int(topk_ids.numel() + e * bs - topk)
     max_blocks = (max_padded + bs - 1) // bs
     if topk_ids.is_cuda:
-        # device kernels (flyb200_moe_sorting): no host synchronisation, capturable
-        ids32 = topk_ids.to(torch.int32).contiguous()
-        w32 = topk_weights.to(torch.float32).contiguous()
-        sorted_ids = torch.empty((max_padded,), dtype=torch.int32, device=dev)
-        sorted_weights = torch.empty((max_padded,), dtype=torch.float32, device=dev)
-        sorted_expert_ids = torch.empty((max_blocks,), dtype=torch.int32, device=dev)
-        post_pad = torch.empty((2,), dtype=torch.int32, device=dev)
-        counts = torch.empty((e,), dtype=torch.int32, device=dev)
-        with torch.cuda.device(dev):
-            _lib.check(
-                _lib.load().flyb200_moe_sorting(
-                    ids32.data_ptr(), w32.data_ptr(), tokens, topk, e, bs, sorted_ids.data_ptr(), sorted_weights.data_ptr(),
-                    sorted_expert_ids.data_ptr(), post_pad.data_ptr(), counts.data_ptr(),
-                    torch.cuda.current_stream(dev).cuda_stream,
-                ),
-                "moe_sorting",
-            )
-        return sorted_ids, sorted_weights, sorted_expert_ids, post_pad
+        return sort_on_device(topk_ids, topk_weights, e, bs, 0)
     flat = topk_ids.reshape(-1).to(torch.int64)
     flat = torch.where((flat >= 0) & (flat < e), flat, torch.full_like(flat, e))  # ids outside [0, e) are dropped
     order = torch.sort(flat, stable=True).indices  # by expert, then (token, slot)
@@ -134,6 +117,30 @@ def moe_sorting(
     )
     num_tokens_post_pad = torch.tensor([int(padded.sum()), tokens], dtype=torch.int32, device=dev)
     return sorted_ids, sorted_weights, sorted_expert_ids, num_tokens_post_pad
+
+
+def sort_on_device(topk_ids, topk_weights, experts: int, block_size: int, first_expert: int):
+    """``moe_sorting`` for CUDA tensors as one kernel (no host synchronisation, capturable), for the
+    experts ``[first_expert, first_expert + experts)`` renumbered from zero; other routes are dropped."""
+    tokens, topk = topk_ids.shape
+    dev = topk_ids.device
+    ids = topk_ids if topk_ids.dtype in (torch.int32, torch.int64) else topk_ids.to(torch.int32)
+    ids, w32 = ids.contiguous(), topk_weights.to(torch.float32).contiguous()
+    max_padded = tokens * topk + experts * block_size - topk
+    max_blocks = (max_padded + block_size - 1) // block_size
+    sorted_ids = torch.empty((max_padded,), dtype=torch.int32, device=dev)
+    sorted_weights = torch.empty((max_padded,), dtype=torch.float32, device=dev)
+    sorted_expert_ids = torch.empty((max_blocks,), dtype=torch.int32, device=dev)
+    post_pad = torch.empty((2,), dtype=torch.int32, device=dev)
+    with _lib.on_device(dev):
+        rc = _lib.load().flyb200_moe_sorting_range(
+            ids.data_ptr(), ids.element_size(), w32.data_ptr(), tokens, topk, experts, first_expert, block_size,
+            sorted_ids.data_ptr(), sorted_weights.data_ptr(), sorted_expert_ids.data_ptr(), post_pad.data_ptr(),
+            _lib.current_stream(dev),
+        )
+    if rc:
+        _lib.check(rc, "moe_sorting")
+    return sorted_ids, sorted_weights, sorted_expert_ids, post_pad
 
 
 class _MoeStage:

@@ -299,10 +299,16 @@ int flyb200_moe_gemm(int stage, void* out, const void* a_sorted, const void* w_s
  *   sorted_ids / sorted_weights  [tokens * topk + experts * block_size - topk]
  *   sorted_expert_ids            [ceil(that / block_size)]
  *   num_tokens_post_pad          [2] = { sorted rows in use, tokens }
- *   counts_scratch               [experts] int32 (contents irrelevant on entry) */
+ *   counts_scratch               [experts] int32 (not NULL; not used any more) */
 int flyb200_moe_sorting(const int* topk_ids, const float* topk_weights, int tokens, int topk, int experts, int block_size,
                         int* sorted_ids, float* sorted_weights, int* sorted_expert_ids, int* num_tokens_post_pad,
                         int* counts_scratch, void* stream);
+
+/* The same table for the experts [first_expert, first_expert + experts) of a larger set, renumbered from
+ * zero (routes to other experts are dropped), with ids of 4 or 8 bytes and no scratch. */
+int flyb200_moe_sorting_range(const void* topk_ids, int id_bytes, const float* topk_weights, int tokens, int topk, int experts,
+                              long long first_expert, int block_size, int* sorted_ids, float* sorted_weights,
+                              int* sorted_expert_ids, int* num_tokens_post_pad, void* stream);
 
 /* y[token, dim] = sum over slots of x[token, slot, dim] (fp32 sum, one rounding);
  * dtype FLYB200_OUT_BF16 or FLYB200_OUT_FP16, dim even.  With expert_mask

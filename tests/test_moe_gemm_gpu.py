@@ -432,6 +432,32 @@ def test_device_sorting_matches_oracle(dev, tokens, experts, topk, block):
         assert torch.equal(a.cpu(), b), name
 
 
+@pytest.mark.parametrize(
+    "tokens,experts,topk,block,first,total,id_t",
+    [
+        (1, 1, 1, 16, 0, 1, torch.int64),
+        (333, 8, 3, 32, 8, 24, torch.int32),     # 999 pairs: no multiple of four; a middle group of the experts
+        (2049, 16, 2, 64, 16, 32, torch.int64),  # one pair more than a chunk of 4096
+        (40, 5000, 4, 16, 0, 5000, torch.int32), # more experts than one pass of the histogram counts
+        (40, 300, 4, 16, 4200, 5000, torch.int64),
+    ],
+)
+@pytest.mark.parametrize("shift", [0, 1])
+def test_device_sorting_of_a_group_of_experts(dev, tokens, experts, topk, block, first, total, id_t, shift):
+    from flydsl_b200.kernels.moe.moe_gemm_2stage import sort_on_device
+
+    g = torch.Generator().manual_seed(tokens + total)
+    ids = torch.randint(-1, total, (tokens, topk), generator=g)
+    wts = torch.rand(tokens, topk, generator=g)
+    local = torch.where((ids >= first) & (ids < first + experts), ids - first, torch.full_like(ids, -1))
+    want = moe_sorting(local.to(torch.int32), wts, num_experts=experts, block_size=block)  # torch ops on CPU tensors
+    on_dev = torch.empty(tokens * topk + shift, dtype=id_t, device=dev)[shift:].view(tokens, topk)  # 16-byte aligned or not
+    on_dev.copy_(ids)
+    got = sort_on_device(on_dev, wts.to(dev), experts, block, first)
+    for name, a, b in zip(("sorted_ids", "sorted_weights", "sorted_expert_ids", "post_pad"), got, want):
+        assert torch.equal(a.cpu(), b), name
+
+
 def test_device_sorting_skewed_routing(dev):
     """Everything routed to one expert; an expert id outside the range is ignored."""
     ids = torch.full((70, 2), 3, dtype=torch.int32)

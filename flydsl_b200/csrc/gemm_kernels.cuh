@@ -153,6 +153,124 @@ __device__ __forceinline__ float load_bias(const void* bias, int col) {
   }
 }
 
+// 1 / x for 1 <= x < 2^126: the hardware estimate and one Newton-Raphson step whose residual is exact in
+// an FMA (Markstein, "Computation of elementary functions on the IBM RISC System/6000", 1990).  Equal to
+// the IEEE quotient but for at most 32 of the 2^23 mantissas, where it is one unit off with an error of
+// 0.5 + 2^-20 units (tests/test_rows_epilogue_gpu.py), and without its branch.
+__device__ __forceinline__ float reciprocal_of(float x) {
+  float r;
+  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
+  return fmaf(r, fmaf(-x, r, 1.0f), r);
+}
+
+// The activation of epilogue_value on eight values at once: the kind is a template argument and nothing
+// branches per value, so the eight chains (exponential, reciprocal) overlap.  Same operations in the same
+// order, same results.
+template <int EPI>
+__device__ __forceinline__ void activate_eight(float (&v)[8]) {
+  if constexpr (EPI == EPI_BIAS_RELU) {
+#pragma unroll
+    for (int i = 0; i < 8; ++i) v[i] = fmaxf(v[i], 0.0f);
+  } else if constexpr (EPI == EPI_BIAS_SILU) {
+    float d[8];
+    bool plain = true;  // false for a value below -87 (its denominator leaves the range above) or NaN
+#pragma unroll
+    for (int i = 0; i < 8; ++i) {
+      d[i] = 1.0f + __expf(-v[i]);
+      plain &= d[i] < 8.5e37f;
+    }
+    if (plain) {
+#pragma unroll
+      for (int i = 0; i < 8; ++i) v[i] = v[i] * reciprocal_of(d[i]);
+    } else {
+#pragma unroll
+      for (int i = 0; i < 8; ++i) v[i] = v[i] * (1.0f / d[i]);
+    }
+  } else if constexpr (EPI == EPI_BIAS_GELU) {
+#pragma unroll
+    for (int i = 0; i < 8; ++i) {
+      const float y = 0.7978845608f * (v[i] + 0.044715f * (v[i] * v[i] * v[i]));
+      const float e = __expf(-2.0f * fabsf(y));
+      const float num = (y > 0.0f) ? 2.0f : 2.0f * e;
+      v[i] = 0.5f * v[i] * (num * reciprocal_of(1.0f + e));
+    }
+  }
+}
+
+// Channel scales and bias of 32 neighbouring columns from `col` on (a multiple of 8; N is a multiple of
+// 16, so eight columns exist together).  Every lane reads the same addresses: 16-byte loads where the two
+// vectors start on 16 bytes (`vec`), single elements otherwise.  Without scales the factor is one.
+struct ColumnFactors {
+  float sb[32];
+  uint32_t bias[16];  // pairs in the output type
+};
+__device__ __forceinline__ void load_column_factors(ColumnFactors& f, const GemmParams& p, int col, bool scaled, bool vec) {
+  const uint16_t* bias = reinterpret_cast<const uint16_t*>(p.bias);
+  const bool biased = p.epilogue != EPI_NONE;
+#pragma unroll
+  for (int g = 0; g < 4; ++g) {
+    const int c = col + 8 * g;
+    const bool in = c < p.N;
+    if (vec) {
+      float4 s0 = make_float4(1.0f, 1.0f, 1.0f, 1.0f), s1 = s0;
+      uint4 b = make_uint4(0u, 0u, 0u, 0u);
+      if (scaled && in) {
+        s0 = __ldg(reinterpret_cast<const float4*>(p.sb + c));
+        s1 = __ldg(reinterpret_cast<const float4*>(p.sb + c + 4));
+      }
+      if (biased && in) b = __ldg(reinterpret_cast<const uint4*>(bias + c));
+      f.sb[8 * g] = s0.x, f.sb[8 * g + 1] = s0.y, f.sb[8 * g + 2] = s0.z, f.sb[8 * g + 3] = s0.w;
+      f.sb[8 * g + 4] = s1.x, f.sb[8 * g + 5] = s1.y, f.sb[8 * g + 6] = s1.z, f.sb[8 * g + 7] = s1.w;
+      f.bias[4 * g] = b.x, f.bias[4 * g + 1] = b.y, f.bias[4 * g + 2] = b.z, f.bias[4 * g + 3] = b.w;
+    } else {
+#pragma unroll
+      for (int i = 0; i < 8; ++i) f.sb[8 * g + i] = scaled && in ? __ldg(p.sb + c + i) : 1.0f;
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+        const uint32_t lo = biased && in ? __ldg(bias + c + 2 * i) : 0u, hi = biased && in ? __ldg(bias + c + 2 * i + 1) : 0u;
+        f.bias[4 * g + i] = lo | (hi << 16);
+      }
+    }
+  }
+}
+
+// 32 raw accumulators of one row -> scaled, biased, activated, 16-bit; `emit(g, pairs)` takes eight
+// columns (8 g ...).  The order of epilogue_value, every operation rounded by itself.  One value at a
+// time, with its own switch on the activation, its own division and two scalar loads, the four epilogue
+// warps took longer than the mainloop they overlap: int8 997 x 10208 x 5120, bias and gelu, 115.7 us for
+// the kernel (linear layer 130), now 58 (66).
+template <bool IS_INT, int OUTMODE, int EPI, typename EmitFn>
+__device__ __forceinline__ void epilogue_32(const uint32_t (&r)[32], float sa, const ColumnFactors& f, EmitFn emit) {
+#pragma unroll
+  for (int g = 0; g < 4; ++g) {
+    float v[8];
+#pragma unroll
+    for (int i = 0; i < 8; ++i) {
+      const float acc = IS_INT ? static_cast<float>(static_cast<int32_t>(r[8 * g + i])) : __uint_as_float(r[8 * g + i]);
+      v[i] = __fmul_rn(__fmul_rn(acc, sa), f.sb[8 * g + i]);
+      if constexpr (EPI != EPI_NONE) {
+        const uint16_t h = static_cast<uint16_t>(f.bias[4 * g + i / 2] >> (16 * (i & 1)));
+        v[i] = __fadd_rn(v[i], load_bias<OUTMODE>(&h, 0));
+      }
+    }
+    activate_eight<EPI>(v);
+    uint32_t pk[4];
+#pragma unroll
+    for (int i = 0; i < 4; ++i) pk[i] = pack2<OUTMODE>(v[2 * i], v[2 * i + 1]);
+    emit(g, pk);
+  }
+}
+template <bool IS_INT, int OUTMODE, typename EmitFn>
+__device__ __forceinline__ void epilogue_32(int epi, const uint32_t (&r)[32], float sa, const ColumnFactors& f, EmitFn emit) {
+  switch (epi) {
+    case EPI_BIAS: return epilogue_32<IS_INT, OUTMODE, EPI_BIAS>(r, sa, f, emit);
+    case EPI_BIAS_RELU: return epilogue_32<IS_INT, OUTMODE, EPI_BIAS_RELU>(r, sa, f, emit);
+    case EPI_BIAS_SILU: return epilogue_32<IS_INT, OUTMODE, EPI_BIAS_SILU>(r, sa, f, emit);
+    case EPI_BIAS_GELU: return epilogue_32<IS_INT, OUTMODE, EPI_BIAS_GELU>(r, sa, f, emit);
+    default: return epilogue_32<IS_INT, OUTMODE, EPI_NONE>(r, sa, f, emit);
+  }
+}
+
 // One warp's share (32 rows x BN columns) of an accumulator tile: TMEM ->
 // registers -> scale / bias / activation -> bf16|fp16 -> 128-byte-swizzled
 // staging buffer -> TMA store (clipped at M and N), or raw 32-bit stores.
@@ -172,7 +290,7 @@ __device__ __forceinline__ void epilogue_warp_tile(const GemmParams& p, const CU
   constexpr int C_BUF = 32 * 128;
   const bool scaled = (p.sa != nullptr) && (p.sb != nullptr);
   const int row = m0 + lane;
-  const float sa_v = (scaled && row < p.M) ? __ldg(p.sa + row) : 0.0f;
+  const float sa_v = !scaled ? 1.0f : row < p.M ? __ldg(p.sa + row) : 0.0f;
   if constexpr (OUTMODE == OUT_RAW32) {
     uint32_t* out = reinterpret_cast<uint32_t*>(p.c);
 #pragma unroll 1
@@ -196,6 +314,8 @@ __device__ __forceinline__ void epilogue_warp_tile(const GemmParams& p, const CU
     }
     release_tmem();
   } else {
+    const bool vec = ((reinterpret_cast<uintptr_t>(p.sb) | reinterpret_cast<uintptr_t>(p.bias)) & 15u) == 0;
+    ColumnFactors f;
 #pragma unroll 1
     for (int c0 = 0; c0 < BN; c0 += 64) {
       if (c0 + 64 > BN) {
@@ -204,66 +324,42 @@ __device__ __forceinline__ void epilogue_warp_tile(const GemmParams& p, const CU
         // leave the registers directly (64 contiguous bytes per row).
         uint32_t r[32];
         tmem_ld_x32(t_row + c0, r);
+        load_column_factors(f, p, n0 + c0, scaled, vec);
         tmem_ld_wait();
         release_tmem();
         if (row < p.M) {
           uint16_t* out_row = reinterpret_cast<uint16_t*>(p.c) + static_cast<size_t>(row) * p.N;
-#pragma unroll
-          for (int j = 0; j < 32; j += 8) {
-            const int col = n0 + c0 + j;
-            if (col < p.N) {  // N is a multiple of 16: eight columns are in or out together
-              uint32_t pk[4];
-#pragma unroll
-              for (int e = 0; e < 4; ++e) {
-                const int ce = col + 2 * e;
-                const float s0 = scaled ? __ldg(p.sb + ce) : 0.0f, s1 = scaled ? __ldg(p.sb + ce + 1) : 0.0f;
-                const float b0 = p.epilogue != EPI_NONE ? load_bias<OUTMODE>(p.bias, ce) : 0.0f;
-                const float b1 = p.epilogue != EPI_NONE ? load_bias<OUTMODE>(p.bias, ce + 1) : 0.0f;
-                pk[e] = pack2<OUTMODE>(epilogue_value<KT::is_int>(r[j + 2 * e], sa_v, s0, b0, p.epilogue, scaled),
-                                       epilogue_value<KT::is_int>(r[j + 2 * e + 1], sa_v, s1, b1, p.epilogue, scaled));
-              }
-              *reinterpret_cast<uint4*>(out_row + col) = make_uint4(pk[0], pk[1], pk[2], pk[3]);
-            }
-          }
+          epilogue_32<KT::is_int, OUTMODE>(p.epilogue, r, sa_v, f, [&](int g, const uint32_t (&pk)[4]) {
+            const int col = n0 + c0 + 8 * g;
+            if (col < p.N) *reinterpret_cast<uint4*>(out_row + col) = make_uint4(pk[0], pk[1], pk[2], pk[3]);
+          });
         }
         break;
       }
       uint32_t r0[32], r1[32];
       tmem_ld_x32(t_row + c0, r0);
       tmem_ld_x32(t_row + c0 + 32, r1);
+      load_column_factors(f, p, n0 + c0, scaled, vec);
       tmem_ld_wait();
       if (c0 + 64 >= BN) release_tmem();  // accumulator fully read: hand the TMEM buffer back
       // the store that last used this buffer (two chunks ago with two buffers) has to be done reading it
       if (lane == 0) bulk_wait_group_read<CBUFS - 1>();
       __syncwarp();
       const uint32_t cdst = stage_c + cbuf * C_BUF + lane * 128;
-#pragma unroll
+#pragma unroll 1
       for (int h = 0; h < 2; ++h) {
-        uint32_t(&r)[32] = h == 0 ? r0 : r1;
+        if (h == 1) {
+          load_column_factors(f, p, n0 + c0 + 32, scaled, vec);
 #pragma unroll
-        for (int j = 0; j < 32; j += 8) {
-          const int col = n0 + c0 + h * 32 + j;
-          float sbv[8], bv[8];
-#pragma unroll
-          for (int e = 0; e < 8; ++e) {
-            const bool in = (col + e) < p.N;
-            sbv[e] = (scaled && in) ? __ldg(p.sb + col + e) : 0.0f;
-            bv[e] = (p.epilogue != EPI_NONE && in) ? load_bias<OUTMODE>(p.bias, col + e) : 0.0f;
-          }
-          uint32_t pk[4];
-#pragma unroll
-          for (int e = 0; e < 4; ++e) {
-            float lo = epilogue_value<KT::is_int>(r[j + 2 * e], sa_v, sbv[2 * e], bv[2 * e], p.epilogue, scaled);
-            float hi =
-                epilogue_value<KT::is_int>(r[j + 2 * e + 1], sa_v, sbv[2 * e + 1], bv[2 * e + 1], p.epilogue, scaled);
-            pk[e] = pack2<OUTMODE>(lo, hi);
-          }
-          const int chunk = (h * 32 + j) >> 3;  // 16-byte chunk index inside the 128-byte row
+          for (int j = 0; j < 32; ++j) r0[j] = r1[j];
+        }
+        epilogue_32<KT::is_int, OUTMODE>(p.epilogue, r0, sa_v, f, [&](int g, const uint32_t (&pk)[4]) {
+          const int chunk = 4 * h + g;  // 16-byte chunk index inside the 128-byte row
           const uint32_t addr = cdst + static_cast<uint32_t>(((chunk ^ (lane & 7)) << 4));
           asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(addr), "r"(pk[0]), "r"(pk[1]), "r"(pk[2]),
                        "r"(pk[3])
                        : "memory");
-        }
+        });
       }
       fence_proxy_async_smem();
       __syncwarp();

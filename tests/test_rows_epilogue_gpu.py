@@ -1,0 +1,56 @@
+"""The large-M kernel's epilogue: every activation on tile edges, with channel scales and bias that do
+not start on 16 bytes, and the reciprocal it uses instead of a division."""
+
+import numpy as np
+import pytest
+import torch
+
+from oracle import a8w8_oracle as oracle
+from tests.test_gemm_parity_gpu import ATOL, ROWS, RTOL, TALL, run_gemm_generic
+
+
+def test_one_newton_step_gives_the_ieee_reciprocal():
+    """r + r (1 - x r) from any estimate within one unit in the last place, on every float of [1, 2)
+    (powers of two scale exactly): the IEEE reciprocal but for at most 32 of the 2^23, which are one unit
+    off, an error of 0.5 + 2^-20 units (Markstein's exceptions).  float64 holds the residual exactly."""
+    x = (np.arange(1 << 23, dtype=np.uint32) + np.uint32(0x3F800000)).view(np.float32)
+    exact = (np.float32(1) / x).astype(np.float32)
+    for step in (-1, 0, 1):
+        r = (exact.view(np.int32) + step).view(np.float32)
+        e = (1.0 - x.astype(np.float64) * r).astype(np.float32)
+        off = (r + r.astype(np.float64) * e).astype(np.float32).view(np.int32) - exact.view(np.int32)
+        assert np.abs(off).max() <= 1 and np.count_nonzero(off) <= 32
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("epilogue", ["none", "bias", "bias_relu", "bias_silu", "bias_gelu"])
+@pytest.mark.parametrize("in_dtype,out_dtype,offset,hint", [("fp8", "bf16", 0, ROWS | 8), ("int8", "fp16", 1, ROWS | 7), ("int8", "bf16", 2, TALL | 5),
+                                                            ("bf16", "fp16", 3, ROWS | 3), ("fp16", "bf16", 4, 0)])
+def test_epilogue_on_tile_edges(epilogue, in_dtype, out_dtype, offset, hint):
+    """Scales and bias as views `offset` elements into a buffer; N ends inside a tile, M inside a row block.
+    Large negative and positive biases reach both ends of the exponentials."""
+    dev = torch.device("cuda:0")
+    m, n, k = 301, 1040, 512
+    g = torch.Generator().manual_seed(offset)
+    odt = torch.float16 if out_dtype == "fp16" else torch.bfloat16
+    bias = torch.randn(n, generator=g) * 3
+    bias[::7] = -95.0
+    bias[1::7] = 60.0
+    bias = bias.to(odt)
+    if in_dtype in ("bf16", "fp16"):
+        dt = torch.bfloat16 if in_dtype == "bf16" else torch.float16
+        a, b = torch.randn(m, k, generator=g).to(dt), (torch.randn(n, k, generator=g) * 0.05).to(dt)
+        sa = sb = sb_dev = None
+    else:
+        a, b, sa, sb = oracle.make_inputs(m, n, k, in_dtype, seed=offset)
+        sb_buf = torch.empty(n + 8, dtype=torch.float32, device=dev)
+        sb_dev = sb_buf[offset : offset + n]
+        sb_dev.copy_(sb.view(-1))
+    bias_buf = torch.empty(n + 8, dtype=odt, device=dev)
+    bias_dev = bias_buf[offset : offset + n]
+    bias_dev.copy_(bias)
+    got = run_gemm_generic(dev, a, b, sa, sb_dev, bias_dev if epilogue != "none" else None, m, n, k, in_dtype, out_dtype=out_dtype,
+                           epilogue=epilogue, hint=hint)
+    acc = a.float() @ b.float().T
+    ref = oracle.epilogue(acc, sa, sb, bias, epilogue, out_dtype=torch.float32)
+    assert not torch.isnan(got).any() and oracle.strict_mismatches(got, ref, RTOL, ATOL) == 0

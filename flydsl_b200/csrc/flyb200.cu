@@ -658,20 +658,37 @@ int launch_shuffle(void* dst, const void* src, int N, int Kb, cudaStream_t s) {
 
 // Row quantiser launch: rows that fit the register-cached single-pass kernel
 // use it (one block per row), longer rows take the two-pass kernel.
+template <typename TIn, bool FP8, int NV, int WPR>
+void launch_quant_rows(uint8_t* y, float* scale, const TIn* x, int rows, int K, cudaStream_t s) {
+  constexpr int PER_BLOCK = 8 / WPR;
+  pertoken_quant_row_kernel<TIn, FP8, NV, WPR><<<(rows + PER_BLOCK - 1) / PER_BLOCK, 256, 0, s>>>(y, scale, x, rows, K);
+}
+// Warps per row: as few as keep a row in eight vectors per thread (a warp that owns its row needs no
+// barrier, and eight loads per thread cover the latency), but at least two blocks per SM: few rows
+// take more warps each.
 template <typename TIn, bool FP8>
 void launch_quant_t(uint8_t* y, float* scale, const TIn* x, int rows, int K, cudaStream_t s) {
-  constexpr int per_vec = 256 * QuantIn<TIn>::VEC;
-  if (K <= per_vec) {
-    pertoken_quant_row_kernel<TIn, FP8, 1><<<rows, 256, 0, s>>>(y, scale, x, rows, K);
-  } else if (K <= 2 * per_vec) {
-    pertoken_quant_row_kernel<TIn, FP8, 2><<<rows, 256, 0, s>>>(y, scale, x, rows, K);
-  } else if (K <= 4 * per_vec) {
-    pertoken_quant_row_kernel<TIn, FP8, 4><<<rows, 256, 0, s>>>(y, scale, x, rows, K);
-  } else if (K <= 8 * per_vec) {
-    pertoken_quant_row_kernel<TIn, FP8, 8><<<rows, 256, 0, s>>>(y, scale, x, rows, K);
-  } else {
+  const int vecs = K / QuantIn<TIn>::VEC;  // 16-byte vectors of a row
+  int wpr = 1;
+  while (wpr < 8 && (vecs > 256 * wpr || static_cast<long long>(rows) * wpr < 2LL * 148 * 8)) wpr *= 2;
+  const int nv = (vecs + 32 * wpr - 1) / (32 * wpr);  // vectors per thread
+  if (nv > 8) {
     const int grid = rows < 148 * 16 ? rows : 148 * 16;
     pertoken_quant_kernel<TIn, FP8><<<grid, 256, 0, s>>>(y, scale, x, rows, K);
+  } else if (wpr == 1) {
+    if (nv <= 4) launch_quant_rows<TIn, FP8, 4, 1>(y, scale, x, rows, K, s);
+    else launch_quant_rows<TIn, FP8, 8, 1>(y, scale, x, rows, K, s);
+  } else if (wpr == 2) {
+    if (nv <= 4) launch_quant_rows<TIn, FP8, 4, 2>(y, scale, x, rows, K, s);
+    else launch_quant_rows<TIn, FP8, 8, 2>(y, scale, x, rows, K, s);
+  } else if (wpr == 4) {
+    if (nv <= 4) launch_quant_rows<TIn, FP8, 4, 4>(y, scale, x, rows, K, s);
+    else launch_quant_rows<TIn, FP8, 8, 4>(y, scale, x, rows, K, s);
+  } else {
+    if (nv <= 1) launch_quant_rows<TIn, FP8, 1, 8>(y, scale, x, rows, K, s);
+    else if (nv <= 2) launch_quant_rows<TIn, FP8, 2, 8>(y, scale, x, rows, K, s);
+    else if (nv <= 4) launch_quant_rows<TIn, FP8, 4, 8>(y, scale, x, rows, K, s);
+    else launch_quant_rows<TIn, FP8, 8, 8>(y, scale, x, rows, K, s);
   }
 }
 template <typename TIn>

@@ -12,10 +12,9 @@
 // torch's CUDA backend as a multiplication by the fp32 reciprocal, the
 // element-wise division is a true IEEE division.
 //
-// One 256-thread block per row, 16-byte loads, 4..8-byte stores.  Rows of up to
-// 8192 (fp32) / 16384 (16-bit) elements stay in registers between the maximum
-// and the conversion and are read from memory once; longer rows are read twice
-// (the second time from L1/L2).
+// Rows of up to 8192 (fp32) / 16384 (16-bit) elements stay in registers between the
+// maximum and the conversion and are read from memory once; longer rows are read
+// twice (the second time from L1/L2).
 #pragma once
 #include <cstdint>
 #include <cuda_bf16.h>
@@ -81,145 +80,208 @@ __device__ __forceinline__ uint8_t quant_one(float v, float s) {
   }
 }
 
-// Four finite values -> four packed bytes, bit-identical to four quant_one calls
-// but normally without the IEEE divisions.  q' = v * rcp(s) differs from the
-// correctly rounded quotient q = v / s by at most 2.5 ulp, so converting q'
-// gives the same byte unless a rounding boundary of the target type lies
-// within 3 ulp of q': for e4m3 the midpoints between neighbouring values (low
-// 20 mantissa bits == 0x80000) and, conservatively, everything below 2^-5
-// (subnormal spacing); for int8 (truncation) the integers.  If any of the four
-// is that close to a boundary, all four take the exact route.
+// Four finite values -> four packed bytes, bit-identical to four quant_one calls without the IEEE
+// divisions: q0 = v * y with y = RN(1 / s), then one correction with the exact residual,
+// q = q0 + (v - q0 s) y, which rounds to the IEEE quotient (Markstein, "Computation of elementary
+// functions on the IBM RISC System/6000", 1990).  Two values per instruction.  The residual is exact
+// where q matters (from half the smallest e4m3 subnormal, 2^-10, or 1 for int8, up) as long as s is not
+// below 2^-90; the caller divides there.  fp8: the quotient is carried negated, which keeps the sign of a
+// zero (-0 / s = -0) through the correction; the sign bits are flipped back at the end.
+__device__ __forceinline__ unsigned long long f32x2(float lo, float hi) {
+  unsigned long long d;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(d) : "f"(lo), "f"(hi));
+  return d;
+}
+__device__ __forceinline__ float2 f32x2_parts(unsigned long long d) {
+  float2 f;
+  asm("mov.b64 {%0, %1}, %2;" : "=f"(f.x), "=f"(f.y) : "l"(d));
+  return f;
+}
+__device__ __forceinline__ unsigned long long fma_f32x2(unsigned long long a, unsigned long long b, unsigned long long c) {
+  unsigned long long d;
+  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d) : "l"(a), "l"(b), "l"(c));
+  return d;
+}
+__device__ __forceinline__ unsigned long long mul_f32x2(unsigned long long a, unsigned long long b) {
+  unsigned long long d;
+  asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
+  return d;
+}
+
+// What the conversion of a row needs of its scale, each twice: fp8 (s, -1 / s), int8 (-s, 1 / s).
+struct RowDivisor {
+  unsigned long long s, inv;
+};
 template <bool FP8>
-__device__ __forceinline__ uint32_t quant_four(const float* v, float s, float inv_s) {
-  float q[4];
-  bool risky = false;
-#pragma unroll
-  for (int e = 0; e < 4; ++e) {
-    q[e] = v[e] * inv_s;
-    if constexpr (FP8) {
-      const uint32_t b = __float_as_uint(q[e]);
-      const uint32_t mag = b & 0x7FFFFFFFu;
-      risky |= ((b & 0xFFFFFu) - (0x80000u - 3u)) <= 6u;
-      risky |= (mag < 0x3D000000u) && (mag != 0u);
-    } else {
-      risky |= (fabsf(q[e] - rintf(q[e])) < 6.2e-5f) && (q[e] != 0.0f);
-    }
-  }
-  if (risky) {
-    uint32_t b = 0;
-#pragma unroll
-    for (int e = 0; e < 4; ++e) b |= static_cast<uint32_t>(quant_one<FP8>(v[e], s)) << (8 * e);
-    return b;
-  }
+__device__ __forceinline__ RowDivisor row_divisor(float s) {
+  const float inv = __frcp_rn(s);
+  return FP8 ? RowDivisor{f32x2(s, s), f32x2(-inv, -inv)} : RowDivisor{f32x2(-s, -s), f32x2(inv, inv)};
+}
+constexpr float QUANT_TINY_SCALE = 1e-27f;  // above 2^-90
+
+template <bool FP8>
+__device__ __forceinline__ uint32_t quant_four(unsigned long long v01, unsigned long long v23, const RowDivisor& d) {
+  unsigned long long q01 = mul_f32x2(v01, d.inv), q23 = mul_f32x2(v23, d.inv);
+  q01 = fma_f32x2(fma_f32x2(q01, d.s, v01), d.inv, q01);
+  q23 = fma_f32x2(fma_f32x2(q23, d.s, v23), d.inv, q23);
+  const float2 a = f32x2_parts(q01), b = f32x2_parts(q23);
   if constexpr (FP8) {
-    const uint32_t lo = __nv_cvt_float2_to_fp8x2(make_float2(q[0], q[1]), __NV_SATFINITE, __NV_E4M3);
-    const uint32_t hi = __nv_cvt_float2_to_fp8x2(make_float2(q[2], q[3]), __NV_SATFINITE, __NV_E4M3);
-    return lo | (hi << 16);
+    const uint32_t lo = __nv_cvt_float2_to_fp8x2(a, __NV_SATFINITE, __NV_E4M3);
+    const uint32_t hi = __nv_cvt_float2_to_fp8x2(b, __NV_SATFINITE, __NV_E4M3);
+    return (lo | (hi << 16)) ^ 0x80808080u;
   } else {
-    uint32_t b = 0;
-#pragma unroll
-    for (int e = 0; e < 4; ++e) b |= (static_cast<uint32_t>(__float2int_rz(q[e])) & 0xFFu) << (8 * e);
-    return b;
+    const uint32_t lo = __byte_perm(__float2int_rz(a.x), __float2int_rz(a.y), 0x0040);
+    const uint32_t hi = __byte_perm(__float2int_rz(b.x), __float2int_rz(b.y), 0x0040);
+    return __byte_perm(lo, hi, 0x5410);
   }
 }
 
-// Single-pass form for rows of at most 256 * VEC * NV elements: every thread
-// keeps its NV vectors of the row in registers between the maximum and the
-// conversion, so the row is read from memory exactly once and all of a
-// thread's loads are in flight together.  One block per row.
-template <typename TIn, bool FP8, int NV>
-__global__ void __launch_bounds__(256) pertoken_quant_row_kernel(uint8_t* __restrict__ y, float* __restrict__ scale,
-                                                                 const TIn* __restrict__ x, int rows, int K) {
-  constexpr int VEC = QuantIn<TIn>::VEC;
-  constexpr float QMAX = FP8 ? 448.0f : 127.0f;
-  __shared__ float warp_max[8];
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  const int r = blockIdx.x;
-  if (r >= rows) return;
-  const TIn* xr = x + static_cast<size_t>(r) * K;
-  float v[NV][VEC];
-#pragma unroll
-  for (int i = 0; i < NV; ++i) {
-    const int k = (i * 256 + threadIdx.x) * VEC;
-    if (k < K) {
-      QuantIn<TIn>::load(xr + k, v[i]);
-    } else {
-#pragma unroll
-      for (int e = 0; e < VEC; ++e) v[i][e] = 0.0f;
-    }
+// Largest magnitude of a 16-byte vector and what the raw words stand for.  For finite values the order
+// of |x| is the order of the bit patterns without their sign, and any Inf / NaN shows up as a maximum of at
+// least INF_BITS, so the maximum needs no conversion: two 16-bit values per instruction.
+template <typename T>
+struct QuantRaw;
+template <>
+struct QuantRaw<float> {
+  static constexpr uint32_t INF_BITS = 0x7F800000u;
+  __device__ static uint32_t max_abs(uint32_t m, uint32_t w) { return max(m, w & 0x7FFFFFFFu); }
+  __device__ static uint32_t fold(uint32_t m) { return m; }
+  __device__ static float value(uint32_t bits) { return __uint_as_float(bits); }
+  __device__ static void unpack(const uint4& t, float (&v)[4]) {
+    v[0] = __uint_as_float(t.x), v[1] = __uint_as_float(t.y), v[2] = __uint_as_float(t.z), v[3] = __uint_as_float(t.w);
   }
-  // Row maximum on the bit patterns: for finite floats the order of |x| is the
-  // order of (bits & 0x7fffffff) as unsigned integers, and any Inf / NaN in the
-  // row shows up as a maximum >= 0x7f800000, which sends the whole row down the
-  // careful path below.  (The kernel is instruction-bound, not memory-bound, for
-  // 16-bit inputs: every instruction per element counts.)
-  uint32_t bmax = 0u;
+};
+template <typename T>
+struct QuantRaw16 {
+  __device__ static uint32_t max_abs(uint32_t m, uint32_t w) { return __vmaxu2(m, w & 0x7FFF7FFFu); }
+  __device__ static uint32_t fold(uint32_t m) { return max(m & 0xFFFFu, m >> 16); }
+};
+template <>
+struct QuantRaw<__half> : QuantRaw16<__half> {
+  static constexpr uint32_t INF_BITS = 0x7C00u;
+  __device__ static float value(uint32_t bits) { return __half2float(__ushort_as_half(static_cast<unsigned short>(bits))); }
+  __device__ static void unpack(const uint4& t, float (&v)[8]) { QuantIn<__half>::load(reinterpret_cast<const __half*>(&t), v); }
+};
+template <>
+struct QuantRaw<__nv_bfloat16> : QuantRaw16<__nv_bfloat16> {
+  static constexpr uint32_t INF_BITS = 0x7F80u;
+  __device__ static float value(uint32_t bits) { return __uint_as_float(bits << 16); }
+  __device__ static void unpack(const uint4& t, float (&v)[8]) {
+    const uint32_t w[4] = {t.x, t.y, t.z, t.w};
 #pragma unroll
-  for (int i = 0; i < NV; ++i) {
-#pragma unroll
-    for (int e = 0; e < VEC; ++e) bmax = max(bmax, __float_as_uint(v[i][e]) & 0x7FFFFFFFu);
+    for (int i = 0; i < 4; ++i) v[2 * i] = __uint_as_float(w[i] << 16), v[2 * i + 1] = __uint_as_float(w[i] & 0xFFFF0000u);
   }
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) bmax = max(bmax, __shfl_xor_sync(0xffffffffu, bmax, o));
-  if (lane == 0) warp_max[warp] = __uint_as_float(bmax);
-  __syncthreads();
-  uint32_t mb = __float_as_uint(warp_max[lane & 7]);
-#pragma unroll
-  for (int o = 4; o > 0; o >>= 1) mb = max(mb, __shfl_xor_sync(0xffffffffu, mb, o));
-  uint8_t* yr = y + static_cast<size_t>(r) * K;
+};
 
-  if (mb >= 0x7F800000u) {
-    // ---- careful path: the row holds Inf or NaN (block-uniform branch) ----
-    __syncthreads();  // warp_max is reused
+// Quantises one row held as NV raw vectors per thread by the WPR warps that share it (`tid` inside
+// them): vector i covers elements (i * 32 WPR + tid) * VEC.  `red`: 8 words of shared memory of the block,
+// `first_warp`: the row's first warp; barriers are per row (`bar_id`), so rows may take different branches.
+template <typename TIn, bool FP8, int NV, int WPR>
+__device__ __forceinline__ void quant_row_from_registers(const uint4 (&raw)[NV], uint8_t* __restrict__ yr, float* scale_out,
+                                                         int K, int tid, uint32_t* red, int first_warp, int bar_id) {
+  using R = QuantRaw<TIn>;
+  constexpr int VEC = QuantIn<TIn>::VEC;
+  constexpr int TPR = 32 * WPR;
+  constexpr float QMAX = FP8 ? 448.0f : 127.0f;
+  const int lane = tid & 31, warp = tid >> 5;
+  auto row_max = [&](uint32_t m) {
+    m = __reduce_max_sync(0xffffffffu, m);
+    if constexpr (WPR > 1) {
+      if (lane == 0) red[first_warp + warp] = m;
+      asm volatile("bar.sync %0, %1;" ::"r"(bar_id), "n"(TPR) : "memory");
+#pragma unroll
+      for (int w = 0; w < WPR; ++w) m = max(m, red[first_warp + w]);
+    }
+    return m;
+  };
+  uint32_t m = 0u;
+#pragma unroll
+  for (int i = 0; i < NV; ++i) m = R::max_abs(R::max_abs(R::max_abs(R::max_abs(m, raw[i].x), raw[i].y), raw[i].z), raw[i].w);
+  m = row_max(R::fold(m));
+
+  if (m >= R::INF_BITS) {
+    // ---- careful path: the row holds Inf or NaN (the same branch in all of the row's threads) ----
     float amax = 0.0f;
 #pragma unroll
     for (int i = 0; i < NV; ++i) {
+      float v[VEC];
+      R::unpack(raw[i], v);
 #pragma unroll
-      for (int e = 0; e < VEC; ++e) {
-        v[i][e] = scrub(v[i][e], QMAX);
-        amax = fmaxf(amax, fabsf(v[i][e]));
-      }
+      for (int e = 0; e < VEC; ++e) amax = fmaxf(amax, fabsf(scrub(v[e], QMAX)));
     }
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, o));
-    if (lane == 0) warp_max[warp] = amax;
-    __syncthreads();
-    float m = warp_max[lane & 7];
-#pragma unroll
-    for (int o = 4; o > 0; o >>= 1) m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, o));
-    float s = __fmul_rn(m, __fdiv_rn(1.0f, QMAX));
+    if constexpr (WPR > 1) asm volatile("bar.sync %0, %1;" ::"r"(bar_id), "n"(TPR) : "memory");  // red is reused
+    float s = __fmul_rn(__uint_as_float(row_max(__float_as_uint(amax))), __fdiv_rn(1.0f, QMAX));
     if (s == 0.0f) s = 1.0f;
-    if (threadIdx.x == 0) scale[r] = s;
+    if (tid == 0) *scale_out = s;
 #pragma unroll
     for (int i = 0; i < NV; ++i) {
-      const int k = (i * 256 + threadIdx.x) * VEC;
-      if (k < K) {
+      const int k = (i * TPR + tid) * VEC;
+      if (k >= K) break;
+      float v[VEC];
+      R::unpack(raw[i], v);
 #pragma unroll
-        for (int e = 0; e < VEC; ++e) yr[k + e] = quant_one<FP8>(v[i][e], s);
-      }
+      for (int e = 0; e < VEC; ++e) yr[k + e] = quant_one<FP8>(scrub(v[e], QMAX), s);
     }
     return;
   }
 
-  // ---- fast path: all finite ----
-  float s = __fmul_rn(__uint_as_float(mb), __fdiv_rn(1.0f, QMAX));
+  float s = __fmul_rn(R::value(m), __fdiv_rn(1.0f, QMAX));
   if (s == 0.0f) s = 1.0f;
-  if (threadIdx.x == 0) scale[r] = s;
-  const float inv_s = __frcp_rn(s);
+  if (tid == 0) *scale_out = s;
+  const bool tiny = s < QUANT_TINY_SCALE;
+  const RowDivisor d = row_divisor<FP8>(s);
 #pragma unroll
   for (int i = 0; i < NV; ++i) {
-    const int k = (i * 256 + threadIdx.x) * VEC;
-    if (k < K) {
-      uint32_t packed[VEC / 4];
+    const int k = (i * TPR + tid) * VEC;
+    if (k >= K) break;
+    float v[VEC];
+    R::unpack(raw[i], v);
+    uint32_t packed[VEC / 4];
 #pragma unroll
-      for (int w = 0; w < VEC / 4; ++w) packed[w] = quant_four<FP8>(&v[i][4 * w], s, inv_s);
-      if constexpr (VEC == 4) {
-        *reinterpret_cast<uint32_t*>(yr + k) = packed[0];
+    for (int w = 0; w < VEC / 4; ++w) {
+      if (!tiny) {
+        packed[w] = quant_four<FP8>(f32x2(v[4 * w], v[4 * w + 1]), f32x2(v[4 * w + 2], v[4 * w + 3]), d);
       } else {
-        *reinterpret_cast<uint2*>(yr + k) = make_uint2(packed[0], packed[1]);
+        packed[w] = 0u;
+#pragma unroll
+        for (int e = 0; e < 4; ++e) packed[w] |= static_cast<uint32_t>(quant_one<FP8>(v[4 * w + e], s)) << (8 * e);
       }
     }
+    if constexpr (VEC == 4) {
+      *reinterpret_cast<uint32_t*>(yr + k) = packed[0];
+    } else {
+      *reinterpret_cast<uint2*>(yr + k) = make_uint2(packed[0], packed[1]);
+    }
   }
+}
+
+// Single-pass form for rows of at most 32 * WPR * VEC * NV elements.  WPR warps of a 256-thread block
+// share a row; every thread has its NV loads in flight together and keeps the raw vectors in registers
+// (half the registers of the converted values, so more rows in flight).  Memory-bound where there are
+// rows enough; few rows are spread over more warps (launch_quant_t).  One 256-thread block per row, with
+// a conversion of every value before the maximum and a test next to every product for a rounding boundary,
+// was bound by instruction issue and, on short rows, by blocks of a few loads each.  bf16 -> fp8 / int8, us,
+// before and now: 8192 x 8192 51.7 / 49.0 and 39.1 / 44.3 (5.2 / 4.6 TB/s), 8192 x 2048 17.5 / 16.3 and
+// 11.4 / 12.9, 4096 x 14336 61.4 / 58.7 and 37.6 / 42.8, 997 x 5120 6.9 / 7.0 and 4.3 / 5.1, 1 x 8192 2.7 and 1.9.
+// (int8 trails by its float-to-integer conversions, four to a byte quad.)
+template <typename TIn, bool FP8, int NV, int WPR>
+__global__ void __launch_bounds__(256) pertoken_quant_row_kernel(uint8_t* __restrict__ y, float* __restrict__ scale,
+                                                                 const TIn* __restrict__ x, int rows, int K) {
+  constexpr int VEC = QuantIn<TIn>::VEC;
+  __shared__ uint32_t red[8];
+  // a GEMM launched as programmatic dependent may set itself up now (it waits for this grid before it reads)
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+  const int group = threadIdx.x / (32 * WPR), tid = threadIdx.x % (32 * WPR);
+  const int r = blockIdx.x * (8 / WPR) + group;
+  if (r >= rows) return;
+  const TIn* xr = x + static_cast<size_t>(r) * K;
+  uint4 raw[NV];
+#pragma unroll
+  for (int i = 0; i < NV; ++i) {
+    const int k = (i * 32 * WPR + tid) * VEC;
+    raw[i] = k < K ? __ldg(reinterpret_cast<const uint4*>(xr + k)) : make_uint4(0u, 0u, 0u, 0u);
+  }
+  quant_row_from_registers<TIn, FP8, NV, WPR>(raw, y + static_cast<size_t>(r) * K, scale + r, K, tid, red, group * WPR, 1 + group);
 }
 
 // General form (any row length): two passes over the row, the second one from L1/L2.

@@ -112,3 +112,43 @@ def test_kernel_bit_identical_on_adversarial_values(qd):
     torch.cuda.synchronize()
     assert torch.equal(s_k, s_t)
     assert torch.equal(y_k.view(torch.uint8), y_t.view(torch.uint8))
+
+
+def boundary_rows(rows, k, dtype, qd, seed):
+    """Rows over the whole exponent range (subnormal to the largest finite), values on and next to the
+    rounding boundaries of the target type relative to the row's scale, both zeros, and a few rows with
+    Inf or NaN among them (every row takes its own branch, whoever shares its block)."""
+    g = torch.Generator().manual_seed(seed)
+    x = torch.randn(rows, k, generator=g)
+    qmax = 448.0 if qd == FP8 else 127.0
+    if qd == FP8:
+        grid = torch.arange(0x7F, dtype=torch.uint8).view(FP8).float()
+        mids = (grid[1:] + grid[:-1]) / 2
+    else:
+        mids = torch.arange(1, 127).float()
+    pick = mids[torch.randint(0, mids.numel(), (rows, k), generator=g)] * torch.where(torch.rand(rows, k, generator=g) < 0.5, -1.0, 1.0)
+    x = torch.where(torch.rand(rows, k, generator=g) < 0.5, pick, x)
+    x[:, 0] = qmax
+    x = (x * (1 + torch.randint(-2, 3, (rows, k), generator=g) * 2.0**-24)) * torch.exp2(
+        torch.randint(-148, 119, (rows, 1), generator=g).float())
+    x[:, 1::9] = 0.0
+    x[:, 2::9] = -0.0
+    x[::11, 3 % k] = float("nan")
+    x[5::13, 5 % k] = float("-inf")
+    x[7::17] = 0.0
+    if dtype == torch.float16:
+        x = x.clamp(-65504, 65504)
+    return x.to(dtype)
+
+
+@pytest.mark.parametrize("qd", [FP8, torch.int8], ids=["fp8", "int8"])
+@pytest.mark.parametrize("dtype", [torch.float32, torch.float16, torch.bfloat16])
+# one, two, four and eight warps per row, four and eight vectors per thread, few rows, the two-pass form
+@pytest.mark.parametrize("rows,k", [(2500, 8), (2501, 1024), (2403, 2048), (2400, 4096), (1500, 3592), (1203, 5120), (700, 8192),
+                                    (299, 16384), (40, 4104), (3, 8200), (65, 16392), (1, 24)])
+def test_every_split_of_a_row_is_bit_identical(qd, dtype, rows, k):
+    x = boundary_rows(rows, k, dtype, qd, rows + k).to("cuda:0")
+    y_k, s_k = pertoken_quant_kernel(x, qd)
+    y_t, s_t = pertoken_quant(x, quant_dtype=qd, use_kernel=False)
+    assert torch.equal(s_k, s_t)
+    assert torch.equal(y_k.view(torch.uint8), y_t.view(torch.uint8))

@@ -21,10 +21,10 @@ namespace {
 
 inline bool aligned16(const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15u) == 0; }
 
-template <int OUTMODE, int BN, bool FP4 = false>
+template <int OUTMODE, int BN, bool FP4, bool SPLIT = false>
 int launch_mx(const CUtensorMap& tmA, const MxParams& p, cudaStream_t s) {
   static std::atomic<uint64_t> done{0};
-  auto kernel = mx_gemm_kernel<OUTMODE, BN, FP4>;
+  auto kernel = mx_gemm_kernel<OUTMODE, BN, FP4, SPLIT>;
   using Smem = MxSmem<BN, FP4>;
   int dev = 0;
   CUDA_TRY(cudaGetDevice(&dev));
@@ -34,11 +34,23 @@ int launch_mx(const CUtensorMap& tmA, const MxParams& p, cudaStream_t s) {
     done.fetch_or(bit, std::memory_order_release);
   }
   int sms = 0;
-  CUDA_TRY(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
+  int rc = host::sm_count(&sms);
+  if (rc) return rc;
   const long long tiles = static_cast<long long>((p.M + BLOCK_ROWS - 1) / BLOCK_ROWS) * (p.N / BN);
-  const int grid = static_cast<int>(tiles < sms ? tiles : sms);
-  kernel<<<grid, NUM_THREADS, Smem::TOTAL, s>>>(tmA, p);
-  CUDA_TRY(cudaGetLastError());
+  cudaLaunchConfig_t cfg;
+  memset(&cfg, 0, sizeof(cfg));
+  cfg.gridDim = dim3(static_cast<unsigned>(SPLIT ? tiles * p.split : tiles < sms ? tiles : sms), 1, 1);
+  cfg.blockDim = dim3(NUM_THREADS, 1, 1);
+  cfg.dynamicSmemBytes = Smem::TOTAL;
+  cfg.stream = s;
+  cudaLaunchAttribute attr;
+  attr.id = cudaLaunchAttributeClusterDimension;
+  attr.val.clusterDim.x = static_cast<unsigned>(p.split);
+  attr.val.clusterDim.y = 1;
+  attr.val.clusterDim.z = 1;
+  cfg.attrs = &attr;
+  cfg.numAttrs = SPLIT ? 1 : 0;
+  CUDA_TRY(cudaLaunchKernelEx(&cfg, kernel, tmA, p));
   return FLYB200_OK;
 }
 
@@ -51,6 +63,79 @@ void launch_mx_quant(uint8_t* codes, uint8_t* scale, uint8_t* raw, const TIn* x,
   else if (fmt == MXQ_FP4) mx_quant_kernel<TIn, MXQ_FP4><<<grid, 256, 0, s>>>(codes, scale, raw, x, units);
   else mx_quant_kernel<TIn, MXQ_FP6><<<grid, 256, 0, s>>>(codes, scale, raw, x, units);
 }
+
+namespace {
+// Up to 128 tokens are a weight stream for the small-M kernel in its block-scaled kind - as long as its
+// CTAs (one per 128 channels) fit one round: on wider outputs its later rounds run part empty and the
+// persistent large-M kernel is 20-45 % faster (MXFP8 128 x 28672 x 8192: 43 against 66 us; MXFP4 128 x
+// 57344 x 8192: 51 against 90 us).  FLYB200_MX_SMALL=0 / 1 forces the choice.
+bool mx_small_m(int M, int N) {
+  if (M > 128) return false;
+  if (const char* e = getenv("FLYB200_MX_SMALL")) {
+    if (e[0] == '0') return false;
+    if (e[0] == '1') return true;
+  }
+  int sms = 0;
+  if (flyb200::host::sm_count(&sms) != FLYB200_OK) return true;
+  return (N + 127) / 128 <= sms;
+}
+// Tile shape of the large-M kernel: 128 x 256 tiles (one accumulator, exposed epilogue) win once a
+// tile's mainloop is a few times longer than its epilogue (2.44-2.47 against 1.82-1.88 PFLOP/s at
+// K = 8192, M >= 4096) - unless the 128 x 128 tiles cover the output in one round of CTAs: then
+// they put twice as many SMs to work (MXFP8 256 x 8192 x 8192: 27.9 against 31.4 us; MXFP4:
+// 18.4 against 20.9 us).  `k_bytes`: bytes of codes per row.
+bool mx_wide_tiles(int M, int N, int k_bytes) {
+  if (N % 256 != 0 || k_bytes < 1024) return false;
+  int sms = 0;
+  if (flyb200::host::sm_count(&sms) != FLYB200_OK) return true;
+  const long long tiles128 = static_cast<long long>((M + 127) / 128) * (N / 128);
+  return tiles128 > sms;
+}
+// K parts of a tile (CTAs of a cluster), 1 = none: the largest of eight, four and two that fits one round of
+// CTAs with at least eight k-blocks each.  Clusters of eight have to find eight free SMs inside one GPC
+// and are placed without delay only while they cover at most half of the SMs.  Measured, split 1 / 2 / 4 /
+// 8, us: MXFP6 x MXFP4 256 x 4096 x 14336 (64 tiles) 46.2 / 27.7 / 36.0 / 66, 128 x 4096 x 14336 (32) 46.2 /
+// 27.0 / 19.9 / 41, 64 x 1024 x 8192 (8) 27.8 / 17.1 / 13.1 / 11.2; MXFP8 200 x 1024 x 14336 (16) 44.0 / 23.9 /
+// 16.5 / 22.5, 600 x 1792 x 2048 (70, 16 k-blocks) 11.4 / 9.6 / 23 / 41, 256 x 4096 x 1024 (64, 8 k-blocks)
+// 7.2 / 8.0 / 16 / 40; MXFP4 256 x 4096 x 14336 27.9 / 18.1 / 26.4 / 54.
+// FLYB200_MX_SPLIT = 1, 2, 4 or 8 forces the factor (tuning and tests).
+int mx_split(int M, int N, int k_bytes) {
+  if (const char* e = getenv("FLYB200_MX_SPLIT"))
+    if (e[0] == '1' || e[0] == '2' || e[0] == '4' || e[0] == '8') return e[0] - '0';
+  int sms = 0;
+  if (flyb200::host::sm_count(&sms) != FLYB200_OK) return 1;
+  const long long tiles = static_cast<long long>((M + 127) / 128) * (N / 128);
+  const int kb = k_bytes / KBLOCK_BYTES;
+  if (16 * tiles <= sms && kb >= 64) return 8;
+  if (4 * tiles <= sms && kb >= 32) return 4;
+  if (2 * tiles <= sms && kb >= 16) return 2;
+  return 1;
+}
+
+template <int OUTMODE, bool FP4>
+int launch_mx_large(const void* a, MxParams& p, cudaStream_t s) {
+  int rc = host::status_word(&p.status);
+  if (rc) return rc;
+  CUtensorMap tmA;
+  rc = host::byte_matrix_map(&tmA, a, static_cast<uint64_t>(p.K_bytes), static_cast<uint64_t>(p.M), BLOCK_ROWS);
+  if (rc) return rc;
+  // FLYB200_MX_BN forces a tile shape without a K split (tuning and tests)
+  bool wide = mx_wide_tiles(p.M, p.N, p.K_bytes);
+  p.split = wide ? 1 : mx_split(p.M, p.N, p.K_bytes);
+  if (const char* e = getenv("FLYB200_MX_BN")) {
+    if (e[0] == '1') wide = false, p.split = 1;
+    if (e[0] == '2' && p.N % 256 == 0) wide = true;
+  }
+  if (wide) return launch_mx<OUTMODE, 256, FP4>(tmA, p, s);
+  if (p.split > 1) return launch_mx<OUTMODE, 128, FP4, true>(tmA, p, s);
+  return launch_mx<OUTMODE, 128, FP4>(tmA, p, s);
+}
+template <bool FP4>
+int launch_mx_large(const void* a, MxParams& p, int out_dtype, void* stream) {
+  cudaStream_t s = static_cast<cudaStream_t>(stream);
+  return out_dtype == FLYB200_OUT_BF16 ? launch_mx_large<MOE_OUT_BF16, FP4>(a, p, s) : launch_mx_large<MOE_OUT_FP16, FP4>(a, p, s);
+}
+}  // namespace
 
 extern "C" {
 
@@ -106,35 +191,6 @@ int flyb200_mx_scale_image(void* dst, const void* src, int rows, int K, void* st
   return FLYB200_OK;
 }
 
-namespace {
-// Up to 128 tokens are a weight stream for the small-M kernel in its block-scaled kind - as long as its
-// CTAs (one per 128 channels) fit one round: on wider outputs its later rounds run part empty and the
-// persistent large-M kernel is 20-45 % faster (MXFP8 128 x 28672 x 8192: 43 against 66 us; MXFP4 128 x
-// 57344 x 8192: 51 against 90 us).  FLYB200_MX_SMALL=0 / 1 forces the choice.
-bool mx_small_m(int M, int N) {
-  if (M > 128) return false;
-  if (const char* e = getenv("FLYB200_MX_SMALL")) {
-    if (e[0] == '0') return false;
-    if (e[0] == '1') return true;
-  }
-  int sms = 0;
-  if (flyb200::host::sm_count(&sms) != FLYB200_OK) return true;
-  return (N + 127) / 128 <= sms;
-}
-// Tile shape of the large-M kernel: 128 x 256 tiles (one accumulator, exposed epilogue) win once a
-// tile's mainloop is a few times longer than its epilogue (2.44-2.47 against 1.82-1.88 PFLOP/s at
-// K = 8192, M >= 4096) - unless the 128 x 128 tiles cover the output in one round of CTAs: then
-// they put twice as many SMs to work (MXFP8 256 x 8192 x 8192: 27.9 against 31.4 us; MXFP4:
-// 18.4 against 20.9 us).  `k_bytes`: bytes of codes per row.
-bool mx_wide_tiles(int M, int N, int k_bytes) {
-  if (N % 256 != 0 || k_bytes < 1024) return false;
-  int sms = 0;
-  if (flyb200::host::sm_count(&sms) != FLYB200_OK) return true;
-  const long long tiles128 = static_cast<long long>((M + 127) / 128) * (N / 128);
-  return tiles128 > sms;
-}
-}  // namespace
-
 int flyb200_gemm_mxfp8(void* c, const void* a, const void* w_shuf, const void* scale_a_image, const void* scale_w_image,
                        int M, int N, int K, int out_dtype, void* stream) {
   if (!c || !a || !w_shuf || !scale_a_image || !scale_w_image || M < 0 || N <= 0 || K <= 0) return FLYB200_E_BAD_ARG;
@@ -157,24 +213,7 @@ int flyb200_gemm_mxfp8(void* c, const void* a, const void* w_shuf, const void* s
   p.N = N;
   p.K_bytes = K;
   p.group_m = 16;
-  int rc = host::status_word(&p.status);
-  if (rc) return rc;
-  CUtensorMap tmA;
-  rc = host::byte_matrix_map(&tmA, a, static_cast<uint64_t>(K), static_cast<uint64_t>(M), BLOCK_ROWS);
-  if (rc) return rc;
-  cudaStream_t s = static_cast<cudaStream_t>(stream);
-  // FLYB200_MX_BN forces a tile shape (tuning and tests)
-  bool wide = mx_wide_tiles(M, N, K);
-  if (const char* e = getenv("FLYB200_MX_BN")) {
-    if (e[0] == '1') wide = false;
-    if (e[0] == '2' && N % 256 == 0) wide = true;
-  }
-  if (wide) {
-    if (out_dtype == FLYB200_OUT_BF16) return launch_mx<MOE_OUT_BF16, 256>(tmA, p, s);
-    return launch_mx<MOE_OUT_FP16, 256>(tmA, p, s);
-  }
-  if (out_dtype == FLYB200_OUT_BF16) return launch_mx<MOE_OUT_BF16, 128>(tmA, p, s);
-  return launch_mx<MOE_OUT_FP16, 128>(tmA, p, s);
+  return launch_mx_large<false>(a, p, out_dtype, stream);
 }
 
 int flyb200_gemm_mx_mixed(void* c, const void* a, const void* w_shuf, const void* scale_a_image, const void* scale_w_image,
@@ -199,19 +238,7 @@ int flyb200_gemm_mx_mixed(void* c, const void* a, const void* w_shuf, const void
   p.K_bytes = K;  // one byte per code: sub-byte codes travel in byte containers
   p.group_m = 16;
   p.fmt_bits = (static_cast<uint32_t>(a_format) << 7) | (static_cast<uint32_t>(w_format) << 10);
-  int rc = host::status_word(&p.status);
-  if (rc) return rc;
-  CUtensorMap tmA;
-  rc = host::byte_matrix_map(&tmA, a, static_cast<uint64_t>(K), static_cast<uint64_t>(M), BLOCK_ROWS);
-  if (rc) return rc;
-  cudaStream_t s = static_cast<cudaStream_t>(stream);
-  const bool wide = mx_wide_tiles(M, N, K);  // byte containers: K bytes per row
-  if (wide) {
-    if (out_dtype == FLYB200_OUT_BF16) return launch_mx<MOE_OUT_BF16, 256>(tmA, p, s);
-    return launch_mx<MOE_OUT_FP16, 256>(tmA, p, s);
-  }
-  if (out_dtype == FLYB200_OUT_BF16) return launch_mx<MOE_OUT_BF16, 128>(tmA, p, s);
-  return launch_mx<MOE_OUT_FP16, 128>(tmA, p, s);
+  return launch_mx_large<false>(a, p, out_dtype, stream);
 }
 
 int flyb200_gemm_mxfp4(void* c, const void* a, const void* w_shuf, const void* scale_a_image, const void* scale_w_image,
@@ -236,23 +263,7 @@ int flyb200_gemm_mxfp4(void* c, const void* a, const void* w_shuf, const void* s
   p.N = N;
   p.K_bytes = K / 2;
   p.group_m = 16;
-  int rc = host::status_word(&p.status);
-  if (rc) return rc;
-  CUtensorMap tmA;
-  rc = host::byte_matrix_map(&tmA, a, static_cast<uint64_t>(K / 2), static_cast<uint64_t>(M), BLOCK_ROWS);
-  if (rc) return rc;
-  cudaStream_t s = static_cast<cudaStream_t>(stream);
-  bool wide = mx_wide_tiles(M, N, K / 2);
-  if (const char* e = getenv("FLYB200_MX_BN")) {
-    if (e[0] == '1') wide = false;
-    if (e[0] == '2' && N % 256 == 0) wide = true;
-  }
-  if (wide) {
-    if (out_dtype == FLYB200_OUT_BF16) return launch_mx<MOE_OUT_BF16, 256, true>(tmA, p, s);
-    return launch_mx<MOE_OUT_FP16, 256, true>(tmA, p, s);
-  }
-  if (out_dtype == FLYB200_OUT_BF16) return launch_mx<MOE_OUT_BF16, 128, true>(tmA, p, s);
-  return launch_mx<MOE_OUT_FP16, 128, true>(tmA, p, s);
+  return launch_mx_large<true>(a, p, out_dtype, stream);
 }
 
 }  // extern "C"

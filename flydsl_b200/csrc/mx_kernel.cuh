@@ -28,6 +28,12 @@
 // of a tile.  Threads as in the large-M kernel: warp 0 producer, warp 1 MMA
 // (copies the two scale atoms to TMEM, then issues the four MMAs of a k-block),
 // warps 2..5 epilogue (thread = token row, 64 contiguous output bytes per chunk).
+//
+// SPLIT: where the 128 x 128 tiles leave at least half of the SMs idle, a cluster of two, four or eight
+// CTAs shares a tile, each with a part of K.  Every CTA parks its fp32 partial tile in its shared memory
+// and, after a cluster barrier, sums a share of the columns over the peers in rank order (deterministic).
+// Bound by the k-blocks a CTA walks (0.36 us each at 6 stages) plus about 5 us of launch, reduction and
+// exit; a workspace and a second kernel would add a launch to that.  Measured, see mx_split.
 #pragma once
 #include "moe_kernel.cuh"
 
@@ -41,6 +47,7 @@ struct MxParams {
   void* c;
   int M, N, K_bytes;
   int group_m;
+  int split;           // SPLIT: CTAs per cluster, K parts of a tile
   uint32_t fmt_bits;   // operand formats of kind::mxf8f6f4 as instruction-descriptor bits: (A format << 7) | (B format << 10)
   int* status;
 };
@@ -69,7 +76,7 @@ struct MxSmem {
   static constexpr int TOTAL = OFF_MISC + 16;
 };
 
-template <int OUTMODE, int BN, bool FP4 = false>
+template <int OUTMODE, int BN, bool FP4 = false, bool SPLIT = false>
 __global__ void __launch_bounds__(NUM_THREADS, 1) mx_gemm_kernel(const __grid_constant__ CUtensorMap tmA, const MxParams p) {
   using L = MxSmem<BN, FP4>;
   constexpr int STAGES = L::STAGES;
@@ -124,7 +131,13 @@ __global__ void __launch_bounds__(NUM_THREADS, 1) mx_gemm_kernel(const __grid_co
   const int num_m = (p.M + BLOCK_ROWS - 1) / BLOCK_ROWS;
   const int num_n = p.N / BN;
   const int num_tiles = num_m * num_n;
-  const int num_kb = p.K_bytes / KBLOCK_BYTES;
+  const int all_kb = p.K_bytes / KBLOCK_BYTES;
+  // this CTA's k-blocks, first tile and step to the next one (SPLIT: one tile per cluster)
+  const int rank = SPLIT ? static_cast<int>(cluster_ctarank()) : 0;
+  const int kb0 = SPLIT ? rank * all_kb / p.split : 0;
+  const int kb1 = SPLIT ? (rank + 1) * all_kb / p.split : all_kb;
+  const int tile0 = SPLIT ? static_cast<int>(blockIdx.x) / p.split : static_cast<int>(blockIdx.x);
+  const int tile_step = SPLIT ? num_tiles : static_cast<int>(gridDim.x);
   auto tile_coords = [&](int t, int& m_blk, int& n_blk) {
     const int per_group = p.group_m * num_n;
     const int g = t / per_group;
@@ -143,10 +156,10 @@ __global__ void __launch_bounds__(NUM_THREADS, 1) mx_gemm_kernel(const __grid_co
       uint32_t phase = 0;
       int issued = 0;
       bool ok = true;
-      for (int t = blockIdx.x; t < num_tiles && ok; t += gridDim.x) {
+      for (int t = tile0; t < num_tiles && ok; t += tile_step) {
         int m_blk, n_blk;
         tile_coords(t, m_blk, n_blk);
-        for (int kb = 0; kb < num_kb; ++kb) {
+        for (int kb = kb0; kb < kb1; ++kb) {
           if (!mbar_wait(bar_empty + 8 * stage, phase ^ 1u, abort_flag)) {
             report_failure(p.status, ST_TIMEOUT, abort_flag);
             ok = false;
@@ -196,14 +209,14 @@ __global__ void __launch_bounds__(NUM_THREADS, 1) mx_gemm_kernel(const __grid_co
       int acc = 0;
       uint32_t acc_phase = 0;
       bool ok = true;
-      for (int t = blockIdx.x; t < num_tiles && ok; t += gridDim.x) {
+      for (int t = tile0; t < num_tiles && ok; t += tile_step) {
         if (!mbar_wait(bar_tempty + 8 * acc, acc_phase ^ 1u, abort_flag)) {
           report_failure(p.status, ST_TIMEOUT, abort_flag);
           break;
         }
         tc_fence_after();
         const uint32_t d_tmem = tmem_base + static_cast<uint32_t>(acc * BN);
-        for (int kb = 0; kb < num_kb; ++kb) {
+        for (int kb = kb0; kb < kb1; ++kb) {
           if (!mbar_wait(bar_full + 8 * stage, phase, abort_flag)) {
             report_failure(p.status, ST_TIMEOUT, abort_flag);
             ok = false;
@@ -231,12 +244,12 @@ __global__ void __launch_bounds__(NUM_THREADS, 1) mx_gemm_kernel(const __grid_co
               const uint32_t id = idesc | (sf_id << 4) | (sf_id << 29);
               umma_mxf4(d_tmem, adesc + static_cast<uint64_t>(k * (UMMA_K_BYTES >> 4)),
                         bdesc + static_cast<uint64_t>(k * (UMMA_K_BYTES >> 4)), id, sfa_t + 4 * (k >> 1),
-                        sfb_t + 4 * L::SFB_ATOMS * (k >> 1), (kb | k) != 0 ? 1u : 0u);
+                        sfb_t + 4 * L::SFB_ATOMS * (k >> 1), (kb != kb0 || k != 0) ? 1u : 0u);
             } else {
               // the k-th 32-element block uses byte k of the scale columns: scale-factor id k for both operands
               const uint32_t id = idesc | (static_cast<uint32_t>(k) << 4) | (static_cast<uint32_t>(k) << 29);
               umma_mxf8(d_tmem, adesc + static_cast<uint64_t>(k * (UMMA_K_BYTES >> 4)),
-                        bdesc + static_cast<uint64_t>(k * (UMMA_K_BYTES >> 4)), id, sfa_t, sfb_t, (kb | k) != 0 ? 1u : 0u);
+                        bdesc + static_cast<uint64_t>(k * (UMMA_K_BYTES >> 4)), id, sfa_t, sfb_t, (kb != kb0 || k != 0) ? 1u : 0u);
             }
           }
           umma_commit(bar_empty + 8 * stage);
@@ -257,7 +270,7 @@ __global__ void __launch_bounds__(NUM_THREADS, 1) mx_gemm_kernel(const __grid_co
     int acc = 0;
     uint32_t acc_phase = 0;
     bool ok = true;
-    for (int t = blockIdx.x; t < num_tiles && ok; t += gridDim.x) {
+    for (int t = tile0; t < num_tiles && ok; t += tile_step) {
       int m_blk, n_blk;
       tile_coords(t, m_blk, n_blk);
       const int row = m_blk * BLOCK_ROWS + q * 32 + lane;
@@ -268,26 +281,45 @@ __global__ void __launch_bounds__(NUM_THREADS, 1) mx_gemm_kernel(const __grid_co
       }
       tc_fence_after();
       const uint32_t t_row = tmem_base + (static_cast<uint32_t>(q * 32) << 16) + static_cast<uint32_t>(acc * BN);
-      // 64 columns per TMEM wait, and each lane then writes one full 128-byte line of its output row
+      if constexpr (SPLIT) {
+        // Park the partial tile at the start of the ring (the barrier above came after the last MMA has
+        // read it): sixteen bytes of row r, columns 4 c ..., at (c * 128 + r) * 16, conflict-free.
+        static_assert(BLOCK_ROWS * BN * 4 <= L::OFF_SFA, "the partial tile must fit into the ring");
 #pragma unroll 1
-      for (int c0 = 0; c0 < BN; c0 += 64) {
-        uint32_t r0[32], r1[32];
-        tmem_ld_x32(t_row + c0, r0);
-        tmem_ld_x32(t_row + c0 + 32, r1);
-        tmem_ld_wait();
-        if (c0 + 64 >= BN) {  // last read of this accumulator: hand it back to the MMA warp
-          tc_fence_before();
-          __syncwarp();
-          if (lane == 0) mbar_arrive(bar_tempty + 8 * acc);
+        for (int c0 = 0; c0 < BN; c0 += 64) {
+          uint32_t r0[32], r1[32];
+          tmem_ld_x32(t_row + c0, r0);
+          tmem_ld_x32(t_row + c0 + 32, r1);
+          tmem_ld_wait();
+          const uint32_t dst = smem_base + static_cast<uint32_t>(((c0 / 4) * BLOCK_ROWS + q * 32 + lane) * 16);
+#pragma unroll
+          for (int j = 0; j < 8; ++j) {
+            st_smem_v4(dst + j * BLOCK_ROWS * 16, r0[4 * j], r0[4 * j + 1], r0[4 * j + 2], r0[4 * j + 3]);
+            st_smem_v4(dst + (j + 8) * BLOCK_ROWS * 16, r1[4 * j], r1[4 * j + 1], r1[4 * j + 2], r1[4 * j + 3]);
+          }
         }
-        if (row < p.M) {
-          float y[32];
+      } else {
+        // 64 columns per TMEM wait, and each lane then writes one full 128-byte line of its output row
+#pragma unroll 1
+        for (int c0 = 0; c0 < BN; c0 += 64) {
+          uint32_t r0[32], r1[32];
+          tmem_ld_x32(t_row + c0, r0);
+          tmem_ld_x32(t_row + c0 + 32, r1);
+          tmem_ld_wait();
+          if (c0 + 64 >= BN) {  // last read of this accumulator: hand it back to the MMA warp
+            tc_fence_before();
+            __syncwarp();
+            if (lane == 0) mbar_arrive(bar_tempty + 8 * acc);
+          }
+          if (row < p.M) {
+            float y[32];
 #pragma unroll
-          for (int j = 0; j < 32; ++j) y[j] = __uint_as_float(r0[j]);
-          moe_store_row32<OUTMODE, false>(p.c, static_cast<size_t>(row) * p.N + n_blk * BN + c0, y, 32);
+            for (int j = 0; j < 32; ++j) y[j] = __uint_as_float(r0[j]);
+            moe_store_row32<OUTMODE, false>(p.c, static_cast<size_t>(row) * p.N + n_blk * BN + c0, y, 32);
 #pragma unroll
-          for (int j = 0; j < 32; ++j) y[j] = __uint_as_float(r1[j]);
-          moe_store_row32<OUTMODE, false>(p.c, static_cast<size_t>(row) * p.N + n_blk * BN + c0 + 32, y, 32);
+            for (int j = 0; j < 32; ++j) y[j] = __uint_as_float(r1[j]);
+            moe_store_row32<OUTMODE, false>(p.c, static_cast<size_t>(row) * p.N + n_blk * BN + c0 + 32, y, 32);
+          }
         }
       }
       acc = (acc + 1) % NACC;
@@ -295,6 +327,43 @@ __global__ void __launch_bounds__(NUM_THREADS, 1) mx_gemm_kernel(const __grid_co
     }
   }
 
+  if constexpr (SPLIT) {
+    // Every thread of every CTA of the cluster comes here, also after a failed wait (all are bounded).
+    __syncwarp();
+    cluster_sync_all();
+    if (warp >= 2) {
+      const int trow = (warp & 3) * 32 + lane;
+      int m_blk, n_blk;
+      tile_coords(tile0, m_blk, n_blk);
+      const int row = m_blk * BLOCK_ROWS + trow;
+      const int share = BN / p.split;  // columns summed and stored by this CTA: 64, 32 or 16
+      for (int c0 = rank * share; c0 < (rank + 1) * share; c0 += 32) {
+        const int n_ok = min(32, share);
+        float y[32];
+#pragma unroll
+        for (int j = 0; j < 32; ++j) y[j] = 0.0f;
+        if (row < p.M) {
+          for (int part = 0; part < p.split; ++part) {
+            const uint32_t src = map_to_cta(smem_base + static_cast<uint32_t>(((c0 / 4) * BLOCK_ROWS + trow) * 16), part);
+            uint4 v[8];
+#pragma unroll
+            for (int j = 0; j < 8; ++j)
+              v[j] = 4 * j < n_ok ? ld_dsmem_v4(src + j * BLOCK_ROWS * 16) : make_uint4(0u, 0u, 0u, 0u);
+#pragma unroll
+            for (int j = 0; j < 8; ++j) {
+              y[4 * j] += __uint_as_float(v[j].x);
+              y[4 * j + 1] += __uint_as_float(v[j].y);
+              y[4 * j + 2] += __uint_as_float(v[j].z);
+              y[4 * j + 3] += __uint_as_float(v[j].w);
+            }
+          }
+          moe_store_row32<OUTMODE, false>(p.c, static_cast<size_t>(row) * p.N + n_blk * BN + c0, y, n_ok);
+        }
+      }
+    }
+    __syncwarp();
+    cluster_sync_all();  // nobody leaves while a peer may still read its shared memory
+  }
   tc_fence_before();
   __syncthreads();
   if (warp == 1) {

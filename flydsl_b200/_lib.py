@@ -21,6 +21,7 @@ DT_FP8, DT_INT8, DT_FP16, DT_BF16 = range(4)
 OUT_BF16, OUT_FP16, OUT_F32 = range(3)
 EPI_NONE, EPI_BIAS, EPI_BIAS_RELU, EPI_BIAS_SILU, EPI_BIAS_GELU = range(5)
 SRC_ROW_MAJOR, SRC_MFMA_16x16 = range(2)
+MOE_QUANT_MAX_K = 16384
 
 IN_DTYPES = {"fp8": DT_FP8, "int8": DT_INT8, "fp16": DT_FP16, "bf16": DT_BF16}
 OUT_DTYPES = {"bf16": OUT_BF16, "fp16": OUT_FP16}
@@ -53,6 +54,7 @@ SIGNATURES = {
     "flyb200_read_status": (_i, [ctypes.POINTER(_i)]),
     "flyb200_selftest_bounded_wait": (_i, [ctypes.c_uint, _vp]),
     "flyb200_moe_gather_rows": (_i, [_vp, _vp, _vp, _vp, _vp, _vp, _i, _i, _i, _i, _i, _vp]),
+    "flyb200_moe_quant_sorted": (_i, [_vp, _vp, _vp, _vp, _vp, _i, _i, _i, _i, _i, _vp]),
     "flyb200_moe_gemm": (_i, [_i, _vp, _vp, _vp, _vp, _vp, _vp, _vp, _vp, _vp] + [_i] * 12 + [_vp]),
     "flyb200_moe_reduce": (_i, [_vp, _vp, _i, _i, _i, _i, _vp, _vp, _i, _vp]),
     "flyb200_moe_sorting": (_i, [_vp, _vp, _i, _i, _i, _i, _vp, _vp, _vp, _vp, _vp, _vp]),

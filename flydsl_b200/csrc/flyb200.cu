@@ -658,37 +658,16 @@ int launch_shuffle(void* dst, const void* src, int N, int Kb, cudaStream_t s) {
 
 // Row quantiser launch: rows that fit the register-cached single-pass kernel
 // use it (one block per row), longer rows take the two-pass kernel.
-template <typename TIn, bool FP8, int NV, int WPR>
-void launch_quant_rows(uint8_t* y, float* scale, const TIn* x, int rows, int K, cudaStream_t s) {
-  constexpr int PER_BLOCK = 8 / WPR;
-  pertoken_quant_row_kernel<TIn, FP8, NV, WPR><<<(rows + PER_BLOCK - 1) / PER_BLOCK, 256, 0, s>>>(y, scale, x, rows, K);
-}
-// Warps per row: as few as keep a row in eight vectors per thread (a warp that owns its row needs no
-// barrier, and eight loads per thread cover the latency), but at least two blocks per SM: few rows
-// take more warps each.
 template <typename TIn, bool FP8>
 void launch_quant_t(uint8_t* y, float* scale, const TIn* x, int rows, int K, cudaStream_t s) {
-  const int vecs = K / QuantIn<TIn>::VEC;  // 16-byte vectors of a row
-  int wpr = 1;
-  while (wpr < 8 && (vecs > 256 * wpr || static_cast<long long>(rows) * wpr < 2LL * 148 * 8)) wpr *= 2;
-  const int nv = (vecs + 32 * wpr - 1) / (32 * wpr);  // vectors per thread
-  if (nv > 8) {
+  const bool fits = quant_row_dispatch(rows, K / QuantIn<TIn>::VEC, [&](auto nv, auto wpr) {
+    constexpr int PER_BLOCK = 8 / decltype(wpr)::value;
+    pertoken_quant_row_kernel<TIn, FP8, decltype(nv)::value, decltype(wpr)::value>
+        <<<(rows + PER_BLOCK - 1) / PER_BLOCK, 256, 0, s>>>(y, scale, x, rows, K);
+  });
+  if (!fits) {
     const int grid = rows < 148 * 16 ? rows : 148 * 16;
     pertoken_quant_kernel<TIn, FP8><<<grid, 256, 0, s>>>(y, scale, x, rows, K);
-  } else if (wpr == 1) {
-    if (nv <= 4) launch_quant_rows<TIn, FP8, 4, 1>(y, scale, x, rows, K, s);
-    else launch_quant_rows<TIn, FP8, 8, 1>(y, scale, x, rows, K, s);
-  } else if (wpr == 2) {
-    if (nv <= 4) launch_quant_rows<TIn, FP8, 4, 2>(y, scale, x, rows, K, s);
-    else launch_quant_rows<TIn, FP8, 8, 2>(y, scale, x, rows, K, s);
-  } else if (wpr == 4) {
-    if (nv <= 4) launch_quant_rows<TIn, FP8, 4, 4>(y, scale, x, rows, K, s);
-    else launch_quant_rows<TIn, FP8, 8, 4>(y, scale, x, rows, K, s);
-  } else {
-    if (nv <= 1) launch_quant_rows<TIn, FP8, 1, 8>(y, scale, x, rows, K, s);
-    else if (nv <= 2) launch_quant_rows<TIn, FP8, 2, 8>(y, scale, x, rows, K, s);
-    else if (nv <= 4) launch_quant_rows<TIn, FP8, 4, 8>(y, scale, x, rows, K, s);
-    else launch_quant_rows<TIn, FP8, 8, 8>(y, scale, x, rows, K, s);
   }
 }
 template <typename TIn>
@@ -764,7 +743,7 @@ namespace host {
 // Block-scaled GEMM (MXFP8, or MXFP4 with `fp4`) for up to 128 tokens on the small-M (weight-streaming)
 // kernel; K = bytes of codes per row.
 int gemm_mx_small(void* c, const void* a, const void* w, const void* sf_a, const void* sf_w, int M, int N, int K,
-                  int outmode, bool fp4, void* stream) {
+                  int outmode, bool fp4, void* stream, int a_format, int w_format) {
   DeviceState* st = nullptr;
   int rc = device_state(&st);
   if (rc) return rc;
@@ -791,6 +770,7 @@ int gemm_mx_small(void* c, const void* a, const void* w, const void* sf_a, const
   p.sf_w = static_cast<const uint8_t*>(sf_w);
   p.sf_a = static_cast<const uint8_t*>(sf_a);
   p.sf_a_tiles = (M + 127) / 128;
+  p.fmt_bits = (static_cast<uint32_t>(w_format) << 7) | (static_cast<uint32_t>(a_format) << 10);
   p.status = st->status;
   CUtensorMap tmA;
   rc = make_map(&tmA, CU_TENSOR_MAP_DATA_TYPE_UINT8, 1, a, static_cast<uint64_t>(K), static_cast<uint64_t>(M), KBLOCK_BYTES,

@@ -191,6 +191,29 @@ int flyb200_moe_gather_rows(void* dst, float* dst_scale, const void* src, const 
   return FLYB200_OK;
 }
 
+int flyb200_moe_quant_sorted(void* dst, float* dst_scale, const void* src, const int* sorted_ids, const int* num_valid_ids,
+                             int tokens, int topk, int K, int rows, int quant_dtype, void* stream) {
+  if (!dst || !dst_scale || !src || !sorted_ids || !num_valid_ids) return FLYB200_E_BAD_ARG;
+  if (tokens < 0 || topk <= 0 || topk > 255 || K <= 0 || rows < 0) return FLYB200_E_BAD_ARG;
+  if (quant_dtype != FLYB200_DT_FP8 && quant_dtype != FLYB200_DT_INT8) return FLYB200_E_BAD_ARG;
+  if (K % 16 != 0 || K > FLYB200_MOE_QUANT_MAX_K) return FLYB200_E_UNSUPPORTED;
+  if (!aligned16(dst) || !aligned16(src)) return FLYB200_E_BAD_ALIGN;
+  if (rows == 0) return FLYB200_OK;
+  cudaStream_t s = static_cast<cudaStream_t>(stream);
+  quant_row_dispatch(rows, K / 8, [&](auto nv, auto wpr) {
+    constexpr int NV = decltype(nv)::value, WPR = decltype(wpr)::value;
+    const int grid = (rows + 8 / WPR - 1) / (8 / WPR);
+    const __nv_bfloat16* x = static_cast<const __nv_bfloat16*>(src);
+    uint8_t* y = static_cast<uint8_t*>(dst);
+    if (quant_dtype == FLYB200_DT_FP8)
+      moe_quant_sorted_kernel<true, NV, WPR><<<grid, 256, 0, s>>>(y, dst_scale, x, sorted_ids, num_valid_ids, tokens, topk, K, rows);
+    else
+      moe_quant_sorted_kernel<false, NV, WPR><<<grid, 256, 0, s>>>(y, dst_scale, x, sorted_ids, num_valid_ids, tokens, topk, K, rows);
+  });
+  CUDA_TRY(cudaGetLastError());
+  return FLYB200_OK;
+}
+
 int flyb200_moe_gemm(int stage, void* out, const void* a_sorted, const void* w_shuf, const float* scale_a_sorted,
                      const float* scale_w, const int* sorted_ids, const int* expert_ids, const float* sorted_weights,
                      const int* num_valid_ids, int tokens, int topk, int experts, int model_dim, int inter_dim,

@@ -17,6 +17,7 @@
 // twice (the second time from L1/L2).
 #pragma once
 #include <cstdint>
+#include <type_traits>
 #include <cuda_bf16.h>
 #include <cuda_fp16.h>
 #include <cuda_fp8.h>
@@ -258,7 +259,7 @@ __device__ __forceinline__ void quant_row_from_registers(const uint4 (&raw)[NV],
 // Single-pass form for rows of at most 32 * WPR * VEC * NV elements.  WPR warps of a 256-thread block
 // share a row; every thread has its NV loads in flight together and keeps the raw vectors in registers
 // (half the registers of the converted values, so more rows in flight).  Memory-bound where there are
-// rows enough; few rows are spread over more warps (launch_quant_t).  One 256-thread block per row, with
+// rows enough; few rows are spread over more warps (quant_warps_per_row).  One 256-thread block per row, with
 // a conversion of every value before the maximum and a test next to every product for a rounding boundary,
 // was bound by instruction issue and, on short rows, by blocks of a few loads each.  bf16 -> fp8 / int8, us,
 // before and now: 8192 x 8192 51.7 / 49.0 and 39.1 / 44.3 (5.2 / 4.6 TB/s), 8192 x 2048 17.5 / 16.3 and
@@ -282,6 +283,38 @@ __global__ void __launch_bounds__(256) pertoken_quant_row_kernel(uint8_t* __rest
     raw[i] = k < K ? __ldg(reinterpret_cast<const uint4*>(xr + k)) : make_uint4(0u, 0u, 0u, 0u);
   }
   quant_row_from_registers<TIn, FP8, NV, WPR>(raw, y + static_cast<size_t>(r) * K, scale + r, K, tid, red, group * WPR, 1 + group);
+}
+
+// Warps per row: as few as keep a row in eight vectors per thread (a warp that owns its row needs no
+// barrier, and eight loads per thread cover the latency), but at least two blocks per SM: few rows
+// take more warps each.  `vecs`: 16-byte vectors of a row.
+inline int quant_warps_per_row(int rows, int vecs) {
+  int wpr = 1;
+  while (wpr < 8 && (vecs > 256 * wpr || static_cast<long long>(rows) * wpr < 2LL * 148 * 8)) wpr *= 2;
+  return wpr;
+}
+// Calls launch(NV, WPR) with integral constants for a row of `vecs` vectors; false where it does not fit registers.
+template <typename LaunchFn>
+bool quant_row_dispatch(int rows, int vecs, LaunchFn launch) {
+  using std::integral_constant;
+  const int wpr = quant_warps_per_row(rows, vecs);
+  const int nv = (vecs + 32 * wpr - 1) / (32 * wpr);  // vectors per thread
+  if (nv > 8) return false;
+  const bool four = nv <= 4;
+  if (wpr == 1) {
+    four ? launch(integral_constant<int, 4>(), integral_constant<int, 1>()) : launch(integral_constant<int, 8>(), integral_constant<int, 1>());
+  } else if (wpr == 2) {
+    four ? launch(integral_constant<int, 4>(), integral_constant<int, 2>()) : launch(integral_constant<int, 8>(), integral_constant<int, 2>());
+  } else if (wpr == 4) {
+    four ? launch(integral_constant<int, 4>(), integral_constant<int, 4>()) : launch(integral_constant<int, 8>(), integral_constant<int, 4>());
+  } else if (nv <= 1) {
+    launch(integral_constant<int, 1>(), integral_constant<int, 8>());
+  } else if (nv <= 2) {
+    launch(integral_constant<int, 2>(), integral_constant<int, 8>());
+  } else {
+    four ? launch(integral_constant<int, 4>(), integral_constant<int, 8>()) : launch(integral_constant<int, 8>(), integral_constant<int, 8>());
+  }
+  return true;
 }
 
 // General form (any row length): two passes over the row, the second one from L1/L2.

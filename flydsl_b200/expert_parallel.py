@@ -110,7 +110,6 @@ class ExpertParallelMoe:
 
     def forward_local(self, x_q, scale_x, topk_ids, topk_weights):
         """This rank's partial output [tokens, model_dim] (routes to other ranks' experts contribute nothing)."""
-        from . import pertoken_quant
         from .kernels.moe.moe_gemm_2stage import sort_on_device
 
         if self._w1 is None:
@@ -121,22 +120,17 @@ class ExpertParallelMoe:
         srt, wts, e_ids, post = sort_on_device(topk_ids, topk_weights, self.shard.experts_local, self.tile_m, self.shard.e0)
         blocks = int(e_ids.numel())
         st = torch.cuda.current_stream(dev)
-        # rows of routes that belong to other ranks are not written; the quantiser takes whatever they hold
-        # (Inf and NaN included) and nothing reads what it makes of them
+        # rows of routes that belong to other ranks are neither written nor read
         out1 = torch.empty(tokens * self.topk, self.inter_dim, dtype=torch.bfloat16, device=dev)
         self._g1(out1, x_q.reshape(-1), self._w1.reshape(-1), scale_x.reshape(-1), self._sw1, srt, e_ids, wts, post, tokens,
                  self.inter_dim, self.model_dim, blocks, st)
-        qd = torch.float8_e4m3fn if self.in_dtype == "fp8" else torch.int8
-        a2, sa2 = pertoken_quant(out1, quant_dtype=qd)
         if self.out_dtype == "f32":
             y = torch.zeros(tokens, self.model_dim, dtype=torch.float32, device=dev)
-            self._g2(y, a2.reshape(-1), self._w2.reshape(-1), sa2.reshape(-1), self._sw2, srt, e_ids, wts, post, tokens,
-                     self.model_dim, self.inter_dim, blocks, st)
+            self._g2._launch_quantising(y, out1, self._w2, self._sw2, srt, e_ids, wts, post, tokens, blocks, st)
             return y
         # rows of routes that belong to other ranks are never written; the masked reduction skips them
         out2 = torch.empty(tokens * self.topk, self.model_dim, dtype=torch.bfloat16, device=dev)
-        self._g2(out2, a2.reshape(-1), self._w2.reshape(-1), sa2.reshape(-1), self._sw2, srt, e_ids, wts, post, tokens,
-                 self.model_dim, self.inter_dim, blocks, st)
+        self._g2._launch_quantising(out2, out1, self._w2, self._sw2, srt, e_ids, wts, post, tokens, blocks, st)
         if self._mask is None or self._mask.device != dev:
             mask = torch.zeros(self.shard.experts_total, dtype=torch.int32, device=dev)
             mask[self.shard.e0 : self.shard.e1] = 1

@@ -269,26 +269,55 @@ class _MoeStage:
             with torch.cuda.device(dev):
                 return self._launch(out, x, w, scale_x, scale_w, sorted_token_ids, sorted_expert_ids, sorted_weights,
                                     num_valid_ids, tokens, blocks, stream)
-        lib = _lib.load()
         s = _stream_handle(stream) or None
         rows = blocks * self.tile_m
-        if self.in_dtype == "int4":
-            w = self._weights_for_kernel(w, self.experts * (2 * self.inter_dim if self.stage == 1 else self.model_dim) * self._k)
         a_sorted, sa_sorted = self._sorted_buffers(dev, rows, s)
-        a_ptr, sa_ptr, ids_ptr, nv_ptr = a_sorted.data_ptr(), sa_sorted.data_ptr(), sorted_token_ids.data_ptr(), num_valid_ids.data_ptr()
-        rc = lib.flyb200_moe_gather_rows(a_ptr, sa_ptr, x.data_ptr(), scale_x.data_ptr(), ids_ptr, nv_ptr, tokens, self.topk,
-                                         self._gather_mode, self._k, rows, s)
+        rc = _lib.load().flyb200_moe_gather_rows(
+            a_sorted.data_ptr(), sa_sorted.data_ptr(), x.data_ptr(), scale_x.data_ptr(), sorted_token_ids.data_ptr(),
+            num_valid_ids.data_ptr(), tokens, self.topk, self._gather_mode, self._k, rows, s)
         if rc:
             _lib.check(rc, "moe_gather_rows")
-        rc = lib.flyb200_moe_gemm(
-            self.stage, out.data_ptr(), a_ptr, w.data_ptr(), sa_ptr, scale_w.data_ptr(), ids_ptr, sorted_expert_ids.data_ptr(),
-            sorted_weights.data_ptr() if sorted_weights is not None and sorted_weights.numel() else None, nv_ptr,
+        self._gemm(out, a_sorted, sa_sorted, w, scale_w, sorted_token_ids, sorted_expert_ids, sorted_weights, num_valid_ids,
+                   tokens, blocks, s)
+        return None
+
+    def _launch_quantising(self, out, x16, w, scale_w, sorted_token_ids, sorted_expert_ids, sorted_weights, num_valid_ids,
+                           tokens, blocks, stream):
+        """Stage 2 on the bf16 rows ``x16 [tokens * topk, inter_dim]`` of stage 1: the quantiser writes the codes
+        straight into sorted order (``pertoken_quant`` and the gather as one kernel).  Same results as both in turn."""
+        if self._k > _lib.MOE_QUANT_MAX_K or blocks == 0 or tokens == 0:
+            from ....utils import pertoken_quant
+
+            x, sx = pertoken_quant(x16, quant_dtype=self._torch_in)
+            return self._launch(out, x, w, sx, scale_w, sorted_token_ids, sorted_expert_ids, sorted_weights, num_valid_ids,
+                                tokens, blocks, stream)
+        dev = out.device
+        with _lib.on_device(dev):
+            s = _stream_handle(stream) or None
+            rows = blocks * self.tile_m
+            a_sorted, sa_sorted = self._sorted_buffers(dev, rows, s)
+            rc = _lib.load().flyb200_moe_quant_sorted(
+                a_sorted.data_ptr(), sa_sorted.data_ptr(), x16.data_ptr(), sorted_token_ids.data_ptr(), num_valid_ids.data_ptr(),
+                tokens, self.topk, self._k, rows, self._dt, s)
+            if rc:
+                _lib.check(rc, "moe_quant_sorted")
+            self._gemm(out, a_sorted, sa_sorted, w, scale_w, sorted_token_ids, sorted_expert_ids, sorted_weights, num_valid_ids,
+                       tokens, blocks, s)
+        return None
+
+    def _gemm(self, out, a_sorted, sa_sorted, w, scale_w, sorted_token_ids, sorted_expert_ids, sorted_weights, num_valid_ids,
+              tokens, blocks, s):
+        if self.in_dtype == "int4":
+            w = self._weights_for_kernel(w, self.experts * (2 * self.inter_dim if self.stage == 1 else self.model_dim) * self._k)
+        rc = _lib.load().flyb200_moe_gemm(
+            self.stage, out.data_ptr(), a_sorted.data_ptr(), w.data_ptr(), sa_sorted.data_ptr(), scale_w.data_ptr(),
+            sorted_token_ids.data_ptr(), sorted_expert_ids.data_ptr(),
+            sorted_weights.data_ptr() if sorted_weights is not None and sorted_weights.numel() else None, num_valid_ids.data_ptr(),
             tokens, self.topk, self.experts, self.model_dim, self.inter_dim, self.tile_m, blocks, self._dt, self._out,
             int(self.doweight), int(self.accumulate), 1, s,
         )
         if rc:
             _lib.check(rc, "moe_gemm")
-        return None
 
 
 def _check_common(model_dim, inter_dim, experts, topk, tile_m, tile_n, tile_k, in_dtype, k):

@@ -263,6 +263,15 @@ int flyb200_moe_gather_rows(void* dst, float* dst_scale, const void* src, const 
                             const int* num_valid_ids, int tokens, int topk, int by_slot, int row_bytes, int rows,
                             void* stream);
 
+/* The per-token quantiser and the stage-2 gather as one pass: dst[p, :], dst_scale[p] =
+ * flyb200_pertoken_quant of the bf16 row src[token * topk + slot, :], bit-identical; padding
+ * rows and rows >= num_valid_ids[0] become zero with scale zero.  rows = blocks * tile_m,
+ * K a multiple of 16, at most FLYB200_MOE_QUANT_MAX_K.  Counts as the gather pass of
+ * flyb200_moe_gemm's after_gather. */
+#define FLYB200_MOE_QUANT_MAX_K 16384
+int flyb200_moe_quant_sorted(void* dst, float* dst_scale, const void* src, const int* sorted_ids, const int* num_valid_ids,
+                             int tokens, int topk, int K, int rows, int quant_dtype, void* stream);
+
 /* stage 1: out[token, slot, inter_dim] = silu(g) * u [* routed weight],
  *          g/u = (x . W1[e, gate/up rows]^T) * scale_w * scale_x
  * stage 2: accumulate = 1: out[token, model_dim] += y (atomic adds; the caller zeroes out),

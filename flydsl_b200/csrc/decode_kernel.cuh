@@ -419,7 +419,7 @@ __global__ void __launch_bounds__(DECODE_THREADS, 1) gemm_decode_kernel(const __
                         (kb >= 2 || k != 0) ? 1u : 0u);
             }
           } else {
-            constexpr uint32_t mx_idesc = umma_idesc_mxf8(WROWS, BN);
+            const uint32_t mx_idesc = umma_idesc_mxf8(WROWS, BN) | p.fmt_bits;
 #pragma unroll
             for (int k = 0; k < KBLOCK_BYTES / UMMA_K_BYTES; ++k) {
               const uint32_t id = mx_idesc | (static_cast<uint32_t>(k) << 4) | (static_cast<uint32_t>(k) << 29);

@@ -79,6 +79,16 @@ bool mx_small_m(int M, int N) {
   if (flyb200::host::sm_count(&sms) != FLYB200_OK) return true;
   return (N + 127) / 128 <= sms;
 }
+// The mixed kinds (byte containers) the same way, except for 65..128 tokens where the large-M kernel can
+// only split K in two or not at all: there the two are even or the large-M kernel is ahead.  Small-M /
+// large-M with its K split, us, MXFP6 x MXFP4: 32 x 8192 x 8192 18.2 / 18.7, 64 x 8192 x 8192 18.9 / 19.4, 64 x 1024
+// x 8192 9.8 / 11.2, 16 x 4096 x 14336 16.1 / 17.0, 100 x 2048 x 4096 9.9 / 11.1, 128 x 8192 x 8192 21.8 / 20.4.
+bool mx_mixed_small_m(int M, int N) {
+  if (!mx_small_m(M, N)) return false;
+  int sms = 0;
+  if (M <= 64 || getenv("FLYB200_MX_SMALL") || flyb200::host::sm_count(&sms) != FLYB200_OK) return true;
+  return 4 * ((N + 127) / 128) <= sms;
+}
 // Tile shape of the large-M kernel: 128 x 256 tiles (one accumulator, exposed epilogue) win once a
 // tile's mainloop is a few times longer than its epilogue (2.44-2.47 against 1.82-1.88 PFLOP/s at
 // K = 8192, M >= 4096) - unless the 128 x 128 tiles cover the output in one round of CTAs: then
@@ -227,6 +237,9 @@ int flyb200_gemm_mx_mixed(void* c, const void* a, const void* w_shuf, const void
   if (!aligned16(c) || !aligned16(a) || !aligned16(w_shuf) || !aligned16(scale_a_image) || !aligned16(scale_w_image))
     return FLYB200_E_BAD_ALIGN;
   if (M == 0) return FLYB200_OK;
+  if (mx_mixed_small_m(M, N))
+    return host::gemm_mx_small(c, a, w_shuf, scale_a_image, scale_w_image, M, N, K, out_dtype == FLYB200_OUT_FP16 ? 1 : 0,
+                               false, stream, a_format, w_format);
   MxParams p;
   memset(&p, 0, sizeof(p));
   p.w = static_cast<const uint8_t*>(w_shuf);

@@ -54,6 +54,7 @@ struct GemmParams {
   const uint8_t* sf_w;   // decode kernel, MX kind: scale image of the weights [K/128][N/128][512]
   const uint8_t* sf_a;   // decode kernel, MX kind: scale image of the activations [K/128][sf_a_tiles][512]
   int sf_a_tiles;        // ceil(M / 128)
+  uint32_t fmt_bits;     // decode kernel, MX kind on bytes: operand formats as instruction-descriptor bits (weights << 7 | tokens << 10)
   int bn;                // large-M kernel: output channels per tile (multiple of 32, 32..256)
   int rows_stages;       // large-M kernel: depth of the shared-memory ring
   int n_dst;             // scatter kernel: number of output buffers

@@ -11,9 +11,10 @@ namespace host {
 // 128 bytes x box_rows rows, 128-byte swizzle, out-of-bounds rows read as zero.
 int byte_matrix_map(CUtensorMap* m, const void* base, uint64_t row_bytes, uint64_t rows, uint32_t box_rows);
 // Block-scaled GEMM (MXFP8, or MXFP4 with `fp4`) of up to 128 tokens on the small-M (weight-streaming)
-// kernel; K = bytes of codes per row; outmode 0 bf16, 1 fp16.
+// kernel; K = bytes of codes per row; outmode 0 bf16, 1 fp16.  a_format, w_format: codes in byte containers
+// (FLYB200_MXFMT_*; 0 = E4M3, and for `fp4`).
 int gemm_mx_small(void* c, const void* a, const void* w, const void* sf_a, const void* sf_w, int M, int N, int K,
-                  int outmode, bool fp4, void* stream);
+                  int outmode, bool fp4, void* stream, int a_format = 0, int w_format = 0);
 // Pointer to the current device's status word (first failed bounded wait wins).
 int status_word(int** out);
 // SM count of the current device.

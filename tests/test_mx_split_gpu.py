@@ -56,3 +56,17 @@ def test_split_equals_unsplit_to_the_last_rounding(monkeypatch, fmt, m, n, k, ou
         got = product(fmt, x, w, out_dtype).float()
         assert bool(((got - whole).abs() <= 2 * unit * whole.abs() + slack).all())
         assert torch.equal(got, product(fmt, x, w, out_dtype).float())  # summed in rank order: repeatable
+
+
+@pytest.mark.parametrize("m,n,k", [(1, 256, 512), (17, 384, 4096), (128, 1024, 2304)])
+def test_mixed_kinds_on_the_small_m_kernel(monkeypatch, m, n, k):
+    """MXFP6 x MXFP4 of up to 128 tokens: the small-M kernel (weights on the other operand side) against
+    the large-M kernel, apart from the rounding of sums and output."""
+    g = torch.Generator(device="cuda").manual_seed(m)
+    x = torch.randn(m, k, generator=g, device="cuda", dtype=torch.float32).to(torch.bfloat16)
+    w = (torch.randn(n, k, generator=g, device="cuda", dtype=torch.float32) * 0.05).to(torch.bfloat16)
+    monkeypatch.setenv("FLYB200_MX_SMALL", "0")
+    large = product("mxfp6", x, w, "fp16").float()
+    monkeypatch.setenv("FLYB200_MX_SMALL", "1")
+    small = product("mxfp6", x, w, "fp16").float()
+    assert bool(((small - large).abs() <= 2.0**-10 * large.abs() + k * 2.0**-24 * float(large.abs().max())).all())

@@ -8,6 +8,8 @@ from __future__ import annotations
 
 import contextlib
 import ctypes
+import importlib.machinery
+import importlib.util
 import threading
 
 import torch
@@ -73,6 +75,7 @@ SIGNATURES = {
 
 _lock = threading.Lock()
 _lib = None
+_ops = None
 _NO_GUARD = contextlib.nullcontext()
 
 
@@ -99,6 +102,23 @@ def load() -> ctypes.CDLL:
     return _lib
 
 
+def ops():
+    """The CPython extension with the operators' host path (csrc/ops.cpp), loaded (built first if missing
+    or stale) on first use.  Its functions return None for arguments that are not of the common form,
+    an int for a library error."""
+    global _ops
+    if _ops is not None:
+        return _ops
+    load()
+    with _lock:
+        if _ops is None:
+            loader = importlib.machinery.ExtensionFileLoader("flyb200_ops", _build.build_ops())
+            mod = importlib.util.module_from_spec(importlib.util.spec_from_loader("flyb200_ops", loader))
+            loader.exec_module(mod)
+            _ops = mod
+    return _ops
+
+
 def check(code: int, what: str = "libflyb200") -> None:
     if code == OK:
         return
@@ -116,7 +136,7 @@ def on_device(device):
 
 def current_stream(device) -> int:
     """Raw handle of torch's current stream on ``device`` (0 = default)."""
-    return torch.cuda.current_stream(device).cuda_stream
+    return torch._C._cuda_getCurrentRawStream(device.index)
 
 
 PLAN_FIELDS = ("kernel", "bn", "split_k", "kb_per_split", "reduce", "stages", "pdl", "token_blocks")

@@ -1,4 +1,5 @@
-"""Build libflyb200.so (CUDA kernels + C ABI) in-tree for sm_100a.
+"""Build libflyb200.so (CUDA kernels + C ABI) in-tree for sm_100a, and the CPython extension
+flyb200_ops.so (the operators' host path) next to it.
 
     python -m flydsl_b200.build [--force] [-v]
 
@@ -24,6 +25,9 @@ from concurrent.futures import ThreadPoolExecutor
 CSRC = os.path.join(os.path.dirname(os.path.abspath(__file__)), "csrc")
 LIB_PATH = os.path.join(CSRC, "libflyb200.so")
 STAMP_PATH = os.path.join(CSRC, "libflyb200.stamp")  # digest of the inputs the library was built from
+OPS_PATH = os.path.join(CSRC, "flyb200_ops.so")  # CPython extension: the operators' host path over the library
+OPS_STAMP_PATH = os.path.join(CSRC, "flyb200_ops.stamp")
+OPS_SOURCES = ["ops.cpp", os.path.join("..", "..", "include", "flyb200.h")]
 OBJ_DIR = os.path.join(CSRC, "build")
 SOURCES = [
     "flyb200.cu",
@@ -150,5 +154,63 @@ def build_library(force: bool = False, verbose: bool = False) -> str:
     return LIB_PATH
 
 
+def _ops_digest() -> str:
+    import torch
+
+    h = hashlib.sha256(f"{torch.__version__} {sys.version}".encode())  # the extension is built against these
+    for f in OPS_SOURCES:
+        with open(os.path.join(CSRC, f), "rb") as fh:
+            h.update(fh.read())
+    return h.hexdigest()
+
+
+def _ops_stale() -> bool:
+    if not os.path.exists(OPS_PATH) or not os.path.exists(OPS_STAMP_PATH):
+        return True
+    with open(OPS_STAMP_PATH) as fh:
+        return fh.read().strip() != _ops_digest()
+
+
+def build_ops(force: bool = False) -> str:
+    """Compile the extension if it is missing or older than its sources (after the library it links to)."""
+    build_library()
+    if not force and not _ops_stale():
+        return OPS_PATH
+    import sysconfig
+
+    import torch
+
+    cxx = shutil.which("g++")
+    nvcc = find_nvcc()
+    if cxx is None or nvcc is None:
+        raise RuntimeError("g++ or the CUDA toolkit not found: cannot build flyb200_ops.so")
+    root = os.path.dirname(torch.__file__)
+    include = [os.path.join(root, "include"), os.path.join(root, "include", "torch", "csrc", "api", "include"),
+               sysconfig.get_paths()["include"], os.path.join(os.path.dirname(os.path.dirname(nvcc)), "include")]
+    os.makedirs(OBJ_DIR, exist_ok=True)
+    with open(os.path.join(OBJ_DIR, ".lock"), "w") as lock:
+        fcntl.flock(lock, fcntl.LOCK_EX)
+        try:
+            if not force and not _ops_stale():
+                return OPS_PATH
+            tmp = OPS_PATH + f".{os.getpid()}.tmp"
+            cmd = [cxx, "-O2", "-std=c++17", "-fPIC", "-shared", f"-D_GLIBCXX_USE_CXX11_ABI={int(torch._C._GLIBCXX_USE_CXX11_ABI)}"]
+            for d in include:
+                cmd += ["-isystem", d]
+            cmd += ["ops.cpp", "-o", tmp, "-L.", "-l:libflyb200.so", f"-L{os.path.join(root, 'lib')}", "-lc10", "-lc10_cuda",
+                    "-ltorch_cpu", "-ltorch_python", "-Wl,-rpath,$ORIGIN"]
+            res = subprocess.run(cmd, cwd=CSRC, capture_output=True, text=True)
+            if res.returncode != 0:
+                raise RuntimeError(f"g++ failed on ops.cpp ({res.returncode}):\n{res.stdout}\n{res.stderr}")
+            os.replace(tmp, OPS_PATH)
+            with open(OPS_STAMP_PATH + f".{os.getpid()}.tmp", "w") as fh:
+                fh.write(_ops_digest() + "\n")
+            os.replace(OPS_STAMP_PATH + f".{os.getpid()}.tmp", OPS_STAMP_PATH)
+        finally:
+            fcntl.flock(lock, fcntl.LOCK_UN)
+    return OPS_PATH
+
+
 if __name__ == "__main__":
     print(build_library(force="--force" in sys.argv, verbose="-v" in sys.argv))
+    print(build_ops(force="--force" in sys.argv))

@@ -22,6 +22,7 @@ from dataclasses import dataclass
 import torch
 import torch.distributed as dist
 
+from . import _lib
 from .column_parallel import check_agreement
 
 
@@ -116,6 +117,10 @@ class ExpertParallelMoe:
             raise RuntimeError("load_expert_weights has not been called")
         tokens = x_q.shape[0]
         dev = x_q.device
+        if self.out_dtype == "bf16" and self.in_dtype in ("fp8", "int8") and x_q.is_cuda and tokens > 0:
+            y = self._forward_native(x_q, scale_x, topk_ids, topk_weights, tokens, dev)
+            if y is not None:
+                return y
         # routes of this rank's experts only, in their numbering (local_routing inside the sort)
         srt, wts, e_ids, post = sort_on_device(topk_ids, topk_weights, self.shard.experts_local, self.tile_m, self.shard.e0)
         blocks = int(e_ids.numel())
@@ -131,12 +136,30 @@ class ExpertParallelMoe:
         # rows of routes that belong to other ranks are never written; the masked reduction skips them
         out2 = torch.empty(tokens * self.topk, self.model_dim, dtype=torch.bfloat16, device=dev)
         self._g2._launch_quantising(out2, out1, self._w2, self._sw2, srt, e_ids, wts, post, tokens, blocks, st)
+        y = torch.empty(tokens, self.model_dim, dtype=torch.bfloat16, device=dev)
+        self._reduce(out2, y, self._expert_mask(dev), topk_ids.to(torch.int32).contiguous(), tokens, st)
+        return y
+
+    def _expert_mask(self, dev):
         if self._mask is None or self._mask.device != dev:
             mask = torch.zeros(self.shard.experts_total, dtype=torch.int32, device=dev)
             mask[self.shard.e0 : self.shard.e1] = 1
             self._mask = mask
-        y = torch.empty(tokens, self.model_dim, dtype=torch.bfloat16, device=dev)
-        self._reduce(out2, y, self._mask, topk_ids.to(torch.int32).contiguous(), tokens, st)
+        return self._mask
+
+    def _forward_native(self, x_q, scale_x, topk_ids, topk_weights, tokens, dev):
+        """The same sequence as one call of the host extension; None where an argument is not of the common
+        form (the statements of forward_local then take it, or say what is wrong with it)."""
+        el = self.shard.experts_local
+        blocks = (tokens * self.topk + el * self.tile_m - self.topk + self.tile_m - 1) // self.tile_m
+        st = _lib.current_stream(dev)
+        a1, sa1 = self._g1._sorted_buffers(dev, blocks * self.tile_m, st)
+        a2, sa2 = self._g2._sorted_buffers(dev, blocks * self.tile_m, st)
+        y = _lib.ops().moe_layer(x_q, scale_x, topk_ids, topk_weights, self._w1, self._sw1, self._w2, self._sw2, self._expert_mask(dev),
+                                 a1, sa1, a2, sa2, el, self.shard.e0, self.shard.experts_total, self.model_dim, self.inter_dim,
+                                 self.topk, self.tile_m, _lib.IN_DTYPES[self.in_dtype])
+        if type(y) is int:
+            _lib.check(y, "moe_layer")
         return y
 
     def forward(self, x_q, scale_x, topk_ids, topk_weights, handshake_group=None):

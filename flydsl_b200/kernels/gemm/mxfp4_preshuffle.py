@@ -64,7 +64,7 @@ def per_1x32_f4_quant(x: torch.Tensor):
     q = quant_kernel(x, _FORMATS["fp4"])
     if q is None:
         return per_1x32_f4_quant_torch(x)
-    return q[0].view(*shape[:-1], shape[-1] // 2), q[1].view(*shape[:-1], shape[-1] // 32)
+    return q[0], q[1]
 
 
 def per_1x32_f4_quant_torch(x: torch.Tensor):
@@ -150,7 +150,7 @@ def per_1x32_f6_quant(x: torch.Tensor):
     q = quant_kernel(x, _FORMATS["fp6"])
     if q is None:
         return per_1x32_f6_quant_torch(x)
-    return q[0].view(m, k), q[1].view(m, k // 32), q[2].view(m, k)
+    return q
 
 
 def per_1x32_f6_quant_torch(x: torch.Tensor):
@@ -232,6 +232,13 @@ class MxMixedGemm:
             raise ValueError(f"N passed at call time ({n_rt}) differs from the N the launcher was built for ({self.N})")
         if M < 0:
             raise ValueError("M must be non-negative")
+        if arg_bias is None or arg_bias.numel() == 0:
+            rc = _lib.ops().mx_gemm(_FORMATS[self.a_dtype], _FORMATS["fp4"], arg_c, arg_a, arg_b, arg_scale_a, arg_scale_b, M, self.N, self.K,
+                                    self._out, _stream_handle(stream))
+            if rc is not None:
+                if rc:
+                    _lib.check(rc, "gemm_mx_mixed")
+                return None
         lib = _lib.load()
         for name, t in (("c", arg_c), ("a", arg_a), ("b", arg_b), ("scale_a", arg_scale_a), ("scale_b", arg_scale_b)):
             if not isinstance(t, torch.Tensor) or not t.is_cuda or not t.is_contiguous():
@@ -286,6 +293,12 @@ class MxFp4Gemm:
             raise ValueError(f"N passed at call time ({n_rt}) differs from the N the launcher was built for ({self.N})")
         if M < 0:
             raise ValueError("M must be non-negative")
+        if arg_bias is None or arg_bias.numel() == 0:
+            rc = _lib.ops().mx_gemm(5, 5, arg_c, arg_a, arg_b, arg_scale_a, arg_scale_b, M, self.N, self.K, self._out, _stream_handle(stream))
+            if rc is not None:
+                if rc:
+                    _lib.check(rc, "gemm_mxfp4")
+                return None
         lib = _lib.load()
         need = (
             ("c", arg_c, M * self.N), ("a", arg_a, M * self.K // 2), ("b", arg_b, self.N * self.K // 2),

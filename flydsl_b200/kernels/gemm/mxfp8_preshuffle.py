@@ -27,30 +27,16 @@ _TORCH_OUT = {"bf16": torch.bfloat16, "fp16": torch.float16, "f16": torch.float1
 FP8_MAX = 448.0
 
 
-_QUANT_IN = {torch.float32: 0, torch.float16: 1, torch.bfloat16: 2}
-
-
 def quant_kernel(x: torch.Tensor, fmt: int):
     """The per-1x32 quantisers as ONE kernel (the torch statements launch 30 to 250): ``(codes, scales, raw)``
-    as flat uint8 tensors on x's device, or None where the kernel cannot take ``x`` (CPU tensors, other
+    on x's device and of its leading shape, or None where the kernel cannot take ``x`` (CPU tensors, other
     dtypes, no elements).  ``fmt``: 0 E4M3, 3 E2M3, 5 E2M1; ``raw`` (the codes one per byte) is None unless E2M3."""
-    if not x.is_cuda or x.dtype not in _QUANT_IN:
+    if not x.is_cuda:
         return None
-    n = x.numel()
-    x = x.contiguous()
-    ptr = x.data_ptr()
-    if n == 0 or ptr % 16 != 0:
-        return None
-    dev = x.device
-    codes = torch.empty(n // 2 if fmt == 5 else n, dtype=torch.uint8, device=dev)
-    scale = torch.empty(n // 32, dtype=torch.uint8, device=dev)
-    raw = torch.empty(n, dtype=torch.uint8, device=dev) if fmt == 3 else None
-    with _lib.on_device(dev):
-        rc = _lib.load().flyb200_mx_quant(codes.data_ptr(), scale.data_ptr(), raw.data_ptr() if fmt == 3 else None, ptr, n,
-                                          _QUANT_IN[x.dtype], fmt, _lib.current_stream(dev))
-    if rc:
-        _lib.check(rc, "mx_quant")
-    return codes, scale, raw
+    r = _lib.ops().mx_quant(x, fmt)
+    if type(r) is int:
+        _lib.check(r, "mx_quant")
+    return r
 
 
 def per_1x32_f8_quant(x: torch.Tensor):
@@ -64,7 +50,7 @@ def per_1x32_f8_quant(x: torch.Tensor):
     q = quant_kernel(x, 0)
     if q is None:
         return per_1x32_f8_quant_torch(x)
-    return q[0].view(torch.float8_e4m3fn).view(shape), q[1].view(*shape[:-1], shape[-1] // 32)
+    return q[0], q[1]
 
 
 def per_1x32_f8_quant_torch(x: torch.Tensor):
@@ -95,6 +81,11 @@ def shuffle_scale(scale: torch.Tensor) -> torch.Tensor:
         raise ValueError("K must be a multiple of 128")
     if not scale.is_cuda:
         raise ValueError("scale must be a CUDA tensor")
+    r = _lib.ops().mx_scale_image(scale)
+    if r is not None:
+        if type(r) is int:
+            _lib.check(r, "mx_scale_image")
+        return r
     dev = scale.device
     src = scale.contiguous()
     out = torch.empty(scale_image_bytes(rows, kb32 * 32), dtype=torch.uint8, device=dev)
@@ -123,6 +114,12 @@ class MxFp8Gemm:
             raise ValueError(f"N passed at call time ({n_rt}) differs from the N the launcher was built for ({self.N})")
         if M < 0:
             raise ValueError("M must be non-negative")
+        if arg_bias is None or arg_bias.numel() == 0:
+            rc = _lib.ops().mx_gemm(0, 0, arg_c, arg_a, arg_b, arg_scale_a, arg_scale_b, M, self.N, self.K, self._out, _stream_handle(stream))
+            if rc is not None:
+                if rc:
+                    _lib.check(rc, "gemm_mxfp8")
+                return None
         lib = _lib.load()
         need = (
             ("c", arg_c, M * self.N), ("a", arg_a, M * self.K), ("b", arg_b, self.N * self.K),

@@ -211,7 +211,7 @@ class CompiledPreshuffleGemm:
 
     def __init__(self, op: "PreshuffleGemm"):
         self.op = op
-        self._fn = _lib.load().flyb200_gemm_a8w8
+        self._fn = _lib.ops().gemm_a8w8
 
     def __call__(self, arg_c, arg_a, arg_b, arg_scale_a, arg_scale_b, arg_bias, i32_m, i32_n, stream=None):
         op = self.op
@@ -233,11 +233,11 @@ class CompiledPreshuffleGemm:
             with torch.cuda.device(dev):
                 return self.__call__(arg_c, arg_a, arg_b, arg_scale_a, arg_scale_b, arg_bias, i32_m, i32_n, stream)
         rc = self._fn(
-            arg_c.data_ptr(), arg_a.data_ptr(), arg_b.data_ptr(),
-            arg_scale_a.data_ptr() if eight else None, arg_scale_b.data_ptr() if eight else None,
-            arg_bias.data_ptr() if op._epi else None,
-            M, op.N, op.K, op._dt, op._out, op._epi, op.variant_hint, ws[0] or None, ws[1], s or None,
+            arg_c, arg_a, arg_b, arg_scale_a if eight else None, arg_scale_b if eight else None, arg_bias if op._epi else None,
+            M, op.N, op.K, op._dt, op._out, op._epi, op.variant_hint, ws[0], ws[1], s,
         )  # fmt: skip
+        if rc is None:
+            raise TypeError("preshuffle_gemm: c, a, b, scales and bias must be tensors")
         if rc:
             _lib.check(rc, "preshuffle_gemm")
         return None

@@ -122,6 +122,11 @@ def moe_sorting(
 def sort_on_device(topk_ids, topk_weights, experts: int, block_size: int, first_expert: int):
     """``moe_sorting`` for CUDA tensors as one kernel (no host synchronisation, capturable), for the
     experts ``[first_expert, first_expert + experts)`` renumbered from zero; other routes are dropped."""
+    r = _lib.ops().moe_sort(topk_ids, topk_weights, experts, block_size, first_expert)
+    if r is not None:
+        if type(r) is int:
+            _lib.check(r, "moe_sorting")
+        return r
     tokens, topk = topk_ids.shape
     dev = topk_ids.device
     ids = topk_ids if topk_ids.dtype in (torch.int32, torch.int64) else topk_ids.to(torch.int32)
@@ -272,13 +277,16 @@ class _MoeStage:
         s = _stream_handle(stream) or None
         rows = blocks * self.tile_m
         a_sorted, sa_sorted = self._sorted_buffers(dev, rows, s)
-        rc = _lib.load().flyb200_moe_gather_rows(
-            a_sorted.data_ptr(), sa_sorted.data_ptr(), x.data_ptr(), scale_x.data_ptr(), sorted_token_ids.data_ptr(),
-            num_valid_ids.data_ptr(), tokens, self.topk, self._gather_mode, self._k, rows, s)
+        if self.in_dtype == "int4":
+            w = self._weights_for_kernel(w, self.experts * (2 * self.inter_dim if self.stage == 1 else self.model_dim) * self._k)
+        rc = _lib.ops().moe_stage(
+            out, x, w, scale_x, scale_w, sorted_token_ids, sorted_expert_ids, sorted_weights, num_valid_ids, a_sorted, sa_sorted,
+            self.stage, tokens, self.topk, self._gather_mode, self._k, self.experts, self.model_dim, self.inter_dim, self.tile_m,
+            blocks, self._dt, self._out, self.doweight, self.accumulate, s or 0)
+        if rc is None:
+            raise TypeError("moe_gemm: all arguments but the routed weights must be tensors")
         if rc:
-            _lib.check(rc, "moe_gather_rows")
-        self._gemm(out, a_sorted, sa_sorted, w, scale_w, sorted_token_ids, sorted_expert_ids, sorted_weights, num_valid_ids,
-                   tokens, blocks, s)
+            _lib.check(rc, "moe_gemm")
         return None
 
     def _launch_quantising(self, out, x16, w, scale_w, sorted_token_ids, sorted_expert_ids, sorted_weights, num_valid_ids,

@@ -23,6 +23,9 @@ def get_dtype_max(dtype: torch.dtype) -> float:
 
 
 _X_DTYPES = {torch.float32: 0, torch.float16: 1, torch.bfloat16: 2}
+_QUANT_CODES = {torch.int8: _lib.DT_INT8}
+if hasattr(torch, "float8_e4m3fn"):
+    _QUANT_CODES[torch.float8_e4m3fn] = _lib.DT_FP8
 
 
 def _kernel_can_quantise(x, scale, x_scale, scale_dtype, quant_dtype, dtypeMax) -> bool:
@@ -41,18 +44,10 @@ def pertoken_quant_kernel(x: torch.Tensor, quant_dtype=torch.int8):
     fused; the torch statement below launches about ten element-wise kernels
     and materialises fp32 temporaries).  Bit-identical to :func:`pertoken_quant`
     evaluated by torch on the same GPU tensor."""
-    lib = _lib.load()
-    k = x.shape[-1]
-    rows = x.numel() // k
-    y = torch.empty(x.shape, dtype=quant_dtype, device=x.device)
-    s = torch.empty(*x.shape[:-1], 1, dtype=torch.float32, device=x.device)
-    qd = _lib.DT_INT8 if quant_dtype == torch.int8 else _lib.DT_FP8
-    with torch.cuda.device(x.device):
-        rc = lib.flyb200_pertoken_quant(
-            y.data_ptr(), s.data_ptr(), x.data_ptr(), rows, k, _X_DTYPES[x.dtype], qd, _stream_ptr(x.device)
-        )
-    _lib.check(rc, "pertoken_quant")
-    return y, s
+    r = _lib.ops().pertoken_quant(x, _QUANT_CODES[quant_dtype])
+    if type(r) is not tuple:
+        _lib.check(_lib.E_UNSUPPORTED if r is None else r, "pertoken_quant")
+    return r
 
 
 def pertoken_quant(
@@ -69,6 +64,11 @@ def pertoken_quant(
     dtypeMax) go through the fused kernel (:func:`pertoken_quant_kernel`);
     ``use_kernel=False`` forces the torch statement, ``use_kernel=True`` raises
     if the kernel cannot take the arguments."""
+    if (use_kernel is not False and scale is None and x_scale is None and dtypeMax is None and scale_dtype == torch.float32
+            and quant_dtype in _QUANT_CODES and isinstance(x, torch.Tensor) and x.is_cuda):
+        r = _lib.ops().pertoken_quant(x, _QUANT_CODES[quant_dtype])  # checks what _kernel_can_quantise does
+        if type(r) is tuple:
+            return r
     can = _kernel_can_quantise(x, scale, x_scale, scale_dtype, quant_dtype, dtypeMax)
     if use_kernel and not can:
         raise ValueError("the fused quantiser needs a contiguous CUDA fp32/fp16/bf16 tensor and default options")

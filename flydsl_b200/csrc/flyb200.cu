@@ -659,21 +659,22 @@ int launch_shuffle(void* dst, const void* src, int N, int Kb, cudaStream_t s) {
 // Row quantiser launch: rows that fit the register-cached single-pass kernel
 // use it (one block per row), longer rows take the two-pass kernel.
 template <typename TIn, bool FP8>
-void launch_quant_t(uint8_t* y, float* scale, const TIn* x, int rows, int K, cudaStream_t s) {
+cudaError_t launch_quant_t(uint8_t* y, float* scale, const TIn* x, int rows, int K, cudaStream_t s) {
+  cudaError_t err = cudaSuccess;
   const bool fits = quant_row_dispatch(rows, K / QuantIn<TIn>::VEC, [&](auto nv, auto wpr) {
     constexpr int PER_BLOCK = 8 / decltype(wpr)::value;
-    pertoken_quant_row_kernel<TIn, FP8, decltype(nv)::value, decltype(wpr)::value>
-        <<<(rows + PER_BLOCK - 1) / PER_BLOCK, 256, 0, s>>>(y, scale, x, rows, K);
+    err = host::launch_dependent(pertoken_quant_row_kernel<TIn, FP8, decltype(nv)::value, decltype(wpr)::value>,
+                                 dim3((rows + PER_BLOCK - 1) / PER_BLOCK), 256, 0, s, y, scale, x, rows, K);
   });
   if (!fits) {
     const int grid = rows < 148 * 16 ? rows : 148 * 16;
-    pertoken_quant_kernel<TIn, FP8><<<grid, 256, 0, s>>>(y, scale, x, rows, K);
+    err = host::launch_dependent(pertoken_quant_kernel<TIn, FP8>, dim3(grid), 256, 0, s, y, scale, x, rows, K);
   }
+  return err;
 }
 template <typename TIn>
-void launch_quant(uint8_t* y, float* scale, const TIn* x, int rows, int K, bool fp8, cudaStream_t s) {
-  if (fp8) launch_quant_t<TIn, true>(y, scale, x, rows, K, s);
-  else launch_quant_t<TIn, false>(y, scale, x, rows, K, s);
+cudaError_t launch_quant(uint8_t* y, float* scale, const TIn* x, int rows, int K, bool fp8, cudaStream_t s) {
+  return fp8 ? launch_quant_t<TIn, true>(y, scale, x, rows, K, s) : launch_quant_t<TIn, false>(y, scale, x, rows, K, s);
 }
 
 bool ranges_overlap(const void* a, const void* b, size_t bytes) {
@@ -975,13 +976,12 @@ int flyb200_pertoken_quant(void* y, float* scale, const void* x, int rows, int K
   uint8_t* yo = static_cast<uint8_t*>(y);
   const bool fp8 = quant_dtype == FLYB200_DT_FP8;
   if (x_dtype == QX_F32) {
-    launch_quant<float>(yo, scale, static_cast<const float*>(x), rows, K, fp8, s);
+    CUDA_TRY(launch_quant<float>(yo, scale, static_cast<const float*>(x), rows, K, fp8, s));
   } else if (x_dtype == QX_F16) {
-    launch_quant<__half>(yo, scale, static_cast<const __half*>(x), rows, K, fp8, s);
+    CUDA_TRY(launch_quant<__half>(yo, scale, static_cast<const __half*>(x), rows, K, fp8, s));
   } else {
-    launch_quant<__nv_bfloat16>(yo, scale, static_cast<const __nv_bfloat16*>(x), rows, K, fp8, s);
+    CUDA_TRY(launch_quant<__nv_bfloat16>(yo, scale, static_cast<const __nv_bfloat16*>(x), rows, K, fp8, s));
   }
-  CUDA_TRY(cudaGetLastError());
   return FLYB200_OK;
 }
 

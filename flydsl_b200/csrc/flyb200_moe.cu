@@ -97,8 +97,7 @@ int launch_moe_rows(const CUtensorMap& tmA, const MoeParams& p, int blocks, cuda
   const int pairs = STAGE == 1 ? (p.n_out + BLOCK_ROWS - 1) / BLOCK_ROWS : (p.n_out + MOE_ROWS_BN - 1) / MOE_ROWS_BN;
   const long long items = row_blocks * pairs;
   const int grid = static_cast<int>(items < sms ? items : sms);
-  kernel<<<grid, NUM_THREADS, MoeRowsSmem::TOTAL, s>>>(tmA, p);
-  CUDA_TRY(cudaGetLastError());
+  CUDA_TRY(host::launch_dependent(kernel, dim3(grid), NUM_THREADS, MoeRowsSmem::TOTAL, s, tmA, p));
   return FLYB200_OK;
 }
 
@@ -155,16 +154,16 @@ int launch_moe_bn(int bn, int stage, int out_dtype, bool accumulate, const CUten
 
 // Vectors of eight where every row starts on a 16-byte boundary, else pairs.
 template <typename T>
-void launch_moe_reduce(void* y, const void* x, int tokens, int topk, int dim, const int* expert_mask, const int* topk_ids,
+cudaError_t launch_moe_reduce(void* y, const void* x, int tokens, int topk, int dim, const int* expert_mask, const int* topk_ids,
                        int num_experts, cudaStream_t s) {
   T* yt = static_cast<T*>(y);
   const T* xt = static_cast<const T*>(x);
   if (dim % 8 == 0 && aligned16(y) && aligned16(x)) {
     const dim3 grid(tokens, (dim / 8 + 255) / 256);
-    moe_reduce_kernel<T, 8><<<grid, 256, 0, s>>>(yt, xt, topk, dim, expert_mask, topk_ids, num_experts);
+    return host::launch_dependent(moe_reduce_kernel<T, 8>, grid, 256, 0, s, yt, xt, topk, dim, expert_mask, topk_ids, num_experts);
   } else {
     const dim3 grid(tokens, (dim / 2 + 255) / 256);
-    moe_reduce_kernel<T, 2><<<grid, 256, 0, s>>>(yt, xt, topk, dim, expert_mask, topk_ids, num_experts);
+    return host::launch_dependent(moe_reduce_kernel<T, 2>, grid, 256, 0, s, yt, xt, topk, dim, expert_mask, topk_ids, num_experts);
   }
 }
 
@@ -184,10 +183,9 @@ int flyb200_moe_gather_rows(void* dst, float* dst_scale, const void* src, const 
   const int warps = 8;
   int grid = (rows + warps - 1) / warps;
   if (grid > 148 * 8) grid = 148 * 8;
-  moe_gather_rows_kernel<<<grid, warps * 32, 0, static_cast<cudaStream_t>(stream)>>>(
-      static_cast<uint8_t*>(dst), dst_scale, static_cast<const uint8_t*>(src), src_scale, sorted_ids, num_valid_ids,
-      tokens, topk, by_slot, row_bytes, rows);
-  CUDA_TRY(cudaGetLastError());
+  CUDA_TRY(host::launch_dependent(moe_gather_rows_kernel, dim3(grid), warps * 32, 0, static_cast<cudaStream_t>(stream),
+                                  static_cast<uint8_t*>(dst), dst_scale, static_cast<const uint8_t*>(src), src_scale, sorted_ids,
+                                  num_valid_ids, tokens, topk, by_slot, row_bytes, rows));
   return FLYB200_OK;
 }
 
@@ -200,17 +198,16 @@ int flyb200_moe_quant_sorted(void* dst, float* dst_scale, const void* src, const
   if (!aligned16(dst) || !aligned16(src)) return FLYB200_E_BAD_ALIGN;
   if (rows == 0) return FLYB200_OK;
   cudaStream_t s = static_cast<cudaStream_t>(stream);
+  cudaError_t err = cudaSuccess;
   quant_row_dispatch(rows, K / 8, [&](auto nv, auto wpr) {
     constexpr int NV = decltype(nv)::value, WPR = decltype(wpr)::value;
     const int grid = (rows + 8 / WPR - 1) / (8 / WPR);
     const __nv_bfloat16* x = static_cast<const __nv_bfloat16*>(src);
     uint8_t* y = static_cast<uint8_t*>(dst);
-    if (quant_dtype == FLYB200_DT_FP8)
-      moe_quant_sorted_kernel<true, NV, WPR><<<grid, 256, 0, s>>>(y, dst_scale, x, sorted_ids, num_valid_ids, tokens, topk, K, rows);
-    else
-      moe_quant_sorted_kernel<false, NV, WPR><<<grid, 256, 0, s>>>(y, dst_scale, x, sorted_ids, num_valid_ids, tokens, topk, K, rows);
+    err = host::launch_dependent(quant_dtype == FLYB200_DT_FP8 ? moe_quant_sorted_kernel<true, NV, WPR> : moe_quant_sorted_kernel<false, NV, WPR>,
+                                 dim3(grid), 256, 0, s, y, dst_scale, x, sorted_ids, num_valid_ids, tokens, topk, K, rows);
   });
-  CUDA_TRY(cudaGetLastError());
+  CUDA_TRY(err);
   return FLYB200_OK;
 }
 
@@ -297,16 +294,13 @@ int flyb200_moe_sorting_range(const void* topk_ids, int id_bytes, const float* t
   // four pairs per thread, and enough threads for the histogram and the padding of small calls
   long long threads = (n_pairs / 4 + 31) / 32 * 32;
   threads = threads < 128 ? 128 : threads > MOE_SORT_MAX_THREADS ? MOE_SORT_MAX_THREADS : threads;
-  if (id_bytes == 4) {
-    moe_sort_kernel<int><<<experts, static_cast<int>(threads), 0, s>>>(
-        static_cast<const int*>(topk_ids), topk_weights, static_cast<int>(n_pairs), topk, tokens, experts, first_expert,
-        block_size, sorted_ids, sorted_weights, sorted_expert_ids, num_tokens_post_pad, static_cast<int>(max_padded), max_blocks);
-  } else {
-    moe_sort_kernel<long long><<<experts, static_cast<int>(threads), 0, s>>>(
-        static_cast<const long long*>(topk_ids), topk_weights, static_cast<int>(n_pairs), topk, tokens, experts, first_expert,
-        block_size, sorted_ids, sorted_weights, sorted_expert_ids, num_tokens_post_pad, static_cast<int>(max_padded), max_blocks);
-  }
-  CUDA_TRY(cudaGetLastError());
+  auto launch = [&](auto* ids) {
+    using ID = std::remove_const_t<std::remove_pointer_t<decltype(ids)>>;
+    return host::launch_dependent(moe_sort_kernel<ID>, dim3(experts), static_cast<int>(threads), 0, s, ids, topk_weights,
+                                  static_cast<int>(n_pairs), topk, tokens, experts, first_expert, block_size, sorted_ids, sorted_weights,
+                                  sorted_expert_ids, num_tokens_post_pad, static_cast<int>(max_padded), max_blocks);
+  };
+  CUDA_TRY(id_bytes == 4 ? launch(static_cast<const int*>(topk_ids)) : launch(static_cast<const long long*>(topk_ids)));
   return FLYB200_OK;
 }
 
@@ -327,9 +321,8 @@ int flyb200_moe_reduce(void* y, const void* x, int tokens, int topk, int dim, in
   if (tokens == 0) return FLYB200_OK;
   cudaStream_t s = static_cast<cudaStream_t>(stream);
   if (dtype != FLYB200_OUT_BF16 && dtype != FLYB200_OUT_FP16) return FLYB200_E_UNSUPPORTED;
-  if (dtype == FLYB200_OUT_BF16) launch_moe_reduce<__nv_bfloat16>(y, x, tokens, topk, dim, expert_mask, topk_ids, num_experts, s);
-  else launch_moe_reduce<__half>(y, x, tokens, topk, dim, expert_mask, topk_ids, num_experts, s);
-  CUDA_TRY(cudaGetLastError());
+  if (dtype == FLYB200_OUT_BF16) CUDA_TRY(launch_moe_reduce<__nv_bfloat16>(y, x, tokens, topk, dim, expert_mask, topk_ids, num_experts, s));
+  else CUDA_TRY(launch_moe_reduce<__half>(y, x, tokens, topk, dim, expert_mask, topk_ids, num_experts, s));
   return FLYB200_OK;
 }
 

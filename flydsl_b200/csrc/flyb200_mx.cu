@@ -43,13 +43,20 @@ int launch_mx(const CUtensorMap& tmA, const MxParams& p, cudaStream_t s) {
   cfg.blockDim = dim3(NUM_THREADS, 1, 1);
   cfg.dynamicSmemBytes = Smem::TOTAL;
   cfg.stream = s;
-  cudaLaunchAttribute attr;
-  attr.id = cudaLaunchAttributeClusterDimension;
-  attr.val.clusterDim.x = static_cast<unsigned>(p.split);
-  attr.val.clusterDim.y = 1;
-  attr.val.clusterDim.z = 1;
-  cfg.attrs = &attr;
-  cfg.numAttrs = SPLIT ? 1 : 0;
+  cudaLaunchAttribute attrs[2];
+  attrs[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;  // as launch_dependent
+  attrs[0].val.programmaticStreamSerializationAllowed = 1;
+  const char* e = getenv("FLYB200_PDL");
+  int na = e && e[0] == '0' ? 0 : 1;
+  if (SPLIT) {
+    attrs[na].id = cudaLaunchAttributeClusterDimension;
+    attrs[na].val.clusterDim.x = static_cast<unsigned>(p.split);
+    attrs[na].val.clusterDim.y = 1;
+    attrs[na].val.clusterDim.z = 1;
+    ++na;
+  }
+  cfg.attrs = attrs;
+  cfg.numAttrs = na;
   CUDA_TRY(cudaLaunchKernelEx(&cfg, kernel, tmA, p));
   return FLYB200_OK;
 }
@@ -57,11 +64,10 @@ int launch_mx(const CUtensorMap& tmA, const MxParams& p, cudaStream_t s) {
 }  // namespace
 
 template <typename TIn>
-void launch_mx_quant(uint8_t* codes, uint8_t* scale, uint8_t* raw, const TIn* x, long long units, int fmt, cudaStream_t s) {
+cudaError_t launch_mx_quant(uint8_t* codes, uint8_t* scale, uint8_t* raw, const TIn* x, long long units, int fmt, cudaStream_t s) {
   const unsigned grid = static_cast<unsigned>((units + 255) / 256);
-  if (fmt == MXQ_FP8) mx_quant_kernel<TIn, MXQ_FP8><<<grid, 256, 0, s>>>(codes, scale, raw, x, units);
-  else if (fmt == MXQ_FP4) mx_quant_kernel<TIn, MXQ_FP4><<<grid, 256, 0, s>>>(codes, scale, raw, x, units);
-  else mx_quant_kernel<TIn, MXQ_FP6><<<grid, 256, 0, s>>>(codes, scale, raw, x, units);
+  auto kernel = fmt == MXQ_FP8 ? mx_quant_kernel<TIn, MXQ_FP8> : fmt == MXQ_FP4 ? mx_quant_kernel<TIn, MXQ_FP4> : mx_quant_kernel<TIn, MXQ_FP6>;
+  return host::launch_dependent(kernel, dim3(grid), 256, 0, s, codes, scale, raw, x, units);
 }
 
 namespace {
@@ -166,10 +172,9 @@ int flyb200_mx_quant(void* codes, void* scale, void* raw, const void* x, long lo
   const long long units = elements / MXQ_UNIT;
   cudaStream_t s = static_cast<cudaStream_t>(stream);
   uint8_t *c = static_cast<uint8_t*>(codes), *sc = static_cast<uint8_t*>(scale), *r = static_cast<uint8_t*>(raw);
-  if (x_dtype == 0) launch_mx_quant(c, sc, r, static_cast<const float*>(x), units, format, s);
-  else if (x_dtype == 1) launch_mx_quant(c, sc, r, static_cast<const __half*>(x), units, format, s);
-  else launch_mx_quant(c, sc, r, static_cast<const __nv_bfloat16*>(x), units, format, s);
-  CUDA_TRY(cudaGetLastError());
+  if (x_dtype == 0) CUDA_TRY(launch_mx_quant(c, sc, r, static_cast<const float*>(x), units, format, s));
+  else if (x_dtype == 1) CUDA_TRY(launch_mx_quant(c, sc, r, static_cast<const __half*>(x), units, format, s));
+  else CUDA_TRY(launch_mx_quant(c, sc, r, static_cast<const __nv_bfloat16*>(x), units, format, s));
   return FLYB200_OK;
 }
 
@@ -181,9 +186,8 @@ int flyb200_mx_fp6_containers(void* dst, const void* src, long long bytes, void*
   const long long blocks32 = bytes / 32;
   long long grid = (blocks32 + 255) / 256;
   if (grid > 148 * 16) grid = 148 * 16;
-  mx_fp6_containers_kernel<<<static_cast<int>(grid), 256, 0, static_cast<cudaStream_t>(stream)>>>(
-      static_cast<uint4*>(dst), static_cast<const uint4*>(src), blocks32);
-  CUDA_TRY(cudaGetLastError());
+  CUDA_TRY(host::launch_dependent(mx_fp6_containers_kernel, dim3(static_cast<unsigned>(grid)), 256, 0, static_cast<cudaStream_t>(stream),
+                                  static_cast<uint4*>(dst), static_cast<const uint4*>(src), blocks32));
   return FLYB200_OK;
 }
 
@@ -195,9 +199,8 @@ int flyb200_mx_scale_image(void* dst, const void* src, int rows, int K, void* st
   const long long total = static_cast<long long>(flyb200_mx_scale_image_bytes(rows, K)) / 4;
   long long blocks = (total + 255) / 256;
   if (blocks > 148 * 8) blocks = 148 * 8;
-  mx_scale_image_kernel<<<static_cast<int>(blocks), 256, 0, static_cast<cudaStream_t>(stream)>>>(
-      static_cast<uint32_t*>(dst), static_cast<const uint8_t*>(src), rows, K / 32, row_tiles);
-  CUDA_TRY(cudaGetLastError());
+  CUDA_TRY(host::launch_dependent(mx_scale_image_kernel, dim3(static_cast<unsigned>(blocks)), 256, 0, static_cast<cudaStream_t>(stream),
+                                  static_cast<uint32_t*>(dst), static_cast<const uint8_t*>(src), rows, K / 32, row_tiles));
   return FLYB200_OK;
 }
 

@@ -251,6 +251,7 @@ __global__ void __launch_bounds__(MOE_THREADS) moe_gemm_kernel(const __grid_cons
           phase ^= 1u;
         }
       }
+      if (p.pdl) pdl_trigger();  // after its wait: the next kernel may be scheduled as the CTAs finish
       if (!ok || *abort_flag) {
         // wait (bounded) for copies still in flight so none lands after the CTA is gone
         const int pending = min(issued, stages);
@@ -497,12 +498,14 @@ __global__ void __launch_bounds__(NUM_THREADS, 1) moe_rows_kernel(const __grid_c
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem_base = *tmem_slot;
+  const int* num_valid = p.num_valid;
+  pdl_wait(num_valid);  // launched as a programmatic dependent: nothing in global memory is touched before this
 
   // Work items: (row block of 128 sorted rows, channel pair).  Row blocks run
   // fastest, so CTAs working side by side share the weight tiles of an expert,
   // and they are taken in groups of MOE_ROWS_GROUP whose activation rows stay in
   // L2 while the group walks all channel pairs.
-  const int n_rows = __ldg(p.num_valid);
+  const int n_rows = __ldg(num_valid);
   const int row_blocks = (n_rows + BLOCK_ROWS - 1) / BLOCK_ROWS;
   const int pairs = STAGE == 1 ? (p.n_out + BLOCK_ROWS - 1) / BLOCK_ROWS : (p.n_out + BN - 1) / BN;
   // Routing blocks of 64 rows: a 128-row block holds two of them.  Where both have
@@ -596,6 +599,7 @@ __global__ void __launch_bounds__(NUM_THREADS, 1) moe_rows_kernel(const __grid_c
           }
         }
       }
+      pdl_trigger();  // the last loads are on their way: the next kernel may be scheduled as the CTAs finish
       if (!ok || *abort_flag) {
         const int pending = min(issued, STAGES);
         for (int i = 0; i < pending; ++i) {
@@ -774,8 +778,8 @@ static __global__ void moe_gather_rows_kernel(uint8_t* __restrict__ dst, float* 
                                        const uint8_t* __restrict__ src, const float* __restrict__ src_scale,
                                        const int* __restrict__ sorted_ids, const int* __restrict__ num_valid, int tokens,
                                        int topk, int by_slot, int K_bytes, int rows) {
-  // a GEMM launched as programmatic dependent may start its weight stream now
-  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+  pdl_wait(dst, dst_scale, src, src_scale, sorted_ids, num_valid);
+  pdl_trigger();  // a GEMM launched as programmatic dependent may start its weight stream now
   const int warps_per_block = blockDim.x >> 5;
   const int lane = threadIdx.x & 31;
   const int n_valid = __ldg(num_valid);
@@ -813,8 +817,8 @@ moe_quant_sorted_kernel(uint8_t* __restrict__ y, float* __restrict__ scale, cons
                         const int* __restrict__ sorted_ids, const int* __restrict__ num_valid, int tokens, int topk, int K, int rows) {
   constexpr int VEC = 8, TPR = 32 * WPR;
   __shared__ uint32_t red[8];
-  // a GEMM launched as programmatic dependent may start its weight stream now
-  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+  pdl_wait(y, scale, x, sorted_ids, num_valid);
+  pdl_trigger();  // a GEMM launched as programmatic dependent may start its weight stream now
   const int group = threadIdx.x / TPR, tid = threadIdx.x % TPR;
   const int r = blockIdx.x * (8 / WPR) + group;
   if (r >= rows) return;
@@ -889,6 +893,8 @@ moe_sort_kernel(const ID* __restrict__ topk_ids, const float* __restrict__ topk_
   __shared__ int bins[MOE_SORT_BINS];
   __shared__ int warp_sums[2][32];
   __shared__ int s_start, s_total, s_mine;
+  pdl_wait(topk_ids, topk_weights, sorted_ids, sorted_weights, sorted_expert_ids, post_pad);
+  pdl_trigger();
   const int me = blockIdx.x;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int threads = blockDim.x, warps = threads >> 5;
@@ -995,6 +1001,8 @@ __global__ void __launch_bounds__(256) moe_reduce_kernel(T* __restrict__ y, cons
                                                          const int* __restrict__ expert_mask,
                                                          const int* __restrict__ topk_ids, int num_experts) {
   static_assert(VEC == 2 || VEC == 8, "pairs or 16-byte vectors");
+  pdl_wait(y, x, expert_mask, topk_ids);
+  pdl_trigger();
   const long long t = blockIdx.x;
   const int c = (blockIdx.y * 256 + threadIdx.x) * VEC;
   if (c >= dim) return;

@@ -127,6 +127,7 @@ __global__ void __launch_bounds__(NUM_THREADS, 1) mx_gemm_kernel(const __grid_co
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem_base = *tmem_slot;
+  pdl_wait<>();  // launched as a programmatic dependent: nothing in global memory is touched before this
 
   const int num_m = (p.M + BLOCK_ROWS - 1) / BLOCK_ROWS;
   const int num_n = p.N / BN;
@@ -186,6 +187,7 @@ __global__ void __launch_bounds__(NUM_THREADS, 1) mx_gemm_kernel(const __grid_co
           }
         }
       }
+      pdl_trigger();  // the last loads are on their way: the next kernel may be scheduled as the CTAs finish
       if (!ok || *abort_flag) {
         const int pending = min(issued, STAGES);
         for (int i = 0; i < pending; ++i) {
@@ -379,6 +381,8 @@ __global__ void __launch_bounds__(NUM_THREADS, 1) mx_gemm_kernel(const __grid_co
 // rows of K = 8192 takes 2.0 to 2.4 us, the floor of a launch.
 static __global__ void mx_scale_image_kernel(uint32_t* __restrict__ dst, const uint8_t* __restrict__ src, int rows, int kb32,
                                       int row_tiles) {
+  pdl_wait(dst, src);
+  pdl_trigger();
   const long long total = static_cast<long long>(kb32 / 4) * row_tiles * (MX_SF_ATOM / 4);
   const bool aligned = (reinterpret_cast<uintptr_t>(src) & 3u) == 0;  // rows of kb32 bytes, a multiple of four
   for (long long i = blockIdx.x * static_cast<long long>(blockDim.x) + threadIdx.x; i < total;

@@ -82,6 +82,8 @@ template <typename TIn, int FMT>
 __global__ void __launch_bounds__(256) mx_quant_kernel(uint8_t* __restrict__ codes, uint8_t* __restrict__ scale,
                                                        uint8_t* __restrict__ raw, const TIn* __restrict__ x,
                                                        long long units) {
+  pdl_wait(codes, scale, raw, x);
+  pdl_trigger();
   const long long u = blockIdx.x * 256ll + threadIdx.x;
   // units is even (whole blocks of 32), so both lanes of a pair are in or out together; the others of the
   // warp stay for the shuffle
@@ -169,6 +171,8 @@ __global__ void __launch_bounds__(256) mx_quant_kernel(uint8_t* __restrict__ cod
 // followed by 4 bytes of padding.  One thread per block of 32 codes.
 static __global__ void __launch_bounds__(256) mx_fp6_containers_kernel(uint4* __restrict__ dst, const uint4* __restrict__ src,
                                                                        long long blocks) {
+  pdl_wait(dst, src);
+  pdl_trigger();
   for (long long i = blockIdx.x * 256ll + threadIdx.x; i < blocks; i += gridDim.x * 256ll) {
     const uint4 a = __ldg(src + 2 * i);
     const uint2 b = __ldg(reinterpret_cast<const uint2*>(src + 2 * i + 1));

@@ -363,6 +363,20 @@ __device__ __forceinline__ void tmem_ld_x16(uint32_t taddr, uint32_t (&r)[16]) {
 }
 __device__ __forceinline__ void tmem_ld_wait() { asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory"); }
 
+// ---- programmatic dependent launch ----
+// Wait until the kernels this one depends on have completed and their writes are visible; nothing happens
+// for a kernel launched without the attribute.  The pointers pass through the statement, so that no load
+// through them can be scheduled ahead of it.
+template <typename... P>
+__device__ __forceinline__ void pdl_wait(P&... ptrs) {
+  asm volatile("griddepcontrol.wait;" ::: "memory");
+  auto pass = [](auto& p) { asm volatile("" : "+l"(p)::"memory"); };
+  (pass(ptrs), ...);
+}
+// The next kernel on the stream may be scheduled once every CTA of this one has come here or is gone.  Only
+// after pdl_wait: a kernel that started early can then count on everything before its direct predecessor.
+__device__ __forceinline__ void pdl_trigger() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+
 // ---- thread-block clusters ----
 __device__ __forceinline__ uint32_t cluster_ctarank() {
   uint32_t r;

@@ -18,6 +18,7 @@
 #pragma once
 #include <cstdint>
 #include <type_traits>
+#include "ptx.cuh"
 #include <cuda_bf16.h>
 #include <cuda_fp16.h>
 #include <cuda_fp8.h>
@@ -270,8 +271,8 @@ __global__ void __launch_bounds__(256) pertoken_quant_row_kernel(uint8_t* __rest
                                                                  const TIn* __restrict__ x, int rows, int K) {
   constexpr int VEC = QuantIn<TIn>::VEC;
   __shared__ uint32_t red[8];
-  // a GEMM launched as programmatic dependent may set itself up now (it waits for this grid before it reads)
-  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+  pdl_wait(x, y, scale);
+  pdl_trigger();
   const int group = threadIdx.x / (32 * WPR), tid = threadIdx.x % (32 * WPR);
   const int r = blockIdx.x * (8 / WPR) + group;
   if (r >= rows) return;
@@ -325,6 +326,8 @@ __global__ void __launch_bounds__(256) pertoken_quant_kernel(uint8_t* __restrict
   constexpr float QMAX = FP8 ? 448.0f : 127.0f;
   __shared__ float warp_max[8];
   __shared__ float row_scale;
+  pdl_wait(x, y, scale);
+  pdl_trigger();
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   for (int r = blockIdx.x; r < rows; r += gridDim.x) {
     const TIn* xr = x + static_cast<size_t>(r) * K;

@@ -97,7 +97,7 @@ int launch_moe_rows(const CUtensorMap& tmA, const MoeParams& p, int blocks, cuda
   const int pairs = STAGE == 1 ? (p.n_out + BLOCK_ROWS - 1) / BLOCK_ROWS : (p.n_out + MOE_ROWS_BN - 1) / MOE_ROWS_BN;
   const long long items = row_blocks * pairs;
   const int grid = static_cast<int>(items < sms ? items : sms);
-  CUDA_TRY(host::launch_dependent(kernel, dim3(grid), NUM_THREADS, MoeRowsSmem::TOTAL, s, tmA, p));
+  CUDA_TRY(host::launch_dependent(kernel, dim3(grid), MOE_ROWS_THREADS, MoeRowsSmem::TOTAL, s, tmA, p));
   return FLYB200_OK;
 }
 
@@ -158,13 +158,14 @@ cudaError_t launch_moe_reduce(void* y, const void* x, int tokens, int topk, int 
                        int num_experts, cudaStream_t s) {
   T* yt = static_cast<T*>(y);
   const T* xt = static_cast<const T*>(x);
-  if (dim % 8 == 0 && aligned16(y) && aligned16(x)) {
-    const dim3 grid(tokens, (dim / 8 + 255) / 256);
-    return host::launch_dependent(moe_reduce_kernel<T, 8>, grid, 256, 0, s, yt, xt, topk, dim, expert_mask, topk_ids, num_experts);
-  } else {
-    const dim3 grid(tokens, (dim / 2 + 255) / 256);
-    return host::launch_dependent(moe_reduce_kernel<T, 2>, grid, 256, 0, s, yt, xt, topk, dim, expert_mask, topk_ids, num_experts);
-  }
+  const bool vec = dim % 8 == 0 && aligned16(y) && aligned16(x);
+  const int vecs = dim / (vec ? 8 : 2);
+  auto launch = [&](auto kernel, int unroll) {
+    return host::launch_dependent(kernel, dim3(tokens, (vecs + 256 * unroll - 1) / (256 * unroll)), 256, 0, s, yt, xt, topk, dim, expert_mask,
+                                  topk_ids, num_experts);
+  };
+  if (!vec) return launch(moe_reduce_kernel<T, 2, 1>, 1);
+  return vecs > 256 && tokens > 256 ? launch(moe_reduce_kernel<T, 8, 2>, 2) : launch(moe_reduce_kernel<T, 8, 1>, 1);
 }
 
 }  // namespace

@@ -40,7 +40,7 @@ int launch_mx(const CUtensorMap& tmA, const MxParams& p, cudaStream_t s) {
   cudaLaunchConfig_t cfg;
   memset(&cfg, 0, sizeof(cfg));
   cfg.gridDim = dim3(static_cast<unsigned>(SPLIT ? tiles * p.split : tiles < sms ? tiles : sms), 1, 1);
-  cfg.blockDim = dim3(NUM_THREADS, 1, 1);
+  cfg.blockDim = dim3(MX_THREADS, 1, 1);
   cfg.dynamicSmemBytes = Smem::TOTAL;
   cfg.stream = s;
   cudaLaunchAttribute attrs[2];
@@ -75,7 +75,11 @@ namespace {
 // CTAs (one per 128 channels) fit one round: on wider outputs its later rounds run part empty and the
 // persistent large-M kernel is 20-45 % faster (MXFP8 128 x 28672 x 8192: 43 against 66 us; MXFP4 128 x
 // 57344 x 8192: 51 against 90 us).  FLYB200_MX_SMALL=0 / 1 forces the choice.
-bool mx_small_m(int M, int N) {
+// With more than half as many channel tiles as SMs the small-M kernel has no K split to balance its token
+// tile with, and from 65 tokens up (MXFP4, half the weight bytes: 33) the large-M kernel is ahead: MXFP8 96 x
+// 12288 x 4096 16.6 against 20.1 us, 128 x 16384 x 8192 29.0 / 34.7 (64: 16.2 / 16.4, 28 / 28); MXFP4 128 x 12288 x
+// 4096 11.5 / 18.3, 64 x 10240 x 8192 16.8 / 18.1 (16: 11.4 / 9.7).
+bool mx_small_m(int M, int N, bool fp4 = false) {
   if (M > 128) return false;
   if (const char* e = getenv("FLYB200_MX_SMALL")) {
     if (e[0] == '0') return false;
@@ -83,7 +87,8 @@ bool mx_small_m(int M, int N) {
   }
   int sms = 0;
   if (flyb200::host::sm_count(&sms) != FLYB200_OK) return true;
-  return (N + 127) / 128 <= sms;
+  const int tiles = (N + 127) / 128;
+  return tiles <= sms && (2 * tiles <= sms || M <= (fp4 ? 32 : 64));
 }
 // The mixed kinds (byte containers) the same way, except for 65..128 tokens where the large-M kernel can
 // only split K in two or not at all: there the two are even or the large-M kernel is ahead.  Small-M /
@@ -266,7 +271,7 @@ int flyb200_gemm_mxfp4(void* c, const void* a, const void* w_shuf, const void* s
     return FLYB200_E_BAD_ALIGN;
   if (M == 0) return FLYB200_OK;
   // up to 128 tokens: a weight stream (half the bytes of 8-bit codes), run by the small-M kernel
-  if (mx_small_m(M, N))
+  if (mx_small_m(M, N, true))
     return host::gemm_mx_small(c, a, w_shuf, scale_a_image, scale_w_image, M, N, K / 2,
                                out_dtype == FLYB200_OUT_FP16 ? 1 : 0, true, stream);
   MxParams p;

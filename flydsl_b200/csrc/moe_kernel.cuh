@@ -391,13 +391,16 @@ constexpr int MOE_ROWS_STAGES = 4;
 constexpr int MOE_ROWS_BN = 2 * BLOCK_ROWS;
 constexpr int MOE_ROWS_GROUP = 32;  // row blocks per rasterisation group (16 MiB of activations at K = 4096)
 
+constexpr int STORE_STAGE = 32 * 64;  // shared memory of a warp for store_rows32, bytes
+constexpr int MOE_ROWS_THREADS = 64 + 8 * 32;  // producer, MMA issuer, eight epilogue warps
 struct MoeRowsSmem {
   static constexpr int A_STAGE = BLOCK_ROWS * KBLOCK_BYTES;
   static constexpr int B_STAGE = MOE_ROWS_BN * KBLOCK_BYTES;
   static constexpr int OFF_A = 0;
   static constexpr int OFF_B = OFF_A + MOE_ROWS_STAGES * A_STAGE;
-  static constexpr int OFF_SW = OFF_B + MOE_ROWS_STAGES * B_STAGE;   // 4 warps x 256 weight scales
-  static constexpr int OFF_BAR = OFF_SW + 4 * MOE_ROWS_BN * 4;       // full[S], empty[S], tfull[2], tempty[2]
+  static constexpr int OFF_C = OFF_B + MOE_ROWS_STAGES * B_STAGE;    // 8 warps x one store stage
+  static constexpr int OFF_SW = OFF_C + 8 * STORE_STAGE;             // 8 warps x 128 weight scales
+  static constexpr int OFF_BAR = OFF_SW + 8 * BLOCK_ROWS * 4;        // full[S], empty[S], tfull[2], tempty[2]
   static constexpr int OFF_MISC = OFF_BAR + 8 * (2 * MOE_ROWS_STAGES + 4);
   static constexpr int TOTAL = OFF_MISC + 16;
 };
@@ -421,39 +424,62 @@ __device__ __forceinline__ void moe_red16(void* dst, const uint32_t (&v)[4]) {
   }
 }
 
-// 32 consecutive channels of one output row in 16-byte accesses; n_ok (a multiple of 16) of them exist.
-// Rows are multiples of 16 channels, so every access is 16-byte aligned.  Accumulating one packed pair
-// at a time bound the down projection: 515 tokens x top-4 x 2048 fp16 (int8, K = 1408) 94.4 us, now 22.2.
+// 32 rows (one per lane) x 32 consecutive channels of output, n_ok (a multiple of 8) of them existing,
+// in 16-byte accesses.  The lanes' rows lie apart in memory, so a lane that wrote its own row would touch a
+// line of its own with every access; the chunk is turned in 2 KiB of shared memory instead (swizzled, no bank
+// conflicts) and four lanes write 64 contiguous bytes of a row: with that and eight epilogue warps instead of
+// four the down projection of 4096 tokens x top-2 (K = 2048) goes from 70.9 to 67.0 us, the layer from 277 to 274,
+// MXFP8 600 x 1792 x 2048 from 9.6 to 8.2, 384 x 1024 x 4096 from 10.1 to 9.1, 256 x 4096 x 14336 from 25.9 to 24.5.  `rows[k]`: output row of lane 8 k + lane / 4, or
+// negative for none.  Rows are multiples of 16 channels, so every access is 16-byte aligned.  Accumulating one
+// packed pair at a time bound the down projection (515 tokens x top-4 x 2048 fp16, int8, K = 1408: 94.4 us).
 template <int OUTMODE, bool ACCUM>
-__device__ __forceinline__ void moe_store_row32(void* out, size_t elem, const float (&y)[32], int n_ok) {
+__device__ __forceinline__ void store_rows32(void* out, const long long (&rows)[4], int n_out, int col, const float (&y)[32], int n_ok,
+                                             uint32_t stage, int lane) {
   constexpr int PER = OUTMODE == MOE_OUT_F32 ? 4 : 8;  // channels per 16 bytes
-  unsigned char* dst = static_cast<unsigned char*>(out) + elem * (16 / PER);
+  constexpr int COLS = 4 * PER;                        // channels turned at a time: 64 bytes per row
+  const int piece = lane & 3;
+  const uint32_t mine = stage + static_cast<uint32_t>(lane * 64);
 #pragma unroll
-  for (int g = 0; g < 32 / PER; ++g) {
-    if (g * PER >= n_ok) break;
-    uint32_t v[4];
+  for (int c0 = 0; c0 < 32; c0 += COLS) {
 #pragma unroll
-    for (int i = 0; i < 4; ++i) {
-      if constexpr (OUTMODE == MOE_OUT_F32) {
-        v[i] = __float_as_uint(y[g * PER + i]);
-      } else if constexpr (OUTMODE == MOE_OUT_BF16) {
-        const __nv_bfloat162 h = __floats2bfloat162_rn(y[g * PER + 2 * i], y[g * PER + 2 * i + 1]);
-        v[i] = *reinterpret_cast<const uint32_t*>(&h);
+    for (int g = 0; g < 4; ++g) {
+      uint32_t v[4];
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+        const int e = c0 + g * PER;
+        if constexpr (OUTMODE == MOE_OUT_F32) {
+          v[i] = __float_as_uint(y[e + i]);
+        } else if constexpr (OUTMODE == MOE_OUT_BF16) {
+          const __nv_bfloat162 h = __floats2bfloat162_rn(y[e + 2 * i], y[e + 2 * i + 1]);
+          v[i] = *reinterpret_cast<const uint32_t*>(&h);
+        } else {
+          const __half2 h = __floats2half2_rn(y[e + 2 * i], y[e + 2 * i + 1]);
+          v[i] = *reinterpret_cast<const uint32_t*>(&h);
+        }
+      }
+      st_smem_v4(mine + static_cast<uint32_t>((g ^ ((lane >> 1) & 3)) << 4), v[0], v[1], v[2], v[3]);
+    }
+    __syncwarp();
+    const bool exists = c0 + piece * PER < n_ok;
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+      const int r = 8 * k + (lane >> 2);
+      const uint4 q = ld_smem_v4(stage + static_cast<uint32_t>(r * 64 + ((piece ^ ((r >> 1) & 3)) << 4)));
+      if (!exists || rows[k] < 0) continue;
+      unsigned char* dst = static_cast<unsigned char*>(out) + (rows[k] * n_out + col + c0 + piece * PER) * (16 / PER);
+      if constexpr (ACCUM) {
+        const uint32_t v[4] = {q.x, q.y, q.z, q.w};
+        moe_red16<OUTMODE>(dst, v);
       } else {
-        const __half2 h = __floats2half2_rn(y[g * PER + 2 * i], y[g * PER + 2 * i + 1]);
-        v[i] = *reinterpret_cast<const uint32_t*>(&h);
+        *reinterpret_cast<uint4*>(dst) = q;
       }
     }
-    if constexpr (ACCUM) {
-      moe_red16<OUTMODE>(dst + 16 * g, v);
-    } else {
-      *reinterpret_cast<uint4*>(dst + 16 * g) = make_uint4(v[0], v[1], v[2], v[3]);
-    }
+    __syncwarp();  // the stage is free again
   }
 }
 
 template <int KIND, int STAGE, int OUTMODE, bool ACCUM>
-__global__ void __launch_bounds__(NUM_THREADS, 1) moe_rows_kernel(const __grid_constant__ CUtensorMap tmA,
+__global__ void __launch_bounds__(MOE_ROWS_THREADS, 1) moe_rows_kernel(const __grid_constant__ CUtensorMap tmA,
                                                                   const MoeParams p) {
   static_assert(STAGE == 2 || !ACCUM, "only the down projection accumulates");
   using L = MoeRowsSmem;
@@ -482,7 +508,7 @@ __global__ void __launch_bounds__(NUM_THREADS, 1) moe_rows_kernel(const __grid_c
     }
     for (int s = 0; s < 2; ++s) {
       mbar_init(bar_tfull + 8 * s, 1);
-      mbar_init(bar_tempty + 8 * s, 4);
+      mbar_init(bar_tempty + 8 * s, 8);
     }
     abort_flag[0] = 0;
     abort_flag[1] = 0;
@@ -659,8 +685,12 @@ __global__ void __launch_bounds__(NUM_THREADS, 1) moe_rows_kernel(const __grid_c
     }
   } else {
     // ------------------------------ epilogue ------------------------------
+    // Eight warps, two per TMEM lane quadrant; of the 128 channels of each tile (stage 1) or of the two
+    // tiles (stage 2) a warp takes one half.
     const int q = warp & 3;  // TMEM lane quadrant this warp may read
-    float* sw_s = reinterpret_cast<float*>(smem_raw + L::OFF_SW) + (warp - 2) * BN;
+    const int half = (warp - 2) >> 2;
+    float* sw_s = reinterpret_cast<float*>(smem_raw + L::OFF_SW) + (warp - 2) * BLOCK_ROWS;
+    const uint32_t stage_c = smem_base + L::OFF_C + (warp - 2) * STORE_STAGE;
     int acc = 0;
     uint32_t acc_phase = 0;
     bool ok = true;
@@ -685,14 +715,18 @@ __global__ void __launch_bounds__(NUM_THREADS, 1) moe_rows_kernel(const __grid_c
           if (p.doweight) tw = __ldg(p.sorted_w + srow);
         }
       }
-      // weight scales of the 256 columns, one copy per warp
+      long long rows[4];  // output rows this lane stores pieces of
+#pragma unroll
+      for (int k = 0; k < 4; ++k) rows[k] = __shfl_sync(0xffffffffu, orow, 8 * k + (lane >> 2));
+      // weight scales of this warp's columns: stage 1 64 gate channels, then the same 64 up channels
       const float* sw_expert = p.sw + static_cast<size_t>(expert) * p.n_expert;
       __syncwarp();
 #pragma unroll
-      for (int i = 0; i < BN / 32; ++i) {
+      for (int i = 0; i < BLOCK_ROWS / 32; ++i) {
         const int c = i * 32 + lane;
-        const int h = c >> 7, cc = c & 127;
-        sw_s[c] = cc < n_valid[h] ? __ldg(sw_expert + w_row[h] + cc) : 0.0f;
+        const bool second = STAGE == 1 ? c >= 64 : half == 1;
+        const int cc = STAGE == 1 ? half * 64 + (c & 63) : c;
+        sw_s[c] = cc < (second ? n_valid[1] : n_valid[0]) ? __ldg(sw_expert + (second ? w_row[1] : w_row[0]) + cc) : 0.0f;
       }
       __syncwarp();
       if (!mbar_wait(bar_tfull + 8 * acc, acc_phase, abort_flag)) {
@@ -704,14 +738,14 @@ __global__ void __launch_bounds__(NUM_THREADS, 1) moe_rows_kernel(const __grid_c
       const uint32_t t_row = tmem_base + (static_cast<uint32_t>(q * 32) << 16) + static_cast<uint32_t>(acc * BN);
       auto to_f = [](uint32_t r) { return KT::is_int ? static_cast<float>(static_cast<int32_t>(r)) : __uint_as_float(r); };
       if constexpr (STAGE == 1) {
-        const int col0 = pair * BLOCK_ROWS;
 #pragma unroll 1
-        for (int c0 = 0; c0 < BLOCK_ROWS; c0 += 32) {
+        for (int c0 = 0; c0 < 64; c0 += 32) {
+          const int cc = half * 64 + c0;  // channel inside the tile
           uint32_t rg[32], ru[32];
-          tmem_ld_x32(t_row + c0, rg);
-          tmem_ld_x32(t_row + BLOCK_ROWS + c0, ru);
+          tmem_ld_x32(t_row + cc, rg);
+          tmem_ld_x32(t_row + BLOCK_ROWS + cc, ru);
           tmem_ld_wait();
-          if (c0 + 32 >= BLOCK_ROWS) {  // last read of this accumulator: hand it back to the MMA warp
+          if (c0 + 32 >= 64) {  // last read of this accumulator: hand it back to the MMA warp
             tc_fence_before();
             __syncwarp();
             if (lane == 0) mbar_arrive(bar_tempty + 8 * acc);
@@ -720,23 +754,21 @@ __global__ void __launch_bounds__(NUM_THREADS, 1) moe_rows_kernel(const __grid_c
 #pragma unroll
           for (int j = 0; j < 32; ++j) {
             const float g = (to_f(rg[j]) * sw_s[c0 + j]) * sa;
-            const float u = (to_f(ru[j]) * sw_s[BLOCK_ROWS + c0 + j]) * sa;
+            const float u = (to_f(ru[j]) * sw_s[64 + c0 + j]) * sa;
             float v = silu_f32(g) * u;
             if (p.doweight) v *= tw;
             y[j] = v;
           }
-          const int n_ok = min(32, n_valid[0] - c0);
-          if (orow >= 0 && n_ok > 0)
-            moe_store_row32<OUTMODE, ACCUM>(p.out, static_cast<size_t>(orow) * p.n_out + col0 + c0, y, n_ok);
+          const int n_ok = min(32, n_valid[0] - cc);
+          if (n_ok > 0) store_rows32<OUTMODE, ACCUM>(p.out, rows, p.n_out, pair * BLOCK_ROWS + cc, y, n_ok, stage_c, lane);
         }
       } else {
-        const int col0 = pair * BN;
 #pragma unroll 1
-        for (int c0 = 0; c0 < BN; c0 += 32) {
+        for (int c0 = 0; c0 < BLOCK_ROWS; c0 += 32) {
           uint32_t ra[32];
-          tmem_ld_x32(t_row + c0, ra);
+          tmem_ld_x32(t_row + half * BLOCK_ROWS + c0, ra);
           tmem_ld_wait();
-          if (c0 + 32 >= BN) {
+          if (c0 + 32 >= BLOCK_ROWS) {
             tc_fence_before();
             __syncwarp();
             if (lane == 0) mbar_arrive(bar_tempty + 8 * acc);
@@ -747,10 +779,8 @@ __global__ void __launch_bounds__(NUM_THREADS, 1) moe_rows_kernel(const __grid_c
             const float v = (to_f(ra[j]) * sw_s[c0 + j]) * sa;
             y[j] = p.doweight ? v * tw : v;
           }
-          const int h = c0 >> 7;
-          const int n_ok = min(32, n_valid[h] - (c0 & 127));
-          if (orow >= 0 && n_ok > 0)
-            moe_store_row32<OUTMODE, ACCUM>(p.out, static_cast<size_t>(orow) * p.n_out + col0 + c0, y, n_ok);
+          const int n_ok = min(32, (half ? n_valid[1] : n_valid[0]) - c0);
+          if (n_ok > 0) store_rows32<OUTMODE, ACCUM>(p.out, rows, p.n_out, pair * BN + half * BLOCK_ROWS + c0, y, n_ok, stage_c, lane);
         }
       }
       acc ^= 1;
@@ -992,11 +1022,12 @@ moe_sort_kernel(const ID* __restrict__ topk_ids, const float* __restrict__ topk_
 // (the expert-parallel validity mask of kernels/moe/moe_gemm_2stage/moe_reduce.py:3-7
 // in the reference): rows of routes that another rank serves are never read.
 //
-// Memory-bound.  blockIdx.x is the token, a thread owns VEC neighbouring columns: no
-// division by `dim`, and the loads of four slots are in flight together.  VEC = 8 (16-byte
-// accesses) wherever `dim` and the bases allow it, else pairs.  Measured, 4096 tokens x top-2
-// x 4096 bf16 (101 MB): 22.3 us = 4.5 TB/s; one pair per thread with a 64-bit division each 66.4 us.
-template <typename T, int VEC>
+// Memory-bound.  blockIdx.x is the token, a thread owns UNROLL x VEC columns (vectors 256 apart): no division by
+// `dim`, and the loads of up to four slots of all its vectors are in flight together.  VEC = 8 (16-byte
+// accesses) wherever `dim` and the bases allow it, else pairs; UNROLL = 2 where a row holds enough vectors, which
+// halves the blocks.  Measured, 4096 tokens x top-2 x 4096 bf16 (101 MB): 21 us
+// = 4.8 TB/s; one vector per thread 22.3, one pair per thread with a 64-bit division each 66.4.
+template <typename T, int VEC, int UNROLL>
 __global__ void __launch_bounds__(256) moe_reduce_kernel(T* __restrict__ y, const T* __restrict__ x, int topk, int dim,
                                                          const int* __restrict__ expert_mask,
                                                          const int* __restrict__ topk_ids, int num_experts) {
@@ -1004,14 +1035,17 @@ __global__ void __launch_bounds__(256) moe_reduce_kernel(T* __restrict__ y, cons
   pdl_wait(y, x, expert_mask, topk_ids);
   pdl_trigger();
   const long long t = blockIdx.x;
-  const int c = (blockIdx.y * 256 + threadIdx.x) * VEC;
-  if (c >= dim) return;
-  float sum[VEC];
+  const int first = (blockIdx.y * UNROLL * 256 + threadIdx.x) * VEC;
+  constexpr int STEP = 256 * VEC;  // columns between the vectors of a thread
+  float sum[UNROLL][VEC];
 #pragma unroll
-  for (int i = 0; i < VEC; ++i) sum[i] = 0.0f;
+  for (int u = 0; u < UNROLL; ++u) {
+#pragma unroll
+    for (int i = 0; i < VEC; ++i) sum[u][i] = 0.0f;
+  }
   constexpr int W = VEC / 2;  // 32-bit words of a vector
   for (int s0 = 0; s0 < topk; s0 += 4) {
-    uint32_t v[4][W];
+    uint32_t v[4][UNROLL][W];
     bool on[4];
 #pragma unroll
     for (int j = 0; j < 4; ++j) {
@@ -1025,46 +1059,58 @@ __global__ void __launch_bounds__(256) moe_reduce_kernel(T* __restrict__ y, cons
 #pragma unroll
     for (int j = 0; j < 4; ++j) {
       if (!on[j]) continue;
-      const T* src = x + (t * topk + s0 + j) * dim + c;
-      if constexpr (VEC == 8) {
-        const uint4 q = __ldg(reinterpret_cast<const uint4*>(src));
-        v[j][0] = q.x, v[j][1] = q.y, v[j][2] = q.z, v[j][3] = q.w;
-      } else {
-        v[j][0] = __ldg(reinterpret_cast<const uint32_t*>(src));
+#pragma unroll
+      for (int u = 0; u < UNROLL; ++u) {
+        if (first + u * STEP >= dim) continue;
+        const T* src = x + (t * topk + s0 + j) * dim + first + u * STEP;
+        if constexpr (VEC == 8) {
+          const uint4 q = __ldg(reinterpret_cast<const uint4*>(src));
+          v[j][u][0] = q.x, v[j][u][1] = q.y, v[j][u][2] = q.z, v[j][u][3] = q.w;
+        } else {
+          v[j][u][0] = __ldg(reinterpret_cast<const uint32_t*>(src));
+        }
       }
     }
 #pragma unroll
     for (int j = 0; j < 4; ++j) {
       if (!on[j]) continue;
 #pragma unroll
-      for (int i = 0; i < W; ++i) {
-        float2 f;
-        if constexpr (std::is_same<T, __nv_bfloat16>::value) {
-          f = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&v[j][i]));
-        } else {
-          f = __half22float2(*reinterpret_cast<const __half2*>(&v[j][i]));
+      for (int u = 0; u < UNROLL; ++u) {
+#pragma unroll
+        for (int i = 0; i < W; ++i) {
+          float2 f;
+          if constexpr (std::is_same<T, __nv_bfloat16>::value) {
+            f = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&v[j][u][i]));
+          } else {
+            f = __half22float2(*reinterpret_cast<const __half2*>(&v[j][u][i]));
+          }
+          sum[u][2 * i] += f.x;
+          sum[u][2 * i + 1] += f.y;
         }
-        sum[2 * i] += f.x;
-        sum[2 * i + 1] += f.y;
       }
     }
   }
-  uint32_t out[W];
 #pragma unroll
-  for (int i = 0; i < W; ++i) {
-    if constexpr (std::is_same<T, __nv_bfloat16>::value) {
-      const __nv_bfloat162 h = __floats2bfloat162_rn(sum[2 * i], sum[2 * i + 1]);
-      out[i] = *reinterpret_cast<const uint32_t*>(&h);
-    } else {
-      const __half2 h = __floats2half2_rn(sum[2 * i], sum[2 * i + 1]);
-      out[i] = *reinterpret_cast<const uint32_t*>(&h);
+  for (int u = 0; u < UNROLL; ++u) {
+    const int c = first + u * STEP;
+    if (c >= dim) break;
+    uint32_t out[W];
+#pragma unroll
+    for (int i = 0; i < W; ++i) {
+      if constexpr (std::is_same<T, __nv_bfloat16>::value) {
+        const __nv_bfloat162 h = __floats2bfloat162_rn(sum[u][2 * i], sum[u][2 * i + 1]);
+        out[i] = *reinterpret_cast<const uint32_t*>(&h);
+      } else {
+        const __half2 h = __floats2half2_rn(sum[u][2 * i], sum[u][2 * i + 1]);
+        out[i] = *reinterpret_cast<const uint32_t*>(&h);
+      }
     }
-  }
-  T* dst = y + t * dim + c;
-  if constexpr (VEC == 8) {
-    *reinterpret_cast<uint4*>(dst) = make_uint4(out[0], out[1], out[2], out[3]);
-  } else {
-    *reinterpret_cast<uint32_t*>(dst) = out[0];
+    T* dst = y + t * dim + c;
+    if constexpr (VEC == 8) {
+      *reinterpret_cast<uint4*>(dst) = make_uint4(out[0], out[1], out[2], out[3]);
+    } else {
+      *reinterpret_cast<uint32_t*>(dst) = out[0];
+    }
   }
 }
 

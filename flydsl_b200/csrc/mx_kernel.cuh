@@ -27,7 +27,7 @@
 // epilogue is exposed; 4 stages) for long K, where the epilogue is a small part
 // of a tile.  Threads as in the large-M kernel: warp 0 producer, warp 1 MMA
 // (copies the two scale atoms to TMEM, then issues the four MMAs of a k-block),
-// warps 2..5 epilogue (thread = token row, 64 contiguous output bytes per chunk).
+// warps 2..9 epilogue (thread = token row, two warps per 32 rows; stores turned in shared memory, store_rows32).
 //
 // SPLIT: where the 128 x 128 tiles leave at least half of the SMs idle, a cluster of two, four or eight
 // CTAs shares a tile, each with a part of K.  Every CTA parks its fp32 partial tile in its shared memory
@@ -39,6 +39,8 @@
 
 namespace flyb200 {
 
+
+constexpr int MX_THREADS = 64 + 8 * 32;  // producer, MMA issuer, eight epilogue warps
 
 struct MxParams {
   const uint8_t* w;    // weight codes, preshuffled image
@@ -71,13 +73,14 @@ struct MxSmem {
   static constexpr int OFF_B = OFF_A + STAGES * A_STAGE;
   static constexpr int OFF_SFA = OFF_B + STAGES * B_STAGE;
   static constexpr int OFF_SFB = OFF_SFA + STAGES * SFA_STAGE;
-  static constexpr int OFF_BAR = OFF_SFB + STAGES * SFB_STAGE;  // full[S], empty[S], tfull[2], tempty[2]
+  static constexpr int OFF_C = OFF_SFB + STAGES * SFB_STAGE;    // 8 warps x one store stage
+  static constexpr int OFF_BAR = OFF_C + 8 * STORE_STAGE;       // full[S], empty[S], tfull[2], tempty[2]
   static constexpr int OFF_MISC = OFF_BAR + 8 * (2 * STAGES + 4);
   static constexpr int TOTAL = OFF_MISC + 16;
 };
 
 template <int OUTMODE, int BN, bool FP4 = false, bool SPLIT = false>
-__global__ void __launch_bounds__(NUM_THREADS, 1) mx_gemm_kernel(const __grid_constant__ CUtensorMap tmA, const MxParams p) {
+__global__ void __launch_bounds__(MX_THREADS, 1) mx_gemm_kernel(const __grid_constant__ CUtensorMap tmA, const MxParams p) {
   using L = MxSmem<BN, FP4>;
   constexpr int STAGES = L::STAGES;
   constexpr int NACC = L::NACC;
@@ -107,7 +110,7 @@ __global__ void __launch_bounds__(NUM_THREADS, 1) mx_gemm_kernel(const __grid_co
     }
     for (int s = 0; s < 2; ++s) {
       mbar_init(bar_tfull + 8 * s, 1);
-      mbar_init(bar_tempty + 8 * s, 4);
+      mbar_init(bar_tempty + 8 * s, 8);
     }
     abort_flag[0] = 0;
     abort_flag[1] = 0;
@@ -268,14 +271,16 @@ __global__ void __launch_bounds__(NUM_THREADS, 1) mx_gemm_kernel(const __grid_co
     }
   } else {
     // ------------------------------ epilogue ------------------------------
+    // eight warps: two per TMEM lane quadrant, each with one half of the columns
     const int q = warp & 3;
+    const int first_col = ((warp - 2) >> 2) * (BN / 2);
+    const uint32_t stage_c = smem_base + L::OFF_C + (warp - 2) * STORE_STAGE;
     int acc = 0;
     uint32_t acc_phase = 0;
     bool ok = true;
     for (int t = tile0; t < num_tiles && ok; t += tile_step) {
       int m_blk, n_blk;
       tile_coords(t, m_blk, n_blk);
-      const int row = m_blk * BLOCK_ROWS + q * 32 + lane;
       if (!mbar_wait(bar_tfull + 8 * acc, acc_phase, abort_flag)) {
         if (lane == 0) report_failure(p.status, ST_TIMEOUT, abort_flag);
         ok = false;
@@ -288,7 +293,7 @@ __global__ void __launch_bounds__(NUM_THREADS, 1) mx_gemm_kernel(const __grid_co
         // read it): sixteen bytes of row r, columns 4 c ..., at (c * 128 + r) * 16, conflict-free.
         static_assert(BLOCK_ROWS * BN * 4 <= L::OFF_SFA, "the partial tile must fit into the ring");
 #pragma unroll 1
-        for (int c0 = 0; c0 < BN; c0 += 64) {
+        for (int c0 = first_col; c0 < first_col + BN / 2; c0 += 64) {
           uint32_t r0[32], r1[32];
           tmem_ld_x32(t_row + c0, r0);
           tmem_ld_x32(t_row + c0 + 32, r1);
@@ -301,27 +306,30 @@ __global__ void __launch_bounds__(NUM_THREADS, 1) mx_gemm_kernel(const __grid_co
           }
         }
       } else {
-        // 64 columns per TMEM wait, and each lane then writes one full 128-byte line of its output row
+        long long rows[4];  // output rows this lane stores pieces of
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+          const int r = m_blk * BLOCK_ROWS + q * 32 + 8 * k + (lane >> 2);
+          rows[k] = r < p.M ? r : -1;
+        }
 #pragma unroll 1
-        for (int c0 = 0; c0 < BN; c0 += 64) {
+        for (int c0 = first_col; c0 < first_col + BN / 2; c0 += 64) {  // 64 columns per TMEM wait
           uint32_t r0[32], r1[32];
           tmem_ld_x32(t_row + c0, r0);
           tmem_ld_x32(t_row + c0 + 32, r1);
           tmem_ld_wait();
-          if (c0 + 64 >= BN) {  // last read of this accumulator: hand it back to the MMA warp
+          if (c0 + 64 >= first_col + BN / 2) {  // last read of this accumulator: hand it back to the MMA warp
             tc_fence_before();
             __syncwarp();
             if (lane == 0) mbar_arrive(bar_tempty + 8 * acc);
           }
-          if (row < p.M) {
-            float y[32];
+          float y[32];
 #pragma unroll
-            for (int j = 0; j < 32; ++j) y[j] = __uint_as_float(r0[j]);
-            moe_store_row32<OUTMODE, false>(p.c, static_cast<size_t>(row) * p.N + n_blk * BN + c0, y, 32);
+          for (int j = 0; j < 32; ++j) y[j] = __uint_as_float(r0[j]);
+          store_rows32<OUTMODE, false>(p.c, rows, p.N, n_blk * BN + c0, y, 32, stage_c, lane);
 #pragma unroll
-            for (int j = 0; j < 32; ++j) y[j] = __uint_as_float(r1[j]);
-            moe_store_row32<OUTMODE, false>(p.c, static_cast<size_t>(row) * p.N + n_blk * BN + c0 + 32, y, 32);
-          }
+          for (int j = 0; j < 32; ++j) y[j] = __uint_as_float(r1[j]);
+          store_rows32<OUTMODE, false>(p.c, rows, p.N, n_blk * BN + c0 + 32, y, 32, stage_c, lane);
         }
       }
       acc = (acc + 1) % NACC;
@@ -334,34 +342,36 @@ __global__ void __launch_bounds__(NUM_THREADS, 1) mx_gemm_kernel(const __grid_co
     __syncwarp();
     cluster_sync_all();
     if (warp >= 2) {
-      const int trow = (warp & 3) * 32 + lane;
+      const int q = warp & 3;
+      const uint32_t stage_c = smem_base + L::OFF_C + (warp - 2) * STORE_STAGE;
       int m_blk, n_blk;
       tile_coords(tile0, m_blk, n_blk);
-      const int row = m_blk * BLOCK_ROWS + trow;
-      const int share = BN / p.split;  // columns summed and stored by this CTA: 64, 32 or 16
-      for (int c0 = rank * share; c0 < (rank + 1) * share; c0 += 32) {
-        const int n_ok = min(32, share);
-        float y[32];
+      long long rows[4];
 #pragma unroll
-        for (int j = 0; j < 32; ++j) y[j] = 0.0f;
-        if (row < p.M) {
-          for (int part = 0; part < p.split; ++part) {
-            const uint32_t src = map_to_cta(smem_base + static_cast<uint32_t>(((c0 / 4) * BLOCK_ROWS + trow) * 16), part);
-            uint4 v[8];
+      for (int k = 0; k < 4; ++k) {
+        const int r = m_blk * BLOCK_ROWS + q * 32 + 8 * k + (lane >> 2);
+        rows[k] = r < p.M ? r : -1;
+      }
+      // columns summed and stored by this CTA (64, 32 or 16), half of them by each of a quadrant's two warps
+      const int share = BN / p.split / 2;
+      const int c0 = rank * 2 * share + ((warp - 2) >> 2) * share;
+      float y[32];
 #pragma unroll
-            for (int j = 0; j < 8; ++j)
-              v[j] = 4 * j < n_ok ? ld_dsmem_v4(src + j * BLOCK_ROWS * 16) : make_uint4(0u, 0u, 0u, 0u);
+      for (int j = 0; j < 32; ++j) y[j] = 0.0f;
+      for (int part = 0; part < p.split; ++part) {
+        const uint32_t src = map_to_cta(smem_base + static_cast<uint32_t>(((c0 / 4) * BLOCK_ROWS + q * 32 + lane) * 16), part);
+        uint4 v[8];
 #pragma unroll
-            for (int j = 0; j < 8; ++j) {
-              y[4 * j] += __uint_as_float(v[j].x);
-              y[4 * j + 1] += __uint_as_float(v[j].y);
-              y[4 * j + 2] += __uint_as_float(v[j].z);
-              y[4 * j + 3] += __uint_as_float(v[j].w);
-            }
-          }
-          moe_store_row32<OUTMODE, false>(p.c, static_cast<size_t>(row) * p.N + n_blk * BN + c0, y, n_ok);
+        for (int j = 0; j < 8; ++j) v[j] = 4 * j < share ? ld_dsmem_v4(src + j * BLOCK_ROWS * 16) : make_uint4(0u, 0u, 0u, 0u);
+#pragma unroll
+        for (int j = 0; j < 8; ++j) {
+          y[4 * j] += __uint_as_float(v[j].x);
+          y[4 * j + 1] += __uint_as_float(v[j].y);
+          y[4 * j + 2] += __uint_as_float(v[j].z);
+          y[4 * j + 3] += __uint_as_float(v[j].w);
         }
       }
+      store_rows32<OUTMODE, false>(p.c, rows, p.N, n_blk * BN + c0, y, share, stage_c, lane);
     }
     __syncwarp();
     cluster_sync_all();  // nobody leaves while a peer may still read its shared memory

@@ -40,7 +40,7 @@ int launch_rows(const CUtensorMap& tmA, const CUtensorMap& tmC, const GemmParams
   if (L.total > SMEM_LIMIT || p.bn < 32 || p.bn > 256 || (p.bn & 31)) return FLYB200_E_UNSUPPORTED;
   const long long tiles = static_cast<long long>((p.M + BLOCK_ROWS - 1) / BLOCK_ROWS) * ((p.N + p.bn - 1) / p.bn);
   const int grid = static_cast<int>(tiles < sms ? tiles : sms);
-  return launch_plain_or_pdl(kernel, grid, NUM_THREADS, L.total, s, p.pdl != 0, tmA, tmC, p);
+  return launch_plain_or_pdl(kernel, grid, ROWS_THREADS, L.total, s, p.pdl != 0, tmA, tmC, p);
 }
 
 // One CTA per 256 x bn tile (tmA: boxes of 256 rows).
@@ -106,7 +106,7 @@ int launch_rows_scatter(const CUtensorMap& tmA, const OutputMaps& outs, const Ge
   if (L.total > SMEM_LIMIT || p.bn < 64 || p.bn > 256 || (p.bn & 63)) return FLYB200_E_UNSUPPORTED;
   const long long tiles = static_cast<long long>((p.M + BLOCK_ROWS - 1) / BLOCK_ROWS) * ((p.N + p.bn - 1) / p.bn);
   const int grid = static_cast<int>(tiles < sms ? tiles : sms);
-  kernel<<<grid, NUM_THREADS, L.total, s>>>(tmA, outs, p);
+  kernel<<<grid, ROWS_THREADS, L.total, s>>>(tmA, outs, p);
   FLYB200_CUDA_TRY(cudaGetLastError());
   return FLYB200_OK;
 }

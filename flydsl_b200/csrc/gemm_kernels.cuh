@@ -164,37 +164,45 @@ __device__ __forceinline__ float reciprocal_of(float x) {
   return fmaf(r, fmaf(-x, r, 1.0f), r);
 }
 
-// The activation of epilogue_value on eight values at once: the kind is a template argument and nothing
-// branches per value, so the eight chains (exponential, reciprocal) overlap.  Same operations in the same
+// The activation of epilogue_value on N values at once: the kind is a template argument and nothing
+// branches per value, so the chains (exponential, reciprocal) overlap.  Same operations in the same
 // order, same results.
-template <int EPI>
-__device__ __forceinline__ void activate_eight(float (&v)[8]) {
+template <int EPI, int N>
+__device__ __forceinline__ void activate(float (&v)[N]) {
   if constexpr (EPI == EPI_BIAS_RELU) {
 #pragma unroll
-    for (int i = 0; i < 8; ++i) v[i] = fmaxf(v[i], 0.0f);
+    for (int i = 0; i < N; ++i) v[i] = fmaxf(v[i], 0.0f);
   } else if constexpr (EPI == EPI_BIAS_SILU) {
-    float d[8];
+    float d[N];
     bool plain = true;  // false for a value below -87 (its denominator leaves the range above) or NaN
 #pragma unroll
-    for (int i = 0; i < 8; ++i) {
+    for (int i = 0; i < N; ++i) {
       d[i] = 1.0f + __expf(-v[i]);
       plain &= d[i] < 8.5e37f;
     }
     if (plain) {
 #pragma unroll
-      for (int i = 0; i < 8; ++i) v[i] = v[i] * reciprocal_of(d[i]);
+      for (int i = 0; i < N; ++i) v[i] = v[i] * reciprocal_of(d[i]);
     } else {
 #pragma unroll
-      for (int i = 0; i < 8; ++i) v[i] = v[i] * (1.0f / d[i]);
+      for (int i = 0; i < N; ++i) v[i] = v[i] * (1.0f / d[i]);
     }
   } else if constexpr (EPI == EPI_BIAS_GELU) {
 #pragma unroll
-    for (int i = 0; i < 8; ++i) {
+    for (int i = 0; i < N; ++i) {
       const float y = 0.7978845608f * (v[i] + 0.044715f * (v[i] * v[i] * v[i]));
       const float e = __expf(-2.0f * fabsf(y));
       const float num = (y > 0.0f) ? 2.0f : 2.0f * e;
       v[i] = 0.5f * v[i] * (num * reciprocal_of(1.0f + e));
     }
+  }
+}
+template <int N>
+__device__ __forceinline__ void activate(int epi, float (&v)[N]) {
+  switch (epi) {
+    case EPI_BIAS_RELU: return activate<EPI_BIAS_RELU>(v);
+    case EPI_BIAS_SILU: return activate<EPI_BIAS_SILU>(v);
+    case EPI_BIAS_GELU: return activate<EPI_BIAS_GELU>(v);
   }
 }
 
@@ -237,27 +245,28 @@ __device__ __forceinline__ void load_column_factors(ColumnFactors& f, const Gemm
 
 // 32 raw accumulators of one row -> scaled, biased, activated, 16-bit; `emit(g, pairs)` takes eight
 // columns (8 g ...).  The order of epilogue_value, every operation rounded by itself.  One value at a
-// time, with its own switch on the activation, its own division and two scalar loads, the four epilogue
-// warps took longer than the mainloop they overlap: int8 997 x 10208 x 5120, bias and gelu, 115.7 us for
-// the kernel (linear layer 130), now 58 (66).
+// time, with its own switch on the activation, its own division and two scalar loads, the epilogue warps
+// took longer than the mainloop they overlap: int8 997 x 10208 x 5120, bias and gelu, 115.7 us for the
+// kernel, 52 this way.  Eight epilogue warps instead of four matter where K is short: 2048 x 8192 x 2048 with
+// bias and silu 64.4 -> 44.7 us, gelu 54.0 -> 42.5, none 32.2 -> 32.0.
 template <bool IS_INT, int OUTMODE, int EPI, typename EmitFn>
 __device__ __forceinline__ void epilogue_32(const uint32_t (&r)[32], float sa, const ColumnFactors& f, EmitFn emit) {
+  float v[32];
+#pragma unroll
+  for (int i = 0; i < 32; ++i) {
+    const float acc = IS_INT ? static_cast<float>(static_cast<int32_t>(r[i])) : __uint_as_float(r[i]);
+    v[i] = __fmul_rn(__fmul_rn(acc, sa), f.sb[i]);
+    if constexpr (EPI != EPI_NONE) {
+      const uint16_t h = static_cast<uint16_t>(f.bias[i / 2] >> (16 * (i & 1)));
+      v[i] = __fadd_rn(v[i], load_bias<OUTMODE>(&h, 0));
+    }
+  }
+  activate<EPI>(v);
 #pragma unroll
   for (int g = 0; g < 4; ++g) {
-    float v[8];
-#pragma unroll
-    for (int i = 0; i < 8; ++i) {
-      const float acc = IS_INT ? static_cast<float>(static_cast<int32_t>(r[8 * g + i])) : __uint_as_float(r[8 * g + i]);
-      v[i] = __fmul_rn(__fmul_rn(acc, sa), f.sb[8 * g + i]);
-      if constexpr (EPI != EPI_NONE) {
-        const uint16_t h = static_cast<uint16_t>(f.bias[4 * g + i / 2] >> (16 * (i & 1)));
-        v[i] = __fadd_rn(v[i], load_bias<OUTMODE>(&h, 0));
-      }
-    }
-    activate_eight<EPI>(v);
     uint32_t pk[4];
 #pragma unroll
-    for (int i = 0; i < 4; ++i) pk[i] = pack2<OUTMODE>(v[2 * i], v[2 * i + 1]);
+    for (int i = 0; i < 4; ++i) pk[i] = pack2<OUTMODE>(v[8 * g + 2 * i], v[8 * g + 2 * i + 1]);
     emit(g, pk);
   }
 }
@@ -283,10 +292,11 @@ __device__ __forceinline__ void epilogue_32(int epi, const uint32_t (&r)[32], fl
 // the same time.
 // CBUFS: staging buffers of this warp at `stage_c` (two: the store of one chunk overlaps the
 // conversion of the next; one: where shared memory is short).
-template <int KIND, int OUTMODE, int CBUFS = 2, typename ReleaseFn>
+// SHARE: warps that share these 32 rows; this one, `part`, takes every SHARE-th chunk of 64 columns.
+template <int KIND, int OUTMODE, int CBUFS = 2, int SHARE = 1, typename ReleaseFn>
 __device__ __forceinline__ void epilogue_warp_tile(const GemmParams& p, const CUtensorMap* tmC, int n_dst, int dst_first,
                                                    uint32_t t_row, int m0, int n0, int BN, int lane, uint32_t stage_c,
-                                                   int& cbuf, ReleaseFn release_tmem) {
+                                                   int& cbuf, ReleaseFn release_tmem, int part = 0) {
   using KT = KindTraits<KIND>;
   constexpr int C_BUF = 32 * 128;
   const bool scaled = (p.sa != nullptr) && (p.sb != nullptr);
@@ -295,7 +305,7 @@ __device__ __forceinline__ void epilogue_warp_tile(const GemmParams& p, const CU
   if constexpr (OUTMODE == OUT_RAW32) {
     uint32_t* out = reinterpret_cast<uint32_t*>(p.c);
 #pragma unroll 1
-    for (int c0 = 0; c0 < BN; c0 += 32) {
+    for (int c0 = 32 * part; c0 < BN; c0 += 32 * SHARE) {
       uint32_t r[32];
       tmem_ld_x32(t_row + c0, r);
       tmem_ld_wait();
@@ -317,8 +327,9 @@ __device__ __forceinline__ void epilogue_warp_tile(const GemmParams& p, const CU
   } else {
     const bool vec = ((reinterpret_cast<uintptr_t>(p.sb) | reinterpret_cast<uintptr_t>(p.bias)) & 15u) == 0;
     ColumnFactors f;
+    if (64 * part >= BN) release_tmem();  // nothing to do for this warp
 #pragma unroll 1
-    for (int c0 = 0; c0 < BN; c0 += 64) {
+    for (int c0 = 64 * part; c0 < BN; c0 += 64 * SHARE) {
       if (c0 + 64 > BN) {
         // Last 32 columns of a tile whose width is not a multiple of 64: a
         // 64-column TMA box would reach into the neighbouring tile, so these
@@ -337,29 +348,21 @@ __device__ __forceinline__ void epilogue_warp_tile(const GemmParams& p, const CU
         }
         break;
       }
-      uint32_t r0[32], r1[32];
-      tmem_ld_x32(t_row + c0, r0);
-      tmem_ld_x32(t_row + c0 + 32, r1);
-      load_column_factors(f, p, n0 + c0, scaled, vec);
-      tmem_ld_wait();
-      if (c0 + 64 >= BN) release_tmem();  // accumulator fully read: hand the TMEM buffer back
       // the store that last used this buffer (two chunks ago with two buffers) has to be done reading it
       if (lane == 0) bulk_wait_group_read<CBUFS - 1>();
       __syncwarp();
       const uint32_t cdst = stage_c + cbuf * C_BUF + lane * 128;
 #pragma unroll 1
       for (int h = 0; h < 2; ++h) {
-        if (h == 1) {
-          load_column_factors(f, p, n0 + c0 + 32, scaled, vec);
-#pragma unroll
-          for (int j = 0; j < 32; ++j) r0[j] = r1[j];
-        }
-        epilogue_32<KT::is_int, OUTMODE>(p.epilogue, r0, sa_v, f, [&](int g, const uint32_t (&pk)[4]) {
+        uint32_t r[32];
+        tmem_ld_x32(t_row + c0 + 32 * h, r);
+        load_column_factors(f, p, n0 + c0 + 32 * h, scaled, vec);
+        tmem_ld_wait();
+        // this warp's last read of the accumulator: hand the TMEM buffer back
+        if (h == 1 && c0 + 64 * SHARE >= BN) release_tmem();
+        epilogue_32<KT::is_int, OUTMODE>(p.epilogue, r, sa_v, f, [&](int g, const uint32_t (&pk)[4]) {
           const int chunk = 4 * h + g;  // 16-byte chunk index inside the 128-byte row
-          const uint32_t addr = cdst + static_cast<uint32_t>(((chunk ^ (lane & 7)) << 4));
-          asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(addr), "r"(pk[0]), "r"(pk[1]), "r"(pk[2]),
-                       "r"(pk[3])
-                       : "memory");
+          st_smem_v4(cdst + static_cast<uint32_t>(((chunk ^ (lane & 7)) << 4)), pk[0], pk[1], pk[2], pk[3]);
         });
       }
       fence_proxy_async_smem();
@@ -387,14 +390,15 @@ struct RowsLayout {
   int a_stage, b_stage, off_b, off_c, off_bar, off_misc, total;
 };
 constexpr int ROWS_C_BUF = 32 * 128;  // staging buffer: 32 rows x 64 two-byte columns
+constexpr int ROWS_THREADS = 64 + 8 * 32;  // producer, MMA issuer, eight epilogue warps (two per 32 rows)
 constexpr int ROWS_ACC_COLS = 256;    // TMEM columns between the two accumulator buffers
 __host__ __device__ inline RowsLayout rows_layout(int bn, int stages) {
   RowsLayout l;
   l.a_stage = BLOCK_ROWS * KBLOCK_BYTES;
   l.b_stage = bn * KBLOCK_BYTES;
   l.off_b = stages * l.a_stage;
-  l.off_c = l.off_b + stages * l.b_stage;       // 4 warps x 2 buffers
-  l.off_bar = l.off_c + 4 * 2 * ROWS_C_BUF;     // full[S], empty[S], tfull[2], tempty[2]
+  l.off_c = l.off_b + stages * l.b_stage;       // one buffer per epilogue warp
+  l.off_bar = l.off_c + 8 * ROWS_C_BUF;         // full[S], empty[S], tfull[2], tempty[2]
   l.off_misc = l.off_bar + 8 * (2 * stages + 4);
   l.total = l.off_misc + 16;
   return l;
@@ -449,7 +453,7 @@ __device__ __forceinline__ void gemm_rows_body(const CUtensorMap& tmA, const CUt
     }
     for (int s = 0; s < 2; ++s) {
       mbar_init(bar_tfull + 8 * s, 1);
-      mbar_init(bar_tempty + 8 * s, 4);
+      mbar_init(bar_tempty + 8 * s, 8);
     }
     abort_flag[0] = 0;
     abort_flag[1] = 0;  // stays zero: lets the drain below wait on time alone
@@ -594,7 +598,7 @@ __device__ __forceinline__ void gemm_rows_body(const CUtensorMap& tmA, const CUt
     // ------------------------------ epilogue ------------------------------
     const int q = warp & 3;  // TMEM lane quadrant this warp may read
     const int ew = warp - 2; // staging buffer owner
-    const uint32_t stage_c = smem_base + L.off_c + ew * 2 * ROWS_C_BUF;
+    const uint32_t stage_c = smem_base + L.off_c + ew * ROWS_C_BUF;
     int acc = 0;
     uint32_t acc_phase = 0;
     int cbuf = 0;
@@ -614,11 +618,11 @@ __device__ __forceinline__ void gemm_rows_body(const CUtensorMap& tmA, const CUt
           tmem_base + (static_cast<uint32_t>(q * 32) << 16) + static_cast<uint32_t>(acc * ROWS_ACC_COLS);
       // own buffer first for the first tile; every further tile and warp starts one destination later
       const int first = n_dst > 1 ? (dst_first + (t / static_cast<int>(gridDim.x)) + ew) % n_dst : 0;
-      epilogue_warp_tile<KIND, OUTMODE>(p, tmC_ptr, n_dst, first, t_row, m0, n0, BN, lane, stage_c, cbuf, [&]() {
+      epilogue_warp_tile<KIND, OUTMODE, 1, 2>(p, tmC_ptr, n_dst, first, t_row, m0, n0, BN, lane, stage_c, cbuf, [&]() {
         tc_fence_before();
         __syncwarp();
         if (lane == 0) mbar_arrive(bar_tempty + 8 * acc);
-      });
+      }, ew >> 2);
       acc ^= 1;
       if (acc == 0) acc_phase ^= 1u;
     }
@@ -651,7 +655,7 @@ __device__ __forceinline__ void gemm_rows_body(const CUtensorMap& tmA, const CUt
 
 // One output buffer (the regular GEMM).
 template <int KIND, int OUTMODE>
-__global__ void __launch_bounds__(NUM_THREADS, 1)
+__global__ void __launch_bounds__(ROWS_THREADS, 1)
 gemm_rows_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmC,
                  const GemmParams p) {
   gemm_rows_body<KIND, OUTMODE>(tmA, &tmC, 1, 0, p);
@@ -662,7 +666,7 @@ gemm_rows_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
 // memory; plain TMA stores, per CTA, no multicast): the all-gather of the
 // shards happens tile by tile inside the GEMM.
 template <int KIND, int OUTMODE>
-__global__ void __launch_bounds__(NUM_THREADS, 1)
+__global__ void __launch_bounds__(ROWS_THREADS, 1)
 gemm_rows_scatter_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ OutputMaps outs,
                          const GemmParams p) {
   gemm_rows_body<KIND, OUTMODE>(tmA, outs.m, p.n_dst, p.dst_first, p);

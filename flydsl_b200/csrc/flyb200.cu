@@ -375,11 +375,15 @@ int auto_rows_bn(int M, int N, int K_bytes, int sms) {
   for (int bn = 256; bn >= 64; bn -= 32) {
     const long long tiles = num_m * ((N + bn - 1) / bn);
     const long long rounds = (tiles + sms - 1) / sms;
-    long long per_kb = 2 * bn;
-    if (per_kb < ROWS_ISSUE_CYCLES) per_kb = ROWS_ISSUE_CYCLES;
-    const long long load = (BLOCK_ROWS * KBLOCK_BYTES + bn * KBLOCK_BYTES) / ROWS_LOAD_BYTES_PER_CYCLE;
-    if (per_kb < load) per_kb = load;
-    const long long cost = rounds * (kb * per_kb + 4 * bn) + ROWS_TILE_OVERHEAD_CYCLES;
+    auto tile_cost = [&](int width) {
+      long long per_kb = 2 * width;
+      if (per_kb < ROWS_ISSUE_CYCLES) per_kb = ROWS_ISSUE_CYCLES;
+      const long long load = (BLOCK_ROWS * KBLOCK_BYTES + width * KBLOCK_BYTES) / ROWS_LOAD_BYTES_PER_CYCLE;
+      if (per_kb < load) per_kb = load;
+      return kb * per_kb + 4 * width;
+    };
+    const int parts = host::rows_tail_parts(bn, tiles, sms);  // the last round may go in column strips
+    const long long cost = (rounds - 1) * tile_cost(bn) + tile_cost(bn / parts) + ROWS_TILE_OVERHEAD_CYCLES;
     if (best_cost < 0 || cost < best_cost) {
       best_cost = cost;
       best = bn;

@@ -57,6 +57,7 @@ struct GemmParams {
   uint32_t fmt_bits;     // decode kernel, MX kind on bytes: operand formats as instruction-descriptor bits (weights << 7 | tokens << 10)
   int bn;                // large-M kernel: output channels per tile (multiple of 32, 32..256)
   int rows_stages;       // large-M kernel: depth of the shared-memory ring
+  int tail_parts;        // large-M kernel: column parts of the tiles of the last, partial round (1, 2 or 4; bn / parts a multiple of 64)
   int n_dst;             // scatter kernel: number of output buffers
   int dst_first;         // scatter kernel: buffer stored to first
   int* status;           // device status word (first failure wins)
@@ -496,6 +497,28 @@ __device__ __forceinline__ void gemm_rows_body(const CUtensorMap& tmA, const CUt
     if (g & 1) n_blk = num_n - 1 - n_blk;
   };
 
+  // Work items: the tiles of the whole rounds, then those of the last, partial round in `parts` column
+  // strips each, so that the round costs a strip instead of a tile (host: rows_tail_parts).
+  const int parts = p.tail_parts;
+  const int whole = parts > 1 ? num_tiles - num_tiles % static_cast<int>(gridDim.x) : num_tiles;
+  const int items = whole + (num_tiles - whole) * parts;
+  const int strip = BN / parts;
+  // item -> row tile, first column and width; false where the strip lies past the last column
+  auto item_coords = [&](int i, int& m_blk, int& n0, int& width) {
+    int n_blk;
+    if (i < whole) {
+      tile_coords(i, m_blk, n_blk);
+      n0 = n_blk * BN;
+      width = BN;
+      return true;
+    }
+    const int j = i - whole;
+    tile_coords(whole + j / parts, m_blk, n_blk);
+    n0 = n_blk * BN + j % parts * strip;
+    width = strip;
+    return n0 < p.N;
+  };
+
   if (warp == 0) {
     // ------------------------------ producer ------------------------------
     if (lane == 0) {
@@ -505,11 +528,10 @@ __device__ __forceinline__ void gemm_rows_body(const CUtensorMap& tmA, const CUt
       uint32_t phase = 0;
       int issued = 0;
       bool ok = true;
-      for (int t = blockIdx.x; t < num_tiles && ok; t += gridDim.x) {
-        int m_blk, n_blk;
-        tile_coords(t, m_blk, n_blk);
-        const int n0 = n_blk * BN;
-        const uint32_t w_rows = static_cast<uint32_t>(min(BN, p.N - n0));
+      for (int t = blockIdx.x; t < items && ok; t += gridDim.x) {
+        int m_blk, n0, width;
+        if (!item_coords(t, m_blk, n0, width)) continue;
+        const uint32_t w_rows = static_cast<uint32_t>(min(width, p.N - n0));
         const uint32_t w_bytes = w_rows * KBLOCK_BYTES;
         // The ring holds a few k-blocks; the weights of the next `prefetch`
         // k-blocks are already on their way from DRAM into L2, so the depth
@@ -555,13 +577,15 @@ __device__ __forceinline__ void gemm_rows_body(const CUtensorMap& tmA, const CUt
   } else if (warp == 1) {
     // ------------------------------ MMA issue -----------------------------
     if (lane == 0) {
-      const uint32_t idesc = umma_idesc(KT::dfmt, KT::abfmt, BLOCK_ROWS, static_cast<uint32_t>(BN));
       int stage = 0;
       uint32_t phase = 0;
       int acc = 0;
       uint32_t acc_phase = 0;
       bool ok = true;
-      for (int t = blockIdx.x; t < num_tiles && ok; t += gridDim.x) {
+      for (int t = blockIdx.x; t < items && ok; t += gridDim.x) {
+        int m_blk, n0, width;
+        if (!item_coords(t, m_blk, n0, width)) continue;
+        const uint32_t idesc = umma_idesc(KT::dfmt, KT::abfmt, BLOCK_ROWS, static_cast<uint32_t>(width));
         if (!mbar_wait(bar_tempty + 8 * acc, acc_phase ^ 1u, abort_flag FLYB200_PROF_ARG(&prof_wait[1]))) {
           report_failure(p.status, ST_TIMEOUT, abort_flag);
           break;
@@ -603,11 +627,10 @@ __device__ __forceinline__ void gemm_rows_body(const CUtensorMap& tmA, const CUt
     uint32_t acc_phase = 0;
     int cbuf = 0;
     bool ok = true;
-    for (int t = blockIdx.x; t < num_tiles && ok; t += gridDim.x) {
-      int m_blk, n_blk;
-      tile_coords(t, m_blk, n_blk);
+    for (int t = blockIdx.x; t < items && ok; t += gridDim.x) {
+      int m_blk, n0, width;
+      if (!item_coords(t, m_blk, n0, width)) continue;
       const int m0 = m_blk * BLOCK_ROWS + q * 32;
-      const int n0 = n_blk * BN;
       if (!mbar_wait(bar_tfull + 8 * acc, acc_phase, abort_flag FLYB200_PROF_ARG(&prof_wait[3]))) {
         if (lane == 0) report_failure(p.status, ST_TIMEOUT, abort_flag);
         ok = false;
@@ -618,7 +641,7 @@ __device__ __forceinline__ void gemm_rows_body(const CUtensorMap& tmA, const CUt
           tmem_base + (static_cast<uint32_t>(q * 32) << 16) + static_cast<uint32_t>(acc * ROWS_ACC_COLS);
       // own buffer first for the first tile; every further tile and warp starts one destination later
       const int first = n_dst > 1 ? (dst_first + (t / static_cast<int>(gridDim.x)) + ew) % n_dst : 0;
-      epilogue_warp_tile<KIND, OUTMODE, 1, 2>(p, tmC_ptr, n_dst, first, t_row, m0, n0, BN, lane, stage_c, cbuf, [&]() {
+      epilogue_warp_tile<KIND, OUTMODE, 1, 2>(p, tmC_ptr, n_dst, first, t_row, m0, n0, width, lane, stage_c, cbuf, [&]() {
         tc_fence_before();
         __syncwarp();
         if (lane == 0) mbar_arrive(bar_tempty + 8 * acc);

@@ -39,6 +39,18 @@ inline int rows_stages_for(int bn) {
   return s;
 }
 
+// Column strips of the tiles of the large-M kernel's last round, where that is at most half full (1: none): two or
+// four strips per tile while every SM gets at most one; strips are multiples of 64 columns (the stores' box).  The
+// round is short of power rather than of time (fewer busy SMs clock higher), so the gain is small: whole tiles /
+// strips, us, fp16 4096 x 4096 x 4096 (3.46 rounds of tiles) 104.1 / 102.8, fp8 55.4 / 54.2; even where the last
+// round is more than half full (no strips) or one of many.
+inline int rows_tail_parts(int bn, long long tiles, int sms) {
+  const long long rest = tiles % sms;
+  if (tiles < sms || rest == 0 || bn % 128 != 0) return 1;
+  if (bn == 256 && 4 * rest <= sms) return 4;
+  return 2 * rest <= sms ? 2 : 1;
+}
+
 // Large-M kernel (p.bn, p.rows_stages set) in one of three forms: one CTA per 128 x bn tile, CTA pairs
 // on 256 x 256 tiles (needs tmW), one CTA per 256 x bn tile (tmA with boxes of 256 rows, three stages).
 // `kind` is KIND_*, `outmode` OUT_*.

@@ -54,3 +54,26 @@ def test_epilogue_on_tile_edges(epilogue, in_dtype, out_dtype, offset, hint):
     acc = a.float() @ b.float().T
     ref = oracle.epilogue(acc, sa, sb, bias, epilogue, out_dtype=torch.float32)
     assert not torch.isnan(got).any() and oracle.strict_mismatches(got, ref, RTOL, ATOL) == 0
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("m,n,width", [(300, 12816, 8), (300, 12704, 8), (300, 14464, 8), (300, 6448, 4), (100, 19104, 4), (520, 7584, 8)])
+@pytest.mark.parametrize("in_dtype", ["int8", "bf16"])
+def test_last_round_in_strips_is_bit_identical(monkeypatch, m, n, width, in_dtype):
+    """Tiles of 32 * width columns of which a few are left for the last round (2 and 4 strips; a last tile of
+    16 columns whose other strips are empty; a strip that N ends in): every output is the same sum."""
+    dev = torch.device("cuda:0")
+    k = 256
+    g = torch.Generator().manual_seed(n)
+    bias = torch.randn(n, generator=g).to(torch.bfloat16)
+    if in_dtype == "bf16":
+        a, b, sa, sb = torch.randn(m, k, generator=g).bfloat16(), torch.randn(n, k, generator=g).bfloat16(), None, None
+    else:
+        a, b, sa, sb = oracle.make_inputs(m, n, k, in_dtype, seed=n)
+    outs = []
+    for tail in ("0", "1"):
+        monkeypatch.setenv("FLYB200_ROWS_TAIL", tail)
+        outs.append(run_gemm_generic(dev, a, b, sa, sb, bias, m, n, k, in_dtype, epilogue="bias_gelu", hint=ROWS | width))
+    assert torch.equal(outs[0], outs[1])
+    ref = oracle.epilogue(a.float() @ b.float().T, sa, sb, bias, "bias_gelu", out_dtype=torch.float32)
+    assert oracle.strict_mismatches(outs[1], ref, RTOL, ATOL) == 0

@@ -31,7 +31,7 @@ enum : int { EPI_NONE = 0, EPI_BIAS = 1, EPI_BIAS_RELU = 2, EPI_BIAS_SILU = 3, E
 constexpr int BLOCK_ROWS = 128;   // UMMA M
 constexpr int KBLOCK_BYTES = 128; // one swizzle row: 128 fp8/int8 or 64 half elements
 constexpr int UMMA_K_BYTES = 32;  // bytes of K consumed by one tcgen05.mma
-constexpr int NUM_THREADS = 192;  // warp 0 producer, warp 1 MMA, warps 2..5 epilogue
+constexpr int NUM_THREADS = 192;  // CTA-pair kernel: warp 0 producer, warp 1 MMA, warps 2..5 epilogue
 
 struct GemmParams {
   const uint8_t* w;      // preshuffled weights

@@ -387,9 +387,9 @@ __global__ void __launch_bounds__(MOE_THREADS) moe_gemm_kernel(const __grid_cons
 // neighbouring tiles), one CTA per SM walking the (row block, channel pair)
 // items, a shared-memory ring that keeps streaming across items and two TMEM
 // accumulators so that the epilogue of an item overlaps the mainloop of the
-// next.  A thread of the epilogue owns one token row: it reads the gate and up
-// columns of the same channel from its own TMEM lane and writes 64 contiguous
-// bytes of its output row per 32-channel chunk.
+// next.  A thread of the epilogue owns one token row (two warps per 32 rows): it
+// reads the gate and up columns of the same channel from its own TMEM lane; the
+// outputs leave through store_rows32.
 constexpr int MOE_ROWS_STAGES = 4;
 constexpr int MOE_ROWS_BN = 2 * BLOCK_ROWS;
 constexpr int MOE_ROWS_GROUP = 32;  // row blocks per rasterisation group (16 MiB of activations at K = 4096)

@@ -12,6 +12,8 @@
 #include "../../include/flyb200.h"
 
 #include <ATen/ATen.h>
+#include <c10/core/GradMode.h>
+#include <c10/core/impl/LocalDispatchKeySet.h>
 #include <c10/cuda/CUDAGuard.h>
 #include <c10/cuda/CUDAStream.h>
 #include <torch/csrc/Exceptions.h>
@@ -93,6 +95,20 @@ T* as(const at::Tensor& t) {
   return static_cast<T*>(ptr(t));
 }
 void* stream_of(const at::Tensor& t) { return c10::cuda::getCurrentCUDAStream(t.device().index()).stream(); }
+// Whether a kernel may stand for torch operations on the tensor `o`: a plain tensor (no subclass, fake,
+// functionalised, functorch-wrapped, lazily negated or conjugated one), with no dispatch mode, trace or transform
+// in force that has to see the operations.  `differentiable`: nor a gradient that they would carry.
+bool runs_eagerly(PyObject* o, bool differentiable) {
+  using K = c10::DispatchKey;
+  constexpr c10::DispatchKeySet wrapped({K::Python, K::PythonTLSSnapshot, K::Functionalize, K::Negative, K::Conjugate, K::ZeroTensor,
+                                         K::FuncTorchBatched, K::FuncTorchGradWrapper, K::BatchedNestedTensor, K::Batched});
+  constexpr c10::DispatchKeySet watching({K::Python, K::PythonTLSSnapshot, K::Functionalize, K::FuncTorchDynamicLayerFrontMode,
+                                          K::FuncTorchVmapMode, K::VmapMode, K::Tracer, K::PreDispatch, K::PythonDispatcher});
+  if (!THPVariable_CheckExact(o)) return false;
+  const at::Tensor& t = THPVariable_Unpack(o);
+  if (t.key_set().has_any(wrapped) || c10::impl::tls_local_dispatch_key_set().included_.has_any(watching)) return false;
+  return !differentiable || !((c10::GradMode::is_enabled() && t.requires_grad()) || t._fw_grad(0).defined());
+}
 void* handle(long long s) { return reinterpret_cast<void*>(static_cast<uintptr_t>(s)); }
 int input_code(const at::Tensor& x) {
   switch (x.scalar_type()) {
@@ -149,13 +165,21 @@ PyObject* gemm_a8w8(PyObject*, PyObject* const* argv, Py_ssize_t n) {
   END_HANDLE_TH_ERRORS
 }
 
-// mx_quant(x, format) -> (codes, scales, raw | None), shaped like x
+// eager(x) -> bool
+PyObject* eager(PyObject*, PyObject* const* argv, Py_ssize_t n) {
+  HANDLE_TH_ERRORS
+  return PyBool_FromLong(n == 1 && runs_eagerly(argv[0], false));
+  END_HANDLE_TH_ERRORS
+}
+
+// mx_quant(x, format) -> (codes, scales, raw | None), shaped like x.  Only E4M3 codes are differentiable as torch
+// operations; the others come out of integer arithmetic.
 PyObject* mx_quant(PyObject*, PyObject* const* argv, Py_ssize_t n) {
   HANDLE_TH_ERRORS
   Args a{argv, n};
   const at::Tensor& arg = a.tensor();
   const int fmt = a.i32();
-  if (!a.done() || !arg.is_cuda() || arg.layout() != at::kStrided || arg.dim() < 1 || arg.numel() == 0 || arg.size(-1) % 32 != 0) return none();
+  if (!a.done() || !runs_eagerly(argv[0], fmt == FLYB200_MXFMT_E4M3) || !arg.is_cuda() || arg.layout() != at::kStrided || arg.dim() < 1 || arg.numel() == 0 || arg.size(-1) % 32 != 0) return none();
   const int in = input_code(arg);
   if (in < 0 || (fmt != FLYB200_MXFMT_E4M3 && fmt != FLYB200_MXFMT_E2M3 && fmt != FLYB200_MXFMT_E2M1)) return none();
   at::Tensor x, codes, scale, raw;
@@ -374,7 +398,7 @@ PyObject* moe_layer(PyObject*, PyObject* const* argv, Py_ssize_t n) {
 }
 
 #define FAST(name) {#name, reinterpret_cast<PyCFunction>(reinterpret_cast<void (*)()>(name)), METH_FASTCALL, nullptr}
-PyMethodDef methods[] = {FAST(pertoken_quant), FAST(gemm_a8w8), FAST(mx_quant), FAST(mx_scale_image), FAST(mx_gemm),
+PyMethodDef methods[] = {FAST(pertoken_quant), FAST(gemm_a8w8), FAST(eager), FAST(mx_quant), FAST(mx_scale_image), FAST(mx_gemm),
                          FAST(moe_sort),       FAST(moe_stage), FAST(moe_layer), {nullptr, nullptr, 0, nullptr}};
 PyModuleDef module = {PyModuleDef_HEAD_INIT, "flyb200_ops", "Host path of the operators.", -1, methods, nullptr, nullptr, nullptr, nullptr};
 

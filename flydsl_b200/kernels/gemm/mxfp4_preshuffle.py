@@ -106,7 +106,8 @@ def fp6_containers_from_padded(a_pad: torch.Tensor) -> torch.Tensor:
     bytes, tests/kernels/utils/gemm_common_utils.py:744-770) -> byte containers [M, K]: every 16
     codes (12 bytes) followed by 4 bytes of padding."""
     m, k = a_pad.shape
-    if a_pad.is_cuda and a_pad.is_contiguous() and a_pad.element_size() == 1 and a_pad.data_ptr() % 16 == 0 and m * k > 0:
+    if (not torch.compiler.is_compiling() and a_pad.is_cuda and _lib.ops().eager(a_pad) and a_pad.is_contiguous()
+            and a_pad.element_size() == 1 and a_pad.data_ptr() % 16 == 0 and m * k > 0):
         dev = a_pad.device
         out = torch.empty(m, k, dtype=torch.uint8, device=dev)
         with _lib.on_device(dev):

@@ -30,8 +30,10 @@ FP8_MAX = 448.0
 def quant_kernel(x: torch.Tensor, fmt: int):
     """The per-1x32 quantisers as ONE kernel (the torch statements launch 30 to 250): ``(codes, scales, raw)``
     on x's device and of its leading shape, or None where the kernel cannot take ``x`` (CPU tensors, other
-    dtypes, no elements).  ``fmt``: 0 E4M3, 3 E2M3, 5 E2M1; ``raw`` (the codes one per byte) is None unless E2M3."""
-    if not x.is_cuda:
+    dtypes, no elements) or torch has to see the operations: tracing and compilation, fake tensors and other
+    subclasses, functional transforms, and for E4M3 an ``x`` whose gradient the codes carry.
+    ``fmt``: 0 E4M3, 3 E2M3, 5 E2M1; ``raw`` (the codes one per byte) is None unless E2M3."""
+    if torch.compiler.is_compiling() or not x.is_cuda:
         return None
     r = _lib.ops().mx_quant(x, fmt)
     if type(r) is int:
@@ -43,7 +45,8 @@ def per_1x32_f8_quant(x: torch.Tensor):
     """Per-1x32 MXFP8 quantiser on the tensor's device: (codes float8_e4m3fn [..., K], E8M0 scales
     uint8 [..., K/32]); same arithmetic as the reference helper
     (tests/kernels/utils/gemm_common_utils.py:53-72, 773-790).  CUDA tensors of fp32, fp16 or bf16
-    take the library's kernel, bit-identical to :func:`per_1x32_f8_quant_torch` on that tensor."""
+    take the library's kernel, bit-identical to :func:`per_1x32_f8_quant_torch` on that tensor, unless the
+    codes carry a gradient or torch traces the call."""
     shape = x.shape
     if shape[-1] % 32 != 0:
         raise ValueError("K must be a multiple of 32")

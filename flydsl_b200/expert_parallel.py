@@ -153,11 +153,12 @@ class ExpertParallelMoe:
         el = self.shard.experts_local
         blocks = (tokens * self.topk + el * self.tile_m - self.topk + self.tile_m - 1) // self.tile_m
         st = _lib.current_stream(dev)
-        a1, sa1 = self._g1._sorted_buffers(dev, blocks * self.tile_m, st)
-        a2, sa2 = self._g2._sorted_buffers(dev, blocks * self.tile_m, st)
-        y = _lib.ops().moe_layer(x_q, scale_x, topk_ids, topk_weights, self._w1, self._sw1, self._w2, self._sw2, self._expert_mask(dev),
-                                 a1, sa1, a2, sa2, el, self.shard.e0, self.shard.experts_total, self.model_dim, self.inter_dim,
-                                 self.topk, self.tile_m, _lib.IN_DTYPES[self.in_dtype])
+        a1, sa1, lock1 = self._g1._sorted_buffers(dev, blocks * self.tile_m, st)
+        a2, sa2, lock2 = self._g2._sorted_buffers(dev, blocks * self.tile_m, st)
+        with lock1, lock2:  # always in this order; a stage called by itself takes its own only
+            y = _lib.ops().moe_layer(x_q, scale_x, topk_ids, topk_weights, self._w1, self._sw1, self._w2, self._sw2, self._expert_mask(dev),
+                                     a1, sa1, a2, sa2, el, self.shard.e0, self.shard.experts_total, self.model_dim, self.inter_dim,
+                                     self.topk, self.tile_m, _lib.IN_DTYPES[self.in_dtype])
         if type(y) is int:
             _lib.check(y, "moe_layer")
         return y

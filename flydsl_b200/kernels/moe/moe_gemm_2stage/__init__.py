@@ -30,6 +30,7 @@ library's counting-sort kernels, on CPU tensors with torch ops.
 
 from __future__ import annotations
 
+import threading
 from typing import Tuple
 
 import torch
@@ -164,6 +165,7 @@ class _MoeStage:
         self._gather_mode = (2 if self._slot_major else 0) if stage == 1 else 1  # how a sorted row finds its activation row
         self._scratch: dict = {}
         self._retired: list = []
+        self._growing = threading.Lock()
         self._w4_expanded: dict = {}  # (data_ptr, numel) of a packed int4 weight tensor -> its int8 image
 
     def _weights_for_kernel(self, w: torch.Tensor, w_elems: int) -> torch.Tensor:
@@ -184,10 +186,18 @@ class _MoeStage:
         """Drop the cached int8 image of a packed int4 weight tensor (its contents changed in place)."""
         self._w4_expanded.pop((w.data_ptr(), w.numel()), None)
 
+    def __getstate__(self):
+        """A copied or unpickled launcher starts without scratch."""
+        return {k: v for k, v in self.__dict__.items() if k not in ("_scratch", "_retired", "_growing")}
+
+    def __setstate__(self, state):
+        self.__dict__.update(state, _scratch={}, _retired=[], _growing=threading.Lock())
+
     def _sorted_buffers(self, device, rows, stream=0):
-        """Gathered activation rows and their scales, one pair per (device, stream): two launches
-        on different streams must not share them.  A buffer that has to grow is replaced but
-        never freed (a kernel still running or a captured graph may hold its address), and
+        """Gathered activation rows, their scales and a lock, one set per (device, stream): two launches
+        on different streams must not share them.  Threads that share a stream share the buffers, so the
+        lock is held from the launch that writes them to the last one that reads them.  A buffer that has
+        to grow is replaced but never freed (a kernel still running or a captured graph may hold its address), and
         growing inside a stream capture is refused: run the shape once before capturing."""
         key = (device.index, stream or 0)
         buf = self._scratch.get(key)
@@ -195,13 +205,17 @@ class _MoeStage:
             if torch.cuda.is_current_stream_capturing():
                 raise RuntimeError("moe_gemm: the gather scratch for this shape does not exist yet; call the launcher "
                                    "once on this stream before capturing a CUDA graph")
-            if buf is not None:
-                self._retired.append(buf)
-            buf = (
-                torch.empty((rows, self._k), dtype=torch.uint8, device=device),
-                torch.empty((rows,), dtype=torch.float32, device=device),
-            )
-            self._scratch[key] = buf
+            with self._growing:
+                buf = self._scratch.get(key)
+                if buf is None or buf[0].shape[0] < rows:
+                    if buf is not None:
+                        self._retired.append(buf)
+                    buf = (
+                        torch.empty((rows, self._k), dtype=torch.uint8, device=device),
+                        torch.empty((rows,), dtype=torch.float32, device=device),
+                        threading.RLock(),
+                    )
+                    self._scratch[key] = buf
         return buf
 
     def __call__(
@@ -276,13 +290,14 @@ class _MoeStage:
                                     num_valid_ids, tokens, blocks, stream)
         s = _stream_handle(stream) or None
         rows = blocks * self.tile_m
-        a_sorted, sa_sorted = self._sorted_buffers(dev, rows, s)
+        a_sorted, sa_sorted, lock = self._sorted_buffers(dev, rows, s)
         if self.in_dtype == "int4":
             w = self._weights_for_kernel(w, self.experts * (2 * self.inter_dim if self.stage == 1 else self.model_dim) * self._k)
-        rc = _lib.ops().moe_stage(
-            out, x, w, scale_x, scale_w, sorted_token_ids, sorted_expert_ids, sorted_weights, num_valid_ids, a_sorted, sa_sorted,
-            self.stage, tokens, self.topk, self._gather_mode, self._k, self.experts, self.model_dim, self.inter_dim, self.tile_m,
-            blocks, self._dt, self._out, self.doweight, self.accumulate, s or 0)
+        with lock:
+            rc = _lib.ops().moe_stage(
+                out, x, w, scale_x, scale_w, sorted_token_ids, sorted_expert_ids, sorted_weights, num_valid_ids, a_sorted, sa_sorted,
+                self.stage, tokens, self.topk, self._gather_mode, self._k, self.experts, self.model_dim, self.inter_dim, self.tile_m,
+                blocks, self._dt, self._out, self.doweight, self.accumulate, s or 0)
         if rc is None:
             raise TypeError("moe_gemm: all arguments but the routed weights must be tensors")
         if rc:
@@ -303,14 +318,15 @@ class _MoeStage:
         with _lib.on_device(dev):
             s = _stream_handle(stream) or None
             rows = blocks * self.tile_m
-            a_sorted, sa_sorted = self._sorted_buffers(dev, rows, s)
-            rc = _lib.load().flyb200_moe_quant_sorted(
-                a_sorted.data_ptr(), sa_sorted.data_ptr(), x16.data_ptr(), sorted_token_ids.data_ptr(), num_valid_ids.data_ptr(),
-                tokens, self.topk, self._k, rows, self._dt, s)
-            if rc:
-                _lib.check(rc, "moe_quant_sorted")
-            self._gemm(out, a_sorted, sa_sorted, w, scale_w, sorted_token_ids, sorted_expert_ids, sorted_weights, num_valid_ids,
-                       tokens, blocks, s)
+            a_sorted, sa_sorted, lock = self._sorted_buffers(dev, rows, s)
+            with lock:
+                rc = _lib.load().flyb200_moe_quant_sorted(
+                    a_sorted.data_ptr(), sa_sorted.data_ptr(), x16.data_ptr(), sorted_token_ids.data_ptr(), num_valid_ids.data_ptr(),
+                    tokens, self.topk, self._k, rows, self._dt, s)
+                if rc:
+                    _lib.check(rc, "moe_quant_sorted")
+                self._gemm(out, a_sorted, sa_sorted, w, scale_w, sorted_token_ids, sorted_expert_ids, sorted_weights, num_valid_ids,
+                           tokens, blocks, s)
         return None
 
     def _gemm(self, out, a_sorted, sa_sorted, w, scale_w, sorted_token_ids, sorted_expert_ids, sorted_weights, num_valid_ids,

@@ -119,14 +119,19 @@ bool mx_wide_tiles(int M, int N, int k_bytes) {
 // 27.0 / 19.9 / 41, 64 x 1024 x 8192 (8) 27.8 / 17.1 / 13.1 / 11.2; MXFP8 200 x 1024 x 14336 (16) 44.0 / 23.9 /
 // 16.5 / 22.5, 600 x 1792 x 2048 (70, 16 k-blocks) 11.4 / 9.6 / 23 / 41, 256 x 4096 x 1024 (64, 8 k-blocks)
 // 7.2 / 8.0 / 16 / 40; MXFP4 256 x 4096 x 14336 27.9 / 18.1 / 26.4 / 54.
-// FLYB200_MX_SPLIT = 1, 2, 4 or 8 forces the factor (tuning and tests).
+// FLYB200_MX_SPLIT = 1, 2, 4 or 8 forces the factor (tuning and tests), halved until every part has a k-block:
+// a CTA without one would add an accumulator that no MMA has written.
 int mx_split(int M, int N, int k_bytes) {
+  const int kb = k_bytes / KBLOCK_BYTES;
   if (const char* e = getenv("FLYB200_MX_SPLIT"))
-    if (e[0] == '1' || e[0] == '2' || e[0] == '4' || e[0] == '8') return e[0] - '0';
+    if (e[0] == '1' || e[0] == '2' || e[0] == '4' || e[0] == '8') {
+      int split = e[0] - '0';
+      while (split > kb) split /= 2;
+      return split;
+    }
   int sms = 0;
   if (flyb200::host::sm_count(&sms) != FLYB200_OK) return 1;
   const long long tiles = static_cast<long long>((M + 127) / 128) * (N / 128);
-  const int kb = k_bytes / KBLOCK_BYTES;
   if (16 * tiles <= sms && kb >= 64) return 8;
   if (4 * tiles <= sms && kb >= 32) return 4;
   if (2 * tiles <= sms && kb >= 16) return 2;

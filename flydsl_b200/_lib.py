@@ -11,6 +11,7 @@ import ctypes
 import importlib.machinery
 import importlib.util
 import threading
+import warnings
 
 import torch
 
@@ -105,16 +106,22 @@ def load() -> ctypes.CDLL:
 def ops():
     """The CPython extension with the operators' host path (csrc/ops.cpp), loaded (built first if missing
     or stale) on first use.  Its functions return None for arguments that are not of the common form,
-    an int for a library error."""
+    an int for a library error.  Where it can be neither built nor loaded, host_statements.py stands for it:
+    the same kernels, with more host time per call."""
     global _ops
     if _ops is not None:
         return _ops
     load()
     with _lock:
         if _ops is None:
-            loader = importlib.machinery.ExtensionFileLoader("flyb200_ops", _build.build_ops())
-            mod = importlib.util.module_from_spec(importlib.util.spec_from_loader("flyb200_ops", loader))
-            loader.exec_module(mod)
+            try:
+                loader = importlib.machinery.ExtensionFileLoader("flyb200_ops", _build.build_ops())
+                mod = importlib.util.module_from_spec(importlib.util.spec_from_loader("flyb200_ops", loader))
+                loader.exec_module(mod)
+            except (RuntimeError, ImportError, OSError) as e:
+                from . import host_statements as mod
+
+                warnings.warn(f"flydsl_b200: no host extension, calls take more host time: {e}", RuntimeWarning, stacklevel=2)
             _ops = mod
     return _ops
 

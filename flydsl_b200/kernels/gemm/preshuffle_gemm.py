@@ -21,7 +21,7 @@ from typing import Optional
 
 import torch
 
-from ... import _lib
+from ... import _lib, host_statements
 
 _IN_DTYPES = ("fp8", "int8", "fp16", "bf16")
 _EPILOGUES = ("none", "bias", "bias_relu", "bias_silu", "bias_gelu")
@@ -232,12 +232,13 @@ class CompiledPreshuffleGemm:
         if torch.cuda.current_device() != dev.index:
             with torch.cuda.device(dev):
                 return self.__call__(arg_c, arg_a, arg_b, arg_scale_a, arg_scale_b, arg_bias, i32_m, i32_n, stream)
-        rc = self._fn(
+        args = (
             arg_c, arg_a, arg_b, arg_scale_a if eight else None, arg_scale_b if eight else None, arg_bias if op._epi else None,
             M, op.N, op.K, op._dt, op._out, op._epi, op.variant_hint, ws[0], ws[1], s,
         )  # fmt: skip
-        if rc is None:
-            raise TypeError("preshuffle_gemm: c, a, b, scales and bias must be tensors")
+        rc = self._fn(*args)
+        if rc is None:  # not tensors, but perhaps with an address
+            rc = host_statements.gemm_a8w8(*args)
         if rc:
             _lib.check(rc, "preshuffle_gemm")
         return None

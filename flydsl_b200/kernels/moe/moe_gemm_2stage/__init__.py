@@ -35,7 +35,7 @@ from typing import Tuple
 
 import torch
 
-from .... import _lib
+from .... import _lib, host_statements
 from ...gemm.preshuffle_gemm import _stream_handle
 
 _OUT = {
@@ -293,13 +293,15 @@ class _MoeStage:
         a_sorted, sa_sorted, lock = self._sorted_buffers(dev, rows, s)
         if self.in_dtype == "int4":
             w = self._weights_for_kernel(w, self.experts * (2 * self.inter_dim if self.stage == 1 else self.model_dim) * self._k)
+        args = (
+            out, x, w, scale_x, scale_w, sorted_token_ids, sorted_expert_ids, sorted_weights, num_valid_ids, a_sorted, sa_sorted,
+            self.stage, tokens, self.topk, self._gather_mode, self._k, self.experts, self.model_dim, self.inter_dim, self.tile_m,
+            blocks, self._dt, self._out, self.doweight, self.accumulate, s or 0,
+        )  # fmt: skip
         with lock:
-            rc = _lib.ops().moe_stage(
-                out, x, w, scale_x, scale_w, sorted_token_ids, sorted_expert_ids, sorted_weights, num_valid_ids, a_sorted, sa_sorted,
-                self.stage, tokens, self.topk, self._gather_mode, self._k, self.experts, self.model_dim, self.inter_dim, self.tile_m,
-                blocks, self._dt, self._out, self.doweight, self.accumulate, s or 0)
-        if rc is None:
-            raise TypeError("moe_gemm: all arguments but the routed weights must be tensors")
+            rc = _lib.ops().moe_stage(*args)
+            if rc is None:  # not tensors, but perhaps with an address
+                rc = host_statements.moe_stage(*args)
         if rc:
             _lib.check(rc, "moe_gemm")
         return None

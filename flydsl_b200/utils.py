@@ -44,10 +44,21 @@ def pertoken_quant_kernel(x: torch.Tensor, quant_dtype=torch.int8):
     fused; the torch statement below launches about ten element-wise kernels
     and materialises fp32 temporaries).  Bit-identical to :func:`pertoken_quant`
     evaluated by torch on the same GPU tensor."""
-    r = _lib.ops().pertoken_quant(x, _QUANT_CODES[quant_dtype])
-    if type(r) is not tuple:
-        _lib.check(_lib.E_UNSUPPORTED if r is None else r, "pertoken_quant")
-    return r
+    qd = _QUANT_CODES[quant_dtype]
+    r = _lib.ops().pertoken_quant(x, qd)
+    if type(r) is tuple:
+        return r
+    if r is None:  # not the common form: the library says what it takes (2^31 elements and more among it)
+        if not x.is_cuda or not x.is_contiguous() or x.dtype not in _X_DTYPES or x.dim() == 0 or x.shape[-1] == 0:
+            _lib.check(_lib.E_UNSUPPORTED, "pertoken_quant")
+        k = x.shape[-1]
+        y = torch.empty(x.shape, dtype=quant_dtype, device=x.device)
+        s = torch.empty(*x.shape[:-1], 1, dtype=torch.float32, device=x.device)
+        with _lib.on_device(x.device):
+            r = _lib.load().flyb200_pertoken_quant(y.data_ptr(), s.data_ptr(), x.data_ptr(), x.numel() // k, k, _X_DTYPES[x.dtype], qd,
+                                                   _lib.current_stream(x.device))
+    _lib.check(r, "pertoken_quant")
+    return y, s
 
 
 def pertoken_quant(

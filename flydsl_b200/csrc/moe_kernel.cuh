@@ -893,22 +893,24 @@ moe_quant_sorted_kernel(uint8_t* __restrict__ y, float* __restrict__ scale, cons
 constexpr int MOE_SORT_MAX_THREADS = 1024;
 constexpr int MOE_SORT_BINS = 4096;  // experts counted per pass over the pairs
 
-// ids of the four pairs at `i` (a multiple of four), -1 past the end; made relative to `first_expert`
+// ids of the four pairs at `i` (a multiple of four), -1 past the end; made relative to `first_expert`.  Of an
+// 8-byte id the low half counts, as in torch's conversion to int32, so that the table and the masked top-k sum
+// (which reads 4-byte ids) agree on every route.
 template <typename ID>
 __device__ __forceinline__ void moe_load_ids(const ID* __restrict__ ids, long long i, long long n_pairs, long long first_expert,
                                              int experts, bool vec, int (&e)[4]) {
-  long long v[4];
+  int v[4];
   if (vec && i + 3 < n_pairs) {
     if constexpr (sizeof(ID) == 4) {
       const int4 q = __ldg(reinterpret_cast<const int4*>(ids + i));
       v[0] = q.x, v[1] = q.y, v[2] = q.z, v[3] = q.w;
     } else {
       const longlong2 q0 = __ldg(reinterpret_cast<const longlong2*>(ids + i)), q1 = __ldg(reinterpret_cast<const longlong2*>(ids + i + 2));
-      v[0] = q0.x, v[1] = q0.y, v[2] = q1.x, v[3] = q1.y;
+      v[0] = static_cast<int>(q0.x), v[1] = static_cast<int>(q0.y), v[2] = static_cast<int>(q1.x), v[3] = static_cast<int>(q1.y);
     }
   } else {
 #pragma unroll
-    for (int j = 0; j < 4; ++j) v[j] = i + j < n_pairs ? static_cast<long long>(__ldg(ids + i + j)) : -1ll;
+    for (int j = 0; j < 4; ++j) v[j] = i + j < n_pairs ? static_cast<int>(__ldg(ids + i + j)) : -1;
   }
 #pragma unroll
   for (int j = 0; j < 4; ++j) {

@@ -314,7 +314,7 @@ int flyb200_moe_sorting(const int* topk_ids, const float* topk_weights, int toke
                         int* counts_scratch, void* stream);
 
 /* The same table for the experts [first_expert, first_expert + experts) of a larger set, renumbered from
- * zero (routes to other experts are dropped), with ids of 4 or 8 bytes and no scratch. */
+ * zero (routes to other experts are dropped), with ids of 4 or 8 bytes (of 8 the low half counts) and no scratch. */
 int flyb200_moe_sorting_range(const void* topk_ids, int id_bytes, const float* topk_weights, int tokens, int topk, int experts,
                               long long first_expert, int block_size, int* sorted_ids, float* sorted_weights,
                               int* sorted_expert_ids, int* num_tokens_post_pad, void* stream);

@@ -174,3 +174,20 @@ def test_routing_table_forms():
         got = moe_sorting(i, w, num_experts=16, block_size=32)
         used = int(want[3][0])
         assert all(torch.equal(a.cpu(), b) for a, b in zip(got, want)), used
+
+
+def test_wide_ids_count_as_int32():
+    """64-bit ids: the low half counts, in the table and in the masked top-k sum alike."""
+    layer, x, sx, ids, wts = layer_and_inputs(tokens=45)
+    want = layer.forward_local(x, sx, ids.int(), wts)
+    wide = ids.clone()
+    wide[::3] += 1 << 32
+    wide[1::3] -= 1 << 40
+    assert torch.equal(layer.forward_local(x, sx, wide, wts), want)
+    for bad in (torch.full_like(ids, (1 << 32) + 8), torch.full_like(ids, 1 << 31)):  # no expert's number, negative
+        assert not layer.forward_local(x, sx, bad, wts).any()
+    for got, ref in zip(moe_sorting(wide, wts, num_experts=8, block_size=16), moe_sorting(ids.int(), wts, num_experts=8, block_size=16)):
+        assert torch.equal(got, ref)
+    odd = torch.empty(wide.numel() + 1, device="cuda", dtype=torch.int64)[1:].view_as(wide).copy_(wide)  # a base of 8 bytes
+    for got, ref in zip(moe_sorting(odd, wts, num_experts=8, block_size=16), moe_sorting(ids.int(), wts, num_experts=8, block_size=16)):
+        assert torch.equal(got, ref)

@@ -160,9 +160,13 @@ cudaError_t launch_moe_reduce(void* y, const void* x, int tokens, int topk, int 
   const T* xt = static_cast<const T*>(x);
   const bool vec = dim % 8 == 0 && aligned16(y) && aligned16(x);
   const int vecs = dim / (vec ? 8 : 2);
+  int log2_cols = 8;
+  while (log2_cols > 0 && vecs <= (128 >> (8 - log2_cols))) --log2_cols;  // threads per token: vecs rounded up to a power of two
+  const int per_block = 256 >> log2_cols;                                 // tokens
   auto launch = [&](auto kernel, int unroll) {
-    return host::launch_dependent(kernel, dim3(tokens, (vecs + 256 * unroll - 1) / (256 * unroll)), 256, 0, s, yt, xt, topk, dim, expert_mask,
-                                  topk_ids, num_experts);
+    const int column_blocks = (vecs - 1) / (unroll << log2_cols) + 1;
+    return host::launch_dependent(kernel, dim3((tokens - 1) / per_block + 1, column_blocks < 65535 ? column_blocks : 65535), 256, 0, s, yt, xt,
+                                  tokens, topk, dim, log2_cols, expert_mask, topk_ids, num_experts);
   };
   if (!vec) return launch(moe_reduce_kernel<T, 2, 1>, 1);
   return vecs > 256 && tokens > 256 ? launch(moe_reduce_kernel<T, 8, 2>, 2) : launch(moe_reduce_kernel<T, 8, 1>, 1);

@@ -631,3 +631,20 @@ def test_int4_nibble_order_matters(dev):
     ref = ref_stage1(d, inter_dim)
     assert moe_oracle.cosine_sim(outs[0].view(tokens, topk, -1), ref) > 0.99
     assert moe_oracle.cosine_sim(outs[1].view(tokens, topk, -1), ref) < 0.9
+
+
+@pytest.mark.parametrize("dim", [2, 8, 16, 18, 40, 64, 66, 128, 254, 256, 520, 1024, 2048, 2056, 2 * 256 * 65536 + 2])
+@pytest.mark.parametrize("tokens", [1, 7, 300])
+def test_topk_sum_of_narrow_and_very_wide_rows(dev, tokens, dim):
+    """Rows of a few vectors share a block, rows past the grid's limit take a second pass: fp32 sum in slot
+    order, one rounding."""
+    topk = 3
+    if dim > 1 << 20:
+        tokens, topk = 1, 2
+    x = torch.randn(tokens, topk, dim, device=dev, dtype=torch.float32).to(torch.bfloat16)
+    y = torch.full((tokens + 1, dim), 7.0, device=dev, dtype=torch.bfloat16)
+    compile_moe_reduction(topk=topk, model_dim=dim, dtype_str="bf16")(x, y[:tokens], None, None, tokens, torch.cuda.current_stream())
+    want = x[:, 0].float()
+    for s in range(1, topk):
+        want = want + x[:, s].float()
+    assert torch.equal(y[:tokens], want.to(torch.bfloat16)) and torch.all(y[tokens:] == 7.0)

@@ -205,12 +205,11 @@ int flyb200_mx_scale_image(void* dst, const void* src, int rows, int K, void* st
   if (!dst || !src || rows <= 0 || K <= 0) return FLYB200_E_BAD_ARG;
   if (K % KBLOCK_BYTES != 0) return FLYB200_E_UNSUPPORTED;
   const int row_tiles = (rows + 127) / 128;
-  if (reinterpret_cast<uintptr_t>(dst) & 3u) return FLYB200_E_BAD_ALIGN;
   const long long total = static_cast<long long>(flyb200_mx_scale_image_bytes(rows, K)) / 4;
   long long blocks = (total + 255) / 256;
   if (blocks > 148 * 8) blocks = 148 * 8;
   CUDA_TRY(host::launch_dependent(mx_scale_image_kernel, dim3(static_cast<unsigned>(blocks)), 256, 0, static_cast<cudaStream_t>(stream),
-                                  static_cast<uint32_t*>(dst), static_cast<const uint8_t*>(src), rows, K / 32, row_tiles));
+                                  static_cast<uint8_t*>(dst), static_cast<const uint8_t*>(src), rows, K / 32, row_tiles));
   return FLYB200_OK;
 }
 

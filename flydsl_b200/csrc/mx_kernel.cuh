@@ -387,14 +387,15 @@ __global__ void __launch_bounds__(MX_THREADS, 1) mx_gemm_kernel(const __grid_con
 
 // Scale image from row-major scales [rows, K/32] (uint8): see the layout above; rows past `rows` read
 // as zero.  A thread moves the four scales of one row and 128-element k-block, a 4-byte word on both
-// sides (at an odd base, where the source words are not aligned, byte by byte).  A call of 1 to 1024
+// sides (byte by byte on a side whose base is not a multiple of four).  A call of 1 to 1024
 // rows of K = 8192 takes 2.0 to 2.4 us, the floor of a launch.
-static __global__ void mx_scale_image_kernel(uint32_t* __restrict__ dst, const uint8_t* __restrict__ src, int rows, int kb32,
+static __global__ void mx_scale_image_kernel(uint8_t* __restrict__ dst, const uint8_t* __restrict__ src, int rows, int kb32,
                                       int row_tiles) {
   pdl_wait(dst, src);
   pdl_trigger();
   const long long total = static_cast<long long>(kb32 / 4) * row_tiles * (MX_SF_ATOM / 4);
   const bool aligned = (reinterpret_cast<uintptr_t>(src) & 3u) == 0;  // rows of kb32 bytes, a multiple of four
+  const bool dst_aligned = (reinterpret_cast<uintptr_t>(dst) & 3u) == 0;
   for (long long i = blockIdx.x * static_cast<long long>(blockDim.x) + threadIdx.x; i < total;
        i += static_cast<long long>(gridDim.x) * blockDim.x) {
     const int w = static_cast<int>(i % (MX_SF_ATOM / 4));  // (r % 32) * 4 + r / 32
@@ -408,7 +409,12 @@ static __global__ void mx_scale_image_kernel(uint32_t* __restrict__ dst, const u
       v = aligned ? __ldg(reinterpret_cast<const uint32_t*>(s))
                   : (__ldg(s) | (__ldg(s + 1) << 8) | (__ldg(s + 2) << 16) | (static_cast<uint32_t>(__ldg(s + 3)) << 24));
     }
-    dst[i] = v;
+    if (dst_aligned) {
+      reinterpret_cast<uint32_t*>(dst)[i] = v;
+    } else {
+#pragma unroll
+      for (int j = 0; j < 4; ++j) dst[4 * i + j] = static_cast<uint8_t>(v >> (8 * j));
+    }
   }
 }
 

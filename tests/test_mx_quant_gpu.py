@@ -4,6 +4,7 @@ codes, scales and (MXFP6) unpacked codes, and the two layout kernels beside them
 import pytest
 import torch
 
+from flydsl_b200 import _lib
 from flydsl_b200.kernels.gemm import mxfp4_preshuffle as mx4
 from flydsl_b200.kernels.gemm import mxfp8_preshuffle as mx8
 
@@ -94,3 +95,14 @@ def test_scale_image_layout(rows, k, offset):
 def test_fp6_containers(rows, k):
     a = torch.randint(0, 256, (rows, k), dtype=torch.uint8)
     assert torch.equal(mx4.fp6_containers_from_padded(a.cuda()).cpu(), mx4.fp6_containers_from_padded(a))
+
+
+@pytest.mark.parametrize("src_shift,dst_shift", [(0, 1), (1, 0), (3, 2), (0, 0)])
+def test_scale_image_at_any_base(src_shift, dst_shift):
+    rows, kb = 200, 16
+    src = torch.randint(0, 256, (rows * kb + src_shift,), device="cuda", dtype=torch.uint8)[src_shift:].view(rows, kb)
+    n = mx8.scale_image_bytes(rows, kb * 32)
+    buf = torch.full((n + dst_shift + 3,), 77, device="cuda", dtype=torch.uint8)
+    rc = _lib.load().flyb200_mx_scale_image(buf.data_ptr() + dst_shift, src.data_ptr(), rows, kb * 32, torch.cuda.current_stream().cuda_stream)
+    assert rc == 0 and torch.equal(buf[dst_shift : dst_shift + n], mx8.shuffle_scale(src.clone()))
+    assert torch.all(buf[:dst_shift] == 77) and torch.all(buf[dst_shift + n :] == 77)

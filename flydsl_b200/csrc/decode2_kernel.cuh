@@ -93,7 +93,6 @@ gemm_decode2_kernel(const __grid_constant__ CUtensorMap tmA, const GemmParams p)
   // stream may still write is read before griddepcontrol.wait (pdl == 2: the
   // weights are static, their first loads go out before it).  An L2 prefetch
   // reads nothing into the SM, so the weights are always requested before it.
-  if (p.pdl) asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
   if (threadIdx.x == 0) {
     for (int s = 0; s < stages; ++s) {
       mbar_init(bar_full + 8 * s, prank == 0 ? 2 : 1);  // leader: its loads and the follower's word
@@ -131,7 +130,10 @@ gemm_decode2_kernel(const __grid_constant__ CUtensorMap tmA, const GemmParams p)
   cluster_barrier_all();  // the barriers of both CTAs exist, the pair's TMEM is allocated
   tc_fence_after();
   const uint32_t tmem_base = *tmem_slot;
-  if (p.pdl && threadIdx.x != 0) asm volatile("griddepcontrol.wait;" ::: "memory");
+  if (p.pdl && threadIdx.x != 0) {
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+    pdl_trigger();  // the next kernel on the stream may be scheduled (its set-up and weight requests overlap this one)
+  }
   // Who sums the K splits after the mainloop: from 64 tokens up all seven warps (the producer and
   // the MMA issuers have nothing left to do by then; measured 2-7 % on the whole kernel at 64-256
   // tokens), below that the four epilogue warps (with so few tokens the extra warps only cost).

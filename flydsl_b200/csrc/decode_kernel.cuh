@@ -248,7 +248,6 @@ __global__ void __launch_bounds__(DECODE_THREADS, 1) gemm_decode_kernel(const __
   //   pdl == 1: no global access at all before the wait.
   //   pdl == 2: the weights are model state that no kernel on the stream
   //             writes, so their first loads are issued before the wait.
-  if (p.pdl) asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
 #ifdef FLYB200_PROFILE
   const unsigned long long prof_t0 = globaltimer_ns();
   if (threadIdx.x == 0) atomicMin(p.prof + 0, prof_t0);
@@ -320,7 +319,10 @@ __global__ void __launch_bounds__(DECODE_THREADS, 1) gemm_decode_kernel(const __
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem_base = *tmem_slot;
-  if (p.pdl && threadIdx.x != 0) asm volatile("griddepcontrol.wait;" ::: "memory");
+  if (p.pdl && threadIdx.x != 0) {
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+    pdl_trigger();  // the next kernel on the stream may be scheduled (its set-up and weight requests overlap this one)
+  }
   // Who sums the K splits after the mainloop: from 64 tokens up all seven warps (the producer and
   // the MMA issuers have nothing left to do by then; measured 2-7 % on the whole kernel at 64-256
   // tokens), below that the four epilogue warps (with so few tokens the extra warps only cost).

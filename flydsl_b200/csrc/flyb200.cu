@@ -271,16 +271,6 @@ struct Plan {
   int prefetch;  // k-blocks of weights requested into L2 ahead of the ring
 };
 
-// 0 = off, 1 = on, 2 = on and the weights are known to be static
-int pdl_default() {
-  static const int mode = []() {
-    const char* e = getenv("FLYB200_PDL");
-    if (!e) return 1;
-    return e[0] == '1' ? 1 : e[0] == '2' ? 2 : 0;
-  }();
-  return mode;
-}
-
 // FLYB200_PREFETCH_DECODE: tuning override of the small-M kernel's prefetch distance (k-blocks); -1 = not set
 int decode_prefetch_override() {
   static const int n = []() {
@@ -503,7 +493,7 @@ int make_plan(Plan* plan, int M, int N, int K_bytes, int variant_hint, size_t wo
   plan->prefetch = 0;  // small-M kernel: set below, once the ring depth is known
   if (plan->decode) plan->prefetch = decode_prefetch_override() >= 0 ? decode_prefetch_override() : plan->stages + 4;
   const int hp = hint_pdl(variant_hint);
-  plan->pdl = hp == 1 ? 1 : hp == 2 ? 0 : hp == 3 ? 2 : pdl_default();
+  plan->pdl = hp == 1 ? 1 : hp == 2 ? 0 : hp == 3 ? 2 : host::pdl_default();
   if (!plan->decode) {
     // Large-M kernels: programmatic dependent launch only for launches of at most two rounds of tiles,
     // where hiding the launch and set-up behind the previous kernel's tail is worth 2-6 % (512 x 4096 x
@@ -661,7 +651,7 @@ int launch_shuffle(void* dst, const void* src, int N, int Kb, cudaStream_t s) {
 }
 
 // Row quantiser launch: rows that fit the register-cached single-pass kernel
-// use it (one block per row), longer rows take the two-pass kernel.
+// use it (one to eight warps per row), longer rows take the two-pass kernel.
 template <typename TIn, bool FP8>
 cudaError_t launch_quant_t(uint8_t* y, float* scale, const TIn* x, int rows, int K, cudaStream_t s) {
   cudaError_t err = cudaSuccess;
@@ -745,6 +735,14 @@ int static_scratch_address(void** out) {
 
 namespace flyb200 {
 namespace host {
+int pdl_default() {
+  static const int mode = []() {
+    const char* e = getenv("FLYB200_PDL");
+    if (!e) return 1;
+    return e[0] == '1' ? 1 : e[0] == '2' ? 2 : 0;
+  }();
+  return mode;
+}
 // Block-scaled GEMM (MXFP8, or MXFP4 with `fp4`) for up to 128 tokens on the small-M (weight-streaming)
 // kernel; K = bytes of codes per row.
 int gemm_mx_small(void* c, const void* a, const void* w, const void* sf_a, const void* sf_w, int M, int N, int K,

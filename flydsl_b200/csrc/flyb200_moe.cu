@@ -273,10 +273,7 @@ int flyb200_moe_gemm(int stage, void* out, const void* a_sorted, const void* w_s
   }
   int bn = 16;
   while (bn < tile_m) bn *= 2;
-  {
-    const char* e = getenv("FLYB200_PDL");
-    p.pdl = (after_gather && !(e && e[0] == '0')) ? 1 : 0;
-  }
+  p.pdl = after_gather && host::pdl_default() != 0 ? 1 : 0;
   rc = host::byte_matrix_map(&tmA, a_sorted, static_cast<uint64_t>(K), static_cast<uint64_t>(blocks) * tile_m, bn);
   if (rc) return rc;
   if (in_dtype == FLYB200_DT_FP8) return launch_moe_bn<KIND_F8>(bn, stage, out_dtype, accumulate != 0, tmA, p, blocks, s);

@@ -46,8 +46,7 @@ int launch_mx(const CUtensorMap& tmA, const MxParams& p, cudaStream_t s) {
   cudaLaunchAttribute attrs[2];
   attrs[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;  // as launch_dependent
   attrs[0].val.programmaticStreamSerializationAllowed = 1;
-  const char* e = getenv("FLYB200_PDL");
-  int na = e && e[0] == '0' ? 0 : 1;
+  int na = host::pdl_default() != 0 ? 1 : 0;
   if (SPLIT) {
     attrs[na].id = cudaLaunchAttributeClusterDimension;
     attrs[na].val.clusterDim.x = static_cast<unsigned>(p.split);

@@ -4,16 +4,16 @@
 #include <cuda_runtime.h>
 #include <cstdint>
 
-#include <cstdlib>
-
 namespace flyb200 {
 namespace host {
+
+// FLYB200_PDL, read once per process: 0 = no programmatic dependent launch, 1 = on, 2 = on and the weights are known to be static.
+int pdl_default();
 
 // Launches a kernel whose first statement is pdl_wait (ptx.cuh) as a programmatic dependent: its launch and
 // set-up overlap the end of the kernel before it on the stream, one to two us each in a chain of small
 // kernels.  Plain stream order / this, us a pass: MoE layer of 32 tokens 57.3 / 49.1, of 4096 282 / 277, its
 // stages one by one (515 tokens) 82.0 / 70.2, MXFP6 layer of 256 tokens 41.4 / 33.9, MXFP8 of 1024 83.5 / 80.3.
-// FLYB200_PDL=0 in the environment launches in plain stream order.
 template <typename... KArgs, typename... Args>
 cudaError_t launch_dependent(void (*kernel)(KArgs...), dim3 grid, int threads, int smem, cudaStream_t s, Args... args) {
   cudaLaunchConfig_t cfg = {};
@@ -24,9 +24,8 @@ cudaError_t launch_dependent(void (*kernel)(KArgs...), dim3 grid, int threads, i
   cudaLaunchAttribute attr;
   attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
   attr.val.programmaticStreamSerializationAllowed = 1;
-  const char* e = getenv("FLYB200_PDL");
   cfg.attrs = &attr;
-  cfg.numAttrs = e && e[0] == '0' ? 0 : 1;
+  cfg.numAttrs = pdl_default() != 0 ? 1 : 0;
   return cudaLaunchKernelEx(&cfg, kernel, static_cast<KArgs>(args)...);
 }
 

@@ -28,3 +28,8 @@ def test_every_trigger_comes_after_a_wait():
             waits = [m.start() for m in re.finditer(r"pdl_wait(<>)?\(|griddepcontrol\.wait;", body)]
             assert waits and waits[0] < first, f"{name}: {body[:120]}"
     assert seen >= 14
+
+
+def test_the_switch_is_read_in_one_place():
+    text = "".join(open(p).read() for p in glob.glob(os.path.join(CSRC, "*")) if p.endswith((".cu", ".cuh", ".h", ".cpp")))
+    assert text.count('getenv("FLYB200_PDL")') == 1

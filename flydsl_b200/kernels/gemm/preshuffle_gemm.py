@@ -17,6 +17,7 @@ reference's runtime ``M`` does.
 from __future__ import annotations
 
 import os
+import threading
 from typing import Optional
 
 import torch
@@ -34,6 +35,7 @@ _TORCH_OUT = {"bf16": torch.bfloat16, "fp16": torch.float16}
 # graph, may hold the address.
 _workspaces: dict = {}
 _retired: list = []
+_growing = threading.Lock()
 _TICKET_BYTES = 16384
 _WORST_CASE_M = (16, 32, 64, 128, 256, 512, 768, 1024)  # every token-block width and count of the small-M kernel
 
@@ -73,11 +75,14 @@ def _workspace(device: torch.device, stream: int, nbytes: int):
                 "preshuffle_gemm: this shape needs a split-K workspace that does not exist yet; call the launcher once "
                 "(or flyc.compile it) on this stream before capturing a CUDA graph"
             )
-        if ws is not None:
-            _retired.append(ws)  # may still be in use by running kernels or captured graphs
-        with _on_stream(device, stream):
-            ws = torch.zeros(nbytes, dtype=torch.uint8, device=device)
-        _workspaces[key] = ws
+        with _growing:  # a buffer that another thread has just handed out must not be replaced unseen
+            ws = _workspaces.get(key)
+            if ws is None or ws.numel() < nbytes:
+                if ws is not None:
+                    _retired.append(ws)  # may still be in use by running kernels or captured graphs
+                with _on_stream(device, stream):
+                    ws = torch.zeros(nbytes, dtype=torch.uint8, device=device)
+                _workspaces[key] = ws
     return ws.data_ptr(), ws.numel()
 
 

@@ -279,13 +279,18 @@ bool routing_takes(const at::Tensor& ids, const at::Tensor& wts, long long exper
   if (wts.device() != ids.device() || wts.layout() != at::kStrided || wts.numel() != ids.numel() || experts <= 0 || block <= 0) return false;
   return ids.numel() + experts * block < (1ll << 31);
 }
+// Sorted rows that the table has room for, and the blocks that cover them.
+int64_t routing_rows(int64_t pairs, int64_t topk, int64_t experts, int64_t block) { return pairs + experts * block - topk; }
+int routing_blocks(int64_t pairs, int64_t topk, int64_t experts, int64_t block) {
+  return static_cast<int>((routing_rows(pairs, topk, experts, block) + block - 1) / block);
+}
 int sort_routes(const at::Tensor& topk_ids, const at::Tensor& topk_weights, int experts, int block, long long first, void* s, Routing& r) {
   const at::ScalarType t = topk_ids.scalar_type();
   const at::Tensor ids = (t == at::kInt || t == at::kLong ? topk_ids : topk_ids.to(at::kInt)).contiguous();
   const at::Tensor w = topk_weights.to(at::kFloat).contiguous();
   const int tokens = static_cast<int>(ids.size(0)), topk = static_cast<int>(ids.size(1));
-  const int64_t padded = static_cast<int64_t>(tokens) * topk + static_cast<int64_t>(experts) * block - topk;
-  r.blocks = static_cast<int>((padded + block - 1) / block);
+  const int64_t padded = routing_rows(ids.numel(), topk, experts, block);
+  r.blocks = routing_blocks(ids.numel(), topk, experts, block);
   const at::TensorOptions i32 = ids.options().dtype(at::kInt);
   r.ids = at::empty({padded}, i32);
   r.weights = at::empty({padded}, ids.options().dtype(at::kFloat));
@@ -360,18 +365,17 @@ PyObject* moe_layer(PyObject*, PyObject* const* argv, Py_ssize_t n) {
   if (!bytes(w1, e * 2 * i * m) || !bytes(w2, e * m * i) || !floats(sw1, e * 2 * i) || !floats(sw2, e * m)) return none();
   for (const at::Tensor* t : {&w1, &w2, &sw1, &sw2, &mask, &a1, &sa1, &a2, &sa2})
     if (t->device() != x.device()) return none();
+  const long long rows = static_cast<long long>(routing_blocks(ids.numel(), topk, experts, tile_m)) * tile_m;
+  if (!bytes(a1, rows * m) || !bytes(a2, rows * i) || !floats(sa1, rows) || !floats(sa2, rows)) return none();
   at::Tensor y;
   int rc;
-  bool fits = true;
   {
     NoGil g;
     const c10::cuda::CUDAGuard dev(x.device());
     void* s = stream_of(x);
     Routing r;
     rc = sort_routes(ids, wts, experts, tile_m, first, s, r);
-    const long long rows = static_cast<long long>(r.blocks) * tile_m;
-    fits = bytes(a1, rows * m) && bytes(a2, rows * i) && floats(sa1, rows) && floats(sa2, rows);
-    if (!rc && fits) {
+    if (!rc) {
       const int t = static_cast<int>(tokens), rn = static_cast<int>(rows);
       const int *ip = as<int>(r.ids), *ep = as<int>(r.experts), *vp = as<int>(r.valid);
       const float* tp = as<float>(r.weights);
@@ -392,7 +396,6 @@ PyObject* moe_layer(PyObject*, PyObject* const* argv, Py_ssize_t n) {
       if (!rc) rc = flyb200_moe_reduce(ptr(y), ptr(out2), t, topk, model, FLYB200_OUT_BF16, as<int>(mask), as<int>(ids32), all, s);
     }
   }
-  if (!fits) return none();
   return rc ? code(rc) : THPVariable_Wrap(y);
   END_HANDLE_TH_ERRORS
 }

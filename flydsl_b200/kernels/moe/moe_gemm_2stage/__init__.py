@@ -309,8 +309,9 @@ class _MoeStage:
     def _launch_quantising(self, out, x16, w, scale_w, sorted_token_ids, sorted_expert_ids, sorted_weights, num_valid_ids,
                            tokens, blocks, stream):
         """Stage 2 on the bf16 rows ``x16 [tokens * topk, inter_dim]`` of stage 1: the quantiser writes the codes
-        straight into sorted order (``pertoken_quant`` and the gather as one kernel).  Same results as both in turn."""
-        if self._k > _lib.MOE_QUANT_MAX_K or blocks == 0 or tokens == 0:
+        straight into sorted order (``pertoken_quant`` and the gather as one kernel).  Same results as both in turn.
+        8-bit weights as the kernel reads them (packed int4 ones go through ``_launch``)."""
+        if self.in_dtype == "int4" or self._k > _lib.MOE_QUANT_MAX_K or blocks == 0 or tokens == 0:
             from ....utils import pertoken_quant
 
             x, sx = pertoken_quant(x16, quant_dtype=self._torch_in)
@@ -327,23 +328,16 @@ class _MoeStage:
                     tokens, self.topk, self._k, rows, self._dt, s)
                 if rc:
                     _lib.check(rc, "moe_quant_sorted")
-                self._gemm(out, a_sorted, sa_sorted, w, scale_w, sorted_token_ids, sorted_expert_ids, sorted_weights, num_valid_ids,
-                           tokens, blocks, s)
+                rc = _lib.load().flyb200_moe_gemm(
+                    self.stage, out.data_ptr(), a_sorted.data_ptr(), w.data_ptr(), sa_sorted.data_ptr(), scale_w.data_ptr(),
+                    sorted_token_ids.data_ptr(), sorted_expert_ids.data_ptr(),
+                    sorted_weights.data_ptr() if sorted_weights is not None and sorted_weights.numel() else None,
+                    num_valid_ids.data_ptr(), tokens, self.topk, self.experts, self.model_dim, self.inter_dim, self.tile_m, blocks,
+                    self._dt, self._out, int(self.doweight), int(self.accumulate), 1, s,
+                )  # fmt: skip
+                if rc:
+                    _lib.check(rc, "moe_gemm")
         return None
-
-    def _gemm(self, out, a_sorted, sa_sorted, w, scale_w, sorted_token_ids, sorted_expert_ids, sorted_weights, num_valid_ids,
-              tokens, blocks, s):
-        if self.in_dtype == "int4":
-            w = self._weights_for_kernel(w, self.experts * (2 * self.inter_dim if self.stage == 1 else self.model_dim) * self._k)
-        rc = _lib.load().flyb200_moe_gemm(
-            self.stage, out.data_ptr(), a_sorted.data_ptr(), w.data_ptr(), sa_sorted.data_ptr(), scale_w.data_ptr(),
-            sorted_token_ids.data_ptr(), sorted_expert_ids.data_ptr(),
-            sorted_weights.data_ptr() if sorted_weights is not None and sorted_weights.numel() else None, num_valid_ids.data_ptr(),
-            tokens, self.topk, self.experts, self.model_dim, self.inter_dim, self.tile_m, blocks, self._dt, self._out,
-            int(self.doweight), int(self.accumulate), 1, s,
-        )
-        if rc:
-            _lib.check(rc, "moe_gemm")
 
 
 def _check_common(model_dim, inter_dim, experts, topk, tile_m, tile_n, tile_k, in_dtype, k):

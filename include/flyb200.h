@@ -302,7 +302,7 @@ int flyb200_moe_gemm(int stage, void* out, const void* a_sorted, const void* w_s
 /* Routing table from the router's choice: the device form of the reference's
  * moe_sorting (layout stated in tests/kernels/test_moe_gemm_2stage.py:99-137; the
  * reference's own device kernel is kernels/moe/moe_sorting_kernel.py).  A stable
- * counting sort of the (token, slot) pairs by expert; three small launches on
+ * counting sort of the (token, slot) pairs by expert; one small launch on
  * the stream, no host synchronisation, so the whole MoE layer can be captured.
  *   topk_ids[tokens, topk] int32, topk_weights[tokens, topk] fp32
  *   sorted_ids / sorted_weights  [tokens * topk + experts * block_size - topk]

@@ -122,11 +122,14 @@ def test_moe_layer_forms(monkeypatch, in_dtype, rank, world):
     wide[:, : x.shape[1]] = x.view(torch.uint8)
     strided = wide[:, : x.shape[1]].view(x.dtype)
     variants = [(x, sx.view(-1), ids.int(), wts), (x, sx, ids.to(torch.int16), wts.double()), (strided, sx, ids, wts),
-                (x, sx, ids.t().contiguous().t(), wts.t().contiguous().t()), (x, sx.view(1, -1), ids, wts.half().float())]
-    for v in variants[:-1]:
+                (x, sx, ids.t().contiguous().t(), wts.t().contiguous().t()), (x, sx.view(1, -1), ids, wts)]
+    for v in variants:
         assert torch.equal(layer.forward_local(*v), want)
+    rounded = layer.forward_local(x, sx.view(1, -1), ids, wts.half())
+    assert not torch.equal(rounded, want)
     monkeypatch.setattr(layer, "_forward_native", lambda *a: None)  # the statements one by one
     assert torch.equal(layer.forward_local(x, sx, ids, wts), want)
+    assert torch.equal(layer.forward_local(x, sx, ids, wts.half()), rounded)
 
 
 def test_moe_layer_on_streams_threads_and_in_a_graph():

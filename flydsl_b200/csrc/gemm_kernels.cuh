@@ -105,13 +105,15 @@ __device__ __forceinline__ void report_failure(int* status, int code, volatile i
 }
 
 // acc (raw 32-bit from TMEM) -> scaled/activated fp32, in the reference's
-// operation order: float(acc); (v * sa[row]) * sb[col]; + bias; activation.
+// operation order: float(acc); (v * sa[row]) * sb[col]; + bias; activation.  Scales
+// and bias are rounded one by one, here and wherever a kernel does the same on
+// several values at once.
 template <bool IS_INT>
 __device__ __forceinline__ float epilogue_value(uint32_t raw, float sa, float sb, float bias, int epi, bool scaled) {
   float v = IS_INT ? static_cast<float>(static_cast<int32_t>(raw)) : __uint_as_float(raw);
-  if (scaled) v = (v * sa) * sb;
+  if (scaled) v = __fmul_rn(__fmul_rn(v, sa), sb);
   if (epi != EPI_NONE) {
-    v = v + bias;
+    v = __fadd_rn(v, bias);
     if (epi == EPI_BIAS_RELU) {
       v = fmaxf(v, 0.0f);
     } else if (epi == EPI_BIAS_SILU) {
@@ -166,8 +168,9 @@ __device__ __forceinline__ float reciprocal_of(float x) {
 }
 
 // The activation of epilogue_value on N values at once: the kind is a template argument and nothing
-// branches per value, so the chains (exponential, reciprocal) overlap.  Same operations in the same
-// order, same results.
+// branches per value, so the chains (exponential, reciprocal) overlap.  The operations and their order
+// are those of epilogue_value but for the reciprocal of the silu and gelu denominators, which
+// reciprocal_of takes without a division: for at most 32 of its 2^23 mantissas one unit of fp32 apart.
 template <int EPI, int N>
 __device__ __forceinline__ void activate(float (&v)[N]) {
   if constexpr (EPI == EPI_BIAS_RELU) {

@@ -842,7 +842,7 @@ static __global__ void moe_gather_rows_kernel(uint8_t* __restrict__ dst, float* 
 // token * topk + slot of `x`, quantises it (quant_kernel.cuh) and writes codes and scale where the down
 // projection reads them; padding rows, and rows past num_valid, become zero with scale zero.  Saves the
 // write and the read of the codes in between and a launch, and rows of routes that nobody sorted are never
-// read.  Bound by memory: 8192 routes x 2048 12.0 us against 12.0 (quantiser) + 8.6 (gather); the layer of 4096
+// read.  Bound by memory: alone, 8192 routes x 2048 12.0 us against 12.0 (quantiser) + 8.6 (gather); the layer of 4096
 // tokens x top-2 x 4096 x 2048 goes from 295 to 284 us, of 32 tokens from 115 to 88 (a launch and two allocations).
 template <bool FP8, int NV, int WPR>
 __global__ void __launch_bounds__(256)
@@ -888,8 +888,9 @@ moe_quant_sorted_kernel(uint8_t* __restrict__ y, float* __restrict__ scale, cons
 // without talking to the others), then walks the pairs once more and writes its own
 // run, its padding and its share of the tail behind the last run.  Latency-bound: a
 // chunk is four pairs per thread, one barrier, so 4096 pairs cost about a microsecond.
-// Measured (pairs / experts, one kernel against memset + count + a walk of 256 pairs at
-// a time, us): 64 / 8 4.4 against 5.0, 2060 / 16 5.4 against 11.5, 8192 / 8 9.5 against 29.
+// Measured alone (pairs / experts, one kernel against memset + count + a walk of 256 pairs at
+// a time, us): 64 / 8 4.4 against 5.0, 2060 / 16 5.4 against 11.5, 8192 / 8 9.5 against 29.  (In a chain of
+// programmatic dependents it starts early and waits, which a profile counts to it: 17.5 us for the last.)
 constexpr int MOE_SORT_MAX_THREADS = 1024;
 constexpr int MOE_SORT_BINS = 4096;  // experts counted per pass over the pairs
 

@@ -5,6 +5,7 @@ import numpy as np
 import pytest
 import torch
 
+from flydsl_b200 import compile_preshuffle_gemm, shuffle_weight
 from oracle import a8w8_oracle as oracle
 from tests.test_gemm_parity_gpu import ATOL, ROWS, RTOL, TALL, run_gemm_generic
 
@@ -77,3 +78,25 @@ def test_last_round_in_strips_is_bit_identical(monkeypatch, m, n, width, in_dtyp
     assert torch.equal(outs[0], outs[1])
     ref = oracle.epilogue(a.float() @ b.float().T, sa, sb, bias, "bias_gelu", out_dtype=torch.float32)
     assert oracle.strict_mismatches(outs[1], ref, RTOL, ATOL) == 0
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("epilogue", ["none", "bias", "bias_relu", "bias_silu", "bias_gelu"])
+@pytest.mark.parametrize("m", [1, 16, 40])
+def test_direct_and_reduced_stores_of_the_small_m_kernel_agree(m, epilogue):
+    """The same integer accumulators through the unsplit kernel (stored from the accumulator layout) and through
+    K splits (summed exactly, stored after the reduction, four values at a time): the same bits."""
+    n, k = 512, 4096
+    g = torch.Generator(device="cuda").manual_seed(m)
+    a = torch.randint(-127, 128, (m, k), generator=g, device="cuda", dtype=torch.int8)
+    b = torch.randint(-127, 128, (n, k), generator=g, device="cuda", dtype=torch.int8)
+    sa, sb = (torch.rand(r, generator=g, device="cuda") * 2e-3 + 1e-4 for r in (m, n))
+    bias = torch.randn(n, generator=g, device="cuda").to(torch.float16)
+    outs = []
+    for hint in (1 << 8 | 1, 1 << 8 | 1 << 12 | 4, 1 << 8 | 2 << 12 | 4):  # unsplit, through a workspace, inside a cluster
+        fn = compile_preshuffle_gemm(N=n, K=k, tile_m=64, tile_n=128, tile_k=128, in_dtype="int8", out_dtype="fp16", epilogue=epilogue,
+                                     variant_hint=hint)
+        c = torch.empty(m, n, device="cuda", dtype=torch.float16)
+        fn(c.view(-1), a.view(-1), shuffle_weight(b).view(-1), sa, sb, bias, m, n, torch.cuda.current_stream())
+        outs.append(c)
+    assert torch.equal(outs[0], outs[1]) and torch.equal(outs[0], outs[2])

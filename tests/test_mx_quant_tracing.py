@@ -64,7 +64,7 @@ def test_codes_carry_the_gradient():
     with fw.dual_level():
         dual = fw.make_dual(x.detach(), up)
         tangents = [fw.unpack_dual(q(dual)[0].float()).tangent for q in (mx8.per_1x32_f8_quant, mx8.per_1x32_f8_quant_torch)]
-        assert torch.equal(*tangents)
+        assert same(*tangents)  # bit by bit: tangents past the range of the codes are NaN
 
 
 class Sub(torch.Tensor):

@@ -45,9 +45,10 @@ def product(fmt, x, w, out_dtype):
 
 
 def bound(exact, magnitude, k, out_dtype):
-    """Half a unit of the output, and the sum in fp32: one addition per 32 products and per part, each off by
-    at most 2^-23 of what has been added so far, which the sum of the magnitudes bounds."""
-    return 2.0 ** (-9 if out_dtype == "bf16" else -12) * exact.abs() + (k / 32 + 10) * 2.0**-23 * magnitude
+    """Half a unit of the output (8 and 11 significant bits: at most 2^-8 and 2^-11 of the value), and the sum in
+    fp32: one addition per 32 products and per part, each off by at most 2^-23 of what has been added so far,
+    which the sum of the magnitudes bounds."""
+    return 2.0 ** (-8 if out_dtype == "bf16" else -11) * exact.abs() + (k / 32 + 10) * 2.0**-23 * magnitude
 
 
 @pytest.mark.parametrize("fmt", ["mxfp8", "mxfp4", "mxfp6"])

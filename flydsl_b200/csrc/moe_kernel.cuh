@@ -153,10 +153,11 @@ __global__ void __launch_bounds__(MOE_THREADS) moe_gemm_kernel(const __grid_cons
   // Blocks past the end of the sorted list, and blocks without an expert, have no work.
   const int blk = blockIdx.x;
   const int row0 = blk * p.tile_m;  // first sorted row of the block
-  // They leave behind the kernel they depend on too: a grid of nothing else must not complete before it.
+  // They leave at once, so that CTAs with work get their SMs - but for the first CTA: a grid of nothing else must
+  // not complete before the kernel it depends on.
   const int expert = row0 >= __ldg(p.num_valid) ? -1 : __ldg(p.expert_ids + blk);
   if (expert < 0 || expert >= p.experts) {
-    if (p.pdl) pdl_wait<>();
+    if (p.pdl && blockIdx.x == 0 && blockIdx.y == 0) pdl_wait<>();
     return;
   }
   if ((smem_base & 1023u) != 0) {

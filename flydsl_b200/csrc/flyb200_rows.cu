@@ -45,7 +45,8 @@ int launch_rows(const CUtensorMap& tmA, const CUtensorMap& tmC, GemmParams p, in
     if (e[0] == '0') p.tail_parts = 1;
   }
   const int grid = static_cast<int>(tiles < sms ? tiles : sms);
-  return launch_plain_or_pdl(kernel, grid, ROWS_THREADS, L.total, s, p.pdl != 0, tmA, tmC, p);
+  const int threads = 64 + 32 * rows_epilogue_warps(p.K_bytes / KBLOCK_BYTES, tiles, sms);
+  return launch_plain_or_pdl(kernel, grid, threads, L.total, s, p.pdl != 0, tmA, tmC, p);
 }
 
 // One CTA per 256 x bn tile (tmA: boxes of 256 rows).
@@ -112,7 +113,8 @@ int launch_rows_scatter(const CUtensorMap& tmA, const OutputMaps& outs, GemmPara
   const long long tiles = static_cast<long long>((p.M + BLOCK_ROWS - 1) / BLOCK_ROWS) * ((p.N + p.bn - 1) / p.bn);
   p.tail_parts = 1;
   const int grid = static_cast<int>(tiles < sms ? tiles : sms);
-  kernel<<<grid, ROWS_THREADS, L.total, s>>>(tmA, outs, p);
+  const int threads = 64 + 32 * rows_epilogue_warps(p.K_bytes / KBLOCK_BYTES, tiles, sms);
+  kernel<<<grid, threads, L.total, s>>>(tmA, outs, p);
   FLYB200_CUDA_TRY(cudaGetLastError());
   return FLYB200_OK;
 }

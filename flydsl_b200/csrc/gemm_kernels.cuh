@@ -294,13 +294,13 @@ __device__ __forceinline__ void epilogue_32(int epi, const uint32_t (&r)[32], fl
 // several GPUs), starting with map `dst_first` (+ a per-tile, per-warp rotation)
 // so that neither the ranks nor the tiles of one rank all hit the same peer at
 // the same time.
-// CBUFS: staging buffers of this warp at `stage_c` (two: the store of one chunk overlaps the
+// cbufs: staging buffers of this warp at `stage_c` (two: the store of one chunk overlaps the
 // conversion of the next; one: where shared memory is short).
-// SHARE: warps that share these 32 rows; this one, `part`, takes every SHARE-th chunk of 64 columns.
-template <int KIND, int OUTMODE, int CBUFS = 2, int SHARE = 1, typename ReleaseFn>
+// share: warps that share these 32 rows; this one, `part`, takes every share-th chunk of 64 columns.
+template <int KIND, int OUTMODE, typename ReleaseFn>
 __device__ __forceinline__ void epilogue_warp_tile(const GemmParams& p, const CUtensorMap* tmC, int n_dst, int dst_first,
                                                    uint32_t t_row, int m0, int n0, int BN, int lane, uint32_t stage_c,
-                                                   int& cbuf, ReleaseFn release_tmem, int part = 0) {
+                                                   int& cbuf, ReleaseFn release_tmem, int cbufs = 2, int share = 1, int part = 0) {
   using KT = KindTraits<KIND>;
   constexpr int C_BUF = 32 * 128;
   const bool scaled = (p.sa != nullptr) && (p.sb != nullptr);
@@ -309,7 +309,7 @@ __device__ __forceinline__ void epilogue_warp_tile(const GemmParams& p, const CU
   if constexpr (OUTMODE == OUT_RAW32) {
     uint32_t* out = reinterpret_cast<uint32_t*>(p.c);
 #pragma unroll 1
-    for (int c0 = 32 * part; c0 < BN; c0 += 32 * SHARE) {
+    for (int c0 = 32 * part; c0 < BN; c0 += 32 * share) {
       uint32_t r[32];
       tmem_ld_x32(t_row + c0, r);
       tmem_ld_wait();
@@ -333,7 +333,7 @@ __device__ __forceinline__ void epilogue_warp_tile(const GemmParams& p, const CU
     ColumnFactors f;
     if (64 * part >= BN) release_tmem();  // nothing to do for this warp
 #pragma unroll 1
-    for (int c0 = 64 * part; c0 < BN; c0 += 64 * SHARE) {
+    for (int c0 = 64 * part; c0 < BN; c0 += 64 * share) {
       if (c0 + 64 > BN) {
         // Last 32 columns of a tile whose width is not a multiple of 64: a
         // 64-column TMA box would reach into the neighbouring tile, so these
@@ -353,7 +353,10 @@ __device__ __forceinline__ void epilogue_warp_tile(const GemmParams& p, const CU
         break;
       }
       // the store that last used this buffer (two chunks ago with two buffers) has to be done reading it
-      if (lane == 0) bulk_wait_group_read<CBUFS - 1>();
+      if (lane == 0) {
+        if (cbufs == 1) bulk_wait_group_read<0>();
+        else bulk_wait_group_read<1>();
+      }
       __syncwarp();
       const uint32_t cdst = stage_c + cbuf * C_BUF + lane * 128;
 #pragma unroll 1
@@ -363,7 +366,7 @@ __device__ __forceinline__ void epilogue_warp_tile(const GemmParams& p, const CU
         load_column_factors(f, p, n0 + c0 + 32 * h, scaled, vec);
         tmem_ld_wait();
         // this warp's last read of the accumulator: hand the TMEM buffer back
-        if (h == 1 && c0 + 64 * SHARE >= BN) release_tmem();
+        if (h == 1 && c0 + 64 * share >= BN) release_tmem();
         epilogue_32<KT::is_int, OUTMODE>(p.epilogue, r, sa_v, f, [&](int g, const uint32_t (&pk)[4]) {
           const int chunk = 4 * h + g;  // 16-byte chunk index inside the 128-byte row
           st_smem_v4(cdst + static_cast<uint32_t>(((chunk ^ (lane & 7)) << 4)), pk[0], pk[1], pk[2], pk[3]);
@@ -380,7 +383,7 @@ __device__ __forceinline__ void epilogue_warp_tile(const GemmParams& p, const CU
         }
         bulk_commit_group();
       }
-      cbuf = (cbuf + 1) % CBUFS;
+      cbuf = cbufs == 1 ? 0 : cbuf ^ 1;
     }
   }
 }
@@ -394,14 +397,14 @@ struct RowsLayout {
   int a_stage, b_stage, off_b, off_c, off_bar, off_misc, total;
 };
 constexpr int ROWS_C_BUF = 32 * 128;  // staging buffer: 32 rows x 64 two-byte columns
-constexpr int ROWS_THREADS = 64 + 8 * 32;  // producer, MMA issuer, eight epilogue warps (two per 32 rows)
+constexpr int ROWS_THREADS = 64 + 8 * 32;  // at most: producer, MMA issuer, eight epilogue warps (two per 32 rows); or four
 constexpr int ROWS_ACC_COLS = 256;    // TMEM columns between the two accumulator buffers
 __host__ __device__ inline RowsLayout rows_layout(int bn, int stages) {
   RowsLayout l;
   l.a_stage = BLOCK_ROWS * KBLOCK_BYTES;
   l.b_stage = bn * KBLOCK_BYTES;
   l.off_b = stages * l.a_stage;
-  l.off_c = l.off_b + stages * l.b_stage;       // one buffer per epilogue warp
+  l.off_c = l.off_b + stages * l.b_stage;       // eight buffers: one per epilogue warp, or two for each of four
   l.off_bar = l.off_c + 8 * ROWS_C_BUF;         // full[S], empty[S], tfull[2], tempty[2]
   l.off_misc = l.off_bar + 8 * (2 * stages + 4);
   l.total = l.off_misc + 16;
@@ -456,7 +459,7 @@ __device__ __forceinline__ void gemm_rows_body(const CUtensorMap& tmA, const CUt
     }
     for (int s = 0; s < 2; ++s) {
       mbar_init(bar_tfull + 8 * s, 1);
-      mbar_init(bar_tempty + 8 * s, 8);
+      mbar_init(bar_tempty + 8 * s, (blockDim.x - 64) >> 5);  // every epilogue warp
     }
     abort_flag[0] = 0;
     abort_flag[1] = 0;  // stays zero: lets the drain below wait on time alone
@@ -627,7 +630,9 @@ __device__ __forceinline__ void gemm_rows_body(const CUtensorMap& tmA, const CUt
     // ------------------------------ epilogue ------------------------------
     const int q = warp & 3;  // TMEM lane quadrant this warp may read
     const int ew = warp - 2; // staging buffer owner
-    const uint32_t stage_c = smem_base + L.off_c + ew * ROWS_C_BUF;
+    const int share = (static_cast<int>(blockDim.x) - 64) >> 7;  // epilogue warps per 32 rows (host: rows_epilogue_warps)
+    const int cbufs = 2 / share;
+    const uint32_t stage_c = smem_base + L.off_c + ew * cbufs * ROWS_C_BUF;
     int acc = 0;
     uint32_t acc_phase = 0;
     int cbuf = 0;
@@ -646,11 +651,11 @@ __device__ __forceinline__ void gemm_rows_body(const CUtensorMap& tmA, const CUt
           tmem_base + (static_cast<uint32_t>(q * 32) << 16) + static_cast<uint32_t>(acc * ROWS_ACC_COLS);
       // own buffer first for the first tile; every further tile and warp starts one destination later
       const int first = n_dst > 1 ? (dst_first + (t / static_cast<int>(gridDim.x)) + ew) % n_dst : 0;
-      epilogue_warp_tile<KIND, OUTMODE, 1, 2>(p, tmC_ptr, n_dst, first, t_row, m0, n0, width, lane, stage_c, cbuf, [&]() {
+      epilogue_warp_tile<KIND, OUTMODE>(p, tmC_ptr, n_dst, first, t_row, m0, n0, width, lane, stage_c, cbuf, [&]() {
         tc_fence_before();
         __syncwarp();
         if (lane == 0) mbar_arrive(bar_tempty + 8 * acc);
-      }, ew >> 2);
+      }, cbufs, share, ew >> 2);
       acc ^= 1;
       if (acc == 0) acc_phase ^= 1u;
     }

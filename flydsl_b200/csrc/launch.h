@@ -5,6 +5,7 @@
 #include "host_common.h"
 
 #include <atomic>
+#include <cstdlib>
 
 namespace flyb200 {
 namespace host {
@@ -40,15 +41,29 @@ inline int rows_stages_for(int bn) {
 }
 
 // Column strips of the tiles of the large-M kernel's last round, where that is at most half full (1: none): two or
-// four strips per tile while every SM gets at most one; strips are multiples of 64 columns (the stores' box).  The
-// round is short of power rather than of time (fewer busy SMs clock higher), so the gain is small: whole tiles /
-// strips, us, fp16 4096 x 4096 x 4096 (3.46 rounds of tiles) 104.1 / 102.8, fp8 55.4 / 54.2; even where the last
-// round is more than half full (no strips) or one of many.
+// four strips per tile while every SM gets at most one; strips are multiples of 64 columns (the stores' box).  At one
+// width the gain is small, as the round is short of power rather than of time (fewer busy SMs clock higher): whole tiles /
+// strips, us, fp16 4096 x 4096 x 4096 (3.46 rounds of tiles) 104.1 / 102.8, fp8 55.4 / 54.2.  But strips also make 256-column tiles
+// of a little more than whole rounds pay, which the planner then prefers to narrower ones in whole rounds: 96 shapes
+// (512..8192 x 3584..28672, K = 2048..8192, fp8 and bf16) whose width changed from 192 or 224 to 256 take 0.85..1.07 of the time
+// (median 0.96; fp8 4096 x 6144 x 2048 55.7 -> 47.2, bf16 3000 x 3584 x 4096 84.1 -> 89.7).
 inline int rows_tail_parts(int bn, long long tiles, int sms) {
   const long long rest = tiles % sms;
   if (tiles < sms || rest == 0 || bn % 128 != 0) return 1;
   if (bn == 256 && 4 * rest <= sms) return 4;
   return 2 * rest <= sms ? 2 : 1;
+}
+
+// Epilogue warps of the large-M kernel.  With few k-blocks a tile's epilogue is as long as the mainloop that it overlaps,
+// and in a launch of few rounds the last one is exposed: eight warps.  In long launches over 32 k-blocks and more the
+// epilogue is hidden either way and four warps leave more power to the tensor cores.  Eight / four, us, fp8:
+// K = 1024 4096 x 14336 74.5 / 108, K = 2048 with silu 2048 x 8192 46.5 / 58.8; K = 8192 (at the power cap) 8192 x 28672 1539 / 1519, with gelu 1587 / 1431,
+// 16384 x 57344 6081 / 5989.
+// FLYB200_ROWS_EPI = 4 or 8 forces the number (tuning and tests).
+inline int rows_epilogue_warps(int kb, long long tiles, int sms) {
+  if (const char* e = getenv("FLYB200_ROWS_EPI"))
+    if (e[0] == '4' || e[0] == '8') return e[0] - '0';
+  return kb >= 32 && tiles >= 8LL * sms ? 4 : 8;
 }
 
 // Large-M kernel (p.bn, p.rows_stages set) in one of three forms: one CTA per 128 x bn tile, CTA pairs

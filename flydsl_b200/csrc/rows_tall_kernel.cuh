@@ -212,11 +212,11 @@ gemm_rows_tall_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_cons
       }
       tc_fence_after();
       const uint32_t t_row = tmem_base + (static_cast<uint32_t>(q * 32) << 16) + static_cast<uint32_t>(half * ROWS_ACC_COLS);
-      epilogue_warp_tile<KIND, OUTMODE, 1>(p, &tmC, 1, 0, t_row, m0, n0, BN, lane, stage_c, cbuf, [&]() {
+      epilogue_warp_tile<KIND, OUTMODE>(p, &tmC, 1, 0, t_row, m0, n0, BN, lane, stage_c, cbuf, [&]() {
         tc_fence_before();
         __syncwarp();
         if (lane == 0) mbar_arrive(bar_tempty);
-      });
+      }, 1);
       acc_phase ^= 1u;
     }
     if (lane == 0) bulk_wait_group<0>();

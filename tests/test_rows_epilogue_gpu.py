@@ -100,3 +100,27 @@ def test_direct_and_reduced_stores_of_the_small_m_kernel_agree(m, epilogue):
         fn(c.view(-1), a.view(-1), shuffle_weight(b).view(-1), sa, sb, bias, m, n, torch.cuda.current_stream())
         outs.append(c)
     assert torch.equal(outs[0], outs[1]) and torch.equal(outs[0], outs[2])
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("epilogue", ["none", "bias_silu"])
+@pytest.mark.parametrize("in_dtype,out_dtype,hint", [("fp8", "bf16", ROWS | 8), ("int8", "fp16", ROWS | 7), ("fp16", "fp16", ROWS | 3), ("bf16", "bf16", ROWS | 1)])
+def test_four_and_eight_epilogue_warps_store_the_same_bits(monkeypatch, in_dtype, out_dtype, epilogue, hint):
+    """Tiles of 256, 224 (a 32-column tail), 96 and 32 columns, several rounds, ragged M and N."""
+    dev = torch.device("cuda:0")
+    m, n, k = 2300, 2064, 512
+    g = torch.Generator().manual_seed(hint)
+    bias = torch.randn(n, generator=g).to(torch.float16 if out_dtype == "fp16" else torch.bfloat16)
+    if in_dtype in ("bf16", "fp16"):
+        dt = torch.bfloat16 if in_dtype == "bf16" else torch.float16
+        a, b, sa, sb = torch.randn(m, k, generator=g).to(dt), (torch.randn(n, k, generator=g) * 0.05).to(dt), None, None
+    else:
+        a, b, sa, sb = oracle.make_inputs(m, n, k, in_dtype, seed=hint)
+    outs = []
+    for warps in ("4", "8"):
+        monkeypatch.setenv("FLYB200_ROWS_EPI", warps)
+        outs.append(run_gemm_generic(dev, a, b, sa, sb, bias if epilogue != "none" else None, m, n, k, in_dtype, out_dtype=out_dtype,
+                                     epilogue=epilogue, hint=hint))
+    assert torch.equal(outs[0], outs[1])
+    ref = oracle.epilogue(a.float() @ b.float().T, sa, sb, bias, epilogue, out_dtype=torch.float32)
+    assert oracle.strict_mismatches(outs[0], ref, RTOL, ATOL) == 0

@@ -97,7 +97,7 @@ int launch_moe_rows(const CUtensorMap& tmA, const MoeParams& p, int blocks, cuda
   const int pairs = STAGE == 1 ? (p.n_out + BLOCK_ROWS - 1) / BLOCK_ROWS : (p.n_out + MOE_ROWS_BN - 1) / MOE_ROWS_BN;
   const long long items = row_blocks * pairs;
   const int grid = static_cast<int>(items < sms ? items : sms);
-  CUDA_TRY(host::launch_dependent(kernel, dim3(grid), MOE_ROWS_THREADS, MoeRowsSmem::TOTAL, s, tmA, p));
+  CUDA_TRY(host::launch_dependent(kernel, dim3(grid), moe_rows_threads(STAGE), MoeRowsSmem::TOTAL, s, tmA, p));
   return FLYB200_OK;
 }
 

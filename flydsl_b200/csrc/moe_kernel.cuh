@@ -388,7 +388,7 @@ __global__ void __launch_bounds__(MOE_THREADS) moe_gemm_kernel(const __grid_cons
 // neighbouring tiles), one CTA per SM walking the (row block, channel pair)
 // items, a shared-memory ring that keeps streaming across items and two TMEM
 // accumulators so that the epilogue of an item overlaps the mainloop of the
-// next.  A thread of the epilogue owns one token row (two warps per 32 rows): it
+// next.  A thread of the epilogue owns one token row (stage 2: two warps per 32 rows): it
 // reads the gate and up columns of the same channel from its own TMEM lane; the
 // outputs leave through store_rows32.
 constexpr int MOE_ROWS_STAGES = 4;
@@ -396,14 +396,18 @@ constexpr int MOE_ROWS_BN = 2 * BLOCK_ROWS;
 constexpr int MOE_ROWS_GROUP = 32;  // row blocks per rasterisation group (16 MiB of activations at K = 4096)
 
 constexpr int STORE_STAGE = 32 * 64;  // shared memory of a warp for store_rows32, bytes
-constexpr int MOE_ROWS_THREADS = 64 + 8 * 32;  // producer, MMA issuer, eight epilogue warps
+// Producer, MMA issuer and epilogue warps: eight where the epilogue is as long as the mainloop it overlaps (the down
+// projection), four for the gate-up stage, whose K is longer: eight / four, us, gather included, 4096 tokens x top-2 x 4096 x
+// 2048 136.0 / 132.8, 515 x top-4 x 2048 x 1408 29.0 / 28.5, 1024 x top-2 x 4096 x 2048 51.5 / 51.2.
+__host__ __device__ constexpr int moe_rows_epilogue_warps(int stage) { return stage == 1 ? 4 : 8; }
+__host__ __device__ constexpr int moe_rows_threads(int stage) { return 64 + 32 * moe_rows_epilogue_warps(stage); }
 struct MoeRowsSmem {
   static constexpr int A_STAGE = BLOCK_ROWS * KBLOCK_BYTES;
   static constexpr int B_STAGE = MOE_ROWS_BN * KBLOCK_BYTES;
   static constexpr int OFF_A = 0;
   static constexpr int OFF_B = OFF_A + MOE_ROWS_STAGES * A_STAGE;
   static constexpr int OFF_C = OFF_B + MOE_ROWS_STAGES * B_STAGE;    // 8 warps x one store stage
-  static constexpr int OFF_SW = OFF_C + 8 * STORE_STAGE;             // 8 warps x 128 weight scales
+  static constexpr int OFF_SW = OFF_C + 8 * STORE_STAGE;             // 1024 weight scales: 8 warps x 128 or 4 x 256
   static constexpr int OFF_BAR = OFF_SW + 8 * BLOCK_ROWS * 4;        // full[S], empty[S], tfull[2], tempty[2]
   static constexpr int OFF_MISC = OFF_BAR + 8 * (2 * MOE_ROWS_STAGES + 4);
   static constexpr int TOTAL = OFF_MISC + 16;
@@ -483,7 +487,7 @@ __device__ __forceinline__ void store_rows32(void* out, const long long (&rows)[
 }
 
 template <int KIND, int STAGE, int OUTMODE, bool ACCUM>
-__global__ void __launch_bounds__(MOE_ROWS_THREADS, 1) moe_rows_kernel(const __grid_constant__ CUtensorMap tmA,
+__global__ void __launch_bounds__(moe_rows_threads(STAGE), 1) moe_rows_kernel(const __grid_constant__ CUtensorMap tmA,
                                                                   const MoeParams p) {
   static_assert(STAGE == 2 || !ACCUM, "only the down projection accumulates");
   using L = MoeRowsSmem;
@@ -512,7 +516,7 @@ __global__ void __launch_bounds__(MOE_ROWS_THREADS, 1) moe_rows_kernel(const __g
     }
     for (int s = 0; s < 2; ++s) {
       mbar_init(bar_tfull + 8 * s, 1);
-      mbar_init(bar_tempty + 8 * s, 8);
+      mbar_init(bar_tempty + 8 * s, moe_rows_epilogue_warps(STAGE));
     }
     abort_flag[0] = 0;
     abort_flag[1] = 0;
@@ -689,11 +693,12 @@ __global__ void __launch_bounds__(MOE_ROWS_THREADS, 1) moe_rows_kernel(const __g
     }
   } else {
     // ------------------------------ epilogue ------------------------------
-    // Eight warps, two per TMEM lane quadrant; of the 128 channels of each tile (stage 1) or of the two
-    // tiles (stage 2) a warp takes one half.
+    // Stage 1: one warp per TMEM lane quadrant, all 128 channels of the gate and of the up tile.  Stage 2: two, each
+    // with the 128 channels of one of the two tiles.
     const int q = warp & 3;  // TMEM lane quadrant this warp may read
     const int half = (warp - 2) >> 2;
-    float* sw_s = reinterpret_cast<float*>(smem_raw + L::OFF_SW) + (warp - 2) * BLOCK_ROWS;
+    constexpr int SCALES = STAGE == 1 ? 2 * BLOCK_ROWS : BLOCK_ROWS;
+    float* sw_s = reinterpret_cast<float*>(smem_raw + L::OFF_SW) + (warp - 2) * SCALES;
     const uint32_t stage_c = smem_base + L::OFF_C + (warp - 2) * STORE_STAGE;
     int acc = 0;
     uint32_t acc_phase = 0;
@@ -722,14 +727,14 @@ __global__ void __launch_bounds__(MOE_ROWS_THREADS, 1) moe_rows_kernel(const __g
       long long rows[4];  // output rows this lane stores pieces of
 #pragma unroll
       for (int k = 0; k < 4; ++k) rows[k] = __shfl_sync(0xffffffffu, orow, 8 * k + (lane >> 2));
-      // weight scales of this warp's columns: stage 1 64 gate channels, then the same 64 up channels
+      // weight scales of this warp's columns: stage 1 the gate channels, then the up channels
       const float* sw_expert = p.sw + static_cast<size_t>(expert) * p.n_expert;
       __syncwarp();
 #pragma unroll
-      for (int i = 0; i < BLOCK_ROWS / 32; ++i) {
+      for (int i = 0; i < SCALES / 32; ++i) {
         const int c = i * 32 + lane;
-        const bool second = STAGE == 1 ? c >= 64 : half == 1;
-        const int cc = STAGE == 1 ? half * 64 + (c & 63) : c;
+        const bool second = STAGE == 1 ? c >= BLOCK_ROWS : half == 1;
+        const int cc = c & (BLOCK_ROWS - 1);
         sw_s[c] = cc < (second ? n_valid[1] : n_valid[0]) ? __ldg(sw_expert + (second ? w_row[1] : w_row[0]) + cc) : 0.0f;
       }
       __syncwarp();
@@ -743,13 +748,12 @@ __global__ void __launch_bounds__(MOE_ROWS_THREADS, 1) moe_rows_kernel(const __g
       auto to_f = [](uint32_t r) { return KT::is_int ? static_cast<float>(static_cast<int32_t>(r)) : __uint_as_float(r); };
       if constexpr (STAGE == 1) {
 #pragma unroll 1
-        for (int c0 = 0; c0 < 64; c0 += 32) {
-          const int cc = half * 64 + c0;  // channel inside the tile
+        for (int c0 = 0; c0 < BLOCK_ROWS; c0 += 32) {
           uint32_t rg[32], ru[32];
-          tmem_ld_x32(t_row + cc, rg);
-          tmem_ld_x32(t_row + BLOCK_ROWS + cc, ru);
+          tmem_ld_x32(t_row + c0, rg);
+          tmem_ld_x32(t_row + BLOCK_ROWS + c0, ru);
           tmem_ld_wait();
-          if (c0 + 32 >= 64) {  // last read of this accumulator: hand it back to the MMA warp
+          if (c0 + 32 >= BLOCK_ROWS) {  // last read of this accumulator: hand it back to the MMA warp
             tc_fence_before();
             __syncwarp();
             if (lane == 0) mbar_arrive(bar_tempty + 8 * acc);
@@ -758,13 +762,13 @@ __global__ void __launch_bounds__(MOE_ROWS_THREADS, 1) moe_rows_kernel(const __g
 #pragma unroll
           for (int j = 0; j < 32; ++j) {
             const float g = (to_f(rg[j]) * sw_s[c0 + j]) * sa;
-            const float u = (to_f(ru[j]) * sw_s[64 + c0 + j]) * sa;
+            const float u = (to_f(ru[j]) * sw_s[BLOCK_ROWS + c0 + j]) * sa;
             float v = silu_f32(g) * u;
             if (p.doweight) v *= tw;
             y[j] = v;
           }
-          const int n_ok = min(32, n_valid[0] - cc);
-          if (n_ok > 0) store_rows32<OUTMODE, ACCUM>(p.out, rows, p.n_out, pair * BLOCK_ROWS + cc, y, n_ok, stage_c, lane);
+          const int n_ok = min(32, n_valid[0] - c0);
+          if (n_ok > 0) store_rows32<OUTMODE, ACCUM>(p.out, rows, p.n_out, pair * BLOCK_ROWS + c0, y, n_ok, stage_c, lane);
         }
       } else {
 #pragma unroll 1

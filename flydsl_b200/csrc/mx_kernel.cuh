@@ -312,8 +312,10 @@ __global__ void __launch_bounds__(MX_THREADS, 1) mx_gemm_kernel(const __grid_con
           const int r = m_blk * BLOCK_ROWS + q * 32 + 8 * k + (lane >> 2);
           rows[k] = r < p.M ? r : -1;
         }
+        const bool any = m_blk * BLOCK_ROWS + q * 32 < p.M;  // few tokens: most warps have no row and nothing to read
+        if (!any && lane == 0) mbar_arrive(bar_tempty + 8 * acc);
 #pragma unroll 1
-        for (int c0 = first_col; c0 < first_col + BN / 2; c0 += 64) {  // 64 columns per TMEM wait
+        for (int c0 = any ? first_col : BN; c0 < first_col + BN / 2; c0 += 64) {  // 64 columns per TMEM wait
           uint32_t r0[32], r1[32];
           tmem_ld_x32(t_row + c0, r0);
           tmem_ld_x32(t_row + c0 + 32, r1);

@@ -89,15 +89,24 @@ bool mx_small_m(int M, int N, bool fp4 = false) {
   const int tiles = (N + 127) / 128;
   return tiles <= sms && (2 * tiles <= sms || M <= (fp4 ? 32 : 64));
 }
-// The mixed kinds (byte containers) the same way, except for 65..128 tokens where the large-M kernel can
-// only split K in two or not at all: there the two are even or the large-M kernel is ahead.  Small-M /
-// large-M with its K split, us, MXFP6 x MXFP4: 32 x 8192 x 8192 18.2 / 18.7, 64 x 8192 x 8192 18.9 / 19.4, 64 x 1024
-// x 8192 9.8 / 11.2, 16 x 4096 x 14336 16.1 / 17.0, 100 x 2048 x 4096 9.9 / 11.1, 128 x 8192 x 8192 21.8 / 20.4.
-bool mx_mixed_small_m(int M, int N) {
+// The mixed kinds (byte containers; kb 128-byte k-blocks).  Small-M / large-M kernel, us, MXFP6 x MXFP4:
+//  * below 12 k-blocks the small-M kernel does not split K and pays about 45 ns a token for its stores: 128 x 2048 x 1024
+//    10.9 / 5.6, 16 x 4096 x 1024 6.4 / 4.9, 4 x 8192 x 512 4.3 / 3.7.  Only on outputs of more than half as many channel tiles as
+//    SMs, where the large-M kernel cannot split K either, a few tokens are faster: 8 x 14336 x 1024 6.2 / 7.0, 16 x 14336 x 512
+//    5.1 / 4.6;
+//  * from 12 to 15 its split is small: 16 x 4096 x 1536 5.1 / 6.2, 33 x 4096 x 1536 7.2 / 6.4, 33 x 14336 x 1536 8.1 / 9.0;
+//  * above, up to 64 tokens (64 x 4096 x 4096 8.0 / 10.0), on wide outputs 48 (48 x 14336 x 2048 9.2 / 11.0, 64 x 14336 x 2048 9.7 / 8.8),
+//    and 128 where the large-M kernel can split K in four: 100 x 2048 x 4096 8.0 / 8.8.
+bool mx_mixed_small_m(int M, int N, int kb) {
   if (!mx_small_m(M, N)) return false;
   int sms = 0;
-  if (M <= 64 || getenv("FLYB200_MX_SMALL") || flyb200::host::sm_count(&sms) != FLYB200_OK) return true;
-  return 4 * ((N + 127) / 128) <= sms;
+  if (getenv("FLYB200_MX_SMALL") || flyb200::host::sm_count(&sms) != FLYB200_OK) return true;
+  const int tiles = (N + 127) / 128;
+  const bool wide = 2 * tiles > sms;
+  if (kb < 12) return wide && M <= kb;
+  if (kb < 16) return M <= (wide ? 48 : 16);
+  if (wide) return M <= 48;
+  return M <= 64 || 4 * tiles <= sms;
 }
 // Tile shape of the large-M kernel: 128 x 256 tiles (one accumulator, exposed epilogue) win once a
 // tile's mainloop is a few times longer than its epilogue (2.44-2.47 against 1.82-1.88 PFLOP/s at
@@ -248,7 +257,7 @@ int flyb200_gemm_mx_mixed(void* c, const void* a, const void* w_shuf, const void
   if (!aligned16(c) || !aligned16(a) || !aligned16(w_shuf) || !aligned16(scale_a_image) || !aligned16(scale_w_image))
     return FLYB200_E_BAD_ALIGN;
   if (M == 0) return FLYB200_OK;
-  if (mx_mixed_small_m(M, N))
+  if (mx_mixed_small_m(M, N, K / KBLOCK_BYTES))
     return host::gemm_mx_small(c, a, w_shuf, scale_a_image, scale_w_image, M, N, K, out_dtype == FLYB200_OUT_FP16 ? 1 : 0,
                                false, stream, a_format, w_format);
   MxParams p;

@@ -152,24 +152,28 @@ int launch_moe_bn(int bn, int stage, int out_dtype, bool accumulate, const CUten
   return FLYB200_E_UNSUPPORTED;
 }
 
-// Vectors of eight where every row starts on a 16-byte boundary, else pairs.
-template <typename T>
-cudaError_t launch_moe_reduce(void* y, const void* x, int tokens, int topk, int dim, const int* expert_mask, const int* topk_ids,
-                       int num_experts, cudaStream_t s) {
-  T* yt = static_cast<T*>(y);
-  const T* xt = static_cast<const T*>(x);
-  const bool vec = dim % 8 == 0 && aligned16(y) && aligned16(x);
-  const int vecs = dim / (vec ? 8 : 2);
+// Vectors of eight where every row starts on a 16-byte boundary, else pairs; a block per token where its threads have
+// work for half a block and more and the grid holds the columns.
+template <typename T, int VEC, int UNROLL>
+cudaError_t launch_moe_reduce_form(T* y, const T* x, int tokens, int topk, int dim, const int* expert_mask, const int* topk_ids, int num_experts,
+                                   cudaStream_t s) {
+  const int vecs = dim / VEC;
   int log2_cols = 8;
   while (log2_cols > 0 && vecs <= (128 >> (8 - log2_cols))) --log2_cols;  // threads per token: vecs rounded up to a power of two
   const int per_block = 256 >> log2_cols;                                 // tokens
-  auto launch = [&](auto kernel, int unroll) {
-    const int column_blocks = (vecs - 1) / (unroll << log2_cols) + 1;
-    return host::launch_dependent(kernel, dim3((tokens - 1) / per_block + 1, column_blocks < 65535 ? column_blocks : 65535), 256, 0, s, yt, xt,
-                                  tokens, topk, dim, log2_cols, expert_mask, topk_ids, num_experts);
-  };
-  if (!vec) return launch(moe_reduce_kernel<T, 2, 1>, 1);
-  return vecs > 256 && tokens > 256 ? launch(moe_reduce_kernel<T, 8, 2>, 2) : launch(moe_reduce_kernel<T, 8, 1>, 1);
+  const int column_blocks = (vecs - 1) / (UNROLL << log2_cols) + 1;
+  const dim3 grid((tokens - 1) / per_block + 1, column_blocks < 65535 ? column_blocks : 65535);
+  auto kernel = log2_cols == 8 && column_blocks <= 65535 ? moe_reduce_kernel<T, VEC, UNROLL, true> : moe_reduce_kernel<T, VEC, UNROLL, false>;
+  return host::launch_dependent(kernel, grid, 256, 0, s, y, x, tokens, topk, dim, log2_cols, expert_mask, topk_ids, num_experts);
+}
+template <typename T>
+cudaError_t launch_moe_reduce(void* y, const void* x, int tokens, int topk, int dim, const int* expert_mask, const int* topk_ids,
+                              int num_experts, cudaStream_t s) {
+  T* yt = static_cast<T*>(y);
+  const T* xt = static_cast<const T*>(x);
+  auto launch = [&](auto form) { return form(yt, xt, tokens, topk, dim, expert_mask, topk_ids, num_experts, s); };
+  if (dim % 8 != 0 || !aligned16(y) || !aligned16(x)) return launch(launch_moe_reduce_form<T, 2, 1>);
+  return dim > 8 * 256 && tokens > 256 ? launch(launch_moe_reduce_form<T, 8, 2>) : launch(launch_moe_reduce_form<T, 8, 1>);
 }
 
 }  // namespace

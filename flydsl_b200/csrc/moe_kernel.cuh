@@ -1033,100 +1033,108 @@ moe_sort_kernel(const ID* __restrict__ topk_ids, const float* __restrict__ topk_
 // (the expert-parallel validity mask of kernels/moe/moe_gemm_2stage/moe_reduce.py:3-7
 // in the reference): rows of routes that another rank serves are never read.
 //
-// Memory-bound.  2^log2_cols threads share a token and own UNROLL x VEC columns each (vectors 2^log2_cols apart),
-// so a block holds 256 / 2^log2_cols tokens and rows of a few vectors leave no warp idle: no division by `dim`, and
-// the loads of up to four slots of all its vectors are in flight together.  VEC = 8 (16-byte
+// Memory-bound: the loads of up to four slots of all vectors of a thread are in flight together.  VEC = 8 (16-byte
 // accesses) wherever `dim` and the bases allow it, else pairs; UNROLL = 2 where a row holds enough vectors, which
-// halves the blocks.  Measured, 4096 tokens x top-2 x 4096 bf16 (101 MB): 21 us
-// = 4.8 TB/s; one vector per thread 22.3, one pair per thread with a 64-bit division each 66.4.
-template <typename T, int VEC, int UNROLL>
+// halves the blocks.  WHOLE: blockIdx.x is the token, a thread owns UNROLL x VEC columns (vectors 256 apart), no division and
+// no run-time stride.  Otherwise 2^log2_cols threads share a token, so that rows of a few vectors leave no warp idle,
+// and rows past the grid's limit take further passes.  Measured, us, 4096 tokens x top-2 x 4096 bf16 (101 MB) as WHOLE 15.6 = 6.4 TB/s,
+// in the other form 25.8, one pair per thread with a 64-bit division each 59; 20000 x top-2 x 256 WHOLE 25.5, other form 7.6, pairs 19.3.
+template <typename T, int VEC, int UNROLL, typename I>
+__device__ __forceinline__ void moe_reduce_columns(T* __restrict__ y, const T* __restrict__ x, long long t, int topk, int dim, I first, int step,
+                                                   const int* __restrict__ expert_mask, const int* __restrict__ topk_ids, int num_experts) {
+  float sum[UNROLL][VEC];
+#pragma unroll
+  for (int u = 0; u < UNROLL; ++u) {
+#pragma unroll
+    for (int i = 0; i < VEC; ++i) sum[u][i] = 0.0f;
+  }
+  constexpr int W = VEC / 2;  // 32-bit words of a vector
+  for (int s0 = 0; s0 < topk; s0 += 4) {
+    uint32_t v[4][UNROLL][W];
+    bool on[4];
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+      const int s = s0 + j;
+      on[j] = s < topk;
+      if (on[j] && expert_mask != nullptr) {
+        const int e = __ldg(topk_ids + t * topk + s);
+        on[j] = e >= 0 && e < num_experts && __ldg(expert_mask + e) != 0;
+      }
+    }
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+      if (!on[j]) continue;
+#pragma unroll
+      for (int u = 0; u < UNROLL; ++u) {
+        if (first + u * step >= dim) continue;
+        const T* src = x + (t * topk + s0 + j) * dim + first + u * step;
+        if constexpr (VEC == 8) {
+          const uint4 q = __ldg(reinterpret_cast<const uint4*>(src));
+          v[j][u][0] = q.x, v[j][u][1] = q.y, v[j][u][2] = q.z, v[j][u][3] = q.w;
+        } else {
+          v[j][u][0] = __ldg(reinterpret_cast<const uint32_t*>(src));
+        }
+      }
+    }
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+      if (!on[j]) continue;
+#pragma unroll
+      for (int u = 0; u < UNROLL; ++u) {
+#pragma unroll
+        for (int i = 0; i < W; ++i) {
+          float2 f;
+          if constexpr (std::is_same<T, __nv_bfloat16>::value) {
+            f = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&v[j][u][i]));
+          } else {
+            f = __half22float2(*reinterpret_cast<const __half2*>(&v[j][u][i]));
+          }
+          sum[u][2 * i] += f.x;
+          sum[u][2 * i + 1] += f.y;
+        }
+      }
+    }
+  }
+#pragma unroll
+  for (int u = 0; u < UNROLL; ++u) {
+    const I c = first + u * step;
+    if (c >= dim) break;
+    uint32_t out[W];
+#pragma unroll
+    for (int i = 0; i < W; ++i) {
+      if constexpr (std::is_same<T, __nv_bfloat16>::value) {
+        const __nv_bfloat162 h = __floats2bfloat162_rn(sum[u][2 * i], sum[u][2 * i + 1]);
+        out[i] = *reinterpret_cast<const uint32_t*>(&h);
+      } else {
+        const __half2 h = __floats2half2_rn(sum[u][2 * i], sum[u][2 * i + 1]);
+        out[i] = *reinterpret_cast<const uint32_t*>(&h);
+      }
+    }
+    T* dst = y + t * dim + c;
+    if constexpr (VEC == 8) {
+      *reinterpret_cast<uint4*>(dst) = make_uint4(out[0], out[1], out[2], out[3]);
+    } else {
+      *reinterpret_cast<uint32_t*>(dst) = out[0];
+    }
+  }
+}
+template <typename T, int VEC, int UNROLL, bool WHOLE>
 __global__ void __launch_bounds__(256) moe_reduce_kernel(T* __restrict__ y, const T* __restrict__ x, int tokens, int topk, int dim,
                                                          int log2_cols, const int* __restrict__ expert_mask,
                                                          const int* __restrict__ topk_ids, int num_experts) {
   static_assert(VEC == 2 || VEC == 8, "pairs or 16-byte vectors");
   pdl_wait(y, x, expert_mask, topk_ids);
   pdl_trigger();
-  const long long t = (static_cast<long long>(blockIdx.x) << (8 - log2_cols)) + (threadIdx.x >> log2_cols);
-  if (t >= tokens) return;
-  const int STEP = VEC << log2_cols;  // columns between the vectors of a thread
-  // one pass but for rows of more than 2^24 vectors, where gridDim.y is at its limit
-  long long first = static_cast<long long>(blockIdx.y) * UNROLL * STEP + (threadIdx.x & ((1 << log2_cols) - 1)) * VEC;
-  for (; first < dim; first += static_cast<long long>(gridDim.y) * UNROLL * STEP) {
-    float sum[UNROLL][VEC];
-#pragma unroll
-    for (int u = 0; u < UNROLL; ++u) {
-#pragma unroll
-      for (int i = 0; i < VEC; ++i) sum[u][i] = 0.0f;
-    }
-    constexpr int W = VEC / 2;  // 32-bit words of a vector
-    for (int s0 = 0; s0 < topk; s0 += 4) {
-      uint32_t v[4][UNROLL][W];
-      bool on[4];
-#pragma unroll
-      for (int j = 0; j < 4; ++j) {
-        const int s = s0 + j;
-        on[j] = s < topk;
-        if (on[j] && expert_mask != nullptr) {
-          const int e = __ldg(topk_ids + t * topk + s);
-          on[j] = e >= 0 && e < num_experts && __ldg(expert_mask + e) != 0;
-        }
-      }
-#pragma unroll
-      for (int j = 0; j < 4; ++j) {
-        if (!on[j]) continue;
-#pragma unroll
-        for (int u = 0; u < UNROLL; ++u) {
-          if (first + u * STEP >= dim) continue;
-          const T* src = x + (t * topk + s0 + j) * dim + first + u * STEP;
-          if constexpr (VEC == 8) {
-            const uint4 q = __ldg(reinterpret_cast<const uint4*>(src));
-            v[j][u][0] = q.x, v[j][u][1] = q.y, v[j][u][2] = q.z, v[j][u][3] = q.w;
-          } else {
-            v[j][u][0] = __ldg(reinterpret_cast<const uint32_t*>(src));
-          }
-        }
-      }
-#pragma unroll
-      for (int j = 0; j < 4; ++j) {
-        if (!on[j]) continue;
-#pragma unroll
-        for (int u = 0; u < UNROLL; ++u) {
-#pragma unroll
-          for (int i = 0; i < W; ++i) {
-            float2 f;
-            if constexpr (std::is_same<T, __nv_bfloat16>::value) {
-              f = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&v[j][u][i]));
-            } else {
-              f = __half22float2(*reinterpret_cast<const __half2*>(&v[j][u][i]));
-            }
-            sum[u][2 * i] += f.x;
-            sum[u][2 * i + 1] += f.y;
-          }
-        }
-      }
-    }
-#pragma unroll
-    for (int u = 0; u < UNROLL; ++u) {
-      const long long c = first + u * STEP;
-      if (c >= dim) break;
-      uint32_t out[W];
-#pragma unroll
-      for (int i = 0; i < W; ++i) {
-        if constexpr (std::is_same<T, __nv_bfloat16>::value) {
-          const __nv_bfloat162 h = __floats2bfloat162_rn(sum[u][2 * i], sum[u][2 * i + 1]);
-          out[i] = *reinterpret_cast<const uint32_t*>(&h);
-        } else {
-          const __half2 h = __floats2half2_rn(sum[u][2 * i], sum[u][2 * i + 1]);
-          out[i] = *reinterpret_cast<const uint32_t*>(&h);
-        }
-      }
-      T* dst = y + t * dim + c;
-      if constexpr (VEC == 8) {
-        *reinterpret_cast<uint4*>(dst) = make_uint4(out[0], out[1], out[2], out[3]);
-      } else {
-        *reinterpret_cast<uint32_t*>(dst) = out[0];
-      }
-    }
+  if constexpr (WHOLE) {
+    moe_reduce_columns<T, VEC, UNROLL, int>(y, x, blockIdx.x, topk, dim, (blockIdx.y * UNROLL * 256 + threadIdx.x) * VEC, 256 * VEC, expert_mask,
+                                            topk_ids, num_experts);
+  } else {
+    const long long t = (static_cast<long long>(blockIdx.x) << (8 - log2_cols)) + (threadIdx.x >> log2_cols);
+    if (t >= tokens) return;
+    const int step = VEC << log2_cols;
+    long long first = static_cast<long long>(blockIdx.y) * UNROLL * step + (threadIdx.x & ((1 << log2_cols) - 1)) * VEC;
+    for (; first < dim; first += static_cast<long long>(gridDim.y) * UNROLL * step)
+      moe_reduce_columns<T, VEC, UNROLL, long long>(y, x, t, topk, dim, first, step, expert_mask, topk_ids, num_experts);
   }
 }
 

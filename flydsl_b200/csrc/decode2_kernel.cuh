@@ -109,13 +109,19 @@ gemm_decode2_kernel(const __grid_constant__ CUtensorMap tmA, const GemmParams p)
     for (int i = 0; i < ahead; ++i)
       bulk_prefetch_l2(p.w + (static_cast<size_t>(kb_begin + i) * p.N + n0) * KBLOCK_BYTES, w_bytes);
     // the ring is empty and the full barriers are this CTA's own: start the stream at once
-    if (p.pdl == 1) asm volatile("griddepcontrol.wait;" ::: "memory");
+    if (p.pdl == 1) {
+      asm volatile("griddepcontrol.wait;" ::: "memory");
+      pdl_trigger();  // the next kernel on the stream may be scheduled: its set-up and weight requests overlap this one
+    }
     for (int i = 0; i < pre; ++i) {
       mbar_expect_tx(bar_full + 8 * i, A_STAGE + w_bytes);
       bulk_load_1d(smem_base + L.off_w + i * W_STAGE, p.w + (static_cast<size_t>(kb_begin + i) * p.N + n0) * KBLOCK_BYTES,
                    w_bytes, bar_full + 8 * i, pol_w);
     }
-    if (p.pdl == 2) asm volatile("griddepcontrol.wait;" ::: "memory");
+    if (p.pdl == 2) {
+      asm volatile("griddepcontrol.wait;" ::: "memory");
+      pdl_trigger();
+    }
     for (int i = 0; i < pre; ++i)
       tma_load_2d(smem_base + L.off_a + i * A_STAGE, &tmA, bar_full + 8 * i, (kb_begin + i) * KBLOCK_BYTES, m_half, pol_a);
   }
@@ -130,10 +136,7 @@ gemm_decode2_kernel(const __grid_constant__ CUtensorMap tmA, const GemmParams p)
   cluster_barrier_all();  // the barriers of both CTAs exist, the pair's TMEM is allocated
   tc_fence_after();
   const uint32_t tmem_base = *tmem_slot;
-  if (p.pdl && threadIdx.x != 0) {
-    asm volatile("griddepcontrol.wait;" ::: "memory");
-    pdl_trigger();  // the next kernel on the stream may be scheduled (its set-up and weight requests overlap this one)
-  }
+  if (p.pdl && threadIdx.x != 0) asm volatile("griddepcontrol.wait;" ::: "memory");
   // Who sums the K splits after the mainloop: from 64 tokens up all seven warps (the producer and
   // the MMA issuers have nothing left to do by then; measured 2-7 % on the whole kernel at 64-256
   // tokens), below that the four epilogue warps (with so few tokens the extra warps only cost).

@@ -288,14 +288,20 @@ __global__ void __launch_bounds__(DECODE_THREADS, 1) gemm_decode_kernel(const __
     const int ahead = min(p.prefetch, num_kb);
     for (int i = 0; i < ahead; ++i)
       bulk_prefetch_l2(p.w + (static_cast<size_t>(kb_begin + i) * p.N + n0) * KBLOCK_BYTES, w_bytes);
-    if (p.pdl == 1) asm volatile("griddepcontrol.wait;" ::: "memory");
+    if (p.pdl == 1) {
+      asm volatile("griddepcontrol.wait;" ::: "memory");
+      pdl_trigger();  // the next kernel on the stream may be scheduled: its set-up and weight requests overlap this one
+    }
     for (int i = 0; i < pre; ++i) {
       mbar_expect_tx(bar_full + 8 * i, A_STAGE + w_bytes + SF_BYTES);
       bulk_load_1d(smem_base + L.off_w + i * W_STAGE,
                    p.w + (static_cast<size_t>(kb_begin + i) * p.N + n0) * KBLOCK_BYTES, w_bytes, bar_full + 8 * i, pol_w);
       load_scale_atoms(smem_base + L.off_sf + i * SF_BYTES, kb_begin + i, bar_full + 8 * i, pol_w, pol_a, true, false);
     }
-    if (p.pdl == 2) asm volatile("griddepcontrol.wait;" ::: "memory");
+    if (p.pdl == 2) {
+      asm volatile("griddepcontrol.wait;" ::: "memory");
+      pdl_trigger();
+    }
     for (int i = 0; i < pre; ++i) {
       tma_load_2d(smem_base + L.off_a + i * A_STAGE, &tmA, bar_full + 8 * i, (kb_begin + i) * KBLOCK_BYTES, m_base, pol_a);
       load_scale_atoms(smem_base + L.off_sf + i * SF_BYTES, kb_begin + i, bar_full + 8 * i, pol_w, pol_a, false, true);
@@ -319,10 +325,7 @@ __global__ void __launch_bounds__(DECODE_THREADS, 1) gemm_decode_kernel(const __
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem_base = *tmem_slot;
-  if (p.pdl && threadIdx.x != 0) {
-    asm volatile("griddepcontrol.wait;" ::: "memory");
-    pdl_trigger();  // the next kernel on the stream may be scheduled (its set-up and weight requests overlap this one)
-  }
+  if (p.pdl && threadIdx.x != 0) asm volatile("griddepcontrol.wait;" ::: "memory");
   // Who sums the K splits after the mainloop: from 64 tokens up all seven warps (the producer and
   // the MMA issuers have nothing left to do by then; measured 2-7 % on the whole kernel at 64-256
   // tokens), below that the four epilogue warps (with so few tokens the extra warps only cost).

@@ -51,6 +51,7 @@ SIGNATURES = {
     "flyb200_pertoken_quant": (_i, [_vp, _vp, _vp, _i, _i, _i, _i, _vp]),
     "flyb200_shuffle_weight": (_i, [_vp, _vp, _i, _i, _i, _i, _vp]),
     "flyb200_unshuffle_weight": (_i, [_vp, _vp, _i, _i, _i, _vp]),
+    "flyb200_pair_width": (_i, [_i, _i, _i, _i, _i, _i]),
     "flyb200_describe_plan": (_i, [_i, _i, _i, _i, _i, _i, ctypes.POINTER(_i)]),
     "flyb200_layout_kind": (_i, [_i, _i, _i]),
     "flyb200_workspace_bytes": (_sz, [_i, _i, _i, _i, _i]),
@@ -154,6 +155,11 @@ def describe_plan(m: int, n: int, k: int, in_dtype: str = "fp8", variant_hint: i
     out = (_i * 8)()
     check(load().flyb200_describe_plan(m, n, k, IN_DTYPES[in_dtype], variant_hint, sm_count, out), "describe_plan")
     return dict(zip(PLAN_FIELDS, list(out)))
+
+
+def pair_width(m: int, n: int, k: int, in_dtype: str = "fp8", variant_hint: int = 0, sm_count: int = 148) -> int:
+    """Tile width with which the call runs as CTA pairs, 0 where the plan of describe_plan runs (no GPU needed)."""
+    return load().flyb200_pair_width(m, n, k, IN_DTYPES[in_dtype], variant_hint, sm_count)
 
 
 _failure_hooks: list = []

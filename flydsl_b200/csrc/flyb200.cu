@@ -14,7 +14,6 @@
 using namespace flyb200;
 using flyb200::host::MAX_DEVICES;
 using flyb200::host::SMEM_LIMIT;
-using flyb200::host::ROWS2_STAGES;
 
 namespace {
 
@@ -382,6 +381,75 @@ int auto_rows_bn(int M, int N, int K_bytes, int sms) {
   return best;
 }
 
+// Large-M kernels: programmatic dependent launch only for launches of at most two rounds of tiles, where hiding the
+// launch and set-up behind the previous kernel's tail is worth 2-6 % (512 x 4096 x 4096: 18.0 -> 16.9 us); on long
+// launches it measured 0.5 % slower.
+int large_pdl(int mode, long long tiles, int ctas) { return tiles > 2LL * ctas ? 0 : mode; }
+
+// Row tiles of a raster group of the pair form: 4096 rows, fewer where their activations would take more than 48 MiB.
+// A group's activations stay in L2 while it walks the channels; larger groups fall out of it, smaller ones read the
+// weights more often, and both cost DRAM energy under the power cap.  us, row tiles per group 4 / 8 / 12 / 16 / 32:
+// bf16 8192 x 8192 x 8192 888 / 859 / 855 / 885 / 941, fp8 8192 x 28672 x 8192 1732 / 1531 / 1494 / 1488 / 1558.
+int pair_group(int K_bytes) {
+  long long rows = (48LL << 20) / K_bytes;
+  rows = rows > 4096 ? 4096 : rows < 512 ? 512 : rows;
+  return static_cast<int>(rows / PAIR_ROWS);
+}
+
+// Estimated cycles of a launch of the pair form with tiles of bn columns, and of the 128-row form: whole rounds (k-blocks
+// plus the hand-over between tiles), the last round, the last epilogue.
+constexpr int TILE_CYCLES = 500;            // hand-over between two tiles of a CTA
+constexpr int EPILOGUE_CYCLES_PER_COL = 12; // of the last tile, which nothing overlaps
+long long pair_cost(int M, int N, long long kb, int bn, int sms) {
+  const int clusters = sms / 2;
+  const long long tiles = host::pair_tiles(M, N, bn), rest = tiles % clusters;
+  const int parts = host::pair_tail_parts(bn, tiles, clusters);
+  const long long last = rest == 0 ? 0 : (tiles < clusters ? 1 : (rest * parts + clusters - 1) / clusters) * host::pair_kb_cycles(bn / parts);
+  return tiles / clusters * (kb * host::pair_kb_cycles(bn) + TILE_CYCLES) + kb * last + EPILOGUE_CYCLES_PER_COL * (bn / parts);
+}
+long long rows_cost(int M, int N, long long kb, int bn, int sms) {
+  auto kb_cycles = [](int width) {
+    long long c = 2LL * width > ROWS_ISSUE_CYCLES ? 2LL * width : ROWS_ISSUE_CYCLES;
+    const long long load = static_cast<long long>(BLOCK_ROWS + width) * KBLOCK_BYTES / 84;
+    return c > load ? c : load;
+  };
+  const long long tiles = static_cast<long long>((M + BLOCK_ROWS - 1) / BLOCK_ROWS) * ((N + bn - 1) / bn);
+  const int parts = host::rows_tail_parts(bn, tiles, sms);
+  return (tiles + sms - 1) / sms * (kb * kb_cycles(bn) + TILE_CYCLES) - kb * (kb_cycles(bn) - kb_cycles(bn / parts)) - TILE_CYCLES +
+         EPILOGUE_CYCLES_PER_COL * (bn / parts);
+}
+
+// Tile width with which a call that leaves the kernel open runs as CTA pairs, or 0 where the planned kernel stays.
+// A pair takes in a third fewer bytes per product than two CTAs of the 128-row form, so it needs less time where the
+// intake binds and less energy where the board's power cap does.  `plan` / pairs, us, fp8 unless stated:
+//   128-row form   4096 x 8192 x 8192 220 / 204, 8192 x 28672 x 8192 1480 / 1420, 2048 x 8192 x 8192 121 / 110, 768 x 8192 x 8192
+//                  56.7 / 48.8; fp16 4096 x 4096 x 4096 118 / 108; int8 997 x 10208 x 5120 54 / 47; bf16 8192 x 5120 x 1024 78 / 72
+//   256-row form   1024 x 8192 x 4096 36.4 / 34.0, 512 x 16384 x 4096 38.3 / 36.1, bf16 1536 x 5120 x 1024 19.0 / 16.8
+//   small-M form   256 x 8192 x 8192 24.7 / 21.9, 256 x 10208 x 5120 26.8 / 18.5, 320 x 4096 x 4096 15.2 / 11.2, bf16 512 x 3584 x 8192 35 / 31.5;
+//                  it stays where it splits K in four or more over at least 64 k-blocks: 256 x 4096 x 14336 22.8 / 24.7,
+//                  512 x 1024 x 8192 14.0 / 14.9, bf16 1024 x 1024 x 8192 21.4 / 24.9
+// Up to 128 tokens half of a pair would have no rows (128 x 8192 x 8192 17.3 / 22.4).  Of the widths the cheapest counts, a
+// narrower one only if it is 2 % cheaper (more bytes per product); over 117 shapes of 264..8192 tokens the choice is
+// within 1 % of the best width and form on average.  With 16 k-blocks or fewer the pairs' set-up (cluster barriers,
+// remote hand-over) weighs more: 320 x 5120 x 1024 bf16 8.5 / 9.5, 1024 x 5120 x 1024 10.2 / 11.3.
+constexpr long long PAIR_SETUP_CYCLES = 2500;
+int pair_choice(const Plan& plan, int M, int N, int K_bytes, int sms) {
+  const long long kb = K_bytes / KBLOCK_BYTES;
+  if (M <= BLOCK_ROWS || sms < 2 || plan.two_sm || plan.pair) return 0;
+  if (plan.decode && plan.split_k >= 4 && kb >= 64) return 0;
+  long long best = -1;
+  int width = 0;
+  for (int bn = 256; bn >= 64; bn -= 32) {
+    const long long c = pair_cost(M, N, kb, bn, sms);
+    if (best < 0 || 100 * c < 98 * best) {
+      best = c;
+      width = bn;
+    }
+  }
+  if (!plan.decode && !plan.tall && rows_cost(M, N, kb, plan.bn, sms) < best + (kb <= 16 ? PAIR_SETUP_CYCLES : 0)) return 0;
+  return width;
+}
+
 // `allow_pair`: the caller's kind has the CTA-pair form of the small-M kernel (the plain kinds do)
 int make_plan(Plan* plan, int M, int N, int K_bytes, int variant_hint, size_t workspace_bytes, bool have_ws, int sms,
               bool allow_pair = true) {
@@ -434,7 +502,7 @@ int make_plan(Plan* plan, int M, int N, int K_bytes, int variant_hint, size_t wo
   if (!plan->decode) {
     // large-M kernel: the split field carries the tile width in units of 32 channels
     if (plan->two_sm) {
-      plan->bn = 256;
+      plan->bn = want_split >= 2 && want_split <= 8 ? 32 * want_split : 256;
     } else if (want_split > 0) {
       if (want_split > 8) return FLYB200_E_BAD_ARG;
       plan->bn = 32 * want_split;
@@ -457,7 +525,7 @@ int make_plan(Plan* plan, int M, int N, int K_bytes, int variant_hint, size_t wo
   }
   // 32 row tiles (32 MiB of 8-bit activations at K = 8192) stay in L2 while a group walks the channels:
   // measured DRAM reads 1.17 x the operands against 1.67 x with groups of 16, at equal time
-  plan->group_m = hint_group(variant_hint) > 0 ? hint_group(variant_hint) : (plan->two_sm ? 8 : plan->tall ? 16 : 32);
+  plan->group_m = hint_group(variant_hint) > 0 ? hint_group(variant_hint) : (plan->two_sm ? pair_group(K_bytes) : plan->tall ? 16 : 32);
   plan->split_k = 1;
   plan->reduce_mode = REDUCE_NONE;
   if (plan->decode) {
@@ -495,12 +563,8 @@ int make_plan(Plan* plan, int M, int N, int K_bytes, int variant_hint, size_t wo
   const int hp = hint_pdl(variant_hint);
   plan->pdl = hp == 1 ? 1 : hp == 2 ? 0 : hp == 3 ? 2 : host::pdl_default();
   if (!plan->decode) {
-    // Large-M kernels: programmatic dependent launch only for launches of at most two rounds of tiles,
-    // where hiding the launch and set-up behind the previous kernel's tail is worth 2-6 % (512 x 4096 x
-    // 4096: 18.0 -> 16.9 us); on long launches it measured 0.5 % slower.  The CTA-pair form runs without it.
-    const long long rows = plan->tall ? 2 * BLOCK_ROWS : BLOCK_ROWS;
-    const long long tiles = ((M + rows - 1) / rows) * ((N + plan->bn - 1) / plan->bn);
-    if (plan->two_sm || tiles > 2LL * sms) plan->pdl = 0;
+    const long long rows = plan->two_sm || plan->tall ? 2 * BLOCK_ROWS : BLOCK_ROWS;
+    plan->pdl = large_pdl(plan->pdl, ((M + rows - 1) / rows) * ((N + plan->bn - 1) / plan->bn), plan->two_sm ? sms / 2 : sms);
   }
   const int kb = K_bytes / KBLOCK_BYTES;
   plan->kb_per_split = kb;
@@ -532,6 +596,24 @@ int make_plan(Plan* plan, int M, int N, int K_bytes, int variant_hint, size_t wo
   return FLYB200_OK;
 }
 
+// make_plan, and CTA pairs where the call leaves the kernel open and they are the better choice.
+int plan_call(Plan* plan, int M, int N, int K_bytes, int variant_hint, size_t workspace_bytes, bool have_ws, int sms) {
+  const int rc = make_plan(plan, M, N, K_bytes, variant_hint, workspace_bytes, have_ws, sms);
+  if (rc || (variant_hint & ~(3 << 28)) != 0 || rows_tall_default() || w64_default()) return rc;
+  const int width = pair_choice(*plan, M, N, K_bytes, sms);
+  if (width == 0) return rc;
+  plan->decode = plan->tall = false;
+  plan->two_sm = true;
+  plan->bn = width;
+  plan->split_k = plan->token_blocks = 1;
+  plan->reduce_mode = REDUCE_NONE;
+  plan->prefetch = 0;
+  plan->group_m = pair_group(K_bytes);
+  const int hp = hint_pdl(variant_hint);
+  plan->pdl = large_pdl(hp == 1 ? 1 : hp == 2 ? 0 : hp == 3 ? 2 : host::pdl_default(), host::pair_tiles(M, N, width), sms / 2);
+  return rc;
+}
+
 int gemm_common(void* c, const void* a, const void* w, const float* sa, const float* sb, const void* bias, int M,
                 int N, int K, int in_dtype, int outmode, int epilogue, int variant_hint, void* workspace,
                 size_t workspace_bytes, void* stream) {
@@ -555,7 +637,7 @@ int gemm_common(void* c, const void* a, const void* w, const float* sa, const fl
   const int K_bytes = K * eb;
 
   Plan plan;
-  rc = make_plan(&plan, M, N, K_bytes, variant_hint, workspace_bytes, workspace != nullptr, st->sms);
+  rc = plan_call(&plan, M, N, K_bytes, variant_hint, workspace_bytes, workspace != nullptr, st->sms);
   if (rc) return rc;
 
   GemmParams p;
@@ -578,33 +660,43 @@ int gemm_common(void* c, const void* a, const void* w, const float* sa, const fl
   p.prefetch = plan.prefetch;
   p.token_blocks = plan.token_blocks;
   p.bn = plan.bn;
-  p.rows_stages = plan.tall ? host::ROWS_TALL_STAGES : host::rows_stages_for(plan.bn);
+  p.rows_stages = plan.two_sm ? host::pair_stages_for(plan.bn) : plan.tall ? host::ROWS_TALL_STAGES : host::rows_stages_for(plan.bn);
+  p.tail_parts = 1;
   p.ws_tickets = static_cast<int*>(workspace);
   p.ws_partials = workspace ? reinterpret_cast<float*>(static_cast<uint8_t*>(workspace) + TICKET_BYTES) : nullptr;
   p.status = st->status;
 
-  CUtensorMap tmA, tmC, tmW;
-  memset(&tmC, 0, sizeof(tmC));
-  memset(&tmW, 0, sizeof(tmW));
-  if (!plan.decode && plan.two_sm) {
-    rc = make_weight_map(&tmW, w, static_cast<uint64_t>(N), static_cast<uint64_t>(K_bytes / KBLOCK_BYTES), BLOCK_ROWS);
-    if (rc) return rc;
-  }
-  rc = make_map(&tmA, CU_TENSOR_MAP_DATA_TYPE_UINT8, 1, a, static_cast<uint64_t>(K_bytes), static_cast<uint64_t>(M),
-                KBLOCK_BYTES, plan.decode ? (plan.pair ? plan.bn / 2 : plan.bn) : plan.tall ? 2 * BLOCK_ROWS : BLOCK_ROWS);
-  if (rc) return rc;
-  if (!plan.decode && outmode != OUT_RAW32) {
-    rc = make_map(&tmC, outmode == OUT_FP16 ? CU_TENSOR_MAP_DATA_TYPE_FLOAT16 : CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, c,
-                  static_cast<uint64_t>(N), static_cast<uint64_t>(M), 64, 32);
-    if (rc) return rc;
-  }
-
   cudaStream_t s = static_cast<cudaStream_t>(stream);
   const int kind = kind_of(in_dtype);
+  const bool maps_c = !plan.decode && outmode != OUT_RAW32;
+  const CUtensorMapDataType c_type = outmode == OUT_FP16 ? CU_TENSOR_MAP_DATA_TYPE_FLOAT16 : CU_TENSOR_MAP_DATA_TYPE_BFLOAT16;
+  auto map_a = [&](CUtensorMap* m, uint32_t box_rows) {
+    return make_map(m, CU_TENSOR_MAP_DATA_TYPE_UINT8, 1, a, static_cast<uint64_t>(K_bytes), static_cast<uint64_t>(M), KBLOCK_BYTES, box_rows);
+  };
+  auto map_c = [&](CUtensorMap* m) {
+    return maps_c ? make_map(m, c_type, 2, c, static_cast<uint64_t>(N), static_cast<uint64_t>(M), 64, 32) : FLYB200_OK;
+  };
+  if (!plan.decode && plan.two_sm) {
+    p.tail_parts = host::pair_tail_parts(plan.bn, host::pair_tiles(M, N, plan.bn), st->sms / 2);
+    auto map_w = [&](CUtensorMap* m, uint32_t box_rows) {
+      return make_weight_map(m, w, static_cast<uint64_t>(N), static_cast<uint64_t>(K_bytes / KBLOCK_BYTES), box_rows);
+    };
+    PairMaps maps;
+    memset(&maps.c, 0, sizeof(maps.c));
+    if ((rc = map_a(&maps.a, BLOCK_ROWS)) || (rc = map_w(&maps.w, plan.bn / 2)) ||
+        (rc = map_w(&maps.w_strip, plan.bn / 2 / p.tail_parts)) || (rc = map_c(&maps.c)))
+      return rc;
+    return host::launch_pair_kind(kind, outmode, maps, p, st->sms, s);
+  }
+  CUtensorMap tmA, tmC;
+  memset(&tmC, 0, sizeof(tmC));
+  rc = map_a(&tmA, plan.decode ? (plan.pair ? plan.bn / 2 : plan.bn) : plan.tall ? 2 * BLOCK_ROWS : BLOCK_ROWS);
+  if (rc) return rc;
+  rc = map_c(&tmC);
+  if (rc) return rc;
   if (plan.decode && plan.pair) return host::launch_decode2_kind(kind, outmode, plan.bn, tmA, p, s);
   if (plan.decode) return host::launch_decode_kind(kind, outmode, plan.bn, plan.w_rows, tmA, p, s);
-  const int form = plan.two_sm ? host::ROWS_FORM_PAIRS : plan.tall ? host::ROWS_FORM_TALL : host::ROWS_FORM_ONE;
-  return host::launch_rows_kind(kind, outmode, form, tmA, tmW, tmC, p, st->sms, s);
+  return host::launch_rows_kind(kind, outmode, plan.tall ? host::ROWS_FORM_TALL : host::ROWS_FORM_ONE, tmA, tmC, p, st->sms, s);
 }
 
 // ---------------------------------------------------------------------------
@@ -1012,10 +1104,19 @@ int flyb200_describe_plan(int M, int N, int K, int in_dtype, int variant_hint, i
   out8[2] = plan.split_k;
   out8[3] = plan.kb_per_split;
   out8[4] = plan.reduce_mode;
-  out8[5] = plan.decode ? plan.stages : (plan.two_sm ? ROWS2_STAGES : plan.tall ? host::ROWS_TALL_STAGES : host::rows_stages_for(plan.bn));
+  out8[5] = plan.decode ? plan.stages : (plan.two_sm ? host::pair_stages_for(plan.bn) : plan.tall ? host::ROWS_TALL_STAGES : host::rows_stages_for(plan.bn));
   out8[6] = plan.pdl;
   out8[7] = plan.token_blocks;
   return FLYB200_OK;
+}
+
+int flyb200_pair_width(int M, int N, int K, int in_dtype, int variant_hint, int sm_count) {
+  if (M <= 0 || N <= 0 || K <= 0 || sm_count <= 0 || in_dtype < FLYB200_DT_FP8 || in_dtype > FLYB200_DT_BF16) return 0;
+  const int eb = elem_bytes_of(in_dtype);
+  if (!flyb200_layout_kind(N, K, eb)) return 0;
+  Plan plan;
+  if (plan_call(&plan, M, N, K * eb, variant_hint, static_cast<size_t>(-1) >> 1, true, sm_count)) return 0;
+  return plan.two_sm ? plan.bn : 0;
 }
 
 int flyb200_layout_kind(int N, int K, int elem_bytes) {

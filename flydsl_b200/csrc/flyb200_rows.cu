@@ -8,6 +8,7 @@
 
 #include <cstdlib>
 #include <cstring>
+#include <type_traits>
 
 namespace flyb200 {
 namespace host {
@@ -63,41 +64,33 @@ int launch_rows_tall(const CUtensorMap& tmA, const CUtensorMap& tmC, const GemmP
   return launch_plain_or_pdl(kernel, grid, TALL_THREADS, L.total, s, p.pdl != 0, tmA, tmC, p);
 }
 
+// CTA pairs on 256 x bn tiles.
 template <int KIND, int OUTMODE>
-int launch_rows2(const CUtensorMap& tmA, const CUtensorMap& tmW, const CUtensorMap& tmC, const GemmParams& p, int sms,
-                 cudaStream_t s) {
-  using L = Rows2Smem<ROWS2_STAGES>;
+int launch_pair(const PairMaps& maps, const GemmParams& p, int sms, cudaStream_t s) {
   static std::atomic<uint64_t> done{0};
-  static int max_clusters[MAX_DEVICES] = {0};
-  auto kernel = gemm_rows2_kernel<KIND, ROWS2_STAGES, OUTMODE>;
-  int rc = ensure_smem(kernel, L::TOTAL, done);
+  auto kernel = gemm_pair_kernel<KIND, OUTMODE>;
+  int rc = ensure_smem(kernel, SMEM_LIMIT, done);
   if (rc) return rc;
+  const RowsLayout L = pair_layout(p.bn, p.rows_stages);
+  if (L.total > SMEM_LIMIT || p.rows_stages < 2 || p.bn < 64 || p.bn > 256 || (p.bn & 31)) return FLYB200_E_UNSUPPORTED;
+  const long long tiles = pair_tiles(p.M, p.N, p.bn);
   cudaLaunchConfig_t cfg;
   memset(&cfg, 0, sizeof(cfg));
-  cfg.blockDim = dim3(NUM_THREADS, 1, 1);
-  cfg.dynamicSmemBytes = L::TOTAL;
-  cfg.stream = s;
-  cudaLaunchAttribute attr;
-  attr.id = cudaLaunchAttributeClusterDimension;
-  attr.val.clusterDim.x = 2;
-  attr.val.clusterDim.y = 1;
-  attr.val.clusterDim.z = 1;
-  cfg.attrs = &attr;
-  cfg.numAttrs = 1;
-  int dev = 0;
-  FLYB200_CUDA_TRY(cudaGetDevice(&dev));
-  if (dev < 0 || dev >= MAX_DEVICES) return FLYB200_E_UNSUPPORTED;
-  if (max_clusters[dev] == 0) {
-    cfg.gridDim = dim3(sms & ~1, 1, 1);
-    int n = 0;
-    FLYB200_CUDA_TRY(cudaOccupancyMaxActiveClusters(&n, kernel, &cfg));
-    if (n < 1) return FLYB200_E_UNSUPPORTED;
-    max_clusters[dev] = n;
-  }
-  const int tiles = ((p.M + 255) / 256) * ((p.N + 255) / 256);
-  const int clusters = tiles < max_clusters[dev] ? tiles : max_clusters[dev];
+  const int clusters = static_cast<int>(tiles < sms / 2 ? tiles : sms / 2);
   cfg.gridDim = dim3(2 * clusters, 1, 1);
-  FLYB200_CUDA_TRY(cudaLaunchKernelEx(&cfg, kernel, tmA, tmW, tmC, p));
+  cfg.blockDim = dim3(64 + 32 * rows_epilogue_warps(p.K_bytes / KBLOCK_BYTES, 2 * tiles, sms), 1, 1);
+  cfg.dynamicSmemBytes = L.total;
+  cfg.stream = s;
+  cudaLaunchAttribute attr[2];
+  attr[0].id = cudaLaunchAttributeClusterDimension;
+  attr[0].val.clusterDim.x = 2;
+  attr[0].val.clusterDim.y = 1;
+  attr[0].val.clusterDim.z = 1;
+  attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[1].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = p.pdl ? 2 : 1;
+  FLYB200_CUDA_TRY(cudaLaunchKernelEx(&cfg, kernel, maps, p));
   return FLYB200_OK;
 }
 
@@ -120,36 +113,38 @@ int launch_rows_scatter(const CUtensorMap& tmA, const OutputMaps& outs, GemmPara
 }
 
 template <int KIND, int OUTMODE>
-int rows_any(int form, const CUtensorMap& tmA, const CUtensorMap& tmW, const CUtensorMap& tmC, const GemmParams& p,
-             int sms, cudaStream_t s) {
-  if (form == ROWS_FORM_PAIRS) return launch_rows2<KIND, OUTMODE>(tmA, tmW, tmC, p, sms, s);
+int rows_any(int form, const CUtensorMap& tmA, const CUtensorMap& tmC, const GemmParams& p, int sms, cudaStream_t s) {
   if (form == ROWS_FORM_TALL) return launch_rows_tall<KIND, OUTMODE>(tmA, tmC, p, sms, s);
   return launch_rows<KIND, OUTMODE>(tmA, tmC, p, sms, s);
 }
 
-}  // namespace
-
-int launch_rows_kind(int kind, int outmode, int form, const CUtensorMap& tmA, const CUtensorMap& tmW,
-                     const CUtensorMap& tmC, const GemmParams& p, int sms, cudaStream_t s) {
+// Calls fn with the kind and the output mode as integral constants.
+template <typename Fn>
+int for_kind(int kind, int outmode, Fn fn) {
+  auto with_out = [&](auto k) {
+    if (outmode == OUT_BF16) return fn(k, std::integral_constant<int, OUT_BF16>());
+    if (outmode == OUT_FP16) return fn(k, std::integral_constant<int, OUT_FP16>());
+    if constexpr (decltype(k)::value == KIND_F8 || decltype(k)::value == KIND_I8) return fn(k, std::integral_constant<int, OUT_RAW32>());
+    return static_cast<int>(FLYB200_E_UNSUPPORTED);
+  };
   switch (kind) {
-    case KIND_F8:
-      if (outmode == OUT_BF16) return rows_any<KIND_F8, OUT_BF16>(form, tmA, tmW, tmC, p, sms, s);
-      if (outmode == OUT_FP16) return rows_any<KIND_F8, OUT_FP16>(form, tmA, tmW, tmC, p, sms, s);
-      return rows_any<KIND_F8, OUT_RAW32>(form, tmA, tmW, tmC, p, sms, s);
-    case KIND_I8:
-      if (outmode == OUT_BF16) return rows_any<KIND_I8, OUT_BF16>(form, tmA, tmW, tmC, p, sms, s);
-      if (outmode == OUT_FP16) return rows_any<KIND_I8, OUT_FP16>(form, tmA, tmW, tmC, p, sms, s);
-      return rows_any<KIND_I8, OUT_RAW32>(form, tmA, tmW, tmC, p, sms, s);
-    case KIND_F16:
-      if (outmode == OUT_BF16) return rows_any<KIND_F16, OUT_BF16>(form, tmA, tmW, tmC, p, sms, s);
-      if (outmode == OUT_FP16) return rows_any<KIND_F16, OUT_FP16>(form, tmA, tmW, tmC, p, sms, s);
-      break;
-    case KIND_BF16:
-      if (outmode == OUT_BF16) return rows_any<KIND_BF16, OUT_BF16>(form, tmA, tmW, tmC, p, sms, s);
-      if (outmode == OUT_FP16) return rows_any<KIND_BF16, OUT_FP16>(form, tmA, tmW, tmC, p, sms, s);
-      break;
+    case KIND_F8: return with_out(std::integral_constant<int, KIND_F8>());
+    case KIND_I8: return with_out(std::integral_constant<int, KIND_I8>());
+    case KIND_F16: return with_out(std::integral_constant<int, KIND_F16>());
+    case KIND_BF16: return with_out(std::integral_constant<int, KIND_BF16>());
   }
   return FLYB200_E_UNSUPPORTED;
+}
+
+}  // namespace
+
+int launch_rows_kind(int kind, int outmode, int form, const CUtensorMap& tmA, const CUtensorMap& tmC, const GemmParams& p,
+                     int sms, cudaStream_t s) {
+  return for_kind(kind, outmode, [&](auto k, auto out) { return rows_any<decltype(k)::value, decltype(out)::value>(form, tmA, tmC, p, sms, s); });
+}
+
+int launch_pair_kind(int kind, int outmode, const PairMaps& maps, const GemmParams& p, int sms, cudaStream_t s) {
+  return for_kind(kind, outmode, [&](auto k, auto out) { return launch_pair<decltype(k)::value, decltype(out)::value>(maps, p, sms, s); });
 }
 
 int launch_rows_scatter_kind(int kind, int outmode, const CUtensorMap& tmA, const OutputMaps& outs, const GemmParams& p,

@@ -31,7 +31,6 @@ enum : int { EPI_NONE = 0, EPI_BIAS = 1, EPI_BIAS_RELU = 2, EPI_BIAS_SILU = 3, E
 constexpr int BLOCK_ROWS = 128;   // UMMA M
 constexpr int KBLOCK_BYTES = 128; // one swizzle row: 128 fp8/int8 or 64 half elements
 constexpr int UMMA_K_BYTES = 32;  // bytes of K consumed by one tcgen05.mma
-constexpr int NUM_THREADS = 192;  // CTA-pair kernel: warp 0 producer, warp 1 MMA, warps 2..5 epilogue
 
 struct GemmParams {
   const uint8_t* w;      // preshuffled weights
@@ -57,7 +56,7 @@ struct GemmParams {
   uint32_t fmt_bits;     // decode kernel, MX kind on bytes: operand formats as instruction-descriptor bits (weights << 7 | tokens << 10)
   int bn;                // large-M kernel: output channels per tile (multiple of 32, 32..256)
   int rows_stages;       // large-M kernel: depth of the shared-memory ring
-  int tail_parts;        // large-M kernel: column parts of the tiles of the last, partial round (1, 2 or 4; bn / parts a multiple of 64)
+  int tail_parts;        // large-M kernels: column parts of the tiles of the last, partial round (1, 2 or 4; bn / parts a multiple of 64)
   int n_dst;             // scatter kernel: number of output buffers
   int dst_first;         // scatter kernel: buffer stored to first
   int* status;           // device status word (first failure wins)

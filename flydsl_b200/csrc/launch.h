@@ -3,6 +3,7 @@
 #pragma once
 #include "decode_kernel.cuh"
 #include "host_common.h"
+#include "rows2_kernel.cuh"
 
 #include <atomic>
 #include <cstdlib>
@@ -13,7 +14,6 @@ namespace host {
 constexpr int SMEM_LIMIT = 232448;  // 227 KiB of dynamic shared memory per CTA
 constexpr int MAX_DEVICES = 64;
 constexpr int ROWS_MAX_STAGES = 8;
-constexpr int ROWS2_STAGES = 6;
 
 #define FLYB200_CUDA_TRY(expr)                                                          \
   do {                                                                                  \
@@ -54,6 +54,36 @@ inline int rows_tail_parts(int bn, long long tiles, int sms) {
   return 2 * rest <= sms ? 2 : 1;
 }
 
+// Pair form: ring depth for a tile width, and the number of 256 x bn tiles.
+inline int pair_stages_for(int bn) {
+  int s = ROWS_MAX_STAGES;
+  while (s > 2 && pair_layout(bn, s).total > SMEM_LIMIT) --s;
+  return s;
+}
+inline long long pair_tiles(int M, int N, int bn) {
+  return static_cast<long long>((M + PAIR_ROWS - 1) / PAIR_ROWS) * ((N + bn - 1) / bn);
+}
+// Cycles a pair spends on one k-block of a tile or strip: the tensor pipe, or the bytes each SM takes in.
+inline long long pair_kb_cycles(int width) {
+  const long long mma = 2LL * width, load = (BLOCK_ROWS + width / 2) * KBLOCK_BYTES / 72;
+  return mma > load ? mma : load;
+}
+// Column strips of the tiles of the last, partial round: the number that makes it shortest.
+inline int pair_tail_parts(int bn, long long tiles, int clusters) {
+  const long long rest = tiles % clusters;
+  if (tiles < clusters || rest == 0) return 1;
+  int best = 1;
+  long long best_cycles = pair_kb_cycles(bn);
+  for (int parts = 2; parts <= 4 && bn % (64 * parts) == 0; parts *= 2) {
+    const long long c = (rest * parts + clusters - 1) / clusters * pair_kb_cycles(bn / parts);
+    if (c < best_cycles) {
+      best_cycles = c;
+      best = parts;
+    }
+  }
+  return best;
+}
+
 // Epilogue warps of the large-M kernel.  With few k-blocks a tile's epilogue is as long as the mainloop that it overlaps,
 // and in a launch of few rounds the last one is exposed: eight warps.  In long launches over 32 k-blocks and more the
 // epilogue is hidden either way and four warps leave more power to the tensor cores.  Eight / four, us, fp8:
@@ -66,13 +96,14 @@ inline int rows_epilogue_warps(int kb, long long tiles, int sms) {
   return kb >= 32 && tiles >= 8LL * sms ? 4 : 8;
 }
 
-// Large-M kernel (p.bn, p.rows_stages set) in one of three forms: one CTA per 128 x bn tile, CTA pairs
-// on 256 x 256 tiles (needs tmW), one CTA per 256 x bn tile (tmA with boxes of 256 rows, three stages).
-// `kind` is KIND_*, `outmode` OUT_*.
-enum : int { ROWS_FORM_ONE = 0, ROWS_FORM_PAIRS = 1, ROWS_FORM_TALL = 2 };
+// Large-M kernel (p.bn, p.rows_stages set): one CTA per 128 x bn tile, or per 256 x bn tile (tmA with boxes of 256 rows,
+// three stages).  `kind` is KIND_*, `outmode` OUT_*.
+enum : int { ROWS_FORM_ONE = 0, ROWS_FORM_TALL = 2 };
 constexpr int ROWS_TALL_STAGES = 3;
-int launch_rows_kind(int kind, int outmode, int form, const CUtensorMap& tmA, const CUtensorMap& tmW,
-                     const CUtensorMap& tmC, const GemmParams& p, int sms, cudaStream_t s);
+int launch_rows_kind(int kind, int outmode, int form, const CUtensorMap& tmA, const CUtensorMap& tmC, const GemmParams& p,
+                     int sms, cudaStream_t s);
+// Large-M kernel, CTA pairs on 256 x bn tiles (p.bn, p.rows_stages, p.tail_parts set).
+int launch_pair_kind(int kind, int outmode, const PairMaps& maps, const GemmParams& p, int sms, cudaStream_t s);
 // Large-M kernel storing every tile through p.n_dst output maps.
 int launch_rows_scatter_kind(int kind, int outmode, const CUtensorMap& tmA, const OutputMaps& outs, const GemmParams& p,
                              int sms, cudaStream_t s);

@@ -61,7 +61,8 @@ extern "C" {
  *   bits 8-11  kernel: 1 = small-M weight-stationary kernel (M <= 1024: up to 256
  *              tokens per CTA, more as token blocks of 256 in grid.z),
  *              2 = large-M persistent kernel, one CTA per 128 x (32..256) tile,
- *              3 = large-M persistent kernel, CTA pairs on 256x256 tiles
+ *              3 = large-M persistent kernel, CTA pairs (tcgen05 cta_group::2) on 256 x (64..256)
+ *              tiles (bits 0-7: the width in units of 32 channels, 2..8; else 256)
  *              4 = small-M kernel with 64-channel weight tiles and no K split
  *              (M <= 64 per token block; twice the CTAs, no reduction step)
  *              5 = small-M kernel as CTA pairs (tcgen05 cta_group::2: 256 channels
@@ -79,7 +80,9 @@ extern "C" {
  *              256 < M <= 1024 -> 1 when 2 * T * ceil(M/256) <= S and K spans at
  *              least 32 blocks of 128 bytes; else M > 256 -> 2, or 3 when FLYB200_ROWS_2SM=1, or 6
  *              when FLYB200_ROWS_TALL=1 or when ceil(M/256) * ceil(N/256) tiles
- *              cover the output in one round that fills at least 80 % of the SMs)
+ *              cover the output in one round that fills at least 80 % of the SMs; a call
+ *              of more than 128 tokens that sets none of the bits 0-27 and 30-31 then runs as 3
+ *              wherever flyb200_pair_width says so)
  *   bits 12-15 how K splits are combined: 1 = global workspace + ticket,
  *              2 = thread-block cluster + distributed shared memory (split <= 8)
  *   bits 16-23 rasterisation group (row tiles per group, large-M kernel)
@@ -220,8 +223,15 @@ size_t flyb200_workspace_bytes(int M, int N, int K, int in_dtype, int variant_hi
  * factor, k-blocks per split, reduction (0 none, 1 workspace, 2 cluster), ring
  * depth, dependent-launch mode, token blocks }.  The B200 counterpart of the
  * per-tile table _TILE_PRELOAD_TABLE / tile arguments the reference's callers
- * tune by hand (kernels/gemm/preshuffle_gemm.py:19-105). */
+ * tune by hand (kernels/gemm/preshuffle_gemm.py:19-105).  A call that leaves the
+ * kernel open runs the planned kernel unless flyb200_pair_width says that CTA
+ * pairs take its place. */
 int flyb200_describe_plan(int M, int N, int K, int in_dtype, int variant_hint, int sm_count, int* out8);
+
+/* Tile width with which the call runs as CTA pairs (256 rows x this many channels
+ * per pair), asked for or because they are estimated to be faster than the plan
+ * of flyb200_describe_plan; 0 where that plan runs.  Pure host function. */
+int flyb200_pair_width(int M, int N, int K, int in_dtype, int variant_hint, int sm_count);
 
 /* Device-side status word of the current device (0 = no failure since the last
  * read).  Synchronises the device; not for the launch path.  The reference only

@@ -92,7 +92,7 @@ __global__ void __launch_bounds__(MX_THREADS, 1) mx_gemm_kernel(const __grid_con
   const uint32_t smem_base = smem_u32(smem_raw);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(smem_raw + L::OFF_MISC + 4);
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(smem_raw + L::OFF_MISC);
-  const int warp = threadIdx.x >> 5;
+  const int warp = warp_index();
   const int lane = threadIdx.x & 31;
   const uint32_t bar_full = smem_base + L::OFF_BAR;
   const uint32_t bar_empty = bar_full + 8 * STAGES;
@@ -154,22 +154,26 @@ __global__ void __launch_bounds__(MX_THREADS, 1) mx_gemm_kernel(const __grid_con
 
   if (warp == 0) {
     // ------------------------------ producer ------------------------------
-    if (lane == 0) {
-      const uint64_t pol = l2_policy_evict_last();
-      int stage = 0;
-      uint32_t phase = 0;
-      int issued = 0;
-      bool ok = true;
-      for (int t = tile0; t < num_tiles && ok; t += tile_step) {
-        int m_blk, n_blk;
-        tile_coords(t, m_blk, n_blk);
-        for (int kb = kb0; kb < kb1; ++kb) {
-          if (!mbar_wait(bar_empty + 8 * stage, phase ^ 1u, abort_flag)) {
-            report_failure(p.status, ST_TIMEOUT, abort_flag);
-            ok = false;
-            break;
-          }
-          const uint32_t fb = bar_full + 8 * stage;
+    // The whole warp runs the loop, here and in the MMA warp, and one lane issues (ptx.cuh).  By themselves the issuing
+    // threads bound this kernel, eleven instructions per k-block in the MMA loop: one lane / whole warp, us, MXFP8 384 x 4096 x 14336
+    // 41.6 / 31.7, 256 x 8192 x 8192 26.4 / 20.1, MXFP4 1024 x 8192 x 8192 36.4 / 29.4, 384 x 4096 x 14336 24.8 / 17.4, MXFP6 256 x 8192 x 8192 26.2 / 20.0.
+    const bool issuer = elect_one();
+    const uint64_t pol = l2_policy_evict_last();
+    int stage = 0;
+    uint32_t phase = 0;
+    int issued = 0;
+    bool ok = true;
+    for (int t = tile0; t < num_tiles && ok; t += tile_step) {
+      int m_blk, n_blk;
+      tile_coords(t, m_blk, n_blk);
+      for (int kb = kb0; kb < kb1; ++kb) {
+        if (!mbar_wait_warp(bar_empty + 8 * stage, phase ^ 1u, abort_flag)) {
+          report_failure(p.status, ST_TIMEOUT, abort_flag);
+          ok = false;
+          break;
+        }
+        const uint32_t fb = bar_full + 8 * stage;
+        if (issuer) {
           mbar_expect_tx(fb, L::A_STAGE + L::B_STAGE + L::SFA_STAGE + L::SFB_STAGE);
           tma_load_2d(smem_base + L::OFF_A + stage * L::A_STAGE, &tmA, fb, kb * KBLOCK_BYTES, m_blk * BLOCK_ROWS, pol);
           bulk_load_1d(smem_base + L::OFF_B + stage * L::B_STAGE,
@@ -183,64 +187,68 @@ __global__ void __launch_bounds__(MX_THREADS, 1) mx_gemm_kernel(const __grid_con
             bulk_load_1d(smem_base + L::OFF_SFB + stage * L::SFB_STAGE + h * L::SFB_HALF,
                          p.sfw + (ekb * (p.N / 128) + n_blk * L::SFB_ATOMS) * MX_SF_ATOM, L::SFB_HALF, fb, pol);
           }
-          ++issued;
-          if (++stage == STAGES) {
-            stage = 0;
-            phase ^= 1u;
-          }
+        }
+        ++issued;
+        if (++stage == STAGES) {
+          stage = 0;
+          phase ^= 1u;
         }
       }
-      pdl_trigger();  // the last loads are on their way: the next kernel may be scheduled as the CTAs finish
-      if (!ok || *abort_flag) {
-        const int pending = min(issued, STAGES);
-        for (int i = 0; i < pending; ++i) {
-          int s = stage - 1 - i;
-          uint32_t ph = phase;
-          if (s < 0) {
-            s += STAGES;
-            ph ^= 1u;
-          }
-          mbar_wait(bar_full + 8 * s, ph, abort_flag + 1);
+    }
+    pdl_trigger();  // the last loads are on their way: the next kernel may be scheduled as the CTAs finish
+    if (!ok || *abort_flag) {
+      const int pending = min(issued, STAGES);
+      for (int i = 0; i < pending; ++i) {
+        int s = stage - 1 - i;
+        uint32_t ph = phase;
+        if (s < 0) {
+          s += STAGES;
+          ph ^= 1u;
         }
+        mbar_wait(bar_full + 8 * s, ph, abort_flag + 1);
       }
     }
   } else if (warp == 1) {
     // ------------------------------ MMA issue -----------------------------
-    if (lane == 0) {
-      // 8-bit containers: E4M3 unless the caller names other formats (E2M3 / E2M1 codes padded to a byte)
-      const uint32_t idesc = FP4 ? umma_idesc_mxf4(BLOCK_ROWS, BN) : (umma_idesc_mxf8(BLOCK_ROWS, BN) | p.fmt_bits);
-      int stage = 0;
-      uint32_t phase = 0;
-      int acc = 0;
-      uint32_t acc_phase = 0;
-      bool ok = true;
-      for (int t = tile0; t < num_tiles && ok; t += tile_step) {
-        if (!mbar_wait(bar_tempty + 8 * acc, acc_phase ^ 1u, abort_flag)) {
+    const bool issuer = elect_one();
+    // 8-bit containers: E4M3 unless the caller names other formats (E2M3 / E2M1 codes padded to a byte)
+    const uint32_t idesc = FP4 ? umma_idesc_mxf4(BLOCK_ROWS, BN) : (umma_idesc_mxf8(BLOCK_ROWS, BN) | p.fmt_bits);
+    const uint64_t adesc0 = umma_desc_sw128_kmajor(smem_base + L::OFF_A), bdesc0 = umma_desc_sw128_kmajor(smem_base + L::OFF_B);
+    const uint64_t sfa_desc0 = sf_smem_desc(smem_base + L::OFF_SFA), sfb_desc0 = sf_smem_desc(smem_base + L::OFF_SFB);
+    int stage = 0;
+    uint32_t phase = 0;
+    int acc = 0;
+    uint32_t acc_phase = 0;
+    bool ok = true;
+    for (int t = tile0; t < num_tiles && ok; t += tile_step) {
+      if (!mbar_wait_warp(bar_tempty + 8 * acc, acc_phase ^ 1u, abort_flag)) {
+        report_failure(p.status, ST_TIMEOUT, abort_flag);
+        break;
+      }
+      tc_fence_after();
+      const uint32_t d_tmem = tmem_base + static_cast<uint32_t>(acc * BN);
+      for (int kb = kb0; kb < kb1; ++kb) {
+        if (!mbar_wait_warp(bar_full + 8 * stage, phase, abort_flag)) {
           report_failure(p.status, ST_TIMEOUT, abort_flag);
+          ok = false;
           break;
         }
         tc_fence_after();
-        const uint32_t d_tmem = tmem_base + static_cast<uint32_t>(acc * BN);
-        for (int kb = kb0; kb < kb1; ++kb) {
-          if (!mbar_wait(bar_full + 8 * stage, phase, abort_flag)) {
-            report_failure(p.status, ST_TIMEOUT, abort_flag);
-            ok = false;
-            break;
-          }
-          tc_fence_after();
-          // scale atoms of this stage: shared memory -> their TMEM columns
-          const uint32_t sfa_t = tmem_base + SF_COL0 + static_cast<uint32_t>(stage * SF_COLS);
-          const uint32_t sfb_t = sfa_t + SFA_COLS;
+        // scale atoms of this stage: shared memory -> their TMEM columns
+        const uint32_t sfa_t = tmem_base + SF_COL0 + static_cast<uint32_t>(stage * SF_COLS);
+        const uint32_t sfb_t = sfa_t + SFA_COLS;
+        const uint64_t adesc = adesc0 + static_cast<uint32_t>(stage * (L::A_STAGE >> 4));
+        const uint64_t bdesc = bdesc0 + static_cast<uint32_t>(stage * (L::B_STAGE >> 4));
+        const uint64_t sfa_desc = sfa_desc0 + static_cast<uint32_t>(stage * (L::SFA_STAGE >> 4));
+        const uint64_t sfb_desc = sfb_desc0 + static_cast<uint32_t>(stage * (L::SFB_STAGE >> 4));
+        if (issuer) {
 #pragma unroll
           for (int h = 0; h < HALVES; ++h) {
-            tmem_cp_sf(sfa_t + 4 * h, sf_smem_desc(smem_base + L::OFF_SFA + stage * L::SFA_STAGE + h * MX_SF_ATOM));
+            tmem_cp_sf(sfa_t + 4 * h, sfa_desc + h * (MX_SF_ATOM >> 4));
 #pragma unroll
             for (int at = 0; at < L::SFB_ATOMS; ++at)
-              tmem_cp_sf(sfb_t + 4 * (h * L::SFB_ATOMS + at),
-                         sf_smem_desc(smem_base + L::OFF_SFB + stage * L::SFB_STAGE + h * L::SFB_HALF + at * MX_SF_ATOM));
+              tmem_cp_sf(sfb_t + 4 * (h * L::SFB_ATOMS + at), sfb_desc + ((h * L::SFB_HALF + at * MX_SF_ATOM) >> 4));
           }
-          const uint64_t adesc = umma_desc_sw128_kmajor(smem_base + L::OFF_A + stage * L::A_STAGE);
-          const uint64_t bdesc = umma_desc_sw128_kmajor(smem_base + L::OFF_B + stage * L::B_STAGE);
 #pragma unroll
           for (int k = 0; k < KBLOCK_BYTES / UMMA_K_BYTES; ++k) {
             if constexpr (FP4) {
@@ -258,16 +266,15 @@ __global__ void __launch_bounds__(MX_THREADS, 1) mx_gemm_kernel(const __grid_con
             }
           }
           umma_commit(bar_empty + 8 * stage);
-          if (++stage == STAGES) {
-            stage = 0;
-            phase ^= 1u;
-          }
+          if (kb == kb1 - 1) umma_commit(bar_tfull + 8 * acc);
         }
-        if (!ok) break;
-        umma_commit(bar_tfull + 8 * acc);
-        acc = (acc + 1) % NACC;
-        if (acc == 0) acc_phase ^= 1u;
+        if (++stage == STAGES) {
+          stage = 0;
+          phase ^= 1u;
+        }
       }
+      acc = (acc + 1) % NACC;
+      if (acc == 0) acc_phase ^= 1u;
     }
   } else {
     // ------------------------------ epilogue ------------------------------

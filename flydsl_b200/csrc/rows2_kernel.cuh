@@ -141,7 +141,7 @@ gemm_pair_kernel(const __grid_constant__ PairMaps maps, const GemmParams p) {
   volatile int* abort_flag = reinterpret_cast<volatile int*>(smem_raw + L.off_misc + 4);
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(smem_raw + L.off_misc);
 
-  const int warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0);  // uniform over the warp
+  const int warp = warp_index();
   const int lane = threadIdx.x & 31;
   const uint32_t rank = cluster_rank();  // 0 = leader
   const uint32_t bar_full = smem_base + L.off_bar;

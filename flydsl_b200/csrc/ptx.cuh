@@ -123,9 +123,9 @@ __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, volatil
 // (rows2_kernel.cuh), 537 with the whole warp.
 __device__ __forceinline__ int warp_index() { return __shfl_sync(0xffffffffu, static_cast<int>(threadIdx.x >> 5), 0); }
 // mbar_wait of all lanes of a warp together; the answer is uniform.
-__device__ __forceinline__ bool mbar_wait_warp(uint32_t bar, uint32_t parity, volatile int* abort_flag) {
+__device__ __forceinline__ bool mbar_wait_warp(uint32_t bar, uint32_t parity, volatile int* abort_flag, long long* waited = nullptr) {
   if (__all_sync(0xffffffffu, mbar_try_wait(bar, parity))) return true;
-  return __all_sync(0xffffffffu, mbar_wait(bar, parity, abort_flag));
+  return __all_sync(0xffffffffu, mbar_wait(bar, parity, abort_flag, waited));
 }
 
 // ---- proxies / fences -------------------------------------------------------

@@ -436,7 +436,7 @@ __device__ __forceinline__ void gemm_rows_body(const CUtensorMap& tmA, const CUt
   volatile int* abort_flag = reinterpret_cast<volatile int*>(smem_raw + L.off_misc + 4);
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(smem_raw + L.off_misc);
 
-  const int warp = threadIdx.x >> 5;
+  const int warp = warp_index();
   const int lane = threadIdx.x & 31;
   const uint32_t bar_full = smem_base + L.off_bar;
   const uint32_t bar_empty = bar_full + 8 * STAGES;
@@ -528,102 +528,96 @@ __device__ __forceinline__ void gemm_rows_body(const CUtensorMap& tmA, const CUt
 
   if (warp == 0) {
     // ------------------------------ producer ------------------------------
-    if (lane == 0) {
-      const uint64_t pol_a = l2_policy_evict_last();
-      const uint64_t pol_w = l2_policy_evict_last();
-      int stage = 0;
-      uint32_t phase = 0;
-      int issued = 0;
-      bool ok = true;
-      for (int t = blockIdx.x; t < items && ok; t += gridDim.x) {
-        int m_blk, n0, width;
-        if (!item_coords(t, m_blk, n0, width)) continue;
-        const uint32_t w_rows = static_cast<uint32_t>(min(width, p.N - n0));
-        const uint32_t w_bytes = w_rows * KBLOCK_BYTES;
-        // The ring holds a few k-blocks; the weights of the next `prefetch`
-        // k-blocks are already on their way from DRAM into L2, so the depth
-        // of the ring only has to cover the L2 latency.
-        const int ahead = min(p.prefetch, num_kb);
-        for (int kb = 0; kb < ahead; ++kb)
-          bulk_prefetch_l2(p.w + (static_cast<size_t>(kb) * p.N + n0) * KBLOCK_BYTES, w_bytes);
-        for (int kb = 0; kb < num_kb; ++kb) {
-          if (ahead > 0 && kb + ahead < num_kb)
-            bulk_prefetch_l2(p.w + (static_cast<size_t>(kb + ahead) * p.N + n0) * KBLOCK_BYTES, w_bytes);
-          if (!mbar_wait(bar_empty + 8 * stage, phase ^ 1u, abort_flag FLYB200_PROF_ARG(&prof_wait[0]))) {
-            report_failure(p.status, ST_TIMEOUT, abort_flag);
-            ok = false;
-            break;
-          }
-          const uint32_t fb = bar_full + 8 * stage;
+    const bool issuer = elect_one();  // the whole warp runs the loop, here and in the MMA warp, and one lane issues (ptx.cuh)
+    const uint64_t pol_a = l2_policy_evict_last();
+    const uint64_t pol_w = l2_policy_evict_last();
+    int stage = 0;
+    uint32_t phase = 0;
+    int issued = 0;
+    bool ok = true;
+    for (int t = blockIdx.x; t < items && ok; t += gridDim.x) {
+      int m_blk, n0, width;
+      if (!item_coords(t, m_blk, n0, width)) continue;
+      const uint32_t w_rows = static_cast<uint32_t>(min(width, p.N - n0));
+      const uint32_t w_bytes = w_rows * KBLOCK_BYTES;
+      for (int kb = 0; kb < num_kb; ++kb) {
+        if (!mbar_wait_warp(bar_empty + 8 * stage, phase ^ 1u, abort_flag FLYB200_PROF_ARG(&prof_wait[0]))) {
+          report_failure(p.status, ST_TIMEOUT, abort_flag);
+          ok = false;
+          break;
+        }
+        const uint32_t fb = bar_full + 8 * stage;
+        if (issuer) {
           mbar_expect_tx(fb, L.a_stage + w_bytes);
           tma_load_2d(smem_base + stage * L.a_stage, &tmA, fb, kb * KBLOCK_BYTES, m_blk * BLOCK_ROWS, pol_a);
           bulk_load_1d(smem_base + L.off_b + stage * L.b_stage,
                        p.w + (static_cast<size_t>(kb) * p.N + n0) * KBLOCK_BYTES, w_bytes, fb, pol_w);
-          ++issued;
-          if (++stage == STAGES) {
-            stage = 0;
-            phase ^= 1u;
-          }
+        }
+        ++issued;
+        if (++stage == STAGES) {
+          stage = 0;
+          phase ^= 1u;
         }
       }
-      if (!ok || *abort_flag) {
-        // Drain: wait (bounded) for the copies this thread still has in flight
-        // so that none lands in shared memory after the CTA has gone.
-        const int pending = min(issued, STAGES);
-        for (int i = 0; i < pending; ++i) {
-          int s = stage - 1 - i;
-          uint32_t ph = phase;
-          if (s < 0) {
-            s += STAGES;
-            ph ^= 1u;
-          }
-          mbar_wait(bar_full + 8 * s, ph, abort_flag + 1 /* never set: wait on time only */);
+    }
+    if (!ok || *abort_flag) {
+      // Drain: wait (bounded) for the copies this warp still has in flight
+      // so that none lands in shared memory after the CTA has gone.
+      const int pending = min(issued, STAGES);
+      for (int i = 0; i < pending; ++i) {
+        int s = stage - 1 - i;
+        uint32_t ph = phase;
+        if (s < 0) {
+          s += STAGES;
+          ph ^= 1u;
         }
+        mbar_wait(bar_full + 8 * s, ph, abort_flag + 1 /* never set: wait on time only */);
       }
     }
   } else if (warp == 1) {
     // ------------------------------ MMA issue -----------------------------
-    if (lane == 0) {
-      int stage = 0;
-      uint32_t phase = 0;
-      int acc = 0;
-      uint32_t acc_phase = 0;
-      bool ok = true;
-      for (int t = blockIdx.x; t < items && ok; t += gridDim.x) {
-        int m_blk, n0, width;
-        if (!item_coords(t, m_blk, n0, width)) continue;
-        const uint32_t idesc = umma_idesc(KT::dfmt, KT::abfmt, BLOCK_ROWS, static_cast<uint32_t>(width));
-        if (!mbar_wait(bar_tempty + 8 * acc, acc_phase ^ 1u, abort_flag FLYB200_PROF_ARG(&prof_wait[1]))) {
+    const bool issuer = elect_one();
+    const uint64_t adesc0 = umma_desc_sw128_kmajor(smem_base), bdesc0 = umma_desc_sw128_kmajor(smem_base + L.off_b);
+    int stage = 0;
+    uint32_t phase = 0;
+    int acc = 0;
+    uint32_t acc_phase = 0;
+    bool ok = true;
+    for (int t = blockIdx.x; t < items && ok; t += gridDim.x) {
+      int m_blk, n0, width;
+      if (!item_coords(t, m_blk, n0, width)) continue;
+      const uint32_t idesc = umma_idesc(KT::dfmt, KT::abfmt, BLOCK_ROWS, static_cast<uint32_t>(width));
+      if (!mbar_wait_warp(bar_tempty + 8 * acc, acc_phase ^ 1u, abort_flag FLYB200_PROF_ARG(&prof_wait[1]))) {
+        report_failure(p.status, ST_TIMEOUT, abort_flag);
+        break;
+      }
+      tc_fence_after();
+      const uint32_t d_tmem = tmem_base + static_cast<uint32_t>(acc * ROWS_ACC_COLS);
+      for (int kb = 0; kb < num_kb; ++kb) {
+        if (!mbar_wait_warp(bar_full + 8 * stage, phase, abort_flag FLYB200_PROF_ARG(&prof_wait[2]))) {
           report_failure(p.status, ST_TIMEOUT, abort_flag);
+          ok = false;
           break;
         }
         tc_fence_after();
-        const uint32_t d_tmem = tmem_base + static_cast<uint32_t>(acc * ROWS_ACC_COLS);
-        for (int kb = 0; kb < num_kb; ++kb) {
-          if (!mbar_wait(bar_full + 8 * stage, phase, abort_flag FLYB200_PROF_ARG(&prof_wait[2]))) {
-            report_failure(p.status, ST_TIMEOUT, abort_flag);
-            ok = false;
-            break;
-          }
-          tc_fence_after();
-          const uint64_t adesc = umma_desc_sw128_kmajor(smem_base + stage * L.a_stage);
-          const uint64_t bdesc = umma_desc_sw128_kmajor(smem_base + L.off_b + stage * L.b_stage);
+        const uint64_t adesc = adesc0 + static_cast<uint32_t>(stage * (L.a_stage >> 4));
+        const uint64_t bdesc = bdesc0 + static_cast<uint32_t>(stage * (L.b_stage >> 4));
+        if (issuer) {
 #pragma unroll
           for (int k = 0; k < KBLOCK_BYTES / UMMA_K_BYTES; ++k) {
             umma_ss<KIND>(d_tmem, adesc + static_cast<uint64_t>(k * (UMMA_K_BYTES >> 4)),
                           bdesc + static_cast<uint64_t>(k * (UMMA_K_BYTES >> 4)), idesc, (kb | k) != 0 ? 1u : 0u);
           }
           umma_commit(bar_empty + 8 * stage);
-          if (++stage == STAGES) {
-            stage = 0;
-            phase ^= 1u;
-          }
+          if (kb == num_kb - 1) umma_commit(bar_tfull + 8 * acc);
         }
-        if (!ok) break;
-        umma_commit(bar_tfull + 8 * acc);
-        acc ^= 1;
-        if (acc == 0) acc_phase ^= 1u;
+        if (++stage == STAGES) {
+          stage = 0;
+          phase ^= 1u;
+        }
       }
+      acc ^= 1;
+      if (acc == 0) acc_phase ^= 1u;
     }
   } else {
     // ------------------------------ epilogue ------------------------------

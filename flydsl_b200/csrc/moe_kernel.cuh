@@ -144,7 +144,7 @@ __global__ void __launch_bounds__(MOE_THREADS) moe_gemm_kernel(const __grid_cons
   float* sa_s = reinterpret_cast<float*>(smem_raw + L.off_sa);
   float* tw_s = reinterpret_cast<float*>(smem_raw + L.off_tw);
 
-  const int warp = threadIdx.x >> 5;
+  const int warp = warp_index();
   const int lane = threadIdx.x & 31;
   const uint32_t bar_full = smem_base + L.off_bar;
   const uint32_t bar_empty = bar_full + 8 * stages;
@@ -214,92 +214,100 @@ __global__ void __launch_bounds__(MOE_THREADS) moe_gemm_kernel(const __grid_cons
 
   if (warp == 0) {
     // ------------------------------ producer ------------------------------
-    if (lane == 0) {
-      const uint64_t pol_a = l2_policy_evict_last();
-      const uint64_t pol_w = l2_policy_evict_normal();  // other blocks of the same expert read the same tiles
-      int stage = 0;
-      uint32_t phase = 0;
-      int issued = 0;
-      auto load_weights = [&](int kb, int st, uint32_t fb) {
-        mbar_expect_tx(fb, A_STAGE + w_bytes0 + w_bytes1);
-        const uint32_t wdst = smem_base + L.off_w + st * W_STAGE;
-        bulk_load_1d(wdst, w_expert + (static_cast<size_t>(kb) * p.n_expert + w_row[0]) * KBLOCK_BYTES, w_bytes0, fb,
-                     pol_w);
-        if (has_b)
-          bulk_load_1d(wdst + W_TILE, w_expert + (static_cast<size_t>(kb) * p.n_expert + w_row[1]) * KBLOCK_BYTES,
-                       w_bytes1, fb, pol_w);
-      };
-      // As a programmatic dependent of the gather pass the kernel may run before
-      // the gathered activations exist.  The weights are model state: the ring is
-      // filled with them first; everything the gather pass writes is touched only
-      // after griddepcontrol.wait.
-      const int pre = p.pdl ? min(stages, num_kb) : 0;
+    const bool issuer = elect_one();  // the whole warp runs the loop, here and in the MMA warps, and one lane issues (ptx.cuh)
+    const uint64_t pol_a = l2_policy_evict_last();
+    const uint64_t pol_w = l2_policy_evict_normal();  // other blocks of the same expert read the same tiles
+    int stage = 0;
+    uint32_t phase = 0;
+    int issued = 0;
+    auto load_weights = [&](int kb, int st, uint32_t fb) {
+      mbar_expect_tx(fb, A_STAGE + w_bytes0 + w_bytes1);
+      const uint32_t wdst = smem_base + L.off_w + st * W_STAGE;
+      bulk_load_1d(wdst, w_expert + (static_cast<size_t>(kb) * p.n_expert + w_row[0]) * KBLOCK_BYTES, w_bytes0, fb,
+                   pol_w);
+      if (has_b)
+        bulk_load_1d(wdst + W_TILE, w_expert + (static_cast<size_t>(kb) * p.n_expert + w_row[1]) * KBLOCK_BYTES,
+                     w_bytes1, fb, pol_w);
+    };
+    // As a programmatic dependent of the gather pass the kernel may run before
+    // the gathered activations exist.  The weights are model state: the ring is
+    // filled with them first; everything the gather pass writes is touched only
+    // after griddepcontrol.wait.
+    const int pre = p.pdl ? min(stages, num_kb) : 0;
+    if (issuer)
       for (int i = 0; i < pre; ++i) load_weights(i, i, bar_full + 8 * i);
-      if (p.pdl) asm volatile("griddepcontrol.wait;" ::: "memory");
+    if (p.pdl) asm volatile("griddepcontrol.wait;" ::: "memory");
+    if (issuer)
       for (int i = 0; i < pre; ++i)
         tma_load_2d(smem_base + L.off_a + i * A_STAGE, &tmA, bar_full + 8 * i, i * KBLOCK_BYTES, row0, pol_a);
-      issued = pre;
-      if (pre == stages) phase = 1u; else stage = pre;
-      for (int kb = pre; kb < num_kb; ++kb) {
-        if (!mbar_wait(bar_empty + 8 * stage, phase ^ 1u, abort_flag)) {
-          report_failure(p.status, ST_TIMEOUT, abort_flag);
-          ok = false;
-          break;
-        }
-        const uint32_t fb = bar_full + 8 * stage;
+    issued = pre;
+    if (pre == stages) phase = 1u; else stage = pre;
+    for (int kb = pre; kb < num_kb; ++kb) {
+      if (!mbar_wait_warp(bar_empty + 8 * stage, phase ^ 1u, abort_flag)) {
+        report_failure(p.status, ST_TIMEOUT, abort_flag);
+        ok = false;
+        break;
+      }
+      const uint32_t fb = bar_full + 8 * stage;
+      if (issuer) {
         load_weights(kb, stage, fb);
         tma_load_2d(smem_base + L.off_a + stage * A_STAGE, &tmA, fb, kb * KBLOCK_BYTES, row0, pol_a);
-        ++issued;
-        if (++stage == stages) {
-          stage = 0;
-          phase ^= 1u;
-        }
       }
-      if (p.pdl) pdl_trigger();  // after its wait: the next kernel may be scheduled as the CTAs finish
-      if (!ok || *abort_flag) {
-        // wait (bounded) for copies still in flight so none lands after the CTA is gone
-        const int pending = min(issued, stages);
-        for (int i = 0; i < pending; ++i) {
-          int s = stage - 1 - i;
-          uint32_t ph = phase;
-          if (s < 0) {
-            s += stages;
-            ph ^= 1u;
-          }
-          mbar_wait(bar_full + 8 * s, ph, abort_flag + 1);
+      ++issued;
+      if (++stage == stages) {
+        stage = 0;
+        phase ^= 1u;
+      }
+    }
+    if (p.pdl) pdl_trigger();  // after its wait: the next kernel may be scheduled as the CTAs finish
+    if (!ok || *abort_flag) {
+      // wait (bounded) for copies still in flight so none lands after the CTA is gone
+      const int pending = min(issued, stages);
+      for (int i = 0; i < pending; ++i) {
+        int s = stage - 1 - i;
+        uint32_t ph = phase;
+        if (s < 0) {
+          s += stages;
+          ph ^= 1u;
         }
+        mbar_wait(bar_full + 8 * s, ph, abort_flag + 1);
       }
     }
     __syncwarp();
   } else if (warp == 1 || warp == 6) {
     // ------------------------------ MMA issue -----------------------------
     const int which = warp == 1 ? 0 : 1;  // tile A / tile B
-    if (lane == 0 && (which == 0 || has_b)) {
+    if (which == 0 || has_b) {
+      const bool issuer = elect_one();
       constexpr uint32_t idesc = umma_idesc(KT::dfmt, KT::abfmt, BLOCK_ROWS, BN);
       const uint32_t d_tmem = tmem_base + static_cast<uint32_t>(which * BN);
+      const uint64_t wdesc0 = umma_desc_sw128_kmajor(smem_base + L.off_w + which * W_TILE);
+      const uint64_t adesc0 = umma_desc_sw128_kmajor(smem_base + L.off_a);
       int stage = 0;
       uint32_t phase = 0;
       for (int kb = 0; kb < num_kb; ++kb) {
-        if (!mbar_wait(bar_full + 8 * stage, phase, abort_flag)) {
+        if (!mbar_wait_warp(bar_full + 8 * stage, phase, abort_flag)) {
           report_failure(p.status, ST_TIMEOUT, abort_flag);
           ok = false;
           break;
         }
         tc_fence_after();
-        const uint64_t wdesc = umma_desc_sw128_kmajor(smem_base + L.off_w + stage * W_STAGE + which * W_TILE);
-        const uint64_t adesc = umma_desc_sw128_kmajor(smem_base + L.off_a + stage * A_STAGE);
+        const uint64_t wdesc = wdesc0 + static_cast<uint32_t>(stage * (W_STAGE >> 4));
+        const uint64_t adesc = adesc0 + static_cast<uint32_t>(stage * (A_STAGE >> 4));
+        if (issuer) {
 #pragma unroll
-        for (int k = 0; k < KBLOCK_BYTES / UMMA_K_BYTES; ++k) {
-          umma_ss<KIND>(d_tmem, wdesc + static_cast<uint64_t>(k * (UMMA_K_BYTES >> 4)),
-                        adesc + static_cast<uint64_t>(k * (UMMA_K_BYTES >> 4)), idesc, (kb != 0 || k != 0) ? 1u : 0u);
+          for (int k = 0; k < KBLOCK_BYTES / UMMA_K_BYTES; ++k) {
+            umma_ss<KIND>(d_tmem, wdesc + static_cast<uint64_t>(k * (UMMA_K_BYTES >> 4)),
+                          adesc + static_cast<uint64_t>(k * (UMMA_K_BYTES >> 4)), idesc, (kb != 0 || k != 0) ? 1u : 0u);
+          }
+          umma_commit(bar_empty + 8 * stage);
+          if (kb == num_kb - 1) umma_commit(bar_tfull);
         }
-        umma_commit(bar_empty + 8 * stage);
         if (++stage == stages) {
           stage = 0;
           phase ^= 1u;
         }
       }
-      if (ok) umma_commit(bar_tfull);
     }
     __syncwarp();
   } else {
@@ -498,7 +506,7 @@ __global__ void __launch_bounds__(moe_rows_threads(STAGE), 1) moe_rows_kernel(co
   const uint32_t smem_base = smem_u32(smem_raw);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(smem_raw + L::OFF_MISC + 4);
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(smem_raw + L::OFF_MISC);
-  const int warp = threadIdx.x >> 5;
+  const int warp = warp_index();
   const int lane = threadIdx.x & 31;
   const uint32_t bar_full = smem_base + L::OFF_BAR;
   const uint32_t bar_empty = bar_full + 8 * STAGES;
@@ -598,98 +606,100 @@ __global__ void __launch_bounds__(moe_rows_threads(STAGE), 1) moe_rows_kernel(co
 
   if (warp == 0) {
     // ------------------------------ producer ------------------------------
-    if (lane == 0) {
-      const uint64_t pol = l2_policy_evict_last();
-      int stage = 0;
-      uint32_t phase = 0;
-      int issued = 0;
-      bool ok = true;
-      for (int t = blockIdx.x; t < items && ok; t += gridDim.x) {
-        int rb, pair, lo, hi;
-        const int expert = item_of(t, rb, pair, lo, hi);
-        if (expert < 0) continue;
-        int w_row[2], n_valid[2];
-        tiles_of(pair, w_row, n_valid);
-        const uint8_t* w_expert = p.w + static_cast<size_t>(expert) * p.n_expert * p.K_bytes;
-        const uint32_t b0 = static_cast<uint32_t>(n_valid[0]) * KBLOCK_BYTES, b1 = static_cast<uint32_t>(n_valid[1]) * KBLOCK_BYTES;
-        for (int kb = 0; kb < num_kb; ++kb) {
-          if (!mbar_wait(bar_empty + 8 * stage, phase ^ 1u, abort_flag)) {
-            report_failure(p.status, ST_TIMEOUT, abort_flag);
-            ok = false;
-            break;
-          }
-          const uint32_t fb = bar_full + 8 * stage;
+    const bool issuer = elect_one();
+    const uint64_t pol = l2_policy_evict_last();
+    int stage = 0;
+    uint32_t phase = 0;
+    int issued = 0;
+    bool ok = true;
+    for (int t = blockIdx.x; t < items && ok; t += gridDim.x) {
+      int rb, pair, lo, hi;
+      const int expert = __shfl_sync(0xffffffffu, item_of(t, rb, pair, lo, hi), 0);
+      if (expert < 0) continue;
+      int w_row[2], n_valid[2];
+      tiles_of(pair, w_row, n_valid);
+      const uint8_t* w_expert = p.w + static_cast<size_t>(expert) * p.n_expert * p.K_bytes;
+      const uint32_t b0 = static_cast<uint32_t>(n_valid[0]) * KBLOCK_BYTES, b1 = static_cast<uint32_t>(n_valid[1]) * KBLOCK_BYTES;
+      for (int kb = 0; kb < num_kb; ++kb) {
+        if (!mbar_wait_warp(bar_empty + 8 * stage, phase ^ 1u, abort_flag)) {
+          report_failure(p.status, ST_TIMEOUT, abort_flag);
+          ok = false;
+          break;
+        }
+        const uint32_t fb = bar_full + 8 * stage;
+        const uint32_t bdst = smem_base + L::OFF_B + stage * L::B_STAGE;
+        if (issuer) {
           mbar_expect_tx(fb, L::A_STAGE + b0 + b1);
           tma_load_2d(smem_base + L::OFF_A + stage * L::A_STAGE, &tmA, fb, kb * KBLOCK_BYTES, rb * BLOCK_ROWS, pol);
-          const uint32_t bdst = smem_base + L::OFF_B + stage * L::B_STAGE;
           bulk_load_1d(bdst, w_expert + (static_cast<size_t>(kb) * p.n_expert + w_row[0]) * KBLOCK_BYTES, b0, fb, pol);
           if (b1)
             bulk_load_1d(bdst + BLOCK_ROWS * KBLOCK_BYTES,
                          w_expert + (static_cast<size_t>(kb) * p.n_expert + w_row[1]) * KBLOCK_BYTES, b1, fb, pol);
-          ++issued;
-          if (++stage == STAGES) {
-            stage = 0;
-            phase ^= 1u;
-          }
+        }
+        ++issued;
+        if (++stage == STAGES) {
+          stage = 0;
+          phase ^= 1u;
         }
       }
-      pdl_trigger();  // the last loads are on their way: the next kernel may be scheduled as the CTAs finish
-      if (!ok || *abort_flag) {
-        const int pending = min(issued, STAGES);
-        for (int i = 0; i < pending; ++i) {
-          int s = stage - 1 - i;
-          uint32_t ph = phase;
-          if (s < 0) {
-            s += STAGES;
-            ph ^= 1u;
-          }
-          mbar_wait(bar_full + 8 * s, ph, abort_flag + 1);
+    }
+    pdl_trigger();  // the last loads are on their way: the next kernel may be scheduled as the CTAs finish
+    if (!ok || *abort_flag) {
+      const int pending = min(issued, STAGES);
+      for (int i = 0; i < pending; ++i) {
+        int s = stage - 1 - i;
+        uint32_t ph = phase;
+        if (s < 0) {
+          s += STAGES;
+          ph ^= 1u;
         }
+        mbar_wait(bar_full + 8 * s, ph, abort_flag + 1);
       }
     }
   } else if (warp == 1) {
     // ------------------------------ MMA issue -----------------------------
-    if (lane == 0) {
-      constexpr uint32_t idesc = umma_idesc(KT::dfmt, KT::abfmt, BLOCK_ROWS, BN);
-      int stage = 0;
-      uint32_t phase = 0;
-      int acc = 0;
-      uint32_t acc_phase = 0;
-      bool ok = true;
-      for (int t = blockIdx.x; t < items && ok; t += gridDim.x) {
-        int rb, pair, lo, hi;
-        if (item_of(t, rb, pair, lo, hi) < 0) continue;
-        if (!mbar_wait(bar_tempty + 8 * acc, acc_phase ^ 1u, abort_flag)) {
+    const bool issuer = elect_one();
+    constexpr uint32_t idesc = umma_idesc(KT::dfmt, KT::abfmt, BLOCK_ROWS, BN);
+    const uint64_t adesc0 = umma_desc_sw128_kmajor(smem_base + L::OFF_A), bdesc0 = umma_desc_sw128_kmajor(smem_base + L::OFF_B);
+    int stage = 0;
+    uint32_t phase = 0;
+    int acc = 0;
+    uint32_t acc_phase = 0;
+    bool ok = true;
+    for (int t = blockIdx.x; t < items && ok; t += gridDim.x) {
+      int rb, pair, lo, hi;
+      if (__shfl_sync(0xffffffffu, item_of(t, rb, pair, lo, hi), 0) < 0) continue;
+      if (!mbar_wait_warp(bar_tempty + 8 * acc, acc_phase ^ 1u, abort_flag)) {
+        report_failure(p.status, ST_TIMEOUT, abort_flag);
+        break;
+      }
+      tc_fence_after();
+      const uint32_t d_tmem = tmem_base + static_cast<uint32_t>(acc * BN);
+      for (int kb = 0; kb < num_kb; ++kb) {
+        if (!mbar_wait_warp(bar_full + 8 * stage, phase, abort_flag)) {
           report_failure(p.status, ST_TIMEOUT, abort_flag);
+          ok = false;
           break;
         }
         tc_fence_after();
-        const uint32_t d_tmem = tmem_base + static_cast<uint32_t>(acc * BN);
-        for (int kb = 0; kb < num_kb; ++kb) {
-          if (!mbar_wait(bar_full + 8 * stage, phase, abort_flag)) {
-            report_failure(p.status, ST_TIMEOUT, abort_flag);
-            ok = false;
-            break;
-          }
-          tc_fence_after();
-          const uint64_t adesc = umma_desc_sw128_kmajor(smem_base + L::OFF_A + stage * L::A_STAGE);
-          const uint64_t bdesc = umma_desc_sw128_kmajor(smem_base + L::OFF_B + stage * L::B_STAGE);
+        const uint64_t adesc = adesc0 + static_cast<uint32_t>(stage * (L::A_STAGE >> 4));
+        const uint64_t bdesc = bdesc0 + static_cast<uint32_t>(stage * (L::B_STAGE >> 4));
+        if (issuer) {
 #pragma unroll
           for (int k = 0; k < KBLOCK_BYTES / UMMA_K_BYTES; ++k) {
             umma_ss<KIND>(d_tmem, adesc + static_cast<uint64_t>(k * (UMMA_K_BYTES >> 4)),
                           bdesc + static_cast<uint64_t>(k * (UMMA_K_BYTES >> 4)), idesc, (kb | k) != 0 ? 1u : 0u);
           }
           umma_commit(bar_empty + 8 * stage);
-          if (++stage == STAGES) {
-            stage = 0;
-            phase ^= 1u;
-          }
+          if (kb == num_kb - 1) umma_commit(bar_tfull + 8 * acc);
         }
-        if (!ok) break;
-        umma_commit(bar_tfull + 8 * acc);
-        acc ^= 1;
-        if (acc == 0) acc_phase ^= 1u;
+        if (++stage == STAGES) {
+          stage = 0;
+          phase ^= 1u;
+        }
       }
+      acc ^= 1;
+      if (acc == 0) acc_phase ^= 1u;
     }
   } else {
     // ------------------------------ epilogue ------------------------------

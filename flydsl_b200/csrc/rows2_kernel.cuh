@@ -141,7 +141,8 @@ gemm_pair_kernel(const __grid_constant__ PairMaps maps, const GemmParams p) {
   volatile int* abort_flag = reinterpret_cast<volatile int*>(smem_raw + L.off_misc + 4);
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(smem_raw + L.off_misc);
 
-  const int warp = warp_index();
+  const int warp = threadIdx.x >> 5;
+  const int role = warp_index();  // for the loops that issue
   const int lane = threadIdx.x & 31;
   const uint32_t rank = cluster_rank();  // 0 = leader
   const uint32_t bar_full = smem_base + L.off_bar;
@@ -220,7 +221,7 @@ gemm_pair_kernel(const __grid_constant__ PairMaps maps, const GemmParams p) {
     return n0 < p.N;
   };
 
-  if (warp == 0) {
+  if (role == 0) {
     // ---------------- producer (both CTAs): own A rows, own half of the weight rows ----------------
     // The whole warp runs the loop and one lane issues, as in the MMA warp.
     const bool issuer = elect_one();
@@ -278,7 +279,7 @@ gemm_pair_kernel(const __grid_constant__ PairMaps maps, const GemmParams p) {
       }
     }
     __syncwarp();
-  } else if (warp == 1) {
+  } else if (role == 1) {
     // ---------------- MMA issue (leader only) ----------------
     // The whole warp runs the loop and one lane issues, so that addresses and descriptors stay uniform over the warp; the
     // same loop in one thread took 779 cycles per k-block, this way 537 (bf16 8192 x 8192 x 8192).

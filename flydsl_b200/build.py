@@ -47,6 +47,7 @@ HEADERS = [
     "decode2_kernel.cuh",
     "quant_kernel.cuh",
     "moe_kernel.cuh",
+    "moe_pair_kernel.cuh",
     "mx_kernel.cuh",
     "mx_quant_kernel.cuh",
     "launch.h",

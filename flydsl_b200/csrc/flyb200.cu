@@ -875,6 +875,9 @@ int gemm_mx_small(void* c, const void* a, const void* w, const void* sf_a, const
   return host::launch_decode_kind(fp4 ? KIND_MXF4 : KIND_MXF8, outmode == OUT_FP16 ? OUT_FP16 : OUT_BF16, plan.bn, plan.w_rows, tmA,
                                   p, s);
 }
+int weight_image_map(CUtensorMap* m, const void* base, uint64_t n_rows, uint64_t k_blocks, uint32_t box_rows) {
+  return make_weight_map(m, base, n_rows, k_blocks, box_rows);
+}
 int byte_matrix_map(CUtensorMap* m, const void* base, uint64_t row_bytes, uint64_t rows, uint32_t box_rows) {
   return make_map(m, CU_TENSOR_MAP_DATA_TYPE_UINT8, 1, base, row_bytes, rows, KBLOCK_BYTES, box_rows);
 }

@@ -2,7 +2,7 @@
 // include/flyb200.h — argument checks, tensor map, kernel selection, launch.
 #include "../../include/flyb200.h"
 #include "host_common.h"
-#include "moe_kernel.cuh"
+#include "moe_pair_kernel.cuh"
 
 #include <atomic>
 #include <cstdlib>
@@ -78,9 +78,43 @@ int sm_count(int* out) {
   return FLYB200_OK;
 }
 
+// CTA pairs on up to 256 rows of an expert.
+template <int KIND, int STAGE, int OUTMODE, bool ACCUM>
+int launch_moe_pair(const CUtensorMap& tmA, const MoePairWeights& tmW, const MoeParams& p, int blocks, int sms, cudaStream_t s) {
+  static std::atomic<uint64_t> done{0};
+  auto kernel = moe_pair_kernel<KIND, STAGE, OUTMODE, ACCUM>;
+  int dev = 0;
+  CUDA_TRY(cudaGetDevice(&dev));
+  const uint64_t bit = 1ull << dev;
+  if (!(done.load(std::memory_order_acquire) & bit)) {
+    CUDA_TRY(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, MoePairSmem::TOTAL));
+    done.fetch_or(bit, std::memory_order_release);
+  }
+  const int pairs = STAGE == 1 ? (p.n_out + BLOCK_ROWS - 1) / BLOCK_ROWS : (p.n_out + MOE_ROWS_BN - 1) / MOE_ROWS_BN;
+  const long long items = static_cast<long long>(blocks) * pairs;  // at most: a tile holds a routing block or more
+  const int clusters = static_cast<int>(items < sms / 2 ? items : sms / 2);
+  cudaLaunchConfig_t cfg;
+  memset(&cfg, 0, sizeof(cfg));
+  cfg.gridDim = dim3(2 * clusters, 1, 1);
+  cfg.blockDim = dim3(moe_rows_threads(STAGE), 1, 1);
+  cfg.dynamicSmemBytes = MoePairSmem::TOTAL;
+  cfg.stream = s;
+  cudaLaunchAttribute attr[2];
+  attr[0].id = cudaLaunchAttributeClusterDimension;
+  attr[0].val.clusterDim.x = 2;
+  attr[0].val.clusterDim.y = 1;
+  attr[0].val.clusterDim.z = 1;
+  attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[1].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = host::pdl_default() != 0 ? 2 : 1;
+  CUDA_TRY(cudaLaunchKernelEx(&cfg, kernel, tmA, tmW, p));
+  return FLYB200_OK;
+}
+
 // Persistent form for routing blocks that are a multiple of 128 rows.
 template <int KIND, int STAGE, int OUTMODE, bool ACCUM>
-int launch_moe_rows(const CUtensorMap& tmA, const MoeParams& p, int blocks, cudaStream_t s) {
+int launch_moe_rows(const CUtensorMap& tmA, const MoeParams& p, int blocks, int sms, cudaStream_t s) {
   static std::atomic<uint64_t> done{0};
   auto kernel = moe_rows_kernel<KIND, STAGE, OUTMODE, ACCUM>;
   int dev = 0;
@@ -90,9 +124,6 @@ int launch_moe_rows(const CUtensorMap& tmA, const MoeParams& p, int blocks, cuda
     CUDA_TRY(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, MoeRowsSmem::TOTAL));
     done.fetch_or(bit, std::memory_order_release);
   }
-  int sms = 0;
-  int rc = sm_count(&sms);
-  if (rc) return rc;
   const long long row_blocks = (static_cast<long long>(blocks) * p.tile_m + BLOCK_ROWS - 1) / BLOCK_ROWS;
   const int pairs = STAGE == 1 ? (p.n_out + BLOCK_ROWS - 1) / BLOCK_ROWS : (p.n_out + MOE_ROWS_BN - 1) / MOE_ROWS_BN;
   const long long items = row_blocks * pairs;
@@ -101,23 +132,56 @@ int launch_moe_rows(const CUtensorMap& tmA, const MoeParams& p, int blocks, cuda
   return FLYB200_OK;
 }
 
+// tmW: the weight images' maps for CTA pairs, or null for one CTA per item.
+template <int KIND, int STAGE, int OUTMODE, bool ACCUM>
+int launch_moe_large(const CUtensorMap& tmA, const MoePairWeights* tmW, const MoeParams& p, int blocks, int sms, cudaStream_t s) {
+  return tmW ? launch_moe_pair<KIND, STAGE, OUTMODE, ACCUM>(tmA, *tmW, p, blocks, sms, s)
+             : launch_moe_rows<KIND, STAGE, OUTMODE, ACCUM>(tmA, p, blocks, sms, s);
+}
 template <int KIND>
-int launch_moe_rows_variant(int stage, int out_dtype, bool accumulate, const CUtensorMap& tmA, const MoeParams& p,
-                            int blocks, cudaStream_t s) {
+int launch_moe_large_variant(int stage, int out_dtype, bool accumulate, const CUtensorMap& tmA, const MoePairWeights* tmW, const MoeParams& p,
+                             int blocks, int sms, cudaStream_t s) {
   if (stage == 1) {
-    if (out_dtype == FLYB200_OUT_BF16) return launch_moe_rows<KIND, 1, MOE_OUT_BF16, false>(tmA, p, blocks, s);
-    if (out_dtype == FLYB200_OUT_FP16) return launch_moe_rows<KIND, 1, MOE_OUT_FP16, false>(tmA, p, blocks, s);
+    if (out_dtype == FLYB200_OUT_BF16) return launch_moe_large<KIND, 1, MOE_OUT_BF16, false>(tmA, tmW, p, blocks, sms, s);
+    if (out_dtype == FLYB200_OUT_FP16) return launch_moe_large<KIND, 1, MOE_OUT_FP16, false>(tmA, tmW, p, blocks, sms, s);
     return FLYB200_E_UNSUPPORTED;
   }
   if (accumulate) {
-    if (out_dtype == FLYB200_OUT_BF16) return launch_moe_rows<KIND, 2, MOE_OUT_BF16, true>(tmA, p, blocks, s);
-    if (out_dtype == FLYB200_OUT_FP16) return launch_moe_rows<KIND, 2, MOE_OUT_FP16, true>(tmA, p, blocks, s);
-    if (out_dtype == FLYB200_OUT_F32) return launch_moe_rows<KIND, 2, MOE_OUT_F32, true>(tmA, p, blocks, s);
+    if (out_dtype == FLYB200_OUT_BF16) return launch_moe_large<KIND, 2, MOE_OUT_BF16, true>(tmA, tmW, p, blocks, sms, s);
+    if (out_dtype == FLYB200_OUT_FP16) return launch_moe_large<KIND, 2, MOE_OUT_FP16, true>(tmA, tmW, p, blocks, sms, s);
+    if (out_dtype == FLYB200_OUT_F32) return launch_moe_large<KIND, 2, MOE_OUT_F32, true>(tmA, tmW, p, blocks, sms, s);
     return FLYB200_E_UNSUPPORTED;
   }
-  if (out_dtype == FLYB200_OUT_BF16) return launch_moe_rows<KIND, 2, MOE_OUT_BF16, false>(tmA, p, blocks, s);
-  if (out_dtype == FLYB200_OUT_FP16) return launch_moe_rows<KIND, 2, MOE_OUT_FP16, false>(tmA, p, blocks, s);
+  if (out_dtype == FLYB200_OUT_BF16) return launch_moe_large<KIND, 2, MOE_OUT_BF16, false>(tmA, tmW, p, blocks, sms, s);
+  if (out_dtype == FLYB200_OUT_FP16) return launch_moe_large<KIND, 2, MOE_OUT_FP16, false>(tmA, tmW, p, blocks, sms, s);
   return FLYB200_E_UNSUPPORTED;
+}
+
+// Whether CTA pairs are estimated to be faster than one CTA per 128-row item.  How the routes fall on the experts is known on
+// the device only, so the estimate spreads them evenly: a last, half-filled tile per expert, and with routing blocks of 64 one
+// more pass of the 128-row form where the expert changes inside an item.  Per k-block a pair needs 512 cycles (tensor pipe)
+// and a CTA by itself 680 (bytes into the SM), per item at least the epilogue's 6000 to 7600; the weights come at 3333 bytes
+// per cycle (6 TB/s), and the second passes read them again once they have left L2.  One CTA / pairs, us, gather included:
+// 4096 tokens x top-2, 8 experts, 4096 x 2048 149 / 139 and 88 / 76 (gate-up, down), 200 tokens 37.3 / 32.3 (gate-up), 800 x top-4, 32
+// experts, 3072 x 1536 99 / 78 and 51 / 45, 515 x top-4, 16 experts, 2048 x 1408 34.3 / 26.8 and 19.3 / 17.2; where items are few and the
+// weights fit L2, or K is short, it is the other way round: 200 x top-2, 8 experts, down 17.2 / 19.6, 1024 x top-4, 8 experts, 2048 x 1024 21.5 /
+// 25.2 and 14.6 / 19.0, 4096 x top-4, 32 experts, 2048 x 768, down 46.3 / 55.6.
+bool moe_pair_pays(int stage, long long routes, int experts, int n_out, int num_kb, int tile_m, int sms) {
+  const double used = routes < experts ? static_cast<double>(routes) : experts, rows = routes / used;
+  const double pairs = (n_out + (stage == 1 ? 127 : 255)) / (stage == 1 ? 128 : 256);
+  const double tiles = rows < 128 ? 1.0 : rows / 256 + 0.5;
+  const double blocks = rows / 128 + (tile_m == 64 || tile_m == 256 ? 1.0 : 0.5);
+  const double weights = used * n_out * (stage == 1 ? 2 : 1) * num_kb * KBLOCK_BYTES;
+  const double again = tile_m == 64 && weights > 100e6 ? 1.4 : 1.0;
+  auto cycles = [&](double x, double kb_cycles, double least, double bytes) {
+    const double part = x - static_cast<long long>(x);
+    const double rounds = x <= 1.0 ? 1.0 : part == 0.0 ? x : part > 0.6 ? x - part + 1.0 : x + 0.4;
+    const double item = num_kb * kb_cycles > least ? num_kb * kb_cycles : least;
+    return rounds * item > bytes / 3333.0 ? rounds * item : bytes / 3333.0;
+  };
+  const double pair = cycles(used * tiles * pairs / (sms / 2), 512.0, stage == 1 ? 7600.0 : 6500.0, weights);
+  const double single = cycles(used * blocks * pairs / sms, 680.0, stage == 1 ? 7000.0 : 6000.0, again * weights);
+  return pair + 1000.0 < single;
 }
 
 template <int KIND, int BN>
@@ -266,14 +330,28 @@ int flyb200_moe_gemm(int stage, void* out, const void* a_sorted, const void* w_s
   cudaStream_t s = static_cast<cudaStream_t>(stream);
   CUtensorMap tmA;
   // Routing blocks of 64, 128 or 256 rows: persistent kernel with the tokens on the
-  // UMMA M side (FLYB200_MOE_KERNEL=1 in the environment forces the other form, for tests and tuning).
+  // UMMA M side (FLYB200_MOE_KERNEL=1 in the environment forces the other form, 2 one CTA per item, 3 CTA pairs, for
+  // tests and tuning).
   const char* force = getenv("FLYB200_MOE_KERNEL");
   const bool rows_form = (tile_m % BLOCK_ROWS == 0 || tile_m == 64) && !(force && force[0] == '1');
   if (rows_form) {
+    int sms = 0;
+    if ((rc = sm_count(&sms))) return rc;
     rc = host::byte_matrix_map(&tmA, a_sorted, static_cast<uint64_t>(K), static_cast<uint64_t>(blocks) * tile_m, BLOCK_ROWS);
     if (rc) return rc;
-    if (in_dtype == FLYB200_DT_FP8) return launch_moe_rows_variant<KIND_F8>(stage, out_dtype, accumulate != 0, tmA, p, blocks, s);
-    return launch_moe_rows_variant<KIND_I8>(stage, out_dtype, accumulate != 0, tmA, p, blocks, s);
+    // CTA pairs where they pay, while the list of their tiles fits shared memory
+    const bool forced = force && (force[0] == '2' || force[0] == '3');
+    const bool pair = blocks <= MOE_PAIR_MAX_BLOCKS && sms > 1 &&
+                      (forced ? force[0] == '3' : moe_pair_pays(stage, static_cast<long long>(tokens) * topk, experts, n_out, K / KBLOCK_BYTES, tile_m, sms));
+    MoePairWeights tmW;
+    for (int i = 0; pair && i < 3; ++i) {
+      rc = host::weight_image_map(&tmW.box[i], w_shuf, static_cast<uint64_t>(p.n_expert), static_cast<uint64_t>(experts) * (K / KBLOCK_BYTES), BLOCK_ROWS >> i);
+      if (rc) return rc;
+    }
+    p.pdl = pair && after_gather && host::pdl_default() != 0 ? 1 : 0;
+    const MoePairWeights* w_map = pair ? &tmW : nullptr;
+    if (in_dtype == FLYB200_DT_FP8) return launch_moe_large_variant<KIND_F8>(stage, out_dtype, accumulate != 0, tmA, w_map, p, blocks, sms, s);
+    return launch_moe_large_variant<KIND_I8>(stage, out_dtype, accumulate != 0, tmA, w_map, p, blocks, sms, s);
   }
   int bn = 16;
   while (bn < tile_m) bn *= 2;

@@ -32,6 +32,9 @@ cudaError_t launch_dependent(void (*kernel)(KArgs...), dim3 grid, int threads, i
 // Tensor map over a row-major byte matrix [rows, row_bytes]: boxes of
 // 128 bytes x box_rows rows, 128-byte swizzle, out-of-bounds rows read as zero.
 int byte_matrix_map(CUtensorMap* m, const void* base, uint64_t row_bytes, uint64_t rows, uint32_t box_rows);
+// Tensor map over preshuffled weights: `k_blocks` images of n_rows x 128 bytes, boxes of box_rows rows of one of them,
+// copied as they are (the image is already swizzled); rows past n_rows read as zero.
+int weight_image_map(CUtensorMap* m, const void* base, uint64_t n_rows, uint64_t k_blocks, uint32_t box_rows);
 // Block-scaled GEMM (MXFP8, or MXFP4 with `fp4`) of up to 128 tokens on the small-M (weight-streaming)
 // kernel; K = bytes of codes per row; outmode 0 bf16, 1 fp16.  a_format, w_format: codes in byte containers
 // (FLYB200_MXFMT_*; 0 = E4M3, and for `fp4`).

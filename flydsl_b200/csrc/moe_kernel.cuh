@@ -494,6 +494,136 @@ __device__ __forceinline__ void store_rows32(void* out, const long long (&rows)[
   }
 }
 
+// First rows in the expert's image of the two tiles of a channel pair, and the channels of each that exist.
+template <int STAGE>
+__device__ __forceinline__ void moe_pair_tiles(const MoeParams& p, int pair, int (&w_row)[2], int (&n_valid)[2]) {
+  if constexpr (STAGE == 1) {
+    const int c = pair * BLOCK_ROWS;
+    w_row[0] = c;
+    w_row[1] = p.n_out + c;
+    n_valid[0] = n_valid[1] = min(BLOCK_ROWS, p.n_out - c);
+  } else {
+    const int c = pair * MOE_ROWS_BN;
+    w_row[0] = c;
+    w_row[1] = c + BLOCK_ROWS;
+    n_valid[0] = min(BLOCK_ROWS, p.n_out - c);
+    n_valid[1] = max(0, min(BLOCK_ROWS, p.n_out - c - BLOCK_ROWS));
+  }
+}
+
+// What one epilogue warp does with the 128-row accumulator tiles of its items: stage 1 both tiles of a channel pair, stage 2
+// one of them.  The factors of the next item (routing id, activation scale, routed weight, weight scales) are asked for
+// before the current one is converted.
+__host__ __device__ constexpr int moe_rows_scales(int stage) { return stage == 1 ? 2 * BLOCK_ROWS : BLOCK_ROWS; }  // of a warp
+template <int KIND, int STAGE, int OUTMODE, bool ACCUM>
+struct MoeRowsEpilogue {
+  static constexpr int SCALES = moe_rows_scales(STAGE);
+  const MoeParams& p;
+  float* sw_s;       // shared memory of the warp for the weight scales of its columns
+  uint32_t stage_c;  // ... and for store_rows32
+  int half;          // stage 2: which of the two tiles of a channel pair
+  int lane;
+  // of the item asked for last: this lane's row, its share of the weight scales, output column, channels and tile width
+  int id;
+  float sa, tw, sw[SCALES / 32];
+  int col0_next, cols_next, width_next;
+
+  // This lane's sorted row `srow` (`row_ok`: it belongs to the item) and `width` channels (a multiple of 32) of every tile
+  // of channel pair `pair` from the `c0`-th on.
+  __device__ __forceinline__ void fetch(int expert, int srow, bool row_ok, int pair, int c0, int width) {
+    int w_row[2], n_valid[2];
+    moe_pair_tiles<STAGE>(p, pair, w_row, n_valid);
+    width_next = width;
+    cols_next = (STAGE == 2 && half ? n_valid[1] : n_valid[0]) - c0;
+    col0_next = (STAGE == 1 ? pair * BLOCK_ROWS : pair * MOE_ROWS_BN + half * BLOCK_ROWS) + c0;
+    id = -1;  // token 0xFFFFFF of slot 255: no row
+    sa = 0.0f;
+    tw = 1.0f;
+    if (row_ok) {
+      id = __ldg(p.sorted_ids + srow);
+      sa = __ldg(p.sa + srow);
+      if (p.doweight) tw = __ldg(p.sorted_w + srow);
+    }
+    const float* sw_expert = p.sw + static_cast<size_t>(expert) * p.n_expert + c0;
+#pragma unroll
+    for (int i = 0; i < SCALES / 32; ++i) {
+      const bool second = STAGE == 1 ? i >= BLOCK_ROWS / 32 : half == 1;
+      const int c = (i * 32 + lane) & (BLOCK_ROWS - 1);
+      sw[i] = c < cols_next ? __ldg(sw_expert + (second ? w_row[1] : w_row[0]) + c) : 0.0f;
+    }
+  }
+
+  // The item asked for last.  `next` asks for the one after it; `wait` blocks until the accumulator at `t_row` is complete
+  // (`width` columns of the first tile, then those of the second); `release` (one lane) hands it back after the last
+  // read.  False if the wait failed.
+  template <typename NextFn, typename WaitFn, typename ReleaseFn>
+  __device__ __forceinline__ bool run(uint32_t t_row, NextFn next, WaitFn wait, ReleaseFn release) {
+    const int tok = id & 0xFFFFFF;
+    const int slot = static_cast<int>(static_cast<uint32_t>(id) >> 24);
+    const bool exists = tok < p.tokens && slot < p.topk;
+    const long long orow = !exists ? -1 : (STAGE == 2 && ACCUM) ? tok : static_cast<long long>(tok) * p.topk + slot;
+    const float row_scale = exists ? sa : 0.0f, row_weight = tw;
+    long long rows[4];  // output rows this lane stores pieces of
+#pragma unroll
+    for (int k = 0; k < 4; ++k) rows[k] = __shfl_sync(0xffffffffu, orow, 8 * k + (lane >> 2));
+    __syncwarp();  // the scales of the item before have been read
+#pragma unroll
+    for (int i = 0; i < SCALES / 32; ++i) sw_s[i * 32 + lane] = sw[i];
+    __syncwarp();
+    const int cols = cols_next, col0 = col0_next, width = width_next;
+    next();
+    if (!wait()) return false;
+    tc_fence_after();
+    constexpr bool IS_INT = KindTraits<KIND>::is_int;
+    auto to_f = [](uint32_t r) { return IS_INT ? static_cast<float>(static_cast<int32_t>(r)) : __uint_as_float(r); };
+    auto last_read = [&]() {
+      tc_fence_before();
+      __syncwarp();
+      if (lane == 0) release();
+    };
+    if constexpr (STAGE == 1) {
+      // Not unrolled, here and below, and no accumulators asked for ahead: four times this code was slower, in the gate-up
+      // stage 5.3 us a tile instead of 3.65.
+#pragma unroll 1
+      for (int c = 0; c < width; c += 32) {
+        uint32_t rg[32], ru[32];
+        tmem_ld_x32(t_row + c, rg);
+        tmem_ld_x32(t_row + width + c, ru);
+        tmem_ld_wait();
+        if (c + 32 >= width) last_read();
+        float y[32];
+#pragma unroll
+        for (int j = 0; j < 32; ++j) {
+          const float g = (to_f(rg[j]) * sw_s[c + j]) * row_scale;
+          const float u = (to_f(ru[j]) * sw_s[BLOCK_ROWS + c + j]) * row_scale;
+          float v = silu_f32(g) * u;
+          if (p.doweight) v *= row_weight;
+          y[j] = v;
+        }
+        const int n_ok = min(32, cols - c);
+        if (n_ok > 0) store_rows32<OUTMODE, ACCUM>(p.out, rows, p.n_out, col0 + c, y, n_ok, stage_c, lane);
+      }
+    } else {
+#pragma unroll 1
+      for (int c = 0; c < width; c += 32) {
+        uint32_t r[32];
+        tmem_ld_x32(t_row + half * width + c, r);
+        tmem_ld_wait();
+        if (c + 32 >= width) last_read();
+        float y[32];
+#pragma unroll
+        for (int j = 0; j < 32; ++j) {
+          const float v = (to_f(r[j]) * sw_s[c + j]) * row_scale;
+          y[j] = p.doweight ? v * row_weight : v;
+        }
+        const int n_ok = min(32, cols - c);
+        if (n_ok > 0) store_rows32<OUTMODE, ACCUM>(p.out, rows, p.n_out, col0 + c, y, n_ok, stage_c, lane);
+      }
+    }
+    return true;
+  }
+};
+
 template <int KIND, int STAGE, int OUTMODE, bool ACCUM>
 __global__ void __launch_bounds__(moe_rows_threads(STAGE), 1) moe_rows_kernel(const __grid_constant__ CUtensorMap tmA,
                                                                   const MoeParams p) {
@@ -588,22 +718,6 @@ __global__ void __launch_bounds__(moe_rows_threads(STAGE), 1) moe_rows_kernel(co
     lo = 64;
     return eb == ea ? -1 : eb;
   };
-  // rows of the image and channels that exist for the two tiles of a pair
-  auto tiles_of = [&](int pair, int (&w_row)[2], int (&n_valid)[2]) {
-    if constexpr (STAGE == 1) {
-      const int c = pair * BLOCK_ROWS;
-      w_row[0] = c;
-      w_row[1] = p.n_out + c;
-      n_valid[0] = n_valid[1] = min(BLOCK_ROWS, p.n_out - c);
-    } else {
-      const int c = pair * BN;
-      w_row[0] = c;
-      w_row[1] = c + BLOCK_ROWS;
-      n_valid[0] = min(BLOCK_ROWS, p.n_out - c);
-      n_valid[1] = max(0, min(BLOCK_ROWS, p.n_out - c - BLOCK_ROWS));
-    }
-  };
-
   if (warp == 0) {
     // ------------------------------ producer ------------------------------
     const bool issuer = elect_one();
@@ -617,7 +731,7 @@ __global__ void __launch_bounds__(moe_rows_threads(STAGE), 1) moe_rows_kernel(co
       const int expert = __shfl_sync(0xffffffffu, item_of(t, rb, pair, lo, hi), 0);
       if (expert < 0) continue;
       int w_row[2], n_valid[2];
-      tiles_of(pair, w_row, n_valid);
+      moe_pair_tiles<STAGE>(p, pair, w_row, n_valid);
       const uint8_t* w_expert = p.w + static_cast<size_t>(expert) * p.n_expert * p.K_bytes;
       const uint32_t b0 = static_cast<uint32_t>(n_valid[0]) * KBLOCK_BYTES, b1 = static_cast<uint32_t>(n_valid[1]) * KBLOCK_BYTES;
       for (int kb = 0; kb < num_kb; ++kb) {
@@ -706,101 +820,29 @@ __global__ void __launch_bounds__(moe_rows_threads(STAGE), 1) moe_rows_kernel(co
     // Stage 1: one warp per TMEM lane quadrant, all 128 channels of the gate and of the up tile.  Stage 2: two, each
     // with the 128 channels of one of the two tiles.
     const int q = warp & 3;  // TMEM lane quadrant this warp may read
-    const int half = (warp - 2) >> 2;
-    constexpr int SCALES = STAGE == 1 ? 2 * BLOCK_ROWS : BLOCK_ROWS;
-    float* sw_s = reinterpret_cast<float*>(smem_raw + L::OFF_SW) + (warp - 2) * SCALES;
-    const uint32_t stage_c = smem_base + L::OFF_C + (warp - 2) * STORE_STAGE;
+    MoeRowsEpilogue<KIND, STAGE, OUTMODE, ACCUM> ep{p, reinterpret_cast<float*>(smem_raw + L::OFF_SW) + (warp - 2) * moe_rows_scales(STAGE),
+                                                    smem_base + L::OFF_C + (warp - 2) * STORE_STAGE, (warp - 2) >> 2, lane};
+    // asks for the first item from t on that has work; the item's number, or `items` and more
+    auto fetch_from = [&](int t) {
+      for (; t < items; t += gridDim.x) {
+        int rb, pair, lo, hi;
+        const int expert = item_of(t, rb, pair, lo, hi);
+        if (expert < 0) continue;
+        const int trow = q * 32 + lane;  // this thread's token row
+        const int srow = rb * BLOCK_ROWS + trow;
+        ep.fetch(expert, srow, srow < n_rows && trow >= lo && trow < hi, pair, 0, BLOCK_ROWS);
+        break;
+      }
+      return t;
+    };
     int acc = 0;
     uint32_t acc_phase = 0;
     bool ok = true;
-    for (int t = blockIdx.x; t < items && ok; t += gridDim.x) {
-      int rb, pair, lo, hi;
-      const int expert = item_of(t, rb, pair, lo, hi);
-      if (expert < 0) continue;
-      int w_row[2], n_valid[2];
-      tiles_of(pair, w_row, n_valid);
-      // this thread's token row
-      const int trow = q * 32 + lane;
-      const int srow = rb * BLOCK_ROWS + trow;
-      long long orow = -1;
-      float sa = 0.0f, tw = 1.0f;
-      if (srow < n_rows && trow >= lo && trow < hi) {
-        const int id = __ldg(p.sorted_ids + srow);
-        const int tok = id & 0xFFFFFF;
-        const int slot = static_cast<int>(static_cast<uint32_t>(id) >> 24);
-        if (tok < p.tokens && slot < p.topk) {
-          orow = (STAGE == 2 && ACCUM) ? tok : static_cast<long long>(tok) * p.topk + slot;
-          sa = __ldg(p.sa + srow);
-          if (p.doweight) tw = __ldg(p.sorted_w + srow);
-        }
-      }
-      long long rows[4];  // output rows this lane stores pieces of
-#pragma unroll
-      for (int k = 0; k < 4; ++k) rows[k] = __shfl_sync(0xffffffffu, orow, 8 * k + (lane >> 2));
-      // weight scales of this warp's columns: stage 1 the gate channels, then the up channels
-      const float* sw_expert = p.sw + static_cast<size_t>(expert) * p.n_expert;
-      __syncwarp();
-#pragma unroll
-      for (int i = 0; i < SCALES / 32; ++i) {
-        const int c = i * 32 + lane;
-        const bool second = STAGE == 1 ? c >= BLOCK_ROWS : half == 1;
-        const int cc = c & (BLOCK_ROWS - 1);
-        sw_s[c] = cc < (second ? n_valid[1] : n_valid[0]) ? __ldg(sw_expert + (second ? w_row[1] : w_row[0]) + cc) : 0.0f;
-      }
-      __syncwarp();
-      if (!mbar_wait(bar_tfull + 8 * acc, acc_phase, abort_flag)) {
-        if (lane == 0) report_failure(p.status, ST_TIMEOUT, abort_flag);
-        ok = false;
-        break;
-      }
-      tc_fence_after();
+    for (int t = fetch_from(blockIdx.x); t < items && ok;) {
       const uint32_t t_row = tmem_base + (static_cast<uint32_t>(q * 32) << 16) + static_cast<uint32_t>(acc * BN);
-      auto to_f = [](uint32_t r) { return KT::is_int ? static_cast<float>(static_cast<int32_t>(r)) : __uint_as_float(r); };
-      if constexpr (STAGE == 1) {
-#pragma unroll 1
-        for (int c0 = 0; c0 < BLOCK_ROWS; c0 += 32) {
-          uint32_t rg[32], ru[32];
-          tmem_ld_x32(t_row + c0, rg);
-          tmem_ld_x32(t_row + BLOCK_ROWS + c0, ru);
-          tmem_ld_wait();
-          if (c0 + 32 >= BLOCK_ROWS) {  // last read of this accumulator: hand it back to the MMA warp
-            tc_fence_before();
-            __syncwarp();
-            if (lane == 0) mbar_arrive(bar_tempty + 8 * acc);
-          }
-          float y[32];
-#pragma unroll
-          for (int j = 0; j < 32; ++j) {
-            const float g = (to_f(rg[j]) * sw_s[c0 + j]) * sa;
-            const float u = (to_f(ru[j]) * sw_s[BLOCK_ROWS + c0 + j]) * sa;
-            float v = silu_f32(g) * u;
-            if (p.doweight) v *= tw;
-            y[j] = v;
-          }
-          const int n_ok = min(32, n_valid[0] - c0);
-          if (n_ok > 0) store_rows32<OUTMODE, ACCUM>(p.out, rows, p.n_out, pair * BLOCK_ROWS + c0, y, n_ok, stage_c, lane);
-        }
-      } else {
-#pragma unroll 1
-        for (int c0 = 0; c0 < BLOCK_ROWS; c0 += 32) {
-          uint32_t ra[32];
-          tmem_ld_x32(t_row + half * BLOCK_ROWS + c0, ra);
-          tmem_ld_wait();
-          if (c0 + 32 >= BLOCK_ROWS) {
-            tc_fence_before();
-            __syncwarp();
-            if (lane == 0) mbar_arrive(bar_tempty + 8 * acc);
-          }
-          float y[32];
-#pragma unroll
-          for (int j = 0; j < 32; ++j) {
-            const float v = (to_f(ra[j]) * sw_s[c0 + j]) * sa;
-            y[j] = p.doweight ? v * tw : v;
-          }
-          const int n_ok = min(32, (half ? n_valid[1] : n_valid[0]) - c0);
-          if (n_ok > 0) store_rows32<OUTMODE, ACCUM>(p.out, rows, p.n_out, pair * BN + half * BLOCK_ROWS + c0, y, n_ok, stage_c, lane);
-        }
-      }
+      ok = ep.run(t_row, [&]() { t = fetch_from(t + gridDim.x); }, [&]() { return mbar_wait(bar_tfull + 8 * acc, acc_phase, abort_flag); },
+                  [&]() { mbar_arrive(bar_tempty + 8 * acc); });
+      if (!ok && lane == 0) report_failure(p.status, ST_TIMEOUT, abort_flag);
       acc ^= 1;
       if (acc == 0) acc_phase ^= 1u;
     }

@@ -429,14 +429,18 @@ long long rows_cost(int M, int N, long long kb, int bn, int sms) {
 //                  it stays where it splits K in four or more over at least 64 k-blocks: 256 x 4096 x 14336 22.8 / 24.7,
 //                  512 x 1024 x 8192 14.0 / 14.9, bf16 1024 x 1024 x 8192 21.4 / 24.9
 // Up to 128 tokens half of a pair would have no rows (128 x 8192 x 8192 17.3 / 22.4).  Of the widths the cheapest counts, a
-// narrower one only if it is 2 % cheaper (more bytes per product); over 117 shapes of 264..8192 tokens the choice is
-// within 1 % of the best width and form on average.  With 16 k-blocks or fewer the pairs' set-up (cluster barriers,
-// remote hand-over) weighs more: 320 x 5120 x 1024 bf16 8.5 / 9.5, 1024 x 5120 x 1024 10.2 / 11.3.
-constexpr long long PAIR_SETUP_CYCLES = 2500;
-int pair_choice(const Plan& plan, int M, int N, int K_bytes, int sms) {
+// narrower one only if it is 2 % cheaper (more bytes per product).  A pair's set-up and hand-over of accumulators (cluster
+// barriers, remote arrivals) weigh 5000 cycles, and with few k-blocks, where the epilogue is longer than the mainloop, the 128-row form
+// stays (it also takes the place of the 256-row form there): 128-row form / pairs, us, fp8 8192 x 8192 x 1024 68.5 / 81.1, x 1280 84.8 / 94.7, x
+// 2048 135 / 116, with gelu x 1536 130 / 144, x 2048 153 / 155, x 2560 184 / 170; 512 x 8192 x 2560 11.9 / 13.6.  Over 692 shapes (140..8192 tokens, 1024..28672
+// channels, 12..112 k-blocks) the choice is on average 1.9 % behind the best form and width.
+constexpr long long PAIR_SETUP_CYCLES = 5000;
+constexpr int PAIR_MIN_KB = 13, PAIR_MIN_KB_ACTIVATION = 17;  // the latter with a fused silu or gelu
+int pair_choice(const Plan& plan, int M, int N, int K_bytes, int sms, bool activation) {
   const long long kb = K_bytes / KBLOCK_BYTES;
   if (M <= BLOCK_ROWS || sms < 2 || plan.two_sm || plan.pair) return 0;
   if (plan.decode && plan.split_k >= 4 && kb >= 64) return 0;
+  if (!plan.decode && kb < (activation ? PAIR_MIN_KB_ACTIVATION : PAIR_MIN_KB)) return 0;
   long long best = -1;
   int width = 0;
   for (int bn = 256; bn >= 64; bn -= 32) {
@@ -446,7 +450,7 @@ int pair_choice(const Plan& plan, int M, int N, int K_bytes, int sms) {
       width = bn;
     }
   }
-  if (!plan.decode && !plan.tall && rows_cost(M, N, kb, plan.bn, sms) < best + (kb <= 16 ? PAIR_SETUP_CYCLES : 0)) return 0;
+  if (!plan.decode && rows_cost(M, N, kb, plan.tall ? auto_rows_bn(M, N, K_bytes, sms) : plan.bn, sms) < best + PAIR_SETUP_CYCLES) return 0;
   return width;
 }
 
@@ -597,11 +601,21 @@ int make_plan(Plan* plan, int M, int N, int K_bytes, int variant_hint, size_t wo
 }
 
 // make_plan, and CTA pairs where the call leaves the kernel open and they are the better choice.
-int plan_call(Plan* plan, int M, int N, int K_bytes, int variant_hint, size_t workspace_bytes, bool have_ws, int sms) {
+int plan_call(Plan* plan, int M, int N, int K_bytes, int variant_hint, size_t workspace_bytes, bool have_ws, int sms, bool activation) {
   const int rc = make_plan(plan, M, N, K_bytes, variant_hint, workspace_bytes, have_ws, sms);
   if (rc || (variant_hint & ~(3 << 28)) != 0 || rows_tall_default() || w64_default()) return rc;
-  const int width = pair_choice(*plan, M, N, K_bytes, sms);
-  if (width == 0) return rc;
+  const int width = pair_choice(*plan, M, N, K_bytes, sms, activation);
+  const int hp = hint_pdl(variant_hint);
+  const int pdl = hp == 1 ? 1 : hp == 2 ? 0 : hp == 3 ? 2 : host::pdl_default();
+  if (width == 0) {
+    if (plan->tall) {  // the 128-row form is faster than the 256-row form by now wherever pairs are not: fp8 1500 x 6144 x 1024 12.2 / 15.3 us
+      plan->tall = false;
+      plan->bn = auto_rows_bn(M, N, K_bytes, sms);
+      plan->group_m = 32;
+      plan->pdl = large_pdl(pdl, static_cast<long long>((M + BLOCK_ROWS - 1) / BLOCK_ROWS) * ((N + plan->bn - 1) / plan->bn), sms);
+    }
+    return rc;
+  }
   plan->decode = plan->tall = false;
   plan->two_sm = true;
   plan->bn = width;
@@ -609,8 +623,7 @@ int plan_call(Plan* plan, int M, int N, int K_bytes, int variant_hint, size_t wo
   plan->reduce_mode = REDUCE_NONE;
   plan->prefetch = 0;
   plan->group_m = pair_group(K_bytes);
-  const int hp = hint_pdl(variant_hint);
-  plan->pdl = large_pdl(hp == 1 ? 1 : hp == 2 ? 0 : hp == 3 ? 2 : host::pdl_default(), host::pair_tiles(M, N, width), sms / 2);
+  plan->pdl = large_pdl(pdl, host::pair_tiles(M, N, width), sms / 2);
   return rc;
 }
 
@@ -637,7 +650,7 @@ int gemm_common(void* c, const void* a, const void* w, const float* sa, const fl
   const int K_bytes = K * eb;
 
   Plan plan;
-  rc = plan_call(&plan, M, N, K_bytes, variant_hint, workspace_bytes, workspace != nullptr, st->sms);
+  rc = plan_call(&plan, M, N, K_bytes, variant_hint, workspace_bytes, workspace != nullptr, st->sms, epilogue >= FLYB200_EPI_BIAS_SILU);
   if (rc) return rc;
 
   GemmParams p;
@@ -1118,7 +1131,7 @@ int flyb200_pair_width(int M, int N, int K, int in_dtype, int variant_hint, int 
   const int eb = elem_bytes_of(in_dtype);
   if (!flyb200_layout_kind(N, K, eb)) return 0;
   Plan plan;
-  if (plan_call(&plan, M, N, K * eb, variant_hint, static_cast<size_t>(-1) >> 1, true, sm_count)) return 0;
+  if (plan_call(&plan, M, N, K * eb, variant_hint, static_cast<size_t>(-1) >> 1, true, sm_count, false)) return 0;
   return plan.two_sm ? plan.bn : 0;
 }
 

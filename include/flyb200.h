@@ -230,7 +230,9 @@ int flyb200_describe_plan(int M, int N, int K, int in_dtype, int variant_hint, i
 
 /* Tile width with which the call runs as CTA pairs (256 rows x this many channels
  * per pair), asked for or because they are estimated to be faster than the plan
- * of flyb200_describe_plan; 0 where that plan runs.  Pure host function. */
+ * of flyb200_describe_plan; 0 where that plan runs (as the 128-row form, where it
+ * says 256-row tiles and none were asked for).  For a call without a fused silu or
+ * gelu; with one the pairs begin at a longer K.  Pure host function. */
 int flyb200_pair_width(int M, int N, int K, int in_dtype, int variant_hint, int sm_count);
 
 /* Device-side status word of the current device (0 = no failure since the last

@@ -66,6 +66,8 @@ def test_which_calls_run_as_pairs():
     assert w(128, 8192, 8192) == 0  # half of the pair would have no rows
     assert w(512, 2048, 8192) == 0 and w(512, 2048, 4096) > 0  # K split in four over a long K stays on the small-M kernel
     assert w(320, 10208, 5120, "bf16") == 0  # 384 padded rows against 512
+    assert w(8192, 8192, 1024) == 0 and w(8192, 8192, 2048) > 0  # few k-blocks: the epilogue is longer than the mainloop
+    assert w(512, 8192, 2560) == 0  # one round: the set-up weighs more
     # what a caller asks for is not changed, and a request for the form is honoured at its width
     assert w(4096, 8192, 8192, variant_hint=2 << 8) == 0 and w(4096, 8192, 8192, variant_hint=5) == 0
     assert w(64, 256, 128, variant_hint=PAIR_FORM | 3) == 96 and w(64, 256, 128, variant_hint=PAIR_FORM) == 256

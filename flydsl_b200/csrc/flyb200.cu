@@ -195,6 +195,12 @@ int fill_sms_split_k(int N, int K_bytes, int sms, int token_blocks = 1) {
 // 21 us unsplit and 15 us for split 4), split 4 at 32 tiles of 128 tokens (9.8 us
 // against 12.1 / 19.0 / 21.4 us for 2 / 1 / 8).
 // `pair`: CTA pairs, each CTA stages half of the tokens and the cluster is twice the split.
+constexpr double CROWDED_NS = 10000.0;
+// Clusters have to be placed whole inside a GPC, so fewer CTAs are resident at once than there are
+// SMs: clusters of more than four CTAs are slow to place when they cover more than two thirds of
+// the SMs (16 x 8 CTAs: 12.2 us against 7.3 us for 16 x 4; 12 x 8 is fine), clusters of three or
+// more when they cover more than 90 % (48 x 3 = 144 CTAs: 18.3 us against 12.0 us for 48 x 2).
+bool crowded_clusters(int csize, int ctas, int sms) { return (csize > 4 && 3 * ctas > 2 * sms) || (csize >= 3 && 10 * ctas > 9 * sms); }
 double split_cost_ns(int split, int n_tiles, int kb, int bn, int sms, bool cluster, bool pair = false) {
   const double stage_bytes = static_cast<double>(BLOCK_ROWS * KBLOCK_BYTES + (pair ? bn / 2 : bn) * KBLOCK_BYTES);
   const int rounds = (n_tiles * split + sms - 1) / sms;
@@ -205,13 +211,8 @@ double split_cost_ns(int split, int n_tiles, int kb, int bn, int sms, bool clust
   double reduce = 0.0;
   if (split > 1) {
     const double partial = bn * 512.0;
-    // Clusters have to be placed whole inside a GPC, so fewer CTAs are resident at once than there are
-    // SMs: clusters of more than four CTAs are slow to place when they cover more than two thirds of
-    // the SMs (16 x 8 CTAs: 12.2 us against 7.3 us for 16 x 4; 12 x 8 is fine), clusters of three or
-    // more when they cover more than 90 % (48 x 3 = 144 CTAs: 18.3 us against 12.0 us for 48 x 2).
-    const int csize = pair ? 2 * split : split;
-    const bool crowded = (csize > 4 && 3 * n_tiles * split > 2 * sms) || (csize >= 3 && 10 * n_tiles * split > 9 * sms);
-    reduce = cluster ? 1500.0 + (split - 1.0) / split * partial / 15.0 + (crowded ? 10000.0 : 0.0)
+    const bool crowded = crowded_clusters(pair ? 2 * split : split, n_tiles * split, sms);
+    reduce = cluster ? 1500.0 + (split - 1.0) / split * partial / 15.0 + (crowded ? CROWDED_NS : 0.0)
                      : 3000.0 + split * partial / 14.0;
   }
   return 3000.0 + stream + reduce;
@@ -419,39 +420,65 @@ long long rows_cost(int M, int N, long long kb, int bn, int sms) {
          EPILOGUE_CYCLES_PER_COL * (bn / parts);
 }
 
-// Tile width with which a call that leaves the kernel open runs as CTA pairs, or 0 where the planned kernel stays.
+// Estimated time (ns) of a call of more than 128 tokens that is planned for the small-M kernel, there and on the large-M forms.
+// Fitted to 298 such calls (129..1024 tokens, 512..20480 channels, 8..160 k-blocks, 8 and 16 bits, cold weights), mean error 4 %
+// (pairs 5.5 %): per k-block of a CTA 380 ns, per token of its block the two accumulators and the store, or a share of the K
+// splits' sum; per cycle of pair_cost and rows_cost 0.57 and 0.74 ns.
+double small_ns(const Plan& plan, int M, int N, int sms) {
+  const int ctas = (N + BLOCK_ROWS - 1) / BLOCK_ROWS * plan.token_blocks * plan.split_k;
+  const bool split = plan.split_k > 1;
+  return 4000.0 + 380.0 * ((ctas + sms - 1) / sms) * plan.kb_per_split + (split ? 21.0 : 30.0) * (M < plan.bn ? M : plan.bn) +
+         (split && crowded_clusters(plan.split_k, ctas, sms) ? CROWDED_NS : 0.0);
+}
+double pair_ns(long long cycles) { return 4800.0 + 0.57 * static_cast<double>(cycles); }
+double rows_ns(long long cycles) { return 3400.0 + 0.74 * static_cast<double>(cycles); }
+
+// The large-M form and tile width with which a call that leaves the kernel open runs in place of its plan: CTA pairs, the
+// 128-row form, or none of them (width 0) where the planned kernel stays.
 // A pair takes in a third fewer bytes per product than two CTAs of the 128-row form, so it needs less time where the
 // intake binds and less energy where the board's power cap does.  `plan` / pairs, us, fp8 unless stated:
 //   128-row form   4096 x 8192 x 8192 220 / 204, 8192 x 28672 x 8192 1480 / 1420, 2048 x 8192 x 8192 121 / 110, 768 x 8192 x 8192
 //                  56.7 / 48.8; fp16 4096 x 4096 x 4096 118 / 108; int8 997 x 10208 x 5120 54 / 47; bf16 8192 x 5120 x 1024 78 / 72
 //   256-row form   1024 x 8192 x 4096 36.4 / 34.0, 512 x 16384 x 4096 38.3 / 36.1, bf16 1536 x 5120 x 1024 19.0 / 16.8
-//   small-M form   256 x 8192 x 8192 24.7 / 21.9, 256 x 10208 x 5120 26.8 / 18.5, 320 x 4096 x 4096 15.2 / 11.2, bf16 512 x 3584 x 8192 35 / 31.5;
-//                  it stays where it splits K in four or more over at least 64 k-blocks: 256 x 4096 x 14336 22.8 / 24.7,
-//                  512 x 1024 x 8192 14.0 / 14.9, bf16 1024 x 1024 x 8192 21.4 / 24.9
+//   small-M form   256 x 8192 x 8192 24.7 / 21.9, 256 x 10208 x 5120 26.8 / 18.5, 320 x 4096 x 4096 15.2 / 11.2, bf16 512 x 3584 x 8192 35 / 31.5
 // Up to 128 tokens half of a pair would have no rows (128 x 8192 x 8192 17.3 / 22.4).  Of the widths the cheapest counts, a
-// narrower one only if it is 2 % cheaper (more bytes per product).  A pair's set-up and hand-over of accumulators (cluster
+// narrower one only if it is 2 % cheaper (more bytes per product).
+// In place of the small-M kernel the form with the least estimated time runs: it splits K and so keeps narrow outputs over many
+// k-blocks (small-M / pairs, us: 256 x 1024 x 8064 12.5 / 14.7, 130 x 1024 x 8064 9.8 / 14.7, 133 x 5136 x 14336 20.8 / 24.9, 256 x 4096 x
+// 14336 22.8 / 24.7), and the 128-row form is ahead of both with few (small-M / pairs / 128 rows: 200 x 4096 x 1024 12.7 / 7.0 / 5.7).
+// Over the 298 calls the choice is 0.6 % behind the best form and width on average, 12 % at worst (177 x 18464 x 1408 12.7 for
+// 11.3 us), and at most 5.4 % behind the small-M kernel (320 x 2048 x 8064 15.8 for 15.0 us).
+// In place of the large-M forms: a pair's set-up and hand-over of accumulators (cluster
 // barriers, remote arrivals) weigh 5000 cycles, and with few k-blocks, where the epilogue is longer than the mainloop, the 128-row form
 // stays (it also takes the place of the 256-row form there): 128-row form / pairs, us, fp8 8192 x 8192 x 1024 68.5 / 81.1, x 1280 84.8 / 94.7, x
-// 2048 135 / 116, with gelu x 1536 130 / 144, x 2048 153 / 155, x 2560 184 / 170; 512 x 8192 x 2560 11.9 / 13.6.  Over 692 shapes (140..8192 tokens, 1024..28672
-// channels, 12..112 k-blocks) the choice is on average 1.9 % behind the best form and width.
+// 2048 135 / 116, with gelu x 1536 130 / 144, x 2048 153 / 155, x 2560 184 / 170; 512 x 8192 x 2560 11.9 / 13.6.  Over 90 calls of 1025..8192
+// tokens the choice is 1.5 % behind the best on average, 14.5 % at worst (2419 x 4304 x 5632 55.3 for 48.3 us).
 constexpr long long PAIR_SETUP_CYCLES = 5000;
 constexpr int PAIR_MIN_KB = 13, PAIR_MIN_KB_ACTIVATION = 17;  // the latter with a fused silu or gelu
-int pair_choice(const Plan& plan, int M, int N, int K_bytes, int sms, bool activation) {
+struct LargeForm {
+  bool pairs;
+  int width;
+};
+LargeForm large_form(const Plan& plan, int M, int N, int K_bytes, int sms, bool activation) {
+  const LargeForm stay = {false, 0};
   const long long kb = K_bytes / KBLOCK_BYTES;
-  if (M <= BLOCK_ROWS || sms < 2 || plan.two_sm || plan.pair) return 0;
-  if (plan.decode && plan.split_k >= 4 && kb >= 64) return 0;
-  if (!plan.decode && kb < (activation ? PAIR_MIN_KB_ACTIVATION : PAIR_MIN_KB)) return 0;
+  if (M <= BLOCK_ROWS || sms < 2 || plan.two_sm || plan.pair) return stay;
+  if (!plan.decode && kb < (activation ? PAIR_MIN_KB_ACTIVATION : PAIR_MIN_KB)) return stay;
   long long best = -1;
-  int width = 0;
+  LargeForm form = {true, 0};
   for (int bn = 256; bn >= 64; bn -= 32) {
     const long long c = pair_cost(M, N, kb, bn, sms);
     if (best < 0 || 100 * c < 98 * best) {
       best = c;
-      width = bn;
+      form.width = bn;
     }
   }
-  if (!plan.decode && rows_cost(M, N, kb, plan.tall ? auto_rows_bn(M, N, K_bytes, sms) : plan.bn, sms) < best + PAIR_SETUP_CYCLES) return 0;
-  return width;
+  const int rows_bn = !plan.decode && !plan.tall ? plan.bn : auto_rows_bn(M, N, K_bytes, sms);
+  const long long rows = rows_cost(M, N, kb, rows_bn, sms);
+  if (!plan.decode) return rows < best + PAIR_SETUP_CYCLES ? stay : form;
+  const double here = small_ns(plan, M, N, sms), pairs = pair_ns(best), single = rows_ns(rows);
+  if (here <= pairs && here <= single) return stay;
+  return single < pairs ? LargeForm{false, rows_bn} : form;
 }
 
 // `allow_pair`: the caller's kind has the CTA-pair form of the small-M kernel (the plain kinds do)
@@ -600,30 +627,28 @@ int make_plan(Plan* plan, int M, int N, int K_bytes, int variant_hint, size_t wo
   return FLYB200_OK;
 }
 
-// make_plan, and CTA pairs where the call leaves the kernel open and they are the better choice.
+// make_plan, and the large-M form that takes its place where the call leaves the kernel open and another one is the better choice.
 int plan_call(Plan* plan, int M, int N, int K_bytes, int variant_hint, size_t workspace_bytes, bool have_ws, int sms, bool activation) {
   const int rc = make_plan(plan, M, N, K_bytes, variant_hint, workspace_bytes, have_ws, sms);
   if (rc || (variant_hint & ~(3 << 28)) != 0 || rows_tall_default() || w64_default()) return rc;
-  const int width = pair_choice(*plan, M, N, K_bytes, sms, activation);
+  LargeForm form = large_form(*plan, M, N, K_bytes, sms, activation);
+  // the 128-row form is faster than the 256-row form by now wherever pairs are not: fp8 1500 x 6144 x 1024 12.2 / 15.3 us
+  if (form.width == 0 && plan->tall) form = {false, auto_rows_bn(M, N, K_bytes, sms)};
+  if (form.width == 0) return rc;
   const int hp = hint_pdl(variant_hint);
   const int pdl = hp == 1 ? 1 : hp == 2 ? 0 : hp == 3 ? 2 : host::pdl_default();
-  if (width == 0) {
-    if (plan->tall) {  // the 128-row form is faster than the 256-row form by now wherever pairs are not: fp8 1500 x 6144 x 1024 12.2 / 15.3 us
-      plan->tall = false;
-      plan->bn = auto_rows_bn(M, N, K_bytes, sms);
-      plan->group_m = 32;
-      plan->pdl = large_pdl(pdl, static_cast<long long>((M + BLOCK_ROWS - 1) / BLOCK_ROWS) * ((N + plan->bn - 1) / plan->bn), sms);
-    }
-    return rc;
-  }
   plan->decode = plan->tall = false;
-  plan->two_sm = true;
-  plan->bn = width;
+  plan->two_sm = form.pairs;
+  plan->bn = form.width;
+  plan->w_rows = BLOCK_ROWS;
   plan->split_k = plan->token_blocks = 1;
+  plan->kb_per_split = K_bytes / KBLOCK_BYTES;
   plan->reduce_mode = REDUCE_NONE;
   plan->prefetch = 0;
-  plan->group_m = pair_group(K_bytes);
-  plan->pdl = large_pdl(pdl, host::pair_tiles(M, N, width), sms / 2);
+  plan->group_m = form.pairs ? pair_group(K_bytes) : 32;
+  const long long tiles = form.pairs ? host::pair_tiles(M, N, form.width)
+                                     : static_cast<long long>((M + BLOCK_ROWS - 1) / BLOCK_ROWS) * ((N + form.width - 1) / form.width);
+  plan->pdl = large_pdl(pdl, tiles, form.pairs ? sms / 2 : sms);
   return rc;
 }
 

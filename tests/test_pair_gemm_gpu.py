@@ -73,3 +73,15 @@ def test_which_calls_run_as_pairs():
     assert w(64, 256, 128, variant_hint=PAIR_FORM | 3) == 96 and w(64, 256, 128, variant_hint=PAIR_FORM) == 256
     assert w(4096, 8192, 8192, variant_hint=2 << 28) > 0  # (no dependent launch: the kernel is still open)
     assert w(4096, 8192, 8192, sm_count=1) == 0 and w(4096, 8200, 8192) == 0
+
+
+@pytest.mark.parametrize("m,n,k", [(256, 1024, 8064), (256, 2048, 7936), (130, 1024, 6144), (200, 4096, 8064), (133, 5136, 14336), (256, 4096, 14336)])
+def test_narrow_outputs_over_many_k_blocks_keep_the_k_split(m, n, k):
+    """Pairs walk all k-blocks on few SMs there; the choice compares times on both sides of 64 k-blocks."""
+    assert _lib.pair_width(m, n, k) == 0 and _lib.pair_width(m, n, k + 512) == 0
+
+
+@pytest.mark.parametrize("m,n", [(130, 1024), (200, 2048), (256, 4096), (129, 16384)])
+def test_few_k_blocks_do_not_run_as_pairs(m, n):
+    """Eight k-blocks: the 128-row form needs 5.7 us at 200 x 4096, pairs 7.0, the small-M kernel 12.7."""
+    assert _lib.pair_width(m, n, 1024) == 0

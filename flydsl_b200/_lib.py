@@ -60,6 +60,8 @@ SIGNATURES = {
     "flyb200_moe_gather_rows": (_i, [_vp, _vp, _vp, _vp, _vp, _vp, _i, _i, _i, _i, _i, _vp]),
     "flyb200_moe_quant_sorted": (_i, [_vp, _vp, _vp, _vp, _vp, _i, _i, _i, _i, _i, _vp]),
     "flyb200_moe_gemm": (_i, [_i, _vp, _vp, _vp, _vp, _vp, _vp, _vp, _vp, _vp] + [_i] * 12 + [_vp]),
+    "flyb200_moe_gemm_shard": (_i, [_i, _vp, _vp, _vp, _vp, _vp, _vp, _vp, _vp, _vp] + [_i] * 13 + [_vp]),
+    "flyb200_moe_form": (_i, [_i] * 10),
     "flyb200_moe_reduce": (_i, [_vp, _vp, _i, _i, _i, _i, _vp, _vp, _i, _vp]),
     "flyb200_moe_sorting": (_i, [_vp, _vp, _i, _i, _i, _i, _vp, _vp, _vp, _vp, _vp, _vp]),
     "flyb200_moe_sorting_range": (_i, [_vp, _i, _vp, _i, _i, _i, ctypes.c_longlong, _i, _vp, _vp, _vp, _vp, _vp]),
@@ -160,6 +162,14 @@ def describe_plan(m: int, n: int, k: int, in_dtype: str = "fp8", variant_hint: i
 def pair_width(m: int, n: int, k: int, in_dtype: str = "fp8", variant_hint: int = 0, sm_count: int = 148) -> int:
     """Tile width with which the call runs as CTA pairs, 0 where the plan of describe_plan runs (no GPU needed)."""
     return load().flyb200_pair_width(m, n, k, IN_DTYPES[in_dtype], variant_hint, sm_count)
+
+
+def moe_form(stage: int, tokens: int, topk: int, experts: int, model_dim: int, inter_dim: int, tile_m: int, all_experts: int | None = None,
+             sm_count: int = 148) -> int:
+    """The kernel a mixture-of-experts stage runs on, numbered as in FLYB200_MOE_KERNEL (no GPU needed).  ``experts``: of the call,
+    ``all_experts``: of all ranks."""
+    blocks = -(-(tokens * topk + experts * tile_m - topk) // tile_m)  # as many as the routing table has room for
+    return load().flyb200_moe_form(stage, tokens, topk, experts, all_experts or experts, model_dim, inter_dim, tile_m, blocks, sm_count)
 
 
 _failure_hooks: list = []

@@ -157,31 +157,49 @@ int launch_moe_large_variant(int stage, int out_dtype, bool accumulate, const CU
   return FLYB200_E_UNSUPPORTED;
 }
 
-// Whether CTA pairs are estimated to be faster than one CTA per 128-row item.  How the routes fall on the experts is known on
-// the device only, so the estimate spreads them evenly: a last, half-filled tile per expert, and with routing blocks of 64 one
-// more pass of the 128-row form where the expert changes inside an item.  Per k-block a pair needs 512 cycles (tensor pipe)
-// and a CTA by itself 680 (bytes into the SM), per item at least the epilogue's 6000 to 7600; the weights come at 3333 bytes
-// per cycle (6 TB/s), and the second passes read them again once they have left L2.  One CTA / pairs, us, gather included:
-// 4096 tokens x top-2, 8 experts, 4096 x 2048 149 / 139 and 88 / 76 (gate-up, down), 200 tokens 37.3 / 32.3 (gate-up), 800 x top-4, 32
-// experts, 3072 x 1536 99 / 78 and 51 / 45, 515 x top-4, 16 experts, 2048 x 1408 34.3 / 26.8 and 19.3 / 17.2; where items are few and the
-// weights fit L2, or K is short, it is the other way round: 200 x top-2, 8 experts, down 17.2 / 19.6, 1024 x top-4, 8 experts, 2048 x 1024 21.5 /
-// 25.2 and 14.6 / 19.0, 4096 x top-4, 32 experts, 2048 x 768, down 46.3 / 55.6.
-bool moe_pair_pays(int stage, long long routes, int experts, int n_out, int num_kb, int tile_m, int sms) {
-  const double used = routes < experts ? static_cast<double>(routes) : experts, rows = routes / used;
-  const double pairs = (n_out + (stage == 1 ? 127 : 255)) / (stage == 1 ? 128 : 256);
-  const double tiles = rows < 128 ? 1.0 : rows / 256 + 0.5;
-  const double blocks = rows / 128 + (tile_m == 64 || tile_m == 256 ? 1.0 : 0.5);
-  const double weights = used * n_out * (stage == 1 ? 2 : 1) * num_kb * KBLOCK_BYTES;
-  const double again = tile_m == 64 && weights > 100e6 ? 1.4 : 1.0;
-  auto cycles = [&](double x, double kb_cycles, double least, double bytes) {
-    const double part = x - static_cast<long long>(x);
-    const double rounds = x <= 1.0 ? 1.0 : part == 0.0 ? x : part > 0.6 ? x - part + 1.0 : x + 0.4;
-    const double item = num_kb * kb_cycles > least ? num_kb * kb_cycles : least;
-    return rounds * item > bytes / 3333.0 ? rounds * item : bytes / 3333.0;
-  };
-  const double pair = cycles(used * tiles * pairs / (sms / 2), 512.0, stage == 1 ? 7600.0 : 6500.0, weights);
-  const double single = cycles(used * blocks * pairs / sms, 680.0, stage == 1 ? 7000.0 : 6000.0, again * weights);
-  return pair + 1000.0 < single;
+// Estimated time (us, the gather pass left out) of a stage on CTA pairs, or with one CTA per 128-row item.  How the routes fall on the
+// experts is known on the device only, so the estimate spreads `routes` evenly: 128-row items (routing blocks of 64 make one more
+// pass where the expert changes inside an item) or 256-row tiles per expert, rounds of them over the SMs with a part of a
+// last one, per k-block and per item a time, at least the weights at 6.5 TB/s.
+// Fitted to 5038 drawn layers (16..8192 tokens, top-1..8, 8..128 experts of which a rank serves all, a half, a quarter or an eighth, 1024..7168 x
+// 512..4096, routing blocks of 64..256, graph replay, weights rotated past L2).  The form with the smaller estimate is on average 1.0 / 1.0 %
+// (gate-up / down) behind the better one where all experts are served and 1.5 / 1.2 % on a rank's share, 53 % at worst; always
+// pairs 3.8 / 10.0 and 6.8 / 12.2 %, always one CTA 7.9 / 5.0 and 5.2 / 2.9 %.  With all ranks' routes counted on a share 2.6 / 1.9 %.  One
+// CTA / pairs, us, gather included: 4096 tokens x top-2, 8 experts, 4096 x 2048 128 / 122 and 74 / 67 (gate-up, down), 800 x top-4, 32
+// experts, 3072 x 1536 91 / 65 and 48 / 41, 515 x top-4, 16 experts, 2048 x 1408 32.6 / 30.7 and 24.4 / 21.0; where items are few and the
+// weights fit L2, or K is short, it is the other way round: 1024 x top-4, 8 experts, 2048 x 1024, down 19.2 / 20.0, 4096 x top-4, 32 experts, 2048 x
+// 768, down 43.0 / 51.2.
+double moe_form_us(bool pairs, int stage, double routes, int experts, int n_out, int num_kb, int tile_m, int sms) {
+  const bool up = stage == 1;
+  const double used = routes < 1.0 ? 1.0 : routes < experts ? routes : experts, rows = routes / used;
+  const int columns = up ? (n_out + 127) / 128 : (n_out + 255) / 256;
+  const double weights = used * n_out * (up ? 2 : 1) * num_kb * KBLOCK_BYTES / 6.5e6;
+  double rounds, item, fixed;
+  if (pairs) {
+    const double tiles = rows / 256 + (up ? 0.6 : 0.55);
+    rounds = used * (tiles < 1.0 ? 1.0 : tiles) * columns / (sms / 2) + 0.45;
+    item = up ? num_kb * 0.26 + 1.9 : num_kb * 0.28 + 3.1;
+    fixed = up ? 7.8 : 5.7;
+  } else {
+    const double more = tile_m == 64 ? (up ? 1.55 : 1.35) : tile_m == 128 ? (up ? 1.0 : 0.95) : (up ? 1.5 : 1.0);
+    rounds = used * (rows / 128 + more) * columns / sms + (up ? 0.85 : 0.5);
+    item = up ? num_kb * 0.39 + 0.4 : num_kb * 0.45 + 1.6;
+    fixed = 3.7;
+  }
+  const double work = (rounds < 1.0 ? 1.0 : rounds) * item;
+  return fixed + (work > weights ? work : weights);
+}
+
+// Kernel for routing blocks of tile_m rows when nothing forces one, numbered as in FLYB200_MOE_KERNEL: 1 two weight tiles per CTA,
+// 2 one CTA per 128-row item, 3 CTA pairs (while the list of their tiles fits shared memory).  `all_experts`: of which the
+// `experts` of this call get their share of the routes.
+int moe_form(int stage, int tokens, int topk, int experts, int all_experts, int model_dim, int inter_dim, int tile_m, int blocks, int sms) {
+  if (tile_m % BLOCK_ROWS != 0 && tile_m != 64) return 1;
+  if (blocks > MOE_PAIR_MAX_BLOCKS || sms < 2) return 2;
+  const double routes = static_cast<double>(tokens) * topk * experts / all_experts;
+  const int n_out = stage == 1 ? inter_dim : model_dim, num_kb = (stage == 1 ? model_dim : inter_dim) / KBLOCK_BYTES;
+  auto us = [&](bool pairs) { return moe_form_us(pairs, stage, routes, experts, n_out, num_kb, tile_m, sms); };
+  return us(true) < us(false) ? 3 : 2;
 }
 
 template <int KIND, int BN>
@@ -284,16 +302,34 @@ int flyb200_moe_quant_sorted(void* dst, float* dst_scale, const void* src, const
   return FLYB200_OK;
 }
 
+int flyb200_moe_form(int stage, int tokens, int topk, int experts, int all_experts, int model_dim, int inter_dim, int tile_m,
+                     int blocks, int sm_count) {
+  if ((stage != 1 && stage != 2) || tokens <= 0 || topk <= 0 || experts <= 0 || all_experts < experts || model_dim <= 0 || inter_dim <= 0 ||
+      tile_m < 16 || tile_m > 256 || tile_m % 16 != 0 || blocks <= 0 || sm_count <= 0)
+    return 0;
+  return moe_form(stage, tokens, topk, experts, all_experts, model_dim, inter_dim, tile_m, blocks, sm_count);
+}
+
 int flyb200_moe_gemm(int stage, void* out, const void* a_sorted, const void* w_shuf, const float* scale_a_sorted,
                      const float* scale_w, const int* sorted_ids, const int* expert_ids, const float* sorted_weights,
                      const int* num_valid_ids, int tokens, int topk, int experts, int model_dim, int inter_dim,
                      int tile_m, int blocks, int in_dtype, int out_dtype, int doweight, int accumulate, int after_gather,
                      void* stream) {
+  return flyb200_moe_gemm_shard(stage, out, a_sorted, w_shuf, scale_a_sorted, scale_w, sorted_ids, expert_ids, sorted_weights, num_valid_ids,
+                                tokens, topk, experts, experts, model_dim, inter_dim, tile_m, blocks, in_dtype, out_dtype, doweight,
+                                accumulate, after_gather, stream);
+}
+
+int flyb200_moe_gemm_shard(int stage, void* out, const void* a_sorted, const void* w_shuf, const float* scale_a_sorted,
+                           const float* scale_w, const int* sorted_ids, const int* expert_ids, const float* sorted_weights,
+                           const int* num_valid_ids, int tokens, int topk, int experts, int all_experts, int model_dim, int inter_dim,
+                           int tile_m, int blocks, int in_dtype, int out_dtype, int doweight, int accumulate, int after_gather,
+                           void* stream) {
   if (stage != 1 && stage != 2) return FLYB200_E_BAD_ARG;
   if (!out || !a_sorted || !w_shuf || !scale_a_sorted || !scale_w || !sorted_ids || !expert_ids || !num_valid_ids)
     return FLYB200_E_BAD_ARG;
   if (doweight && !sorted_weights) return FLYB200_E_BAD_ARG;
-  if (tokens < 0 || topk <= 0 || topk > 255 || experts <= 0 || model_dim <= 0 || inter_dim <= 0 || blocks < 0)
+  if (tokens < 0 || topk <= 0 || topk > 255 || experts <= 0 || all_experts < experts || model_dim <= 0 || inter_dim <= 0 || blocks < 0)
     return FLYB200_E_BAD_ARG;
   if (tokens >= (1 << 24)) return FLYB200_E_UNSUPPORTED;  // a sorted id keeps the token in 24 bits
   if (in_dtype != FLYB200_DT_FP8 && in_dtype != FLYB200_DT_INT8) return FLYB200_E_UNSUPPORTED;
@@ -339,10 +375,8 @@ int flyb200_moe_gemm(int stage, void* out, const void* a_sorted, const void* w_s
     if ((rc = sm_count(&sms))) return rc;
     rc = host::byte_matrix_map(&tmA, a_sorted, static_cast<uint64_t>(K), static_cast<uint64_t>(blocks) * tile_m, BLOCK_ROWS);
     if (rc) return rc;
-    // CTA pairs where they pay, while the list of their tiles fits shared memory
-    const bool forced = force && (force[0] == '2' || force[0] == '3');
-    const bool pair = blocks <= MOE_PAIR_MAX_BLOCKS && sms > 1 &&
-                      (forced ? force[0] == '3' : moe_pair_pays(stage, static_cast<long long>(tokens) * topk, experts, n_out, K / KBLOCK_BYTES, tile_m, sms));
+    const int form = moe_form(stage, tokens, topk, experts, all_experts, model_dim, inter_dim, tile_m, blocks, sms);
+    const bool pair = force && (force[0] == '2' || force[0] == '3') ? force[0] == '3' && blocks <= MOE_PAIR_MAX_BLOCKS && sms > 1 : form == 3;
     MoePairWeights tmW;
     for (int i = 0; pair && i < 3; ++i) {
       rc = host::weight_image_map(&tmW.box[i], w_shuf, static_cast<uint64_t>(p.n_expert), static_cast<uint64_t>(experts) * (K / KBLOCK_BYTES), BLOCK_ROWS >> i);

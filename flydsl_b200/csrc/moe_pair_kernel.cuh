@@ -7,7 +7,7 @@
 //
 // What bounds it: the weight stream where experts are small (800 tokens x top-4, 32 experts, 3072 x 1536: 321 MB read for 302 MB
 // of weights at 4.8 TB/s, against 444 MB of the 128-row form), the tensor pipe at the clock that the power cap leaves in
-// prefill.  moe_pair_pays in flyb200_moe.cu lists the times of both forms.
+// prefill.  moe_form_us in flyb200_moe.cu lists the times of both forms.
 //
 // A tile starts at every (256 / tile_m)-th routing block of an expert's run of blocks.  One warp finds these in
 // expert_ids before the mainloop and leaves them in shared memory, so that any item can be looked up.

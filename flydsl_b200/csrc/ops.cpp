@@ -320,8 +320,8 @@ PyObject* moe_sort(PyObject*, PyObject* const* argv, Py_ssize_t n) {
 }
 
 // moe_stage(out, x, w, scale_x, scale_w, ids, experts, weights | None, valid, a_sorted, sa_sorted, stage, tokens, topk, gather, k,
-//           n_experts, model, inter, tile_m, blocks, in, out, doweight, accumulate, stream) -> code: gather pass and grouped GEMM.
-// No checks: the launcher's own, or the compiled launcher's.
+//           n_experts, model, inter, tile_m, blocks, in, out, doweight, accumulate, stream, all_experts) -> code: gather pass and
+// grouped GEMM.  No checks: the launcher's own, or the compiled launcher's.
 PyObject* moe_stage(PyObject*, PyObject* const* argv, Py_ssize_t n) {
   HANDLE_TH_ERRORS
   Args a{argv, n};
@@ -330,6 +330,7 @@ PyObject* moe_stage(PyObject*, PyObject* const* argv, Py_ssize_t n) {
   const int stage = a.i32(), tokens = a.i32(), topk = a.i32(), gather = a.i32(), k = a.i32(), experts = a.i32(), model = a.i32(),
             inter = a.i32(), tile_m = a.i32(), blocks = a.i32(), in = a.i32(), out_t = a.i32(), dow = a.i32(), acc = a.i32();
   const long long s = a.integer();
+  const int all = a.i32();
   if (!a.done()) return none();
   void *op = ptr(out), *xp = ptr(x), *wp = ptr(w);
   const float *sxp = as<float>(sx), *swp = as<float>(sw), *tp = wts.defined() && wts.numel() ? as<float>(wts) : nullptr;
@@ -339,8 +340,8 @@ PyObject* moe_stage(PyObject*, PyObject* const* argv, Py_ssize_t n) {
     NoGil g;
     rc = flyb200_moe_gather_rows(ptr(a_s), as<float>(sa_s), xp, sxp, ip, vp, tokens, topk, gather, k, blocks * tile_m, handle(s));
     if (!rc)
-      rc = flyb200_moe_gemm(stage, op, ptr(a_s), wp, as<float>(sa_s), swp, ip, ep, tp, vp, tokens, topk, experts, model, inter, tile_m,
-                            blocks, in, out_t, dow, acc, 1, handle(s));
+      rc = flyb200_moe_gemm_shard(stage, op, ptr(a_s), wp, as<float>(sa_s), swp, ip, ep, tp, vp, tokens, topk, experts, all, model, inter,
+                                  tile_m, blocks, in, out_t, dow, acc, 1, handle(s));
   }
   return code(rc);
   END_HANDLE_TH_ERRORS
@@ -384,13 +385,13 @@ PyObject* moe_layer(PyObject*, PyObject* const* argv, Py_ssize_t n) {
       const at::Tensor out1 = at::empty({tokens * topk, i}, bf16);
       rc = flyb200_moe_gather_rows(ptr(a1), as<float>(sa1), ptr(x), as<float>(sx), ip, vp, t, topk, 0, model, rn, s);
       if (!rc)
-        rc = flyb200_moe_gemm(1, ptr(out1), ptr(a1), ptr(w1), as<float>(sa1), as<float>(sw1), ip, ep, tp, vp, t, topk, experts, model, inter,
-                              tile_m, r.blocks, in, FLYB200_OUT_BF16, 0, 0, 1, s);
+        rc = flyb200_moe_gemm_shard(1, ptr(out1), ptr(a1), ptr(w1), as<float>(sa1), as<float>(sw1), ip, ep, tp, vp, t, topk, experts,
+                                    all, model, inter, tile_m, r.blocks, in, FLYB200_OUT_BF16, 0, 0, 1, s);
       if (!rc) rc = flyb200_moe_quant_sorted(ptr(a2), as<float>(sa2), ptr(out1), ip, vp, t, topk, inter, rn, in, s);
       const at::Tensor out2 = at::empty({tokens * topk, m}, bf16);
       if (!rc)
-        rc = flyb200_moe_gemm(2, ptr(out2), ptr(a2), ptr(w2), as<float>(sa2), as<float>(sw2), ip, ep, tp, vp, t, topk, experts, model, inter,
-                              tile_m, r.blocks, in, FLYB200_OUT_BF16, 1, 0, 1, s);
+        rc = flyb200_moe_gemm_shard(2, ptr(out2), ptr(a2), ptr(w2), as<float>(sa2), as<float>(sw2), ip, ep, tp, vp, t, topk, experts,
+                                    all, model, inter, tile_m, r.blocks, in, FLYB200_OUT_BF16, 1, 0, 1, s);
       const at::Tensor ids32 = ids.to(at::kInt).contiguous();
       y = at::empty({tokens, m}, bf16);
       if (!rc) rc = flyb200_moe_reduce(ptr(y), ptr(out2), t, topk, model, FLYB200_OUT_BF16, as<int>(mask), as<int>(ids32), all, s);

@@ -91,6 +91,7 @@ class ExpertParallelMoe:
             self._reduce = compile_moe_reduction(topk=topk, model_dim=model_dim, dtype_str="bf16", use_mask=True,
                                                  num_experts=experts)
             self._mask = None  # 1 for this rank's experts, built on first use on the layer's device
+        self._g1.all_experts = self._g2.all_experts = experts
         self._w1 = self._w2 = self._sw1 = self._sw2 = None
 
     def describe(self) -> dict:

@@ -31,14 +31,14 @@ def gemm_a8w8(c, a, b, scale_a, scale_b, bias, M, N, K, in_dtype, out_dtype, epi
 
 
 def moe_stage(out, x, w, scale_x, scale_w, ids, expert_ids, weights, valid, a_sorted, sa_sorted, stage, tokens, topk, gather, k, experts,
-              model, inter, tile_m, blocks, in_dtype, out_dtype, doweight, accumulate, stream) -> int:
+              model, inter, tile_m, blocks, in_dtype, out_dtype, doweight, accumulate, stream, all_experts) -> int:
     lib, s = _lib.load(), stream or None
     a, sa, i, v = a_sorted.data_ptr(), sa_sorted.data_ptr(), ids.data_ptr(), valid.data_ptr()
     rc = lib.flyb200_moe_gather_rows(a, sa, x.data_ptr(), scale_x.data_ptr(), i, v, tokens, topk, gather, k, blocks * tile_m, s)
     if rc:
         return rc
-    return lib.flyb200_moe_gemm(
+    return lib.flyb200_moe_gemm_shard(
         stage, out.data_ptr(), a, w.data_ptr(), sa, scale_w.data_ptr(), i, expert_ids.data_ptr(),
-        weights.data_ptr() if weights is not None and weights.numel() else None, v, tokens, topk, experts, model, inter, tile_m, blocks,
-        in_dtype, out_dtype, int(doweight), int(accumulate), 1, s,
+        weights.data_ptr() if weights is not None and weights.numel() else None, v, tokens, topk, experts, all_experts, model, inter, tile_m,
+        blocks, in_dtype, out_dtype, int(doweight), int(accumulate), 1, s,
     )  # fmt: skip

@@ -152,6 +152,10 @@ def sort_on_device(topk_ids, topk_weights, experts: int, block_size: int, first_
 class _MoeStage:
     """Shared launcher: gathers the activation rows into sorted order, then runs the grouped GEMM."""
 
+    # Experts of all ranks where ``experts`` are one rank's share, else 0: the routes are then expected to be spread over
+    # all of them, which decides between the kernels.  The result does not depend on it.
+    all_experts = 0
+
     def __init__(self, stage, model_dim, inter_dim, experts, topk, tile_m, in_dtype, out_dtype, doweight, accumulate):
         self.stage = stage
         self.model_dim, self.inter_dim = int(model_dim), int(inter_dim)
@@ -296,7 +300,7 @@ class _MoeStage:
         args = (
             out, x, w, scale_x, scale_w, sorted_token_ids, sorted_expert_ids, sorted_weights, num_valid_ids, a_sorted, sa_sorted,
             self.stage, tokens, self.topk, self._gather_mode, self._k, self.experts, self.model_dim, self.inter_dim, self.tile_m,
-            blocks, self._dt, self._out, self.doweight, self.accumulate, s or 0,
+            blocks, self._dt, self._out, self.doweight, self.accumulate, s or 0, self.all_experts or self.experts,
         )  # fmt: skip
         with lock:
             rc = _lib.ops().moe_stage(*args)
@@ -328,11 +332,14 @@ class _MoeStage:
                     tokens, self.topk, self._k, rows, self._dt, s)
                 if rc:
                     _lib.check(rc, "moe_quant_sorted")
-                rc = _lib.load().flyb200_moe_gemm(
+                gemm, experts = _lib.load().flyb200_moe_gemm, (self.experts,)
+                if self.all_experts:
+                    gemm, experts = _lib.load().flyb200_moe_gemm_shard, (self.experts, self.all_experts)
+                rc = gemm(
                     self.stage, out.data_ptr(), a_sorted.data_ptr(), w.data_ptr(), sa_sorted.data_ptr(), scale_w.data_ptr(),
                     sorted_token_ids.data_ptr(), sorted_expert_ids.data_ptr(),
                     sorted_weights.data_ptr() if sorted_weights is not None and sorted_weights.numel() else None,
-                    num_valid_ids.data_ptr(), tokens, self.topk, self.experts, self.model_dim, self.inter_dim, self.tile_m, blocks,
+                    num_valid_ids.data_ptr(), tokens, self.topk, *experts, self.model_dim, self.inter_dim, self.tile_m, blocks,
                     self._dt, self._out, int(self.doweight), int(self.accumulate), 1, s,
                 )  # fmt: skip
                 if rc:

@@ -311,6 +311,21 @@ int flyb200_moe_gemm(int stage, void* out, const void* a_sorted, const void* w_s
                      int tile_m, int blocks, int in_dtype, int out_dtype, int doweight, int accumulate, int after_gather,
                      void* stream);
 
+/* The same call where `experts` are one rank's share of `all_experts`: about experts / all_experts of the tokens * topk
+ * routes are in the routing table, which is what the choice of the kernel counts on (flyb200_moe_form).  The
+ * result does not depend on it. */
+int flyb200_moe_gemm_shard(int stage, void* out, const void* a_sorted, const void* w_shuf, const float* scale_a_sorted,
+                           const float* scale_w, const int* sorted_ids, const int* expert_ids, const float* sorted_weights,
+                           const int* num_valid_ids, int tokens, int topk, int experts, int all_experts, int model_dim,
+                           int inter_dim, int tile_m, int blocks, int in_dtype, int out_dtype, int doweight, int accumulate,
+                           int after_gather, void* stream);
+
+/* Which kernel flyb200_moe_gemm_shard runs on a GPU with sm_count SMs when the environment forces none: 1 two weight tiles
+ * per CTA (routing blocks other than 64, 128 and 256), 2 one CTA per 128 sorted rows, 3 CTA pairs; 0 for arguments out
+ * of range.  Pure host function. */
+int flyb200_moe_form(int stage, int tokens, int topk, int experts, int all_experts, int model_dim, int inter_dim, int tile_m,
+                     int blocks, int sm_count);
+
 /* Routing table from the router's choice: the device form of the reference's
  * moe_sorting (layout stated in tests/kernels/test_moe_gemm_2stage.py:99-137; the
  * reference's own device kernel is kernels/moe/moe_sorting_kernel.py).  A stable

@@ -193,18 +193,20 @@ def test_accumulate_ragged_channels(dev, tile_m, out_dtype):
 
 @pytest.mark.parametrize("tile_m,experts,tokens", [(128, 4, 500), (64, 4, 500), (64, 16, 90), (64, 3, 33)])
 def test_both_kernel_forms_agree(dev, monkeypatch, tile_m, experts, tokens):
-    """The persistent form and the two-tiles-per-CTA form do the same arithmetic per output element.
+    """The two persistent forms and the two-tiles-per-CTA form do the same arithmetic per output element.
     With 64-row routing blocks the persistent form works a 128-row block twice where the expert
     changes inside it (many experts with few rows: nearly every block)."""
     model_dim, inter_dim, topk = 512, 384, 2
     d = moe_oracle.make_inputs(tokens, model_dim, inter_dim, experts, topk, "fp8", seed=34)
     kw = dict(model_dim=model_dim, inter_dim=inter_dim, experts=experts, topk=topk, tile_m=tile_m, in_dtype="fp8")
-    a1 = run_stage1(dev, d, **kw, out_dtype="bf16")
-    a2 = run_stage2(dev, d, **kw, out_dtype="bf16", accumulate=False)
     monkeypatch.setenv("FLYB200_MOE_KERNEL", "1")
     b1 = run_stage1(dev, d, **kw, out_dtype="bf16")
     b2 = run_stage2(dev, d, **kw, out_dtype="bf16", accumulate=False)
-    assert torch.equal(a1, b1) and torch.equal(a2, b2)
+    for form in ("2", "3", ""):  # one CTA per 128 rows, CTA pairs, the automatic choice
+        monkeypatch.setenv("FLYB200_MOE_KERNEL", form)
+        a1 = run_stage1(dev, d, **kw, out_dtype="bf16")
+        a2 = run_stage2(dev, d, **kw, out_dtype="bf16", accumulate=False)
+        assert torch.equal(a1, b1) and torch.equal(a2, b2), form
 
 
 def test_stage1_partial_tile_large_block(dev):

@@ -6,6 +6,7 @@ import torch
 
 from flydsl_b200 import _lib, shuffle_weight
 from flydsl_b200.kernels.moe.moe_gemm_2stage import compile_moe_gemm1, compile_moe_gemm2, moe_sorting
+from oracle import moe_oracle
 
 pytestmark = pytest.mark.gpu
 
@@ -89,3 +90,22 @@ def test_blocks_without_expert_and_a_shorter_list(monkeypatch):
                              topk=topk, tile_m=tile_m, in_dtype="int8", out_dtype="bf16", accumulate=False, n_valid=n_valid))
         assert torch.equal(got[0], got[1])
         assert int((got[0] == 0).all(dim=1).sum()) > 0  # some routes had no expert
+
+
+def test_longer_lists_than_the_pair_form_holds(monkeypatch):
+    """7200 experts of one route each are 7200 routing blocks; the pair form's list has room for 7168, so the request for it
+    runs one CTA per item."""
+    experts, model, inter = 7200, 16, 128
+    d = moe_oracle.make_inputs(experts, 128, inter, 2, 1, "int8", seed=5)  # activations and scales of the second stage
+    g = torch.Generator().manual_seed(5)
+    ids = torch.randperm(experts, generator=g).view(-1, 1).int()
+    w2, sw2 = torch.randint(-127, 128, (experts, model, inter), generator=g, dtype=torch.int8), torch.rand(experts, model, 1, generator=g) / 64
+    routing = moe_sorting(ids.cuda(), d["topk_weights"].cuda(), num_experts=experts, block_size=64)
+    assert routing[2].numel() > 7168 and int(routing[3][0]) == 64 * experts
+    monkeypatch.setenv("FLYB200_MOE_KERNEL", "3")
+    got = stage(2, d["a2_q"].view(experts, inter).cuda(), d["scale_a2"].reshape(-1).cuda(), shuffle_weight(w2.cuda()).view(-1), sw2.view(-1).cuda(),
+                routing, model=model, inter=inter, experts=experts, topk=1, tile_m=64, in_dtype="int8", out_dtype="f32", accumulate=True)
+    args = (d["scale_a2"], sw2, ids.long(), d["topk_weights"], model)
+    ref, size = moe_oracle.moe_gemm2(d["a2_q"], w2, *args), moe_oracle.moe_gemm2(d["a2_q"].int().abs(), w2.int().abs(), *args)
+    # the kernel's sum of integers is exact; the oracle rounds both operands, 128 products and sums; four roundings of factors here
+    assert bool(((got[:experts].cpu() - ref).abs() <= (2 * 128 + 6) * 2**-24 * size).all())

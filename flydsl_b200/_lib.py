@@ -52,6 +52,7 @@ SIGNATURES = {
     "flyb200_shuffle_weight": (_i, [_vp, _vp, _i, _i, _i, _i, _vp]),
     "flyb200_unshuffle_weight": (_i, [_vp, _vp, _i, _i, _i, _vp]),
     "flyb200_pair_width": (_i, [_i, _i, _i, _i, _i, _i]),
+    "flyb200_describe_call": (_i, [_i, _i, _i, _i, _i, _i, _i, ctypes.POINTER(_i)]),
     "flyb200_describe_plan": (_i, [_i, _i, _i, _i, _i, _i, ctypes.POINTER(_i)]),
     "flyb200_layout_kind": (_i, [_i, _i, _i]),
     "flyb200_workspace_bytes": (_sz, [_i, _i, _i, _i, _i]),
@@ -149,19 +150,22 @@ def current_stream(device) -> int:
     return torch._C._cuda_getCurrentRawStream(device.index)
 
 
-PLAN_FIELDS = ("kernel", "bn", "split_k", "kb_per_split", "reduce", "stages", "pdl", "token_blocks")
+PLAN_FIELDS = ("kernel", "bn", "split_k", "kb_per_split", "reduce", "stages", "pdl", "token_blocks", "strips")
 
 
-def describe_plan(m: int, n: int, k: int, in_dtype: str = "fp8", variant_hint: int = 0, sm_count: int = 148) -> dict:
-    """The kernel variant the library would pick (no GPU needed)."""
-    out = (_i * 8)()
-    check(load().flyb200_describe_plan(m, n, k, IN_DTYPES[in_dtype], variant_hint, sm_count, out), "describe_plan")
+def describe_plan(m: int, n: int, k: int, in_dtype: str = "fp8", variant_hint: int = 0, sm_count: int = 148, epilogue: str = "none") -> dict:
+    """The kernel variant that the call runs (no GPU needed)."""
+    out = (_i * len(PLAN_FIELDS))()
+    check(load().flyb200_describe_call(m, n, k, IN_DTYPES[in_dtype], EPILOGUES[epilogue], variant_hint, sm_count, out), "describe_plan")
     return dict(zip(PLAN_FIELDS, list(out)))
 
 
-def pair_width(m: int, n: int, k: int, in_dtype: str = "fp8", variant_hint: int = 0, sm_count: int = 148) -> int:
-    """Tile width with which the call runs as CTA pairs, 0 where the plan of describe_plan runs (no GPU needed)."""
-    return load().flyb200_pair_width(m, n, k, IN_DTYPES[in_dtype], variant_hint, sm_count)
+def pair_width(m: int, n: int, k: int, in_dtype: str = "fp8", variant_hint: int = 0, sm_count: int = 148, epilogue: str = "none") -> int:
+    """Tile width with which the call runs as CTA pairs, 0 where it does not (no GPU needed)."""
+    out = (_i * len(PLAN_FIELDS))()
+    if load().flyb200_describe_call(m, n, k, IN_DTYPES[in_dtype], EPILOGUES[epilogue], variant_hint, sm_count, out):
+        return 0
+    return out[1] if out[0] == 3 else 0
 
 
 def moe_form(stage: int, tokens: int, topk: int, experts: int, model_dim: int, inter_dim: int, tile_m: int, all_experts: int | None = None,

@@ -628,10 +628,10 @@ int make_plan(Plan* plan, int M, int N, int K_bytes, int variant_hint, size_t wo
 }
 
 // make_plan, and the large-M form that takes its place where the call leaves the kernel open and another one is the better choice.
-int plan_call(Plan* plan, int M, int N, int K_bytes, int variant_hint, size_t workspace_bytes, bool have_ws, int sms, bool activation) {
+int plan_call(Plan* plan, int M, int N, int K_bytes, int variant_hint, size_t workspace_bytes, bool have_ws, int sms, int epilogue) {
   const int rc = make_plan(plan, M, N, K_bytes, variant_hint, workspace_bytes, have_ws, sms);
   if (rc || (variant_hint & ~(3 << 28)) != 0 || rows_tall_default() || w64_default()) return rc;
-  LargeForm form = large_form(*plan, M, N, K_bytes, sms, activation);
+  LargeForm form = large_form(*plan, M, N, K_bytes, sms, epilogue >= FLYB200_EPI_BIAS_SILU);
   // the 128-row form is faster than the 256-row form by now wherever pairs are not: fp8 1500 x 6144 x 1024 12.2 / 15.3 us
   if (form.width == 0 && plan->tall) form = {false, auto_rows_bn(M, N, K_bytes, sms)};
   if (form.width == 0) return rc;
@@ -650,6 +650,16 @@ int plan_call(Plan* plan, int M, int N, int K_bytes, int variant_hint, size_t wo
                                      : static_cast<long long>((M + BLOCK_ROWS - 1) / BLOCK_ROWS) * ((N + form.width - 1) / form.width);
   plan->pdl = large_pdl(pdl, tiles, form.pairs ? sms / 2 : sms);
   return rc;
+}
+
+// Depth of the shared-memory ring, and column strips of the tiles of the last round, with which a plan is launched.
+int ring_stages(const Plan& plan) {
+  return plan.decode ? plan.stages : plan.two_sm ? host::pair_stages_for(plan.bn) : plan.tall ? host::ROWS_TALL_STAGES : host::rows_stages_for(plan.bn);
+}
+int tail_strips(const Plan& plan, int M, int N, int sms) {
+  if (plan.decode || plan.tall) return 1;
+  if (plan.two_sm) return sms < 2 ? 1 : host::pair_tail_parts(plan.bn, host::pair_tiles(M, N, plan.bn), sms / 2);
+  return host::rows_tail_parts(plan.bn, static_cast<long long>((M + BLOCK_ROWS - 1) / BLOCK_ROWS) * ((N + plan.bn - 1) / plan.bn), sms);
 }
 
 int gemm_common(void* c, const void* a, const void* w, const float* sa, const float* sb, const void* bias, int M,
@@ -675,7 +685,7 @@ int gemm_common(void* c, const void* a, const void* w, const float* sa, const fl
   const int K_bytes = K * eb;
 
   Plan plan;
-  rc = plan_call(&plan, M, N, K_bytes, variant_hint, workspace_bytes, workspace != nullptr, st->sms, epilogue >= FLYB200_EPI_BIAS_SILU);
+  rc = plan_call(&plan, M, N, K_bytes, variant_hint, workspace_bytes, workspace != nullptr, st->sms, epilogue);
   if (rc) return rc;
 
   GemmParams p;
@@ -698,8 +708,8 @@ int gemm_common(void* c, const void* a, const void* w, const float* sa, const fl
   p.prefetch = plan.prefetch;
   p.token_blocks = plan.token_blocks;
   p.bn = plan.bn;
-  p.rows_stages = plan.two_sm ? host::pair_stages_for(plan.bn) : plan.tall ? host::ROWS_TALL_STAGES : host::rows_stages_for(plan.bn);
-  p.tail_parts = 1;
+  p.rows_stages = ring_stages(plan);
+  p.tail_parts = tail_strips(plan, M, N, st->sms);
   p.ws_tickets = static_cast<int*>(workspace);
   p.ws_partials = workspace ? reinterpret_cast<float*>(static_cast<uint8_t*>(workspace) + TICKET_BYTES) : nullptr;
   p.status = st->status;
@@ -715,7 +725,6 @@ int gemm_common(void* c, const void* a, const void* w, const float* sa, const fl
     return maps_c ? make_map(m, c_type, 2, c, static_cast<uint64_t>(N), static_cast<uint64_t>(M), 64, 32) : FLYB200_OK;
   };
   if (!plan.decode && plan.two_sm) {
-    p.tail_parts = host::pair_tail_parts(plan.bn, host::pair_tiles(M, N, plan.bn), st->sms / 2);
     auto map_w = [&](CUtensorMap* m, uint32_t box_rows) {
       return make_weight_map(m, w, static_cast<uint64_t>(N), static_cast<uint64_t>(K_bytes / KBLOCK_BYTES), box_rows);
     };
@@ -1131,33 +1140,40 @@ int flyb200_selftest_bounded_wait(unsigned int limit_us, void* stream) {
   return FLYB200_OK;
 }
 
-int flyb200_describe_plan(int M, int N, int K, int in_dtype, int variant_hint, int sm_count, int* out8) {
-  if (!out8 || M <= 0 || N <= 0 || K <= 0 || sm_count <= 0) return FLYB200_E_BAD_ARG;
+int flyb200_describe_call(int M, int N, int K, int in_dtype, int epilogue, int variant_hint, int sm_count, int* out9) {
+  if (!out9 || M <= 0 || N <= 0 || K <= 0 || sm_count <= 0) return FLYB200_E_BAD_ARG;
   if (in_dtype < FLYB200_DT_FP8 || in_dtype > FLYB200_DT_BF16) return FLYB200_E_BAD_ARG;
+  if (epilogue < FLYB200_EPI_NONE || epilogue > FLYB200_EPI_BIAS_GELU) return FLYB200_E_BAD_ARG;
   const int eb = elem_bytes_of(in_dtype);
   if (!flyb200_layout_kind(N, K, eb)) return FLYB200_E_UNSUPPORTED;
   Plan plan;
   // planned as with an unlimited workspace: the answer says what would be needed
-  int rc = make_plan(&plan, M, N, K * eb, variant_hint, static_cast<size_t>(-1) >> 1, true, sm_count);
+  int rc = plan_call(&plan, M, N, K * eb, variant_hint, static_cast<size_t>(-1) >> 1, true, sm_count, epilogue);
   if (rc) return rc;
-  out8[0] = plan.decode ? (plan.pair ? 5 : plan.w_rows == 64 ? 4 : 1) : (plan.two_sm ? 3 : plan.tall ? 6 : 2);
-  out8[1] = plan.bn;
-  out8[2] = plan.split_k;
-  out8[3] = plan.kb_per_split;
-  out8[4] = plan.reduce_mode;
-  out8[5] = plan.decode ? plan.stages : (plan.two_sm ? host::pair_stages_for(plan.bn) : plan.tall ? host::ROWS_TALL_STAGES : host::rows_stages_for(plan.bn));
-  out8[6] = plan.pdl;
-  out8[7] = plan.token_blocks;
+  out9[0] = plan.decode ? (plan.pair ? 5 : plan.w_rows == 64 ? 4 : 1) : (plan.two_sm ? 3 : plan.tall ? 6 : 2);
+  out9[1] = plan.bn;
+  out9[2] = plan.split_k;
+  out9[3] = plan.kb_per_split;
+  out9[4] = plan.reduce_mode;
+  out9[5] = ring_stages(plan);
+  out9[6] = plan.pdl;
+  out9[7] = plan.token_blocks;
+  out9[8] = tail_strips(plan, M, N, sm_count);
   return FLYB200_OK;
 }
 
+int flyb200_describe_plan(int M, int N, int K, int in_dtype, int variant_hint, int sm_count, int* out8) {
+  if (!out8) return FLYB200_E_BAD_ARG;
+  int out9[9];
+  const int rc = flyb200_describe_call(M, N, K, in_dtype, FLYB200_EPI_NONE, variant_hint, sm_count, out9);
+  if (rc == FLYB200_OK) memcpy(out8, out9, 8 * sizeof(int));
+  return rc;
+}
+
 int flyb200_pair_width(int M, int N, int K, int in_dtype, int variant_hint, int sm_count) {
-  if (M <= 0 || N <= 0 || K <= 0 || sm_count <= 0 || in_dtype < FLYB200_DT_FP8 || in_dtype > FLYB200_DT_BF16) return 0;
-  const int eb = elem_bytes_of(in_dtype);
-  if (!flyb200_layout_kind(N, K, eb)) return 0;
-  Plan plan;
-  if (plan_call(&plan, M, N, K * eb, variant_hint, static_cast<size_t>(-1) >> 1, true, sm_count, false)) return 0;
-  return plan.two_sm ? plan.bn : 0;
+  int out9[9];
+  if (flyb200_describe_call(M, N, K, in_dtype, FLYB200_EPI_NONE, variant_hint, sm_count, out9)) return 0;
+  return out9[0] == 3 ? out9[1] : 0;
 }
 
 int flyb200_layout_kind(int N, int K, int elem_bytes) {
@@ -1178,7 +1194,7 @@ size_t flyb200_workspace_bytes(int M, int N, int K, int in_dtype, int variant_hi
   if (device_state(&st)) return 0;
   // plan as the GEMM would with an unlimited workspace, then size for that plan
   Plan plan;
-  if (make_plan(&plan, M, N, K * eb, variant_hint, static_cast<size_t>(-1) >> 1, true, st->sms)) return 0;
+  if (plan_call(&plan, M, N, K * eb, variant_hint, static_cast<size_t>(-1) >> 1, true, st->sms, FLYB200_EPI_NONE)) return 0;
   if (!plan.decode || plan.reduce_mode != REDUCE_WORKSPACE) return 0;
   return TICKET_BYTES + partial_bytes(plan.split_k, N, plan.bn, plan.token_blocks);
 }

@@ -118,7 +118,7 @@ class PreshuffleGemm:
         """The prebuilt kernel variant a call with ``M`` rows runs on a GPU with
         ``sm_count`` SMs (kernel, tile width, split-K, reduction, ring depth, ...):
         a pure host function of the library, no CUDA call."""
-        return _lib.describe_plan(max(int(M), 1), self.N, self.K, self.in_dtype, self.variant_hint, sm_count)
+        return _lib.describe_plan(max(int(M), 1), self.N, self.K, self.in_dtype, self.variant_hint, sm_count, self.epilogue)
 
     def workspace_bytes(self, device: torch.device) -> int:
         """Scratch this launcher can need on ``device`` for any M: the largest

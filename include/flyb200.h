@@ -79,10 +79,9 @@ extern "C" {
  *              70 % full, or M > 16 (M = 16 with K >= 8192 bytes) when T >= 3 S, go to 2;
  *              256 < M <= 1024 -> 1 when 2 * T * ceil(M/256) <= S and K spans at
  *              least 32 blocks of 128 bytes; else M > 256 -> 2, or 3 when FLYB200_ROWS_2SM=1, or 6
- *              when FLYB200_ROWS_TALL=1 or when ceil(M/256) * ceil(N/256) tiles
- *              cover the output in one round that fills at least 80 % of the SMs; a call
- *              of more than 128 tokens that sets none of the bits 0-27 and 30-31 then runs as 3
- *              wherever flyb200_pair_width says so)
+ *              when FLYB200_ROWS_TALL=1; a call of more than 128 tokens that sets none of the
+ *              bits 0-27 and 30-31 then runs on the one of this kernel, 2 and 3 that is
+ *              estimated to be the fastest: flyb200_describe_call tells)
  *   bits 12-15 how K splits are combined: 1 = global workspace + ticket,
  *              2 = thread-block cluster + distributed shared memory (split <= 8)
  *   bits 16-23 rasterisation group (row tiles per group, large-M kernel)
@@ -217,22 +216,21 @@ int flyb200_layout_kind(int N, int K, int elem_bytes);
  * the current device (0 when the chosen variant keeps its partial sums on chip). */
 size_t flyb200_workspace_bytes(int M, int N, int K, int in_dtype, int variant_hint);
 
-/* Which kernel variant flyb200_gemm_a8w8 would run for this problem on a GPU with
- * sm_count SMs (pure host function, no CUDA call): out8 = { kernel (1 small-M,
- * 2 large-M, 3 large-M as CTA pairs), tile width on the UMMA N side, split-K
- * factor, k-blocks per split, reduction (0 none, 1 workspace, 2 cluster), ring
- * depth, dependent-launch mode, token blocks }.  The B200 counterpart of the
+/* Which kernel variant flyb200_gemm_a8w8 runs for this problem on a GPU with
+ * sm_count SMs (pure host function, no CUDA call; planned as with an unlimited
+ * workspace): out9 = { kernel, numbered as in variant_hint (1 small-M, 2 large-M, 3
+ * large-M as CTA pairs, 4 small-M with 64-channel tiles, 5 small-M as CTA pairs, 6
+ * large-M with 256-row tiles), tile width on the UMMA N side, split-K factor,
+ * k-blocks per split, reduction (0 none, 1 workspace, 2 cluster), ring depth,
+ * dependent-launch mode, token blocks, column strips of the tiles of the last
+ * round }.  The B200 counterpart of the
  * per-tile table _TILE_PRELOAD_TABLE / tile arguments the reference's callers
- * tune by hand (kernels/gemm/preshuffle_gemm.py:19-105).  A call that leaves the
- * kernel open runs the planned kernel unless flyb200_pair_width says that CTA
- * pairs take its place. */
-int flyb200_describe_plan(int M, int N, int K, int in_dtype, int variant_hint, int sm_count, int* out8);
+ * tune by hand (kernels/gemm/preshuffle_gemm.py:19-105). */
+int flyb200_describe_call(int M, int N, int K, int in_dtype, int epilogue, int variant_hint, int sm_count, int* out9);
 
-/* Tile width with which the call runs as CTA pairs (256 rows x this many channels
- * per pair), asked for or because they are estimated to be faster than the plan
- * of flyb200_describe_plan; 0 where that plan runs (as the 128-row form, where it
- * says 256-row tiles and none were asked for).  For a call without a fused silu or
- * gelu; with one the pairs begin at a longer K.  Pure host function. */
+/* The same for a call without an epilogue: its first eight values, and the tile
+ * width where it runs as CTA pairs (256 rows x this many channels per pair), else 0. */
+int flyb200_describe_plan(int M, int N, int K, int in_dtype, int variant_hint, int sm_count, int* out8);
 int flyb200_pair_width(int M, int N, int K, int in_dtype, int variant_hint, int sm_count);
 
 /* Device-side status word of the current device (0 = no failure since the last

@@ -144,18 +144,18 @@ def test_cta_pair_kernel_scaled_output(dev, in_dtype, m, n, k):
 @pytest.mark.parametrize("in_dtype", ["fp8", "int8", "bf16"])
 @pytest.mark.parametrize("m,n,k", [(300, 2048, 4096), (512, 1024, 8192), (1024, 2048, 4096), (777, 1040, 4096)])
 def test_narrow_output_mid_m_runs_on_the_small_m_kernel(dev, in_dtype, m, n, k):
-    """257..1024 tokens, few channel tiles, long K: token blocks of 256 on the small-M kernel (automatic)."""
-    fn = compile_preshuffle_gemm(N=n, K=k, tile_m=128, tile_n=128, tile_k=128, in_dtype=in_dtype)
-    assert fn.plan(m)["kernel"] in (1, 5) and fn.plan(m)["token_blocks"] == -(-m // 256)  # 5: pairs, if the environment asks
+    """257..1024 tokens, few channel tiles, long K: token blocks of 256 on the small-M kernel."""
+    fn = compile_preshuffle_gemm(N=n, K=k, tile_m=128, tile_n=128, tile_k=128, in_dtype=in_dtype, variant_hint=DEC)
+    assert fn.plan(m)["kernel"] == 1 and fn.plan(m)["token_blocks"] == -(-m // 256)
     if in_dtype == "bf16":
         g = torch.Generator().manual_seed(m)
         a = (torch.randn(m, k, generator=g) * 0.5).to(torch.bfloat16)
         b = (torch.randn(n, k, generator=g) * 0.5).to(torch.bfloat16)
-        got = run_gemm_generic(dev, a, b, None, None, None, m, n, k, in_dtype)
+        got = run_gemm_generic(dev, a, b, None, None, None, m, n, k, in_dtype, hint=DEC)
         assert oracle.strict_mismatches(got, oracle.run_torch(a, b, None, None), RTOL, ATOL) == 0
         return
     a_q, b_q, sa, sb = oracle.make_inputs(m, n, k, in_dtype, seed=41 + m)
-    c = run_gemm(dev, a_q, b_q, sa, sb, m, n, k, in_dtype)
+    c = run_gemm(dev, a_q, b_q, sa, sb, m, n, k, in_dtype, hint=DEC)
     check_scaled(c, a_q, b_q, sa, sb, m)
 
 
@@ -501,18 +501,21 @@ def test_large_m_kernel_tile_tail_with_fused_epilogue(dev, width, in_dtype):
 
 
 def test_automatic_tile_width_fills_whole_rounds():
-    """The planner picks the width whose tiles cover the 148 SMs in full rounds: 2048 x 8192 gives
-    16 x 37 = 592 tiles of 224 channels (four rounds) instead of 512 tiles of 256 (3.46 rounds); and
-    where 256-row tiles cover the output in one nearly full round (1024 x 8192: 128 tiles) it takes those."""
+    """The planner picks the width whose tiles cover the 148 SMs in full rounds: 128-row tiles of 2048 x 8192 are 16 x 37 = 592 of
+    224 channels (four rounds) instead of 512 of 256 (3.46 rounds); 74 pairs take 8 x 37 = 296 of 224 channels, four rounds again."""
     if os.environ.get("FLYB200_ROWS_TALL") == "1" or os.environ.get("FLYB200_ROWS_2SM") == "1":
         pytest.skip("the environment overrides the automatic choice")
-    plan = _lib.describe_plan(2048, 8192, 8192, "fp8", 0, 148)
+    rows = 2 << 8  # the 128-row form on request
+    plan = _lib.describe_plan(2048, 8192, 8192, "fp8", rows, 148)
     assert plan["kernel"] == 2 and plan["bn"] == 224
-    plan = _lib.describe_plan(1024, 8192, 8192, "fp8", 2 << 8, 148)  # the 128-row form on request
+    plan = _lib.describe_plan(1024, 8192, 8192, "fp8", rows, 148)
     assert plan["kernel"] == 2 and plan["bn"] == 224
-    plan = _lib.describe_plan(1024, 8192, 8192, "fp8", 0, 148)
-    assert plan["kernel"] == 6 and plan["bn"] == 256
-    assert _lib.describe_plan(16384, 57344, 8192, "fp8", 0, 148)["bn"] == 256
+    assert _lib.describe_plan(16384, 57344, 8192, "fp8", rows, 148)["bn"] == 256
+    for m in (1024, 2048):
+        plan = _lib.describe_plan(m, 8192, 8192, "fp8", 0, 148)
+        assert plan["kernel"] == 3 and plan["bn"] == 224
+    plan = _lib.describe_plan(16384, 57344, 8192, "fp8", 0, 148)
+    assert plan["kernel"] == 3 and plan["bn"] == 256
 
 
 def test_reference_example_fp16_4096_cubed():

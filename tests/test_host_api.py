@@ -176,13 +176,19 @@ def test_variant_selection_is_a_pure_host_function():
     assert (p["kernel"], p["bn"], p["split_k"], p["reduce"]) == (4, 32, 1, 0)
     with pytest.raises(_lib.FlyB200Error):
         d(128, 8192, 8192, variant_hint=4 << 8)  # too many tokens for the half-height tiles
-    assert d(1, 8192, 8192)["bn"] == 16 and d(17, 8192, 8192)["bn"] == 32 and d(256, 8192, 8192)["bn"] == 256
+    assert d(1, 8192, 8192)["bn"] == 16 and d(17, 8192, 8192)["bn"] == 32 and d(256, 8192, 8192, variant_hint=1 << 8)["bn"] == 256
     # more channel tiles than SMs: no split
     assert d(8, 57344, 8192)["split_k"] == 1 and d(8, 57344, 8192)["reduce"] == 0
     # benchmark config 1: 32 tiles -> split 4
     assert d(128, 4096, 4096)["split_k"] == 4
-    # large M: persistent kernel, one CTA per tile unless asked otherwise
-    assert d(257, 8192, 8192)["kernel"] == 2 and d(8192, 28672, 8192, variant_hint=3 << 8)["kernel"] == 3
+    # large M: persistent kernels, CTA pairs where they are estimated to be faster than one CTA per 128-row tile
+    assert d(257, 8192, 8192)["kernel"] == 2 and d(8192, 28672, 8192)["kernel"] == 3
+    assert d(8192, 28672, 8192, variant_hint=2 << 8)["kernel"] == 2 and d(257, 8192, 8192, variant_hint=3 << 8)["kernel"] == 3
+    # ... which with silu or gelu takes a longer K
+    assert [d(8192, 8192, 1664, epilogue=e)["kernel"] for e in ("none", "bias_relu", "bias_silu", "bias_gelu")] == [3, 3, 2, 2]
+    assert d(8192, 8192, 2304, epilogue="bias_gelu")["kernel"] == 3
+    # column strips for the few tiles of a last round
+    assert d(4096, 4096, 4096, "fp16")["strips"] == 2 and d(2048, 8192, 8192)["strips"] == 1
     # explicit requests are honoured or refused, never changed silently
     assert d(32, 8192, 8192, variant_hint=(1 << 8) | (1 << 12) | 16)["reduce"] == 1
     with pytest.raises(_lib.FlyB200Error):
@@ -197,24 +203,24 @@ def test_variant_selection_is_a_pure_host_function():
     assert (p["kernel"], p["split_k"], p["reduce"]) == (1, 2, 2)
     # wide outputs (more channel tiles than SMs) go to the persistent kernel above 64 tokens, badly
     # filled rounds from 32, very wide ones from 16; narrow ones stay on the small-M kernel
-    assert d(64, 28672, 8192)["kernel"] == 1 and d(65, 28672, 8192)["kernel"] == 2 and d(256, 28672, 8192)["kernel"] == 2
-    assert d(64, 18944, 4096)["kernel"] == 1 and d(200, 18944, 4096)["kernel"] == 1  # exactly one round of CTAs
+    assert d(64, 28672, 8192)["kernel"] == 1 and d(65, 28672, 8192)["kernel"] == 2 and d(256, 28672, 8192)["kernel"] == 3
+    assert d(64, 18944, 4096)["kernel"] == 1 and d(128, 18944, 4096)["kernel"] == 1  # exactly one round of CTAs
     assert d(16, 24576, 8192)["kernel"] == 1 and d(32, 24576, 8192)["kernel"] == 2  # second round 30 % full
     assert d(8, 57344, 8192)["kernel"] == 1 and d(16, 57344, 8192)["kernel"] == 2
-    assert d(256, 16384, 8192)["kernel"] == 1
+    assert d(256, 16384, 8192)["kernel"] == 3 and d(256, 1024, 8192)["kernel"] == 1  # from 129 tokens up what is faster
+    assert d(130, 1024, 8064)["kernel"] == 1 and d(200, 4096, 1024)["kernel"] == 2
     assert d(128, 28672, 8192, variant_hint=1 << 8)["kernel"] == 1  # a request for the small-M kernel stands
-    # 256-row tiles: on request, and by themselves where they cover the output in one nearly full round
-    assert d(4096, 8192, 8192, variant_hint=6 << 8)["kernel"] == 6 and d(4096, 8192, 8192)["kernel"] == 2
-    p = d(1024, 8192, 8192)
+    # 256-row tiles: on request
+    p = d(1024, 8192, 8192, variant_hint=6 << 8)
     assert (p["kernel"], p["bn"], p["stages"]) == (6, 256, 3)
-    assert d(1024, 4096, 8192)["kernel"] == 2 and d(2048, 8192, 8192)["kernel"] == 2
-    assert d(300, 16384, 8192)["kernel"] == 2  # 2 x 64 tiles would fit, but rows 384..511 would be padding
+    for m, n, k in ((1024, 8192, 8192), (1500, 6144, 1024), (4096, 8192, 8192), (512, 16384, 4096)):
+        assert d(m, n, k)["kernel"] != 6
     assert d(128, 37888, 8192)["kernel"] == 2  # wide output routed to the large-M kernel: 128-row tiles
     # 257..1024 tokens on a narrow output with a long K: token blocks of 256 on the small-M kernel
     p = d(512, 2048, 8192)
     assert (p["kernel"], p["bn"], p["token_blocks"], p["split_k"], p["reduce"]) == (1, 256, 2, 4, 2)
-    assert d(1024, 2048, 8192)["token_blocks"] == 4 and d(1025, 2048, 8192)["kernel"] == 2
-    assert d(512, 8192, 8192)["kernel"] == 2 and d(512, 4096, 2048)["kernel"] == 2  # too many tiles; K too short
+    assert d(1024, 1024, 8192)["token_blocks"] == 4 and d(1025, 2048, 8192)["kernel"] == 2
+    assert d(512, 8192, 8192)["kernel"] == 3 and d(512, 4096, 2048)["kernel"] == 2  # too many tiles; K too short
     with pytest.raises(_lib.FlyB200Error):
         d(1025, 2048, 8192, variant_hint=1 << 8)  # four token blocks of 256 are the limit
     # small-M kernel as CTA pairs: on request, for token tiles of 64 and more and an even number of channel tiles

@@ -658,6 +658,8 @@ int ring_stages(const Plan& plan) {
 }
 int tail_strips(const Plan& plan, int M, int N, int sms) {
   if (plan.decode || plan.tall) return 1;
+  const char* e = getenv("FLYB200_ROWS_TAIL");  // 0: whole tiles only (tuning and tests)
+  if (e && e[0] == '0') return 1;
   if (plan.two_sm) return sms < 2 ? 1 : host::pair_tail_parts(plan.bn, host::pair_tiles(M, N, plan.bn), sms / 2);
   return host::rows_tail_parts(plan.bn, static_cast<long long>((M + BLOCK_ROWS - 1) / BLOCK_ROWS) * ((N + plan.bn - 1) / plan.bn), sms);
 }

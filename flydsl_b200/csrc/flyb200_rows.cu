@@ -33,7 +33,7 @@ int launch_plain_or_pdl(KernelT kernel, int grid, int threads, int smem, cudaStr
 }
 
 template <int KIND, int OUTMODE>
-int launch_rows(const CUtensorMap& tmA, const CUtensorMap& tmC, GemmParams p, int sms, cudaStream_t s) {
+int launch_rows(const CUtensorMap& tmA, const CUtensorMap& tmC, const GemmParams& p, int sms, cudaStream_t s) {
   static std::atomic<uint64_t> done{0};
   auto kernel = gemm_rows_kernel<KIND, OUTMODE>;
   int rc = ensure_smem(kernel, SMEM_LIMIT, done);
@@ -41,10 +41,6 @@ int launch_rows(const CUtensorMap& tmA, const CUtensorMap& tmC, GemmParams p, in
   const RowsLayout L = rows_layout(p.bn, p.rows_stages);
   if (L.total > SMEM_LIMIT || p.bn < 32 || p.bn > 256 || (p.bn & 31)) return FLYB200_E_UNSUPPORTED;
   const long long tiles = static_cast<long long>((p.M + BLOCK_ROWS - 1) / BLOCK_ROWS) * ((p.N + p.bn - 1) / p.bn);
-  p.tail_parts = rows_tail_parts(p.bn, tiles, sms);
-  if (const char* e = getenv("FLYB200_ROWS_TAIL")) {  // 0: whole tiles only (tuning and tests)
-    if (e[0] == '0') p.tail_parts = 1;
-  }
   const int grid = static_cast<int>(tiles < sms ? tiles : sms);
   const int threads = 64 + 32 * rows_epilogue_warps(p.K_bytes / KBLOCK_BYTES, tiles, sms);
   return launch_plain_or_pdl(kernel, grid, threads, L.total, s, p.pdl != 0, tmA, tmC, p);

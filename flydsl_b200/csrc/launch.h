@@ -96,8 +96,8 @@ inline int rows_epilogue_warps(int kb, long long tiles, int sms) {
   return kb >= 32 && tiles >= 8LL * sms ? 4 : 8;
 }
 
-// Large-M kernel (p.bn, p.rows_stages set): one CTA per 128 x bn tile, or per 256 x bn tile (tmA with boxes of 256 rows,
-// three stages).  `kind` is KIND_*, `outmode` OUT_*.
+// Large-M kernel (p.bn, p.rows_stages, p.tail_parts set): one CTA per 128 x bn tile, or per 256 x bn tile (tmA with boxes of 256
+// rows, three stages).  `kind` is KIND_*, `outmode` OUT_*.
 enum : int { ROWS_FORM_ONE = 0, ROWS_FORM_TALL = 2 };
 constexpr int ROWS_TALL_STAGES = 3;
 int launch_rows_kind(int kind, int outmode, int form, const CUtensorMap& tmA, const CUtensorMap& tmC, const GemmParams& p,

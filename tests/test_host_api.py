@@ -232,3 +232,11 @@ def test_variant_selection_is_a_pure_host_function():
             d(m, n, 8192, variant_hint=5 << 8)
     with pytest.raises(_lib.FlyB200Error):
         d(64, 8192, 8192, variant_hint=(5 << 8) | (1 << 12) | 2)  # pairs reduce inside their cluster only
+
+
+def test_strips_can_be_switched_off_for_both_large_m_forms(monkeypatch):
+    d = _lib.describe_plan
+    calls = [(4096, 4096, 4096, 2 << 8), (1277, 4080, 256, 3 << 8 | 8), (4096, 4096, 4096, 0)]
+    assert [d(m, n, k, "fp16", variant_hint=h)["strips"] for m, n, k, h in calls] == [2, 4, 2]
+    monkeypatch.setenv("FLYB200_ROWS_TAIL", "0")
+    assert [d(m, n, k, "fp16", variant_hint=h)["strips"] for m, n, k, h in calls] == [1, 1, 1]

@@ -29,6 +29,19 @@ def test_every_width_and_strip_bit_exact(m, n, k, width):
 
 
 @pytest.mark.gpu
+@pytest.mark.parametrize("m,n,k,width", STRIPS)
+def test_last_round_whole_or_in_strips_is_bit_identical(monkeypatch, m, n, k, width):
+    a, b, _, _ = oracle.make_inputs(m, n, k, "int8", seed=m, rne_int8=True)
+    for tail, strips in (("0", {1}), ("1", {2, 4})):
+        monkeypatch.setenv("FLYB200_ROWS_TAIL", tail)
+        assert _lib.describe_plan(m, n, k, "int8", PAIR_FORM | width)["strips"] in strips
+        acc = gpu_acc(a.cuda(), shuffle_weight(b.cuda()), m, n, k, "int8", variant_hint=PAIR_FORM | width)
+        torch.cuda.synchronize()
+        assert device_status() == 0
+        assert torch.equal(acc.cpu(), oracle.int32_acc(a, b))
+
+
+@pytest.mark.gpu
 @pytest.mark.parametrize("epilogue", ["none", "bias_gelu"])
 @pytest.mark.parametrize("in_dtype,out_dtype", [("fp8", "bf16"), ("int8", "fp16"), ("bf16", "bf16"), ("fp16", "fp16")])
 @pytest.mark.parametrize("m,n,k,width", [(200, 1040, 1024, 7), (513, 2064, 2048, 0)] + STRIPS[:1])

@@ -307,7 +307,9 @@ bool decode_pair_default() {
   return on;
 }
 
-// FLYB200_ROWS_TALL=1: 256-row tiles for the large-M kernel wherever no other form is asked for
+// FLYB200_ROWS_TALL=1: 256-row tiles for the large-M kernel wherever no other form is asked for.  Off unless asked for (also per
+// call: kernel field 6 of the hint): pairs or the 128-row form are faster everywhere, one-round shapes included (1024 x 8192 x
+// 4096 36.4 us, pairs 34.0; 1500 x 6144 x 1024 15.3, 128-row form 12.2).
 bool rows_tall_default() {
   static const bool on = []() {
     const char* e = getenv("FLYB200_ROWS_TALL");
@@ -439,7 +441,6 @@ double rows_ns(long long cycles) { return 3400.0 + 0.74 * static_cast<double>(cy
 // intake binds and less energy where the board's power cap does.  `plan` / pairs, us, fp8 unless stated:
 //   128-row form   4096 x 8192 x 8192 220 / 204, 8192 x 28672 x 8192 1480 / 1420, 2048 x 8192 x 8192 121 / 110, 768 x 8192 x 8192
 //                  56.7 / 48.8; fp16 4096 x 4096 x 4096 118 / 108; int8 997 x 10208 x 5120 54 / 47; bf16 8192 x 5120 x 1024 78 / 72
-//   256-row form   1024 x 8192 x 4096 36.4 / 34.0, 512 x 16384 x 4096 38.3 / 36.1, bf16 1536 x 5120 x 1024 19.0 / 16.8
 //   small-M form   256 x 8192 x 8192 24.7 / 21.9, 256 x 10208 x 5120 26.8 / 18.5, 320 x 4096 x 4096 15.2 / 11.2, bf16 512 x 3584 x 8192 35 / 31.5
 // Up to 128 tokens half of a pair would have no rows (128 x 8192 x 8192 17.3 / 22.4).  Of the widths the cheapest counts, a
 // narrower one only if it is 2 % cheaper (more bytes per product).
@@ -450,7 +451,7 @@ double rows_ns(long long cycles) { return 3400.0 + 0.74 * static_cast<double>(cy
 // 11.3 us), and at most 5.4 % behind the small-M kernel (320 x 2048 x 8064 15.8 for 15.0 us).
 // In place of the large-M forms: a pair's set-up and hand-over of accumulators (cluster
 // barriers, remote arrivals) weigh 5000 cycles, and with few k-blocks, where the epilogue is longer than the mainloop, the 128-row form
-// stays (it also takes the place of the 256-row form there): 128-row form / pairs, us, fp8 8192 x 8192 x 1024 68.5 / 81.1, x 1280 84.8 / 94.7, x
+// stays: 128-row form / pairs, us, fp8 8192 x 8192 x 1024 68.5 / 81.1, x 1280 84.8 / 94.7, x
 // 2048 135 / 116, with gelu x 1536 130 / 144, x 2048 153 / 155, x 2560 184 / 170; 512 x 8192 x 2560 11.9 / 13.6.  Over 90 calls of 1025..8192
 // tokens the choice is 1.5 % behind the best on average, 14.5 % at worst (2419 x 4304 x 5632 55.3 for 48.3 us).
 constexpr long long PAIR_SETUP_CYCLES = 5000;
@@ -473,7 +474,7 @@ LargeForm large_form(const Plan& plan, int M, int N, int K_bytes, int sms, bool 
       form.width = bn;
     }
   }
-  const int rows_bn = !plan.decode && !plan.tall ? plan.bn : auto_rows_bn(M, N, K_bytes, sms);
+  const int rows_bn = plan.decode ? auto_rows_bn(M, N, K_bytes, sms) : plan.bn;
   const long long rows = rows_cost(M, N, kb, rows_bn, sms);
   if (!plan.decode) return rows < best + PAIR_SETUP_CYCLES ? stay : form;
   const double here = small_ns(plan, M, N, sms), pairs = pair_ns(best), single = rows_ns(rows);
@@ -515,16 +516,6 @@ int make_plan(Plan* plan, int M, int N, int K_bytes, int variant_hint, size_t wo
   }
   plan->two_sm = want_kernel == 3 ? true : (want_kernel == 2 || want_kernel == 6) ? false : rows_two_sm_default();
   plan->tall = !plan->decode && !plan->two_sm && (want_kernel == 6 || (want_kernel == 0 && rows_tall_default()));
-  if (want_kernel == 0 && !plan->decode && !plan->two_sm && !plan->tall && want_split == 0) {
-    // 256-row tiles where they cover the output in ONE nearly full round of CTAs: every SM then does
-    // the flops of two 128-row tiles but fetches its weight blocks once (1024 x 8192 x 8192: 59-60 us
-    // against 62-65 us).  With more rounds the 128-row form wins: it overlaps the epilogue of a
-    // tile with the mainloop of the next, which the 256-row form (all of TMEM in one tile) cannot.
-    // (Not where the taller tiles would add a padded half tile of rows, nor for M <= 256.)
-    const long long t = static_cast<long long>((M + 255) / 256) * ((N + 255) / 256);
-    const bool no_extra_rows = (M + 255) / 256 * 2 == (M + 127) / 128;
-    plan->tall = M > 256 && no_extra_rows && t <= sms && 5 * t >= 4 * sms;
-  }
   if (plan->decode && M > 1024) return FLYB200_E_UNSUPPORTED;  // up to four token blocks of 256
   if (want_reduce > REDUCE_CLUSTER) return FLYB200_E_BAD_ARG;
   plan->token_blocks = 1;
@@ -630,10 +621,8 @@ int make_plan(Plan* plan, int M, int N, int K_bytes, int variant_hint, size_t wo
 // make_plan, and the large-M form that takes its place where the call leaves the kernel open and another one is the better choice.
 int plan_call(Plan* plan, int M, int N, int K_bytes, int variant_hint, size_t workspace_bytes, bool have_ws, int sms, int epilogue) {
   const int rc = make_plan(plan, M, N, K_bytes, variant_hint, workspace_bytes, have_ws, sms);
-  if (rc || (variant_hint & ~(3 << 28)) != 0 || rows_tall_default() || w64_default()) return rc;
-  LargeForm form = large_form(*plan, M, N, K_bytes, sms, epilogue >= FLYB200_EPI_BIAS_SILU);
-  // the 128-row form is faster than the 256-row form by now wherever pairs are not: fp8 1500 x 6144 x 1024 12.2 / 15.3 us
-  if (form.width == 0 && plan->tall) form = {false, auto_rows_bn(M, N, K_bytes, sms)};
+  if (rc || (variant_hint & ~(3 << 28)) != 0 || rows_tall_default()) return rc;
+  const LargeForm form = large_form(*plan, M, N, K_bytes, sms, epilogue >= FLYB200_EPI_BIAS_SILU);
   if (form.width == 0) return rc;
   const int hp = hint_pdl(variant_hint);
   const int pdl = hp == 1 ? 1 : hp == 2 ? 0 : hp == 3 ? 2 : host::pdl_default();

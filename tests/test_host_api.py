@@ -4,6 +4,8 @@ symbols.  No GPU compute here."""
 import ctypes
 import os
 import re
+import subprocess
+import sys
 
 import pytest
 import torch
@@ -240,3 +242,13 @@ def test_strips_can_be_switched_off_for_both_large_m_forms(monkeypatch):
     assert [d(m, n, k, "fp16", variant_hint=h)["strips"] for m, n, k, h in calls] == [2, 4, 2]
     monkeypatch.setenv("FLYB200_ROWS_TAIL", "0")
     assert [d(m, n, k, "fp16", variant_hint=h)["strips"] for m, n, k, h in calls] == [1, 1, 1]
+
+
+def test_the_switch_for_64_channel_tiles_leaves_other_calls_alone():
+    """FLYB200_DECODE_W64=1 (read once per process) is about calls of up to 64 tokens whose 64-channel tiles fill the SMs."""
+    code = ("from flydsl_b200 import _lib; d = _lib.describe_plan; "
+            "print([d(m, 8192, 8192, 'int8')['kernel'] for m in (1, 64, 128, 256, 4096)])")
+    for value, kernels in (("0", [1, 1, 1, 3, 3]), ("1", [4, 4, 1, 3, 3])):
+        r = subprocess.run([sys.executable, "-c", code], env=dict(os.environ, FLYB200_DECODE_W64=value), capture_output=True, text=True,
+                           cwd=os.path.dirname(os.path.dirname(os.path.abspath(__file__))))
+        assert r.stdout.strip() == str(kernels), r.stderr

@@ -447,6 +447,8 @@ double rows_ns(long long cycles) { return 3400.0 + 0.74 * static_cast<double>(cy
 // In place of the small-M kernel the form with the least estimated time runs: it splits K and so keeps narrow outputs over many
 // k-blocks (small-M / pairs, us: 256 x 1024 x 8064 12.5 / 14.7, 130 x 1024 x 8064 9.8 / 14.7, 133 x 5136 x 14336 20.8 / 24.9, 256 x 4096 x
 // 14336 22.8 / 24.7), and the 128-row form is ahead of both with few (small-M / pairs / 128 rows: 200 x 4096 x 1024 12.7 / 7.0 / 5.7).
+// (Not for silu with a partial last tile: of that the 128-row form loads the existing weight rows alone, what it finds in the place of the others
+// leaves the range of the fast reciprocal, and the division takes 4..6 us in the last epilogue: 180 x 3152 x 2048 14.7, pairs 9.1.)
 // Over the 298 calls the choice is 0.6 % behind the best form and width on average, 12 % at worst (177 x 18464 x 1408 12.7 for
 // 11.3 us), and at most 5.4 % behind the small-M kernel (320 x 2048 x 8064 15.8 for 15.0 us).
 // In place of the large-M forms: a pair's set-up and hand-over of accumulators (cluster
@@ -460,11 +462,11 @@ struct LargeForm {
   bool pairs;
   int width;
 };
-LargeForm large_form(const Plan& plan, int M, int N, int K_bytes, int sms, bool activation) {
+LargeForm large_form(const Plan& plan, int M, int N, int K_bytes, int sms, int epilogue) {
   const LargeForm stay = {false, 0};
   const long long kb = K_bytes / KBLOCK_BYTES;
   if (M <= BLOCK_ROWS || sms < 2 || plan.two_sm || plan.pair) return stay;
-  if (!plan.decode && kb < (activation ? PAIR_MIN_KB_ACTIVATION : PAIR_MIN_KB)) return stay;
+  if (!plan.decode && kb < (epilogue >= FLYB200_EPI_BIAS_SILU ? PAIR_MIN_KB_ACTIVATION : PAIR_MIN_KB)) return stay;
   long long best = -1;
   LargeForm form = {true, 0};
   for (int bn = 256; bn >= 64; bn -= 32) {
@@ -478,8 +480,9 @@ LargeForm large_form(const Plan& plan, int M, int N, int K_bytes, int sms, bool 
   const long long rows = rows_cost(M, N, kb, rows_bn, sms);
   if (!plan.decode) return rows < best + PAIR_SETUP_CYCLES ? stay : form;
   const double here = small_ns(plan, M, N, sms), pairs = pair_ns(best), single = rows_ns(rows);
-  if (here <= pairs && here <= single) return stay;
-  return single < pairs ? LargeForm{false, rows_bn} : form;
+  const bool rows_ok = epilogue != FLYB200_EPI_BIAS_SILU || N % rows_bn == 0;
+  if (rows_ok && single < pairs) return single < here ? LargeForm{false, rows_bn} : stay;
+  return pairs < here ? form : stay;
 }
 
 // `allow_pair`: the caller's kind has the CTA-pair form of the small-M kernel (the plain kinds do)
@@ -622,7 +625,7 @@ int make_plan(Plan* plan, int M, int N, int K_bytes, int variant_hint, size_t wo
 int plan_call(Plan* plan, int M, int N, int K_bytes, int variant_hint, size_t workspace_bytes, bool have_ws, int sms, int epilogue) {
   const int rc = make_plan(plan, M, N, K_bytes, variant_hint, workspace_bytes, have_ws, sms);
   if (rc || (variant_hint & ~(3 << 28)) != 0 || rows_tall_default()) return rc;
-  const LargeForm form = large_form(*plan, M, N, K_bytes, sms, epilogue >= FLYB200_EPI_BIAS_SILU);
+  const LargeForm form = large_form(*plan, M, N, K_bytes, sms, epilogue);
   if (form.width == 0) return rc;
   const int hp = hint_pdl(variant_hint);
   const int pdl = hp == 1 ? 1 : hp == 2 ? 0 : hp == 3 ? 2 : host::pdl_default();

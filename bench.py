@@ -561,11 +561,11 @@ def parity_check(op, a_q, sa, w_q_local, sb_local, local, full_ag, full_fused, d
 
 
 # DRAM traffic of the dominant kernel, from one ncu capture of a smaller case with the
-# same tile order (profiles/gemm_rows_fp8_traffic.md): bytes read + written per launch
+# same tile order (profiles/gemm_pair_fp8_4096x14336x8192.md): bytes read + written per launch
 # there, and that case's algorithmic bytes.  The weights stream once per group of row
 # tiles and the activations once, so the full workload's traffic is estimated group by
 # group (see traffic_estimate), not by plain proportion.
-NCU_TRAFFIC_CASE = {"m": 4096, "n": 14336, "k": 8192, "group_m": 32, "read": 176.1e6, "write": 95.7e6}
+NCU_TRAFFIC_CASE = {"kernel": 3, "m": 4096, "n": 14336, "k": 8192, "group_m": 32, "read": 190.8e6, "write": 99.1e6}
 
 
 def traffic_estimate(m, n, k, group_m):
@@ -758,20 +758,24 @@ def main():
     # the timed steps run after half a second at the power cap: the matching measured figure is the sustained one
     fp8_peak_sustained = 2.0 * (peaks["bf16_sustained"] or peaks["bf16_tflops"])
     plan = op.launch.plan(m)
-    group_m = (args.hint >> 16) & 0xFF or 32
+    form = {2: "gemm_rows_kernel", 3: "gemm_pair_kernel", 6: "gemm_rows_tall_kernel"}.get(plan["kernel"], "gemm_decode_kernel")
+    tile_rows = 256 if plan["kernel"] in (3, 6) else 128
+    # 128-row tiles of a raster group (flyb200.cu: 32, or pair_group(K) tiles of 256 rows)
+    group_m = (args.hint >> 16) & 0xFF or (min(16, max(2, (48 << 20) // k // 256)) if plan["kernel"] == 3 else 32)
+    group_m *= tile_rows // 128
     traffic = None
     traffic_note = "no ncu capture recorded for this build"
-    if NCU_TRAFFIC_CASE:
+    if NCU_TRAFFIC_CASE["kernel"] == plan["kernel"]:
         tc = NCU_TRAFFIC_CASE
         model_small = traffic_estimate(tc["m"], tc["n"], tc["k"], tc["group_m"])
         traffic = (tc["read"] + tc["write"]) / model_small * traffic_estimate(m, nl, k, group_m)
         traffic_note = (f"ncu dram__bytes_read+write of {tc['m']}x{tc['n']}x{tc['k']} (same tile order, group {tc['group_m']}): "
                         f"{(tc['read'] + tc['write']) / 1e6:.0f} MB per launch = {(tc['read'] + tc['write']) / model_small:.2f} x the "
                         "tile-order model (weights once per group of row tiles + activations + output), scaled to this "
-                        "launch by that model; profiles/gemm_rows_fp8_traffic.md")
+                        "launch by that model; profiles/gemm_pair_fp8_4096x14336x8192.md")
     roofline = {
         "bound": "tensor",
-        "kernel": f"gemm_rows_kernel<fp8> (tcgen05 kind::f8f6f4, 128x{plan['bn']} tiles, persistent, {plan['stages']} stages)",
+        "kernel": f"{form}<fp8> (tcgen05 kind::f8f6f4, {tile_rows}x{plan['bn']} tiles, persistent, {plan['stages']} stages)",
         "achieved": achieved,
         "peak": fp8_peak_sustained,
         "unit": "TFLOP/s",

@@ -310,9 +310,9 @@ __global__ void __launch_bounds__(DECODE_THREADS, 1) gemm_decode_kernel(const __
     }
   }
   // Two accumulators (columns [0, BN) and [BN, 2 BN)): even k-blocks are issued by
-  // warp 1 into the first, odd k-blocks by warp 6 into the second, so that the
-  // ~290 cycles one thread needs to issue a k-block's MMAs are spent by two
-  // threads in parallel; the epilogue adds the two.
+  // warp 1 into the first, odd k-blocks by warp 6 into the second, so that the two
+  // issue in parallel (a k-block took about 290 cycles when one lane ran the loop; one warp alone has not been measured
+  // since the whole warp runs it); the epilogue adds the two.
   // MX kinds: 4 more columns per scale atom and ring stage (at most 8 stages) for the atoms in flight
   constexpr int MX_MAX_STAGES = 8;
   constexpr uint32_t SF_COL0 = 2 * BN;
@@ -354,7 +354,10 @@ __global__ void __launch_bounds__(DECODE_THREADS, 1) gemm_decode_kernel(const __
     // ------------------------------ producer ------------------------------
     // The whole warp runs the loop, here and in the MMA warps, and one lane issues (ptx.cuh).  One lane alone / whole warp, us:
     // fp8 1 x 4096 x 4096 6.15 / 5.62, 1 x 10208 x 5120 10.8 / 9.65, 32 x 3072 x 1024 6.35 / 5.54, bf16 1 x 512 x 14336 8.45 / 7.30,
-    // 128 x 8192 x 8192 15.8 / 15.6 (geometric mean over 50 shapes of 1 to 128 tokens 1.06).
+    // 128 x 8192 x 8192 15.8 / 15.6 (geometric mean over 50 shapes of 1 to 128 tokens 1.06); graph replay, cold weights, int8 32 x 8192 x
+    // 8192 14.3 / 13.7.  Slower on some GPUs where L2 has kept a part of the weights between eager launches: three sets of them in
+    // turn, int8 32 x 8192 x 8192 12.5 / 12.8 on two of five, 13.2 / 13.0 on the others.  One lane for the producer alone where K is
+    // split takes the former to 12.6 but costs 0.8 % on average over such shapes (4 x 4176 x 14080 10.1 / 10.5).
     const bool issuer = elect_one();
     const uint64_t pol_a = l2_policy_evict_last();
     const uint64_t pol_w = l2_policy_evict_first();

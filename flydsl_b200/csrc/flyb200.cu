@@ -284,10 +284,9 @@ int decode_prefetch_override() {
 
 bool w64_default() {
   static const bool on = []() {
-    // Off unless asked for: with one CTA streaming a tile's whole K range the
-    // single MMA-issuing thread (about 290 cycles per k-block) becomes the limit;
-    // measured 21 us against 14.5 us for 128-channel tiles with split-K 2
-    // (M = 32, N = K = 8192).
+    // Off unless asked for.  Graph replay with cold weights, us, 64-channel tiles / the automatic choice (128-channel tiles with a
+    // K split): fp8 N = K = 8192 1 token 12.7 / 12.7, 16 13.9 / 13.2, 32 15.2 / 13.9, 64 19.5 / 14.4; N = 9472 (148 of them) 1 token
+    // 13.2 / 13.9, 16 14.3 / 14.4, 32 15.6 / 15.1.
     const char* e = getenv("FLYB200_DECODE_W64");
     return e && e[0] == '1';
   }();
@@ -351,12 +350,13 @@ int auto_token_blocks(int /*M*/, int /*N*/, int /*sms*/) { return 1; }
 // Tile width of the large-M kernel when the caller does not force one.  All
 // tiles are 128 tokens high; the kernel is persistent, so a launch takes
 // ceil(tiles / SMs) rounds of one tile per SM.  Per 128-byte k-block a tile
-// costs the largest of: the tensor pipe (2 * bn cycles), the single thread
-// that issues the MMAs (ROWS_ISSUE_CYCLES), and bringing the operands into
+// costs the largest of: the tensor pipe (2 * bn cycles), what a k-block takes at
+// least (ROWS_MIN_CYCLES; decides for widths below 128 only, 0.21 us per k-block
+// at 130 x 1024), and bringing the operands into
 // shared memory ((16 KiB + bn * 128 B) / ROWS_LOAD_BYTES_PER_CYCLE).  The
 // width with the cheapest whole launch wins; ties go to the wider tile (fewer
 // operand bytes per flop).
-constexpr int ROWS_ISSUE_CYCLES = 300;
+constexpr int ROWS_MIN_CYCLES = 300;
 constexpr int ROWS_LOAD_BYTES_PER_CYCLE = 96;
 constexpr int ROWS_TILE_OVERHEAD_CYCLES = 2000;  // pipeline fill and the last, exposed epilogue of a CTA
 int auto_rows_bn(int M, int N, int K_bytes, int sms) {
@@ -369,7 +369,7 @@ int auto_rows_bn(int M, int N, int K_bytes, int sms) {
     const long long rounds = (tiles + sms - 1) / sms;
     auto tile_cost = [&](int width) {
       long long per_kb = 2 * width;
-      if (per_kb < ROWS_ISSUE_CYCLES) per_kb = ROWS_ISSUE_CYCLES;
+      if (per_kb < ROWS_MIN_CYCLES) per_kb = ROWS_MIN_CYCLES;
       const long long load = (BLOCK_ROWS * KBLOCK_BYTES + width * KBLOCK_BYTES) / ROWS_LOAD_BYTES_PER_CYCLE;
       if (per_kb < load) per_kb = load;
       return kb * per_kb + 4 * width;
@@ -412,7 +412,7 @@ long long pair_cost(int M, int N, long long kb, int bn, int sms) {
 }
 long long rows_cost(int M, int N, long long kb, int bn, int sms) {
   auto kb_cycles = [](int width) {
-    long long c = 2LL * width > ROWS_ISSUE_CYCLES ? 2LL * width : ROWS_ISSUE_CYCLES;
+    long long c = 2LL * width > ROWS_MIN_CYCLES ? 2LL * width : ROWS_MIN_CYCLES;
     const long long load = static_cast<long long>(BLOCK_ROWS + width) * KBLOCK_BYTES / 84;
     return c > load ? c : load;
   };
@@ -578,9 +578,9 @@ int make_plan(Plan* plan, int M, int N, int K_bytes, int variant_hint, size_t wo
     plan->stages += deeper <= SMEM_LIMIT ? 1 : -1;
   }
   // Weights requested into L2 ahead of the ring.  Small-M kernel: four k-blocks
-  // beyond the depth of the ring measured best (INT8 32 x 8192 x 8192 on one GPU:
-  // 13.9 us with 12 blocks ahead of an 8-deep ring, 14.4 us with 8, 14.7 us with
-  // none, 15.3 us with the whole K range requested at once).  Large-M kernel:
+  // beyond the depth of the ring measured best (INT8 32 x 8192 x 8192 on one GPU, cold weights:
+  // 13.76 us with 12 blocks ahead of an 8-deep ring, 14.04 with 8, 13.92 with 18; FP8 1 x
+  // 10208 x 5120 12.0 / 12.3 / 12.7).  Large-M kernel:
   // none; there the weights of a tile are shared by the CTAs of a group and
   // mostly hit L2 already, and the extra requests cost 1-30 %.
   plan->prefetch = 0;  // small-M kernel: set below, once the ring depth is known

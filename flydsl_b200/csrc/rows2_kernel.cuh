@@ -6,8 +6,9 @@
 //
 // What bounds it: the board's power.  A k-block of a 256 x 256 tile takes 523..540 cycles of the 512 that its four
 // MMAs need, at the 1.1..1.3 GHz the 1 kW cap leaves; fewer bytes moved per product are a higher clock.  Next to the
-// 128-row form it is 4..17 % faster from 129 tokens up (pair_choice in flyb200.cu lists both), on bf16 8192 x 8192 x 8192 777..820
-// us against 847 (cuBLAS 786).  Tiles of 512 rows (half of the weight traffic again, all of TMEM in one tile) were built and
+// 128-row form it is 4..17 % faster where it is the choice (large_form in flyb200.cu lists both), in turn on one GPU fp8 16384 x 57344 x 8192
+// 5926 us against 6170, 8192 x 28672 x 8192 1476 against 1554, 16384 x 8192 x 8192 867 against 903; bf16 8192 x 8192 x 8192 777..820
+// against 847 (cuBLAS 786).  Tiles of 512 rows (half of the weight traffic again, all of TMEM in one tile) were built and
 // were slower, 1454 against 1412 us on fp8 8192 x 28672 x 8192, as nothing overlaps their epilogue.
 //
 // Cross-CTA signalling, all without multicast:
